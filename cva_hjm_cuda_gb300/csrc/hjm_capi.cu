@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "../../include/hjm_cva.h"
+#include "hjm_contract.h"
 #include "hjm_eresp.h"
 #include "hjm_kernels.h"
 
@@ -105,39 +106,26 @@ struct hjm_ctx {
     bool keep_exposures = false;
 
     // device buffers
-    DevBuf partials, sums, result, estore, sel, hist, ext, ext_raw, wide, scratch, ck_h, ck_a, vresp, eresp, carry,
+    DevBuf partials, sums, result, estore, sel, hist, ext, ext_raw, wide, scratch, ck_h, ck_a, contract, carry,
         mresp;
     MemBudget budget;
     hjm_ctx()
     {
         for (DevBuf* b : buffers()) b->budget = &budget;
     }
-    std::array<DevBuf*, 16> buffers()
+    std::array<DevBuf*, 15> buffers()
     {
         return {&partials, &sums, &result, &estore, &sel, &hist, &ext, &ext_raw, &wide, &scratch, &ck_h, &ck_a,
-                &vresp, &eresp, &carry, &mresp};
+                &contract, &carry, &mresp};
     }
-    // the response tables in eresp, vresp and mresp hold the run shapes of
-    // their keys; resp_used is recorded after the last kernel that reads one
-    struct ErespKey {  // the response form's table in eresp (Euler or predictor-corrector)
-        bool valid = false, pc = false;
-        int nt = 0, stride = 0, B = 0, np = 0, nres = 0;
-        double c = 0, dtau = 0;
-        std::vector<EulerRespFrame> frames;  // one per window
-        std::vector<double> resid;  // sqrt(dt)-scaled, empty without a residual
-    } eresp_key;
-    struct ErespFirst {  // eresp_first_active_date of the last run shape
-        bool valid = false, pc = false;
-        int nt = 0, stride = 0, B = 0, nres = 0;
-        double c = 0;
-        int first = 2;
-    } eresp_first;
-    struct VrespKey {  // the volatility-table response table in vresp
-        bool valid = false;
+    // the tables in contract and mresp hold the run shapes of their keys;
+    // resp_used is recorded after the last kernel that reads one
+    struct ContractKey {  // the contraction's operand table in contract
+        bool valid = false, ext = false;
         int nt = 0, stride = 0, B = 0, scheme = 0;
         double c = 0;
         std::vector<double> sv;
-    } vresp_key;
+    } contract_key;
     struct MrespKey {  // the mixed-precision response form's slots and its table in mresp
         bool valid = false, on_device = false, pc = false;
         int nt = 0, stride = 0, B = 0, ns = 0;
@@ -797,17 +785,12 @@ static void fill_pc(const hjm_ctx* ctx, const RunShape& sh, double dt, const Pat
     Q.gL = (T)(-c * dtau * dtau);
 }
 
-// FP64 valuation with a decomposition (quadratic factors under either
-// scheme, or cubic ones with a residual table under the Euler step): the
-// response form of hjm_eresp.cu, whose per-step work is on the FP32 pipe and
-// which takes any number of dates (in windows); measured 9.0x the convected
-// form at 20 dates (Euler), and the convected cubic has no form but the table
-// step, so AUTO always takes it.
-//
-// Volatility-table step (no decomposition): the whole stochastic curve in
-// impulse responses, per step and date still to be sampled three
-// double-FP32 terms on the FP32 pipe (in windows of 16 dates), against four
-// FP64 FMAs per live tenor (five for the predictor-corrector) when convected.
+// FP64 valuation: the response form as a contraction on the tensor cores
+// (hjm_contract.cu), for every market and either scheme, so AUTO always takes
+// it: measured 22x the convected decomposed step and 66x the convected table
+// step at 20 dates (5.3 ms against 116.7 and 352 ms at 1M paths), and faster
+// at every size from one path on (200 paths, 25y: 1.7 ms against 9.8 ms for
+// double-FP32 response sums).
 //
 // Mixed precision with polynomial factors (either scheme) and the adjoint
 // without checkpoints (Euler): the FP32 response form of hjm_mresp.cu when
@@ -815,151 +798,62 @@ static void fill_pc(const hjm_ctx* ctx, const RunShape& sh, double dt, const Pat
 // 20 dates in 8), else the convected pairs.
 static bool use_response_form(const hjm_ctx* ctx) { return ctx->remainder != HJM_REMAINDER_CONVECT; }
 
-// The volatility-table response table of the run shape, scheme and loadings
-// sv [kFactors][kMaxTenor] (the path parameters'), on the stream: rebuilt
-// only when it changed, after the kernels of earlier valuations that read it.
-static hjm_status ensure_vol_response_table(hjm_ctx* ctx, const RunShape& sh, double dt, const double* sv,
-                                            cudaStream_t s)
+// The contraction's operand table of the run shape, scheme and loadings sv
+// [kFactors][kMaxTenor] (the path parameters'), on the stream: rebuilt only
+// when it changed, after the kernels of earlier valuations that read it.
+static hjm_status ensure_contract_table(hjm_ctx* ctx, const RunShape& sh, double dt, const double* sv, bool ext,
+                                        cudaStream_t s)
 {
     const double c = dt / ctx->dtau;
     const int nt = ctx->nt;
     std::vector<double> key((size_t)kFactors * nt);
     for (int k = 0; k < kFactors; ++k)
         for (int t = 0; t < nt; ++t) key[(size_t)k * nt + t] = sv[k * kMaxTenor + t];
-    hjm_ctx::VrespKey& k = ctx->vresp_key;
+    hjm_ctx::ContractKey& k = ctx->contract_key;
     if (!ctx->resp_used) HJM_CUDA(ctx, cudaEventCreateWithFlags(&ctx->resp_used, cudaEventDisableTiming));
     if (k.valid && k.nt == nt && k.stride == sh.stride && k.B == sh.B && k.c == c && k.scheme == ctx->scheme &&
-        k.sv == key)
+        k.ext == ext && k.sv == key)
         return HJM_OK;
     k.valid = false;
-    const size_t bytes = sizeof(float4) * response_table_vol_elems(sh.stride, sh.B);
-    if (bytes > ctx->vresp.bytes)
-        HJM_CUDA(ctx, ctx->vresp.ensure(bytes));  // cudaFree waits for the device
+    const size_t bytes = contract_table_bytes(sh.stride, sh.B, ext);
+    if (bytes > ctx->contract.bytes)
+        HJM_CUDA(ctx, ctx->contract.ensure(bytes));  // cudaFree waits for the device
     else
         HJM_CUDA(ctx, cudaStreamWaitEvent(s, ctx->resp_used, 0));
-    HJM_CUDA(ctx, cudaMemsetAsync(ctx->vresp.p, 0, bytes, s));  // entries the kernel reads as exact zeros
-    HJM_CUDA(ctx, launch_response_table_vol(nt, c, sh.stride, sh.B, ctx->scheme == HJM_SCHEME_PREDICTOR_CORRECTOR, sv,
-                                            (float4*)ctx->vresp.p, s));
-    ctx->stat_launches += 1;
+    HJM_CUDA(ctx, launch_contract_table(nt, c, sh.stride, sh.B, ctx->scheme == HJM_SCHEME_PREDICTOR_CORRECTOR, ext,
+                                        sv, ctx->contract.p, s));
+    ctx->stat_launches += 1 + contract_windows(sh.B, sh.stride, ext, nullptr);
     k.nt = nt;
     k.stride = sh.stride;
     k.B = sh.B;
     k.c = c;
     k.scheme = ctx->scheme;
+    k.ext = ext;
     k.sv = key;
     k.valid = true;
     return HJM_OK;
 }
 
-// The response form's table (remainder and residual responses, frame
-// coefficients, active prefixes) for the run shape and decomposition, on the
-// stream: rebuilt only when they changed, after the kernels of earlier
-// valuations that read it.
-static hjm_status ensure_eresp_table(hjm_ctx* ctx, const RunShape& sh, double dt,
-                                     const std::vector<EulerRespFrame>& frames, const std::vector<double>& resid,
-                                     int nres, bool pc, cudaStream_t s)
+// An FP64 valuation in the response form (hjm_contract.cu): the operand table
+// of the market's loadings, the carry of a windowed run, one launch per
+// window.  P: the scheme's parameters (the predictor-corrector's N-projected
+// loadings and deterministic curve).  ext_dev: external normals with their row
+// scales behind them (hjm_run_with_normals), or null.
+static hjm_status enqueue_contract(hjm_ctx* ctx, const RunShape& sh, double dt, const PathParams<double>& P,
+                                   const double* ext_dev, double* estore, cudaStream_t s)
 {
-    const EulerRespFrame& fr = frames[0];
-    const double c = dt / ctx->dtau;
-    hjm_ctx::ErespKey& k = ctx->eresp_key;
-    if (!ctx->resp_used) HJM_CUDA(ctx, cudaEventCreateWithFlags(&ctx->resp_used, cudaEventDisableTiming));
-    if (k.valid && k.pc == pc && k.nt == ctx->nt && k.stride == sh.stride && k.B == sh.B && k.np == fr.np && k.c == c &&
-        k.dtau == ctx->dtau && k.nres == nres && k.frames.size() == frames.size() &&
-        std::memcmp(k.frames.data(), frames.data(), sizeof(EulerRespFrame) * frames.size()) == 0 && k.resid == resid)
-        return HJM_OK;
-    k.valid = false;
-    const size_t bytes = sizeof(float4) * eresp_table_elems(sh.stride, sh.B, fr.np, nres, (int)frames.size());
-    if (bytes > ctx->eresp.bytes)
-        HJM_CUDA(ctx, ctx->eresp.ensure(bytes));  // cudaFree waits for the device
-    else
-        HJM_CUDA(ctx, cudaStreamWaitEvent(s, ctx->resp_used, 0));
-    HJM_CUDA(ctx, launch_eresp_tables(ctx->nt, c, ctx->dtau, sh.stride, sh.B, frames.data(), (int)frames.size(),
-                                      resid.empty() ? nullptr : resid.data(), nres, pc, (float4*)ctx->eresp.p, s));
-    ctx->stat_launches += 3;
-    k.pc = pc;
-    k.nt = ctx->nt;
-    k.stride = sh.stride;
-    k.B = sh.B;
-    k.np = fr.np;
-    k.nres = nres;
-    k.c = c;
-    k.dtau = ctx->dtau;
-    k.frames = frames;
-    k.resid = resid;
-    k.valid = true;
-    return HJM_OK;
-}
-
-// An FP64 valuation in the response form (hjm_eresp.cu): the parts' frame
-// and loadings of the market's decomposition, the table, the carry of a
-// windowed run, and one launch per window.  Q: the predictor-corrector's
-// parameters (its parts' step, N-projected loadings and deterministic
-// curve; quadratic factors), or null for the Euler step.
-static hjm_status enqueue_eresp(hjm_ctx* ctx, const RunShape& sh, double dt, const PathParams<double>& P,
-                                const double* ext_dev, double* estore, cudaStream_t s,
-                                const PcParams<double>* Q = nullptr)
-{
-    const bool pc = Q != nullptr;
-    const bool cubic = !pc && use_cubic_path(ctx);
-    std::vector<double> resid;
-    int nres = 0;
-    if (cubic) {
-        const double sq = std::sqrt(dt);
-        resid.resize(ctx->resid.size());
-        for (size_t i = 0; i < resid.size(); ++i) resid[i] = sq * ctx->resid[i];
-        nres = eresp_residual_factors(ctx->resid.data(), ctx->vol.data(), ctx->nt);
-    }
-    // the earliest date the remainder reaches (the windows hold slots from it on)
-    const double c = dt / ctx->dtau;
-    hjm_ctx::ErespFirst& fa = ctx->eresp_first;
-    if (!(fa.valid && fa.pc == pc && fa.nt == ctx->nt && fa.stride == sh.stride && fa.B == sh.B && fa.nres == nres &&
-          fa.c == c)) {
-        fa.first = eresp_first_active_date(ctx->nt, c, sh.stride, sh.B, nres, pc);
-        fa.pc = pc;
-        fa.nt = ctx->nt;
-        fa.stride = sh.stride;
-        fa.B = sh.B;
-        fa.nres = nres;
-        fa.c = c;
-        fa.valid = true;
-    }
-    int lo[kMaxTenor], hi[kMaxTenor];
-    const int n_windows = eresp_windows(sh.B, fa.first, lo, hi, nullptr, eresp_window_dates(nres));
-    std::vector<EulerRespFrame> frames(n_windows);
-    int degs = 0;
-    double svc_pc[kFactors][3];  // the predictor-corrector's N-projected loadings of 1, T, T^2
-    if (pc)
-        for (int k = 0; k < kFactors; ++k) {
-            svc_pc[k][0] = Q->aS[k];
-            svc_pc[k][1] = Q->aU[k];
-            svc_pc[k][2] = Q->aW[k];
-        }
-    for (int w = 0; w < n_windows; ++w)
-        eresp_make_frame(dt, ctx->dtau, ctx->nt, pc ? svc_pc : P.svc, cubic ? &ctx->cubic[0][0] : nullptr,
-                         ctx->cubic_degs, eresp_window_centre(ctx->dtau, lo[w], hi[w]), frames[w], degs, pc);
-    const EulerRespFrame& fr = frames[0];
-    const size_t smem = eresp_max_smem(sh.B, fr.np, sh.stride, fa.first, nres);
-    if (smem > 227 * 1024) return fail(ctx, HJM_ERR_UNSUPPORTED, "shared memory %zu B exceeds 227 KB", smem);
-    hjm_status st = ensure_eresp_table(ctx, sh, dt, frames, resid, nres, pc, s);
+    hjm_status st = ensure_contract_table(ctx, sh, dt, &P.sv[0][0], ext_dev != nullptr, s);
     if (st != HJM_OK) return st;
-    EulerRespParams E;
-    std::memset(&E, 0, sizeof(E));
-    E.P = P;
-    E.wnew_L = pc ? Q->gL : 0.0;
-    E.tenor_L = ctx->nt - 1;
-    E.frame = block_frame_n(fr.n, sh.stride);
-    E.row = eresp_row(sh.B);
-    // the pairs are renormalised for the residual's terms and for runs of more
-    // than 25 dates, whose dates near the last tenor carry large remainders
-    E.renorm = (cubic || sh.B > kRespSlots + 1) ? 1 : 0;
     double* carry = nullptr;
-    if (n_windows > 1) {
+    if (contract_windows(sh.B, sh.stride, ext_dev != nullptr, nullptr) > 1) {
         HJM_CUDA(ctx, ctx->carry.ensure(sizeof(double) * 2 * (size_t)P.n_paths));
         carry = (double*)ctx->carry.p;
     }
+    const double* ext_scale =
+        ext_dev ? ext_dev + (size_t)P.n_paths * (size_t)sh.B * (size_t)sh.stride * kFactors : nullptr;
     int launches = 0;
-    HJM_CUDA(ctx, launch_path_fp64_eresp(E, frames.data(), degs, nres, (const float4*)ctx->eresp.p, fa.first, ext_dev,
-                                         (double*)ctx->partials.p, estore, carry, s, &launches));
+    HJM_CUDA(ctx, launch_path_contract(ctx->nt, P, ctx->contract.p, ext_dev, ext_scale, (double*)ctx->partials.p,
+                                       estore, carry, (double*)ctx->result.p, ctx->n_sms, s, &launches));
     ctx->stat_launches += launches - 1;
     return HJM_OK;
 }
@@ -1035,23 +929,6 @@ static hjm_status ensure_mresp_table(hjm_ctx* ctx, cudaStream_t s)
     return HJM_OK;
 }
 
-// The volatility-table step in the response form (its table already on the
-// stream): the carry of a windowed run, one launch per window.
-static hjm_status enqueue_vresp(hjm_ctx* ctx, const RunShape& sh, const PathParams<double>& P, const double* ext_dev,
-                                double* estore, cudaStream_t s)
-{
-    double* carry = nullptr;
-    if (vresp_windows(sh.B) > 1) {
-        HJM_CUDA(ctx, ctx->carry.ensure(sizeof(double) * 2 * (size_t)P.n_paths));
-        carry = (double*)ctx->carry.p;
-    }
-    int launches = 0;
-    HJM_CUDA(ctx, launch_path_fp64_vresp(ctx->nt, P, (const float4*)ctx->vresp.p, ext_dev, (double*)ctx->partials.p,
-                                         estore, carry, s, &launches));
-    ctx->stat_launches += launches - 1;
-    return HJM_OK;
-}
-
 static hjm_status enqueue_impl(hjm_ctx* ctx, int64_t n_paths, int32_t n_steps, double dt, uint64_t seed,
                                uint64_t path_offset, int32_t precision, double hazard, double recovery, double pfe_q,
                                const double* ext_dev)
@@ -1074,7 +951,8 @@ static hjm_status enqueue_impl(hjm_ctx* ctx, int64_t n_paths, int32_t n_steps, d
                           use_response_form(ctx))
                              ? mresp_run_slots(ctx, sh, dt, pc)
                              : 0;
-    const int cta = mresp_ns ? kCta
+    const int cta = !mixed && use_response_form(ctx) ? kContractTile
+                    : mresp_ns                       ? kCta
                              : (pc ? pc_cta() : path_cta(mixed, ctx->nt, sh.B, use_poly_path(ctx) || mixed_cubic));
     const int64_t n_ctas = (n_paths + cta - 1) / cta;
     const int64_t ld = (n_paths + 3) / 4 * 4;
@@ -1141,15 +1019,8 @@ static hjm_status enqueue_impl(hjm_ctx* ctx, int64_t n_paths, int32_t n_steps, d
         fill_pc<double>(ctx, sh, dt, P, Q);
         ctx->stat_h2d = sizeof(Q) + sizeof(FinalParams);
         resp = use_response_form(ctx);
-        if (resp && use_poly_path(ctx)) {
-            // the decomposition in the response form of hjm_eresp.cu, with the
-            // two-stage step's parts frame and remainder table (any number of dates)
-            st = enqueue_eresp(ctx, sh, dt, Q.P, ext_dev, store ? (double*)ctx->estore.p : nullptr, s, &Q);
-            if (st != HJM_OK) return st;
-        } else if (resp) {
-            st = ensure_vol_response_table(ctx, sh, dt, &Q.P.sv[0][0], s);
-            if (st != HJM_OK) return st;
-            st = enqueue_vresp(ctx, sh, Q.P, ext_dev, store ? (double*)ctx->estore.p : nullptr, s);
+        if (resp) {
+            st = enqueue_contract(ctx, sh, dt, Q.P, ext_dev, store ? (double*)ctx->estore.p : nullptr, s);
             if (st != HJM_OK) return st;
         } else {
             HJM_CUDA(ctx, launch_path_pc(ctx->nt, Q, use_poly_path(ctx), ext_dev, (double*)ctx->partials.p,
@@ -1181,15 +1052,10 @@ static hjm_status enqueue_impl(hjm_ctx* ctx, int64_t n_paths, int32_t n_steps, d
         PathParams<double> P;
         fill_params<double>(ctx, sh, n_paths, dt, seed, path_offset, hazard, recovery, ld, store, P, F);
         resp = use_response_form(ctx);
-        if (resp && (use_poly_path(ctx) || use_cubic_path(ctx))) {
-            st = enqueue_eresp(ctx, sh, dt, P, ext_dev, store ? (double*)ctx->estore.p : nullptr, s);
+        if (resp) {
+            st = enqueue_contract(ctx, sh, dt, P, ext_dev, store ? (double*)ctx->estore.p : nullptr, s);
             if (st != HJM_OK) return st;
-            run_form = vol_form_code(ctx);
-        } else if (resp) {
-            st = ensure_vol_response_table(ctx, sh, dt, &P.sv[0][0], s);
-            if (st != HJM_OK) return st;
-            st = enqueue_vresp(ctx, sh, P, ext_dev, store ? (double*)ctx->estore.p : nullptr, s);
-            if (st != HJM_OK) return st;
+            if (use_cubic_path(ctx)) run_form = vol_form_code(ctx);
         } else {
             // convected: the quadratic decomposition, else the table step
             HJM_CUDA(ctx, launch_path_fp64(ctx->nt, P, use_poly_path(ctx), ext_dev,
@@ -1261,6 +1127,7 @@ hjm_status hjm_fetch_results(hjm_ctx* ctx, double* ee_out, double* pfe_out, doub
     HJM_CUDA(ctx, cudaMemcpyAsync(res, ctx->result.p, sizeof(res), cudaMemcpyDeviceToHost, ctx->stream));
     HJM_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     ctx->stat_d2h += (int64_t)sizeof(res);
+    if (res[kResErr] != 0.0) return fail(ctx, HJM_ERR_CUDA, "a wait of the path kernel ran out");
     if (ee_out)
         for (int j = 0; j < ctx->nt; ++j) ee_out[j] = res[kResEE + j];
     if (pfe_out)
@@ -1305,11 +1172,13 @@ hjm_status hjm_run_with_normals(hjm_ctx* ctx, int64_t n_paths, int32_t n_steps, 
     if (count > ((size_t)1 << 33)) return fail(ctx, HJM_ERR_INVALID_ARGUMENT, "normals buffer too large");
     HJM_CUDA(ctx, cudaSetDevice(ctx->device));
     HJM_CUDA(ctx, ctx->ext_raw.ensure(sizeof(double) * count));
-    HJM_CUDA(ctx, ctx->ext.ensure(sizeof(double) * count));
+    HJM_CUDA(ctx, ctx->ext.ensure(sizeof(double) * (count + 2 * (size_t)n_paths)));
     HJM_CUDA(ctx, cudaMemcpyAsync(ctx->ext_raw.p, normals_host, sizeof(double) * count, cudaMemcpyHostToDevice,
                                   ctx->stream));
     HJM_CUDA(ctx, launch_transpose_normals((const double*)ctx->ext_raw.p, n_paths, n_steps, (double*)ctx->ext.p,
                                            ctx->stream));
+    HJM_CUDA(ctx, launch_contract_ext_scale((const double*)ctx->ext_raw.p, n_paths, n_steps,
+                                            (double*)ctx->ext.p + count, ctx->stream));
     const double q = pfe_out ? pfe_quantile : 0.0;
     hjm_status st = enqueue_impl(ctx, n_paths, n_steps, dt, 0, 0, precision, hazard_rate, recovery, q,
                                  (const double*)ctx->ext.p);

@@ -1,0 +1,879 @@
+// hjm_contract.cu -- the FP64 valuation's response form as a contraction on
+// the tensor cores (tcgen05), for every volatility market, either time scheme
+// and any number of dates.
+//
+// The pricing of date j reads the stochastic curve h_n = A h_{n-1} + S phi_n
+// (A the upwind step, simulation_cpu.h:96-108, or the predictor-corrector's
+// three-point step) only at tenor j: its value after the date's last step K_j
+// and its sum over the steps, both linear in the path's normals,
+//     h_K[j] = sum_{n,k} phi_{n,k} R_jk(K - n),  R_jk(l) = (A^l S_k)[j],
+// and likewise with CR_jk(l) = sum_{r<=l} R_jk(r).  Over the paths of a tile
+// that is a matrix product: normals [128][steps x 3] times responses
+// [steps x 3][2 per date].
+//
+// FP64 accuracy from FP16 operands.  Each normal is cut into slices on fixed
+// grids, phi = a0 + a1 2^-10 + a2 2^-20 + a3 2^-30: a0, a1, a2 multiples of
+// 2^-7 (the remainder of one is scaled by 2^10 for the next, so |a1|, |a2| <=
+// 4), a3 what is left, rounded to 11 bits (exact for |phi| >= 2^-15; external
+// FP64 normals take a fifth slice).  Each response, scaled per date by a power
+// of two to at most 2^8, is cut likewise into b0 .. b3 (integers up to 2^9) and
+// b4.  Every slice is exact in FP16, every product a_i b_j exact in FP32, and
+// the products of one level s = i + j share one grid, so each level has an FP32
+// accumulator of its own: over 12 chunks of 16 steps (576 products) levels 0
+// and 1 stay below 2^21.1 grid units (rms, for the worst column), 7.5 standard
+// deviations from the 2^24 up to which the accumulators add exactly; level 2's
+// rounding lies 2^-40 below the curve and is met once in 10^5, levels 3 and 4's
+// lies 2^-54 below.  Products of level 5 and above are dropped (2^-48).  After
+// 12 chunks the five accumulators are added, level by level, into double-FP32
+// running sums (Knuth's two-sum) and restart from zero.  Per-path exposures
+// then lie 1e-14 of their scale from the oracle (the convected all-FP64 step:
+// 5e-15; double-FP32 response sums on the FP32 pipe: 5e-14); with three slices
+// fewer bits (grids 2^-12 apart, four levels) it was 6e-13.
+//
+// Roles of a CTA (one per SM, persistent over tiles of 128 paths):
+//   warps 0-15   normals: Philox in registers, Box-Muller, slices; warp w holds
+//                paths 32 (w % 4) + lane and half the steps of every second chunk
+//                and stores the slices to the A operand in tensor memory
+//                (counter-based draws: 16 warps share 128 paths);
+//   warp 20      one lane: B operand tiles by bulk copy (TMA) into shared
+//                memory, tcgen05.mma, commits;
+//   warps 16-19  thread = path: accumulators to running sums, pricing of the
+//                dates in FP64, exposures, partial sums, exposure rows.
+// Accumulator columns are ordered [level][date slot]: the slices b0..b4 of a
+// k-tile are consecutive rows of B, so a_s needs one instruction of (5 - s)
+// npad columns (levels s..4): four instructions per 16-deep k-tile instead of
+// fourteen.
+//
+// What bounds it: instruction issue in the sixteen normal warps, ~180 issue
+// cycles per 32 path-steps (Philox's 18 wide multiplications take four each,
+// the packed slicing operations two).  The matrix instructions of the 10y
+// swap's 20 dates fill 1,008 of a chunk's ~3,100 cycles.  1,048,576 paths x
+// 1,000 steps, FP64, 10y swap: 5.15 ms against 12.9 ms for the same sums in
+// double-FP32 (a date costs no instructions per step any more); a table of any
+// shape 28.3 -> 5.3 ms; the reference driver's 25y call (its PCA table, 50
+// dates) 130 -> 19.7 ms.
+#include <cuda_fp16.h>
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+
+#include "hjm_contract.h"
+#include "hjm_kernels.h"
+#include "hjm_resp.cuh"
+
+namespace hjm {
+
+namespace {
+
+constexpr int kChunk = 16;               // evolved steps per chunk: 48 = 3 x 16 contraction depth
+constexpr int kFlush = 12;               // chunks per accumulator group
+constexpr int kSlices = 4;                // of a normal
+constexpr int kLevels = 5;                // of a response, and accumulators
+constexpr int kProducers = 16;           // warps
+constexpr int kEpilogueWarp = 16;        // first of four
+constexpr int kMmaWarp = 20;
+constexpr int kThreads = 32 * 21;
+constexpr int kAStages = 2, kBStages = 3;
+constexpr int kTmemCols = 512;
+// External FP64 normals take a fifth slice (what FP32 does not hold)
+__host__ __device__ constexpr int slices_of(bool ext) { return ext ? kSlices + 1 : kSlices; }
+// 32-bit tensor-memory columns of a chunk's A slices; the A stages lie behind
+// the accumulators
+__host__ __device__ constexpr int a_stage_cols(bool ext) { return slices_of(ext) * 24; }
+__host__ __device__ constexpr int a_col(bool ext) { return kTmemCols - kAStages * a_stage_cols(ext); }
+static_assert(kLevels * 2 * kContractMaxSlots <= a_col(false) && kLevels * 2 * kContractExtSlots <= a_col(true),
+              "accumulators and A stages share 512 columns");
+
+// bytes of one chunk of the B image: 3 k-tiles of 16 x (kLevels npad) halves
+__host__ __device__ constexpr size_t chunk_bytes(int npad) { return (size_t)3 * kLevels * npad * 32; }
+
+constexpr size_t kScaleBytes = 2 * kMaxTenor * sizeof(double);
+
+// A wait that runs out after this many cycles, about a second (every wait here
+// is for work in flight, so it would be a fault of the program), ends the
+// kernel with result[kResErr] set.
+constexpr long long kWaitCycles = 2000000000;
+
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count)
+{
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint32_t bar)
+{
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity)
+{
+    uint32_t ok;
+    asm volatile(
+        "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+// false when the wait ran out, here or in another warp (*abort_s)
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_s)
+{
+    if (mbar_try(bar, parity)) return true;
+    for (const long long t0 = clock64(); clock64() - t0 < kWaitCycles && !*abort_s;)
+        if (mbar_try(bar, parity)) return true;
+    *abort_s = 1;
+    return false;
+}
+
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t e;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(e));
+    return e != 0;
+}
+
+__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+
+__device__ __forceinline__ void tc_commit(uint32_t bar)
+{
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+// D[128][n] (+)= A[128][16] (tensor memory) B[n][16]^T (shared memory), FP16 in, FP32 accumulators
+__device__ __forceinline__ void tc_mma(uint32_t d, uint32_t a, uint64_t b_desc, uint32_t idesc, uint32_t accumulate)
+{
+    asm volatile(
+        "{\n.reg .pred p;\nsetp.ne.u32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}" ::"r"(d),
+        "r"(a), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+// instruction descriptor: FP32 accumulators, FP16 operands, both K-major, M = 128
+__device__ __forceinline__ uint32_t tc_idesc(int n) { return (1u << 4) | ((uint32_t)(n >> 3) << 17) | (8u << 24); }
+// shared-memory descriptor of a K-major, unswizzled tile: 8 x 16-byte core
+// matrices, consecutive along n (128 bytes), `k_stride` bytes apart along k
+__device__ __forceinline__ uint64_t tc_smem_desc(uint32_t addr, uint32_t k_stride)
+{
+    return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)(k_stride >> 4) << 16) | ((uint64_t)(128u >> 4) << 32) |
+           ((uint64_t)1 << 46);
+}
+
+__device__ __forceinline__ void tmem_st4(uint32_t addr, const uint32_t* r)
+{
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(r[0]), "r"(r[1]),
+                 "r"(r[2]), "r"(r[3])
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_st2(uint32_t addr, const uint32_t* r)
+{
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x2.b32 [%0], {%1, %2};" ::"r"(addr), "r"(r[0]), "r"(r[1])
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_ld8(uint32_t addr, float* r)
+{
+    uint32_t u[8];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7])
+                 : "r"(addr)
+                 : "memory");
+#pragma unroll
+    for (int i = 0; i < 8; ++i) r[i] = __uint_as_float(u[i]);
+}
+
+constexpr float kGrid = 98304.0f;      // 1.5 2^16: adding it rounds to multiples of 2^-7
+constexpr float kShift = 1024.0f;      // 2^10 between slices
+constexpr int kTopBits = 8;            // the largest response of a date is scaled to at most 2^8
+
+// The four slices of two normals, negated (the epilogue's scale carries the
+// sign back): -a_s from the constant minus the rounded sum, so that no
+// instruction negates.  Packed FP32 pairs throughout; every step is exact
+// until the last conversion.
+__device__ __forceinline__ void slice_pair(float2 v, uint32_t (&out)[kSlices])
+{
+    const float2 g = make_float2(kGrid, kGrid), m1 = make_float2(-1.0f, -1.0f), sh = make_float2(kShift, kShift);
+    float2 na = __ffma2_rn(__fadd2_rn(v, g), m1, g);
+    float2 d = __fadd2_rn(v, na);
+#pragma unroll
+    for (int s = 0; s < kSlices - 1; ++s) {
+        const __half2 h = __floats2half2_rn(na.x, na.y);
+        out[s] = *reinterpret_cast<const uint32_t*>(&h);
+        if (s < kSlices - 2) {
+            na = __ffma2_rn(__ffma2_rn(d, sh, g), m1, g);
+            d = __ffma2_rn(d, sh, na);
+        }
+    }
+    d = __fmul2_rn(d, make_float2(-kShift, -kShift));
+    const __half2 h = __floats2half2_rn(d.x, d.y);
+    out[kSlices - 1] = *reinterpret_cast<const uint32_t*>(&h);
+}
+// ... of two FP64 normals (below 8 in magnitude), with a fifth slice for what
+// the fourth leaves; values that FP32 holds give the slices above
+__device__ __forceinline__ void slice_pair(double x, double y, uint32_t (&out)[kSlices + 1])
+{
+    const double g = 52776558133248.0;  // 1.5 2^45: rounds to multiples of 2^-7
+    const bool fx = (double)(float)x == x, fy = (double)(float)y == y;
+#pragma unroll
+    for (int s = 0; s <= kSlices; ++s) {
+        double ax = x, ay = y;
+        if (s < kSlices - 1) {
+            ax = __dsub_rn(__dadd_rn(x, g), g);
+            ay = __dsub_rn(__dadd_rn(y, g), g);
+        }
+        __half2 h = __floats2half2_rn(-(float)ax, -(float)ay);
+        if (s == kSlices) h = __halves2half2(fx ? __half(0.0f) : __low2half(h), fy ? __half(0.0f) : __high2half(h));
+        out[s] = *reinterpret_cast<const uint32_t*>(&h);
+        x = (x + (double)__low2float(h)) * (double)kShift;
+        y = (y + (double)__high2float(h)) * (double)kShift;
+    }
+}
+
+// Philox4x32-10 of counter (step, 0, path): what depends on the path alone is
+// formed once per tile (the first round's product of the path word and the
+// second round's of the result), leaving 18 of the 20 multiplications per step.
+struct PathDraw {
+    uint32_t hi2, lo2;   // second round: high word (with its key) and low word of the path's product
+    uint32_t y2;         // first round's low word with the second round's key
+    uint32_t z1;         // path's high word with the first round's key
+};
+__device__ __forceinline__ PathDraw path_draw(uint64_t path, const uint32_t* rk0, const uint32_t* rk1)
+{
+    const uint64_t p1 = (uint64_t)0xCD9E8D57u * (uint32_t)path;
+    const uint64_t q0 = (uint64_t)0xD2511F53u * ((uint32_t)(p1 >> 32) ^ rk0[0]);
+    PathDraw d;
+    d.hi2 = (uint32_t)(q0 >> 32) ^ rk1[1];
+    d.lo2 = (uint32_t)q0;
+    d.y2 = (uint32_t)p1 ^ rk0[1];
+    d.z1 = (uint32_t)(path >> 32) ^ rk1[0];
+    return d;
+}
+__device__ __forceinline__ uint4 draw_words(const PathDraw& d, uint32_t step, const uint32_t* rk0, const uint32_t* rk1)
+{
+    const uint64_t p0 = (uint64_t)0xD2511F53u * step;
+    const uint64_t p1 = (uint64_t)0xCD9E8D57u * ((uint32_t)(p0 >> 32) ^ d.z1);
+    uint4 c = make_uint4((uint32_t)(p1 >> 32) ^ d.y2, (uint32_t)p1, d.hi2 ^ (uint32_t)p0, d.lo2);
+#pragma unroll
+    for (int r = 2; r < 10; ++r) {
+        const uint64_t a = (uint64_t)0xD2511F53u * c.x;
+        const uint64_t b = (uint64_t)0xCD9E8D57u * c.z;
+        c = make_uint4((uint32_t)(b >> 32) ^ c.y ^ rk0[r], (uint32_t)b, (uint32_t)(a >> 32) ^ c.w ^ rk1[r],
+                       (uint32_t)a);
+    }
+    return c;
+}
+
+__device__ __forceinline__ float2 f2(float x, float y) { return make_float2(x, y); }
+
+// a - b as one packed FMA (a negated operand would take instructions of its own)
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, f2(-1.0f, -1.0f), a); }
+
+// {H, L} += a exactly up to 2^-48 of H: Knuth's two-sum into the high part
+__device__ __forceinline__ void pair_add(float2& H, float2& L, float2 a)
+{
+    const float2 s = __fadd2_rn(H, a);
+    const float2 bp = sub2(s, H);
+    const float2 ap = sub2(s, bp);
+    L = __fadd2_rn(L, __fadd2_rn(sub2(H, ap), sub2(a, bp)));
+    H = s;
+}
+
+__device__ __forceinline__ void epilogue_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+
+}  // namespace
+
+// The launch's constants besides the path parameters.
+struct ContractParams {
+    PathParams<double> P;
+    ContractWindow W;
+    int64_t n_tiles;
+};
+
+template <bool EXT>
+__global__ void __launch_bounds__(kThreads, 1)
+    path_kernel_contract(const __grid_constant__ ContractParams Q, const unsigned char* __restrict__ table,
+                         const double* __restrict__ ext, const double* __restrict__ ext_scale,
+                         double* __restrict__ partials, double* __restrict__ estore, double* __restrict__ carry,
+                         double* __restrict__ result)
+{
+    constexpr int kSl = slices_of(EXT), kAStageCols = a_stage_cols(EXT), kACol = a_col(EXT);
+    const PathParams<double>& P = Q.P;
+    const ContractWindow& W = Q.W;
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ __align__(8) uint64_t bars[2 * kAStages + 2 * kBStages + 3];
+    __shared__ uint32_t tmem_s;
+    __shared__ int abort_flag;
+    __shared__ double red_s[8];
+    volatile int* abort_s = &abort_flag;
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int lo = W.lo, hi = W.hi, npad = W.npad, NC = W.chunks;
+    const size_t cb = chunk_bytes(npad);
+    unsigned char* b_s = smem;                                                       // [kBStages][cb]
+    float4* run_s = reinterpret_cast<float4*>(smem + kBStages * cb);                  // [npad / 2][128] {H x, H sum, L x, L sum}
+    double* cf_s = reinterpret_cast<double*>(run_s + (size_t)(npad / 2) * kContractTile);  // [hi - lo + 3][128]
+
+    const uint32_t a_full = smem_u32(bars), a_empty = a_full + 8 * kAStages, b_full = a_empty + 8 * kAStages,
+                   b_empty = b_full + 8 * kBStages, d_full = b_empty + 8 * kBStages, d_empty = d_full + 8, drain = d_empty + 8;
+    if (warp == kMmaWarp) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_s)),
+                     "n"(kTmemCols)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    if (tid == 0) {
+        for (int i = 0; i < kAStages; ++i) {
+            mbar_init(a_full + 8 * i, kProducers / kAStages);
+            mbar_init(a_empty + 8 * i, 1);
+        }
+        for (int i = 0; i < kBStages; ++i) {
+            mbar_init(b_full + 8 * i, 1);
+            mbar_init(b_empty + 8 * i, 1);
+        }
+        mbar_init(d_full, 1);
+        mbar_init(d_empty, 4);
+        mbar_init(drain, 1);
+        abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_s;
+
+    if (warp < kProducers) {
+        // ---- normals -> A slices in tensor memory.  Two groups of 8 warps take
+        // the chunks of this CTA's sequence in turn, one A stage each, so that
+        // one group's waits and stores lie under the other's arithmetic; a warp
+        // has 8 steps of its chunk, in two halves of 4
+        const int q = warp & 3, sub = (warp >> 2) & 1, st = warp >> 3;
+        const uint32_t a_addr = tmem + ((uint32_t)(32 * q) << 16) + kACol + st * kAStageCols + 12 * sub;
+        const int n_last = P.n_blocks * P.stride - 1;
+        uint32_t ph = 1;
+        bool ok = NC > 0;
+        int c = st;
+        int64_t tile = blockIdx.x;
+        while (ok) {
+            for (; c >= NC; c -= NC) tile += gridDim.x;
+            if (tile >= Q.n_tiles) break;
+            const int64_t lp = tile * kContractTile + 32 * q + lane;
+            const PathDraw pd = path_draw(P.path_offset + (uint64_t)lp, P.rk0, P.rk1);
+            const int64_t lpc = lp < P.n_paths ? lp : 0;
+            double xs = 1.0;
+            if constexpr (EXT) xs = __ldg(ext_scale + 2 * lpc);
+            for (; c < NC; c += kAStages, ph ^= 1u) {
+#pragma unroll 1
+                for (int half = 0; half < 2; ++half) {
+                    const int n0 = P.stride + kChunk * c + 8 * sub + 4 * half;
+                    // value 3 i + k: step n0 + i, factor k; pairs of values are one column
+                    uint32_t w[kSl][6];
+                    if constexpr (EXT) {
+                        double z[12];
+                        const size_t np = (size_t)P.n_paths;
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+#pragma unroll
+                            for (int k = 0; k < 3; ++k)
+                                z[3 * i + k] = __ldg(ext + (size_t)min(n0 + i, n_last) * 3 * np + k * np + lpc) * xs;
+#pragma unroll
+                        for (int u = 0; u < 6; ++u) {
+                            uint32_t o[kSl];
+                            slice_pair(z[2 * u], z[2 * u + 1], o);
+#pragma unroll
+                            for (int s = 0; s < kSl; ++s) w[s][u] = o[s];
+                        }
+                    } else {
+                        float z[12];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const uint4 u = draw_words(pd, (uint32_t)(n0 + i), P.rk0, P.rk1);
+                            normals3(u, z[3 * i], z[3 * i + 1], z[3 * i + 2]);
+                        }
+#pragma unroll
+                        for (int u = 0; u < 6; ++u) {
+                            uint32_t o[kSlices];
+                            slice_pair(f2(z[2 * u], z[2 * u + 1]), o);
+#pragma unroll
+                            for (int s = 0; s < kSlices; ++s) w[s][u] = o[s];
+                        }
+                    }
+                    if (half == 0) {
+                        ok = mbar_wait(a_empty + 8 * st, ph, abort_s);
+                        ok = __all_sync(0xffffffffu, ok);
+                        if (!ok) break;
+                        tc_fence_after();
+                    }
+#pragma unroll
+                    for (int s = 0; s < kSl; ++s) {
+                        const uint32_t a = a_addr + 24 * s + 6 * half;
+                        tmem_st4(a, &w[s][0]);
+                        tmem_st2(a + 4, &w[s][4]);
+                    }
+                }
+                if (!ok) break;
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(a_full + 8 * st);
+            }
+        }
+    } else if (warp == kMmaWarp) {
+        // ---- B tiles and the matrix instructions: the warp waits as one, one
+        // elected lane issues
+        const bool leader = elect_one();
+        const uint32_t bs = smem_u32(b_s);
+        const int64_t tiles = blockIdx.x < Q.n_tiles ? (Q.n_tiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
+        const int64_t total = tiles * NC;
+        const unsigned char* image = table + W.image;
+        int64_t loaded = 0;
+        int load_c = 0, load_s = 0;  // the next load's chunk and stage
+        auto load = [&] {
+            const uint32_t bar = b_full + 8 * load_s;
+            if (leader) {
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"((uint32_t)cb)
+                             : "memory");
+                asm volatile(
+                    "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                        bs + (uint32_t)(load_s * cb)),
+                    "l"(image + (size_t)load_c * cb), "r"((uint32_t)cb), "r"(bar)
+                    : "memory");
+            }
+            ++loaded;
+            if (++load_c == NC) load_c = 0;
+            if (++load_s == kBStages) load_s = 0;
+        };
+        while (loaded < total && loaded < kBStages) load();
+        bool ok = true;
+        // a_s times the response slices b_0 .. b_{levels - 1 - s} gives the
+        // levels s .. 4; beyond 256 columns b_4 takes an instruction of its own
+        const bool split = kLevels * npad > 256;
+        uint32_t idesc[kSl];
+#pragma unroll
+        for (int s = 0; s < kSl; ++s) idesc[s] = tc_idesc((kLevels - s - (s == 0 && split)) * npad);
+        const uint32_t idesc1 = tc_idesc(npad);
+        const uint64_t desc0 = tc_smem_desc(bs, kLevels * npad * 16);
+        const uint32_t kt_step = (uint32_t)(kLevels * npad * 32) >> 4, stage_step = (uint32_t)cb >> 4;
+        int c = 0, st = 0, sb = 0, fl = 0;          // chunk of the tile, A and B stages, chunk of the group
+        uint32_t a_ph = 0, b_ph = 0, d_ph = 1;      // parities
+        for (int64_t g = 0; g < total; ++g) {
+            const bool first = fl == 0;
+            const bool last = fl == kFlush - 1 || c == NC - 1;
+            ok = mbar_wait(a_full + 8 * st, a_ph, abort_s) && mbar_wait(b_full + 8 * sb, b_ph, abort_s) &&
+                 (!first || mbar_wait(d_empty, d_ph, abort_s));
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            tc_fence_after();
+            if (leader) {
+                const uint64_t bd0 = desc0 + (uint64_t)(sb * stage_step);
+                const uint32_t a0 = tmem + kACol + st * kAStageCols;
+#pragma unroll
+                for (int kt = 0; kt < 3; ++kt) {
+                    const uint64_t bd = bd0 + (uint64_t)(kt * kt_step);
+                    const uint32_t a = a0 + 8 * kt;
+                    const uint32_t add = !(first && kt == 0);
+                    tc_mma(tmem, a, bd, idesc[0], add);
+                    if (split)
+                        tc_mma(tmem + (kLevels - 1) * npad, a, bd + (uint64_t)((kLevels - 1) * npad), idesc1, add);
+#pragma unroll
+                    for (int s = 1; s < kSl; ++s) tc_mma(tmem + s * npad, a + 24 * s, bd, idesc[s], 1);
+                }
+                tc_commit(a_empty + 8 * st);
+                tc_commit(b_empty + 8 * sb);
+                if (last) tc_commit(d_full);
+            }
+            // refill the stage of the chunk before (its instructions precede this chunk's)
+            if (g >= 1 && loaded < total) {
+                // that is stage load_s, in the phase before this chunk's if its ring wrapped
+                ok = mbar_wait(b_empty + 8 * load_s, sb == 0 ? b_ph ^ 1u : b_ph, abort_s);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                load();
+            }
+            if (first) d_ph ^= 1u;
+            if (++fl == kFlush || c == NC - 1) fl = 0;
+            if (++c == NC) c = 0;
+            if (++st == kAStages) {
+                st = 0;
+                a_ph ^= 1u;
+            }
+            if (++sb == kBStages) {
+                sb = 0;
+                b_ph ^= 1u;
+            }
+        }
+        if (!ok) {  // copies and matrix instructions in flight end before the CTA does
+            const long long t0 = clock64();
+            if (leader) tc_commit(drain);
+            while (!mbar_try(drain, 0) && clock64() - t0 < kWaitCycles) {
+            }
+            for (int64_t i = loaded > kBStages ? loaded - kBStages : 0; i < loaded; ++i)
+                while (!mbar_try(b_full + 8 * (int)(i % kBStages), (uint32_t)((i / kBStages) & 1)) &&
+                       clock64() - t0 < 2 * kWaitCycles) {
+                }
+        }
+        __syncwarp();
+    } else {
+        // ---- running sums, pricing, exposures: thread = path
+        const int q = warp & 3, p = tid - 32 * kEpilogueWarp;
+        const uint32_t d_addr = tmem + ((uint32_t)(32 * q) << 16);
+        const double* scale = reinterpret_cast<const double*>(table);  // [date][2]
+        const bool top = hi == P.n_blocks, bottom = lo == 1;
+        const int B = P.n_blocks, R = B + 3;
+        const int first_date = lo > 2 ? lo : 2;
+        double* e_s = cf_s + kContractTile;  // exposure row of date j: j - lo + 1 (the cash-flow row of date j + 1)
+        int64_t grp = 0;
+        bool ok = true;
+        for (int64_t tile = blockIdx.x; ok && tile < Q.n_tiles; tile += gridDim.x) {
+            const int64_t base = tile * kContractTile, lp = base + p;
+            const bool active = lp < P.n_paths;
+            double rs = 1.0;
+            if constexpr (EXT) rs = __ldg(ext_scale + 2 * (active ? lp : 0) + 1);
+            auto price = [&](int i) {
+                double x = P.psamp[i], a = P.psum[i];
+                if (i >= 2) {
+                    const float4 r = run_s[(size_t)(hi - i) * kContractTile + p];
+                    double sx = __ldg(scale + 2 * i), sa = __ldg(scale + 2 * i + 1);
+                    if constexpr (EXT) {
+                        sx *= rs;
+                        sa *= rs;
+                    }
+                    x = fma(-(widen_f32(r.x) + widen_f32(r.z)), sx, x);  // (the slices are negated)
+                    a = fma(-(widen_f32(r.y) + widen_f32(r.w)), sa, a);
+                }
+                const double D = exp(-a * P.dt);
+                const double Lb = P.m * (exp(x * P.inv_m) - 1.0);
+                cf_s[(size_t)(i - lo + 1) * kContractTile + p] = D * (P.payA[i] * Lb - P.payB[i]);
+            };
+            if (bottom) price(1);
+            int next = first_date;  // the earliest date not priced yet
+            for (int c = 0; c < NC; c += kFlush, ++grp) {
+                ok = mbar_wait(d_full, (uint32_t)(grp & 1), abort_s);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                tc_fence_after();
+                const int live = hi - next + 1;
+                // four slots at a time, padding included (its columns are zero): the
+                // four two-sum chains interleave
+                for (int r0 = 0; r0 < live; r0 += 4) {
+                    float acc[kLevels][8];
+#pragma unroll
+                    for (int s = 0; s < kLevels; ++s) tmem_ld8(d_addr + s * npad + 2 * r0, acc[s]);
+                    float4 cell[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        cell[u] = c ? run_s[(size_t)(r0 + u) * kContractTile + p] : make_float4(0.f, 0.f, 0.f, 0.f);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    if (r0 + 4 >= live) {  // the accumulators are read: the next group may start
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(d_empty);
+                    }
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        float2 H = f2(cell[u].x, cell[u].y), L = f2(cell[u].z, cell[u].w);
+                        pair_add(H, L, f2(acc[0][2 * u], acc[0][2 * u + 1]));
+                        pair_add(H, L, __fmul2_rn(f2(acc[1][2 * u], acc[1][2 * u + 1]), f2(0x1p-10f, 0x1p-10f)));
+                        pair_add(H, L, __fmul2_rn(f2(acc[2][2 * u], acc[2][2 * u + 1]), f2(0x1p-20f, 0x1p-20f)));
+                        L = __ffma2_rn(f2(acc[3][2 * u], acc[3][2 * u + 1]), f2(0x1p-30f, 0x1p-30f), L);
+                        L = __ffma2_rn(f2(acc[4][2 * u], acc[4][2 * u + 1]), f2(0x1p-40f, 0x1p-40f), L);
+                        const float2 sum = __fadd2_rn(H, L);
+                        L = __fadd2_rn(L, sub2(H, sum));
+                        H = sum;
+                        run_s[(size_t)(r0 + u) * kContractTile + p] = make_float4(H.x, H.y, L.x, L.y);
+                    }
+                }
+                // the dates whose last step this group held
+                const int done = kChunk * min(c + kFlush, NC);
+                for (; next <= hi && (next - 1) * P.stride <= done; ++next) price(next);
+            }
+            if (!ok) break;
+
+            // exposures E_j = max(sum_{i > j} cf_i, 0) of dates lo - 1 .. hi - 1
+            // (and E_B = 0 for the latest window), the later dates' cash flows in carry
+            double v = 0.0, cva_c = 0.0;
+            if (!top && active) {
+                v = carry[lp];
+                cva_c = carry[P.n_paths + lp];
+            }
+            if (top) e_s[(size_t)(B - lo + 1) * kContractTile + p] = 0.0;
+            for (int j = hi - 1; j >= lo - 1; --j) {
+                v += cf_s[(size_t)(j - lo + 2) * kContractTile + p];
+                double e = (v > 0.0) ? v : 0.0;
+                if (!active) e = 0.0;
+                e_s[(size_t)(j - lo + 1) * kContractTile + p] = e;
+                cva_c = fma(P.cvaw[j], e, cva_c);
+            }
+            if (!bottom && active) {
+                carry[lp] = v;
+                carry[P.n_paths + lp] = cva_c;
+            }
+            if (P.store_exposures) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            epilogue_sync();
+            const int j0 = lo - 1, j1 = top ? B : hi - 1;
+            for (int j = j0 + q; j <= j1; j += 4) {
+                double sum = 0.0;
+#pragma unroll
+                for (int u = 0; u < 4; ++u) sum += e_s[(size_t)(j - lo + 1) * kContractTile + lane + 32 * u];
+                sum = warp_sum(sum);
+                if (lane == 0) partials[(size_t)tile * R + j] = sum;
+            }
+            if (bottom) {
+                const double s1 = warp_sum(cva_c), s2 = warp_sum(cva_c * cva_c);
+                if (lane == 0) {
+                    red_s[q] = s1;
+                    red_s[4 + q] = s2;
+                }
+            }
+            if (p == 0 && P.store_exposures) {
+                const int64_t cnt = (P.n_paths - base < kContractTile) ? (P.n_paths - base) : kContractTile;
+                const uint32_t bytes = (uint32_t)(((cnt + 1) / 2) * 2 * sizeof(double));
+                for (int j = j0; j <= j1; ++j) {
+                    double* dst = estore + (size_t)j * (size_t)P.ld + (size_t)base;
+                    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst),
+                                 "r"(smem_u32(e_s + (size_t)(j - lo + 1) * kContractTile)), "r"(bytes)
+                                 : "memory");
+                }
+                asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+            }
+            epilogue_sync();
+            if (p == 0 && bottom) {
+                partials[(size_t)tile * R + B + 1] = (red_s[0] + red_s[1]) + (red_s[2] + red_s[3]);
+                partials[(size_t)tile * R + B + 2] = (red_s[4] + red_s[5]) + (red_s[6] + red_s[7]);
+            }
+        }
+        if (p == 0 && P.store_exposures) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (tid == 0 && abort_flag) result[kResErr] = 1.0;
+    if (warp == kMmaWarp)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(kTmemCols) : "memory");
+}
+
+// ---------------------------------------------------------------------------
+// The operand table
+// ---------------------------------------------------------------------------
+namespace {
+
+struct ContractLoadings {
+    double sv[kFactors][kMaxTenor];
+};
+
+// R_jk(m) = (A^m S_k)[j] and its running sum for dates j = 2..B, m up to the
+// last lag any date reads, in FP64: one warp per factor, lane holding tenors
+// lane and lane + 32, neighbours by shuffles (the recursion is serial in m; a
+// warp-wide step needs no barrier).  resp[(k M + m)(B - 1) + j - 2]; scale
+// [date][2]: the power of two 2^(e - 8) that maps the date's largest response
+// into [2^7, 2^8).
+__global__ void __launch_bounds__(32 * kFactors)
+    contract_response_kernel(int nt, double c, int stride, int B, int pc, const __grid_constant__ ContractLoadings S,
+                             double* __restrict__ scale, double2* __restrict__ resp)
+{
+    __shared__ double top_s[kFactors][2][kMaxTenor];
+    const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int L = nt - 1, M = (B - 1) * stride;
+    const double a0 = 1.0 - c + 0.5 * c * c, a1 = c - c * c, a2 = 0.5 * c * c;
+    const int t0 = lane, t1 = lane + 32;
+    double v0 = t0 < nt ? S.sv[k][t0] : 0.0, v1 = t1 < nt ? S.sv[k][t1] : 0.0;
+    double c0 = 0.0, c1 = 0.0, m0[2] = {0.0, 0.0}, m1[2] = {0.0, 0.0};
+    double2* row = resp + (size_t)k * M * (B - 1);
+    for (int m = 0; m < M; ++m, row += B - 1) {
+        c0 += v0;
+        c1 += v1;
+        if (t0 >= 2 && t0 <= B && m < (t0 - 1) * stride) {
+            row[t0 - 2] = make_double2(v0, c0);
+            m0[0] = fmax(m0[0], fabs(v0));
+            m0[1] = fmax(m0[1], fabs(c0));
+        }
+        if (t1 <= B && m < (t1 - 1) * stride) {
+            row[t1 - 2] = make_double2(v1, c1);
+            m1[0] = fmax(m1[0], fabs(v1));
+            m1[1] = fmax(m1[1], fabs(c1));
+        }
+        const double first1 = __shfl_sync(0xffffffffu, v1, 0), second1 = __shfl_sync(0xffffffffu, v1, 1);
+        double u0 = __shfl_down_sync(0xffffffffu, v0, 1), u1 = __shfl_down_sync(0xffffffffu, v1, 1);
+        if (lane == 31) u0 = first1;
+        const double d1 = __shfl_up_sync(0xffffffffu, v1, 1);  // (the last tenor lies in the upper half)
+        if (!pc) {
+            v0 += c * (u0 - v0);
+            v1 += t1 < L ? c * (u1 - v1) : (t1 == L ? c * (v1 - d1) : 0.0);
+        } else {
+            double w0 = __shfl_down_sync(0xffffffffu, v0, 2);
+            const double w1 = __shfl_down_sync(0xffffffffu, v1, 2);
+            if (lane == 30) w0 = first1;
+            if (lane == 31) w0 = second1;
+            v0 = a0 * v0 + a1 * u0 + a2 * w0;
+            if (t1 < L - 1)
+                v1 = a0 * v1 + a1 * u1 + a2 * w1;
+            else if (t1 == L - 1)
+                v1 += c * (u1 - v1);
+            else if (t1 == L)
+                v1 += c * (v1 - d1);
+        }
+    }
+    for (int w = 0; w < 2; ++w) {
+        top_s[k][w][t0] = m0[w];
+        top_s[k][w][t1] = m1[w];
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < 2 * kMaxTenor; i += blockDim.x) {
+        const int j = i >> 1, w = i & 1;
+        const double top = fmax(top_s[0][w][j], fmax(top_s[1][w][j], top_s[2][w][j]));
+        // top <= 2^e, e = exponent + 1 (responses below 1e-280 count as zero)
+        scale[i] = (top > 1e-280 && top < 1e300) ? scalbn(1.0, ilogb(top) + 1 - kTopBits) : 1.0;
+    }
+}
+
+// The image of one window: per chunk three k-tiles of 16 rows of the
+// contraction (value 3 i + k of the chunk: step i, factor k), per k-tile two
+// halves of 8, each holding the 4 npad rows n = slice npad + 2 slot + {0 value,
+// 1 sum} as consecutive 16-byte rows.
+__global__ void contract_image_kernel(int stride, int B, ContractWindow W, const double* __restrict__ scale,
+                                      const double2* __restrict__ resp, unsigned char* __restrict__ image)
+{
+    const int M = (B - 1) * stride;
+    const int64_t per_chunk = 48 * (int64_t)W.npad;
+    const int64_t total = per_chunk * W.chunks;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
+        const int chunk = (int)(i / per_chunk), rem = (int)(i % per_chunk);
+        const int kk = rem & 7, col = (rem >> 3) % W.npad, oct = (rem >> 3) / W.npad;  // octet of values: 0..5
+        const int val = 8 * oct + kk, step = chunk * kChunk + val / 3, k = val % 3;
+        const int slot = col >> 1, j = W.hi - slot;
+        double x = 0.0;
+        if (slot < W.slots) {
+            const int lag = (j - 1) * stride - 1 - step;
+            if (lag >= 0) {
+                const double2 r = resp[((size_t)k * M + lag) * (B - 1) + (j - 2)];
+                x = ((col & 1) ? r.y : r.x) / scale[2 * j + (col & 1)];
+            }
+        }
+        unsigned char* out = image + (size_t)chunk * chunk_bytes(W.npad) +
+                             (size_t)(oct >> 1) * (kLevels * W.npad * 32) + (size_t)(oct & 1) * (kLevels * W.npad * 16);
+#pragma unroll
+        for (int s = 0; s < kLevels; ++s) {
+            const double b = s < kLevels - 1 ? rint(x) : x;
+            *reinterpret_cast<__half*>(out + (size_t)(s * W.npad + col) * 16 + 2 * kk) = __float2half_rn((float)b);
+            x = (x - b) * (double)kShift;
+        }
+    }
+}
+
+__global__ void contract_ext_scale_kernel(const double* __restrict__ raw, int64_t n_paths, int64_t per_path,
+                                          double* __restrict__ out)
+{
+    const int lane = threadIdx.x & 31;
+    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+    for (int64_t p = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; p < n_paths; p += warps) {
+        int e = 0;  // exponents of finite values only: a non-finite normal spoils its own path and no other
+        for (int64_t i = lane; i < per_path; i += 32) {
+            const uint32_t x = ((uint32_t)(__double_as_longlong(raw[p * per_path + i]) >> 52)) & 0x7ffu;
+            if (x < 0x7ffu) e = max(e, (int)x - 1023 - 2);
+        }
+        e = __reduce_max_sync(0xffffffffu, e);
+        if (lane == 0) {
+            out[2 * p] = scalbn(1.0, -e);
+            out[2 * p + 1] = scalbn(1.0, e);
+        }
+    }
+}
+
+size_t align_up(size_t x) { return (x + 255) & ~(size_t)255; }
+
+size_t contract_smem(const ContractWindow& W)
+{
+    const size_t need = kBStages * chunk_bytes(W.npad) + sizeof(float4) * (size_t)(W.npad / 2) * kContractTile +
+                        sizeof(double) * (size_t)(W.hi - W.lo + 3) * kContractTile;
+    // more than half an SM's shared memory: one CTA per SM, which takes all of its tensor memory
+    return std::max<size_t>(need, 120 * 1024);
+}
+
+}  // namespace
+
+int contract_windows(int n_blocks, int stride, bool ext, ContractWindow* w)
+{
+    const int most = ext ? kContractExtSlots : kContractMaxSlots;
+    int n = 0;
+    size_t image = align_up(kScaleBytes);
+    for (int hi = n_blocks; hi >= 1;) {
+        const int lo = hi - 1 <= most ? 1 : hi - most + 1;
+        ContractWindow x;
+        x.lo = lo;
+        x.hi = hi;
+        x.slots = std::max(hi - std::max(lo, 2) + 1, 0);
+        x.npad = std::max((2 * x.slots + 15) / 16 * 16, 16);
+        x.chunks = ((hi - 1) * stride + kChunk - 1) / kChunk;
+        x.image = image;
+        image += align_up((size_t)x.chunks * chunk_bytes(x.npad));
+        if (w) w[n] = x;
+        ++n;
+        hi = lo - 1;
+    }
+    return n;
+}
+
+size_t contract_table_bytes(int stride, int n_blocks, bool ext)
+{
+    ContractWindow w[kMaxTenor];
+    const int n = contract_windows(n_blocks, stride, ext, w);
+    const ContractWindow& last = w[n - 1];
+    return last.image + align_up((size_t)last.chunks * chunk_bytes(last.npad)) +
+           sizeof(double2) * (size_t)kFactors * std::max(n_blocks - 1, 1) * stride * std::max(n_blocks - 1, 1);
+}
+
+cudaError_t launch_contract_table(int nt, double c, int stride, int n_blocks, bool pc, bool ext, const double* sv,
+                                  void* table, cudaStream_t s)
+{
+    if (nt < 35 || nt > kMaxTenor || n_blocks < 1 || n_blocks >= nt || stride < 1) return cudaErrorInvalidValue;
+    ContractLoadings S;
+    std::memcpy(S.sv, sv, sizeof(S.sv));
+    ContractWindow w[kMaxTenor];
+    const int n = contract_windows(n_blocks, stride, ext, w);
+    double* scale = (double*)table;
+    double2* resp = (double2*)((unsigned char*)table + w[n - 1].image +
+                               align_up((size_t)w[n - 1].chunks * chunk_bytes(w[n - 1].npad)));
+    contract_response_kernel<<<1, 32 * kFactors, 0, s>>>(nt, c, stride, n_blocks, pc ? 1 : 0, S, scale, resp);
+    for (int i = 0; i < n; ++i) {
+        if (w[i].chunks == 0) continue;
+        const int64_t total = 48 * (int64_t)w[i].npad * w[i].chunks;
+        contract_image_kernel<<<(unsigned)std::min<int64_t>((total + 255) / 256, 1216), 256, 0, s>>>(
+            stride, n_blocks, w[i], scale, resp, (unsigned char*)table + w[i].image);
+    }
+    return cudaGetLastError();
+}
+
+cudaError_t launch_contract_ext_scale(const double* raw, int64_t n_paths, int n_steps, double* out, cudaStream_t s)
+{
+    const int64_t blocks = std::min<int64_t>((n_paths + 7) / 8, 4096);
+    contract_ext_scale_kernel<<<(unsigned)blocks, 256, 0, s>>>(raw, n_paths, (int64_t)n_steps * 3, out);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_path_contract(int nt, const PathParams<double>& P, const void* table, const double* ext,
+                                 const double* ext_scale, double* partials, double* estore, double* carry,
+                                 double* result, int n_sms, cudaStream_t s, int* launches)
+{
+    if (!path_tenor_supported(nt) || P.n_blocks < 1 || P.n_blocks >= nt || P.stride < 1 || (ext && !ext_scale))
+        return cudaErrorInvalidValue;
+    ContractWindow w[kMaxTenor];
+    const int n = contract_windows(P.n_blocks, P.stride, ext != nullptr, w);
+    if (n > 1 && !carry) return cudaErrorInvalidValue;
+    auto kernel = ext ? path_kernel_contract<true> : path_kernel_contract<false>;
+    ContractParams Q;
+    Q.P = P;
+    Q.n_tiles = (P.n_paths + kContractTile - 1) / kContractTile;
+    for (int i = 0; i < n; ++i) {
+        Q.W = w[i];
+        const size_t smem = contract_smem(w[i]);
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+        kernel<<<(unsigned)std::min<int64_t>(Q.n_tiles, n_sms), kThreads, smem, s>>>(
+            Q, (const unsigned char*)table, ext, ext_scale, partials, estore, carry, result);
+        e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+    }
+    if (launches) *launches = n;
+    return cudaSuccess;
+}
+
+}  // namespace hjm

@@ -1,0 +1,56 @@
+// hjm_contract.h -- the FP64 response form as an exact-sliced contraction on
+// the tensor cores (hjm_contract.cu): host interface.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <cstddef>
+#include <cstdint>
+
+#include "hjm_device.cuh"
+
+namespace hjm {
+
+constexpr int kContractTile = 128;      // paths per tile: the rows of one tcgen05 M = 128 accumulator
+constexpr int kContractMaxSlots = 32;   // dates a launch carries besides date 1
+constexpr int kContractExtSlots = 24;   // ... with external normals (five slices of each in tensor memory)
+
+// One launch: the dates [lo, hi], slot r holding date hi - r (dates from
+// max(lo, 2)); npad accumulator columns per slice level (two per slot, padded
+// to 16); chunks of 16 evolved steps; its operand image at `image` bytes into
+// the table.
+struct ContractWindow {
+    int lo, hi, slots, npad, chunks;
+    size_t image;
+};
+
+// The windows of a run of n_blocks dates (latest first), at most
+// kContractMaxSlots (ext: kContractExtSlots) slots each: date 1, before any
+// evolution, needs none.  w may be null; returns their number.
+int contract_windows(int n_blocks, int stride, bool ext, ContractWindow* w);
+
+// Bytes of the operand table of a run: scales, images, and the FP64 responses
+// they are cut from.
+size_t contract_table_bytes(int stride, int n_blocks, bool ext);
+
+// Builds the table on the stream (two launches) from the loadings sv
+// [kFactors][kMaxTenor] (sqrt(dt) sigma_k; the predictor-corrector's
+// N-projected ones): the impulse responses of the Euler or the three-point
+// step, sliced for the contraction.
+cudaError_t launch_contract_table(int nt, double c, int stride, int n_blocks, bool pc, bool ext, const double* sv,
+                                  void* table, cudaStream_t s);
+
+// Row scales of external normals [path][step][3]: out[2 p] = 2^-e, out[2 p +
+// 1] = 2^e with e >= 0 the least that brings every |normal| of path p below 8.
+cudaError_t launch_contract_ext_scale(const double* raw, int64_t n_paths, int n_steps, double* out, cudaStream_t s);
+
+// The valuation: one launch per window (carry [2][n_paths] doubles when there
+// is more than one).  partials: one row of n_blocks + 3 doubles per tile of
+// kContractTile paths.  ext: external normals [step][3][path] with their row
+// scales, or null for the generator.  result[kResErr] is set if a wait in the
+// kernel ran out.
+cudaError_t launch_path_contract(int nt, const PathParams<double>& P, const void* table, const double* ext,
+                                 const double* ext_scale, double* partials, double* estore, double* carry,
+                                 double* result, int n_sms, cudaStream_t s, int* launches);
+
+}  // namespace hjm

@@ -20,6 +20,7 @@ constexpr int kResCVA = 2 * kMaxTenor;
 constexpr int kResCVAStderr = kResCVA + 1;
 constexpr int kResDCVADHazard = kResCVA + 2;
 constexpr int kResCVAPathMean = kResCVA + 3;    // mean of per-path CVA contributions
+constexpr int kResErr = kResCVA + 4;         // nonzero: a wait of the contraction kernel ran out
 constexpr int kResLen = kResCVA + 8;
 
 struct FinalParams {

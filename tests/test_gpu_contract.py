@@ -1,0 +1,100 @@
+"""GPU parity of the FP64 contraction kernel (hjm_contract.cu) at the sizes
+where its tiling can go wrong: path counts around the 128-path tiles and the
+SM count, date counts at the edges of the padded accumulator columns (8 dates
+a step) and of a launch's 32 slots (24 with external normals), strides shorter
+and longer than the 16-step chunks, external normals beyond the slices' range.
+
+Tolerances (as the other FP64 tests'): per-path exposures against the all-FP64
+convected step 1e-13 of the exposure scale up to 24 dates, 5e-13 beyond, where
+the two FP64 orderings themselves differ by 1e-13."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from cva_hjm_cuda_gb300.market import Market, RunConfig, Swap
+
+pytestmark = pytest.mark.gpu
+
+
+def _table_market(nt):
+    mk = Market(n_tenor=nt)
+    return Market(n_tenor=nt, vol=mk.vol * (1.0 + 0.1 * np.cos(np.arange(nt) / 7.0))[None, :])
+
+
+def _both(engine, run):
+    """(valuation, exposures) in the response form and convected."""
+    out = []
+    engine.keep_exposures(True)
+    try:
+        for form in ("response", "convect"):
+            engine.set_remainder_form(form)
+            v = run()
+            assert engine.remainder_form() == form
+            out.append((v, engine.exposures()))
+    finally:
+        engine.keep_exposures(False)
+        engine.set_remainder_form("auto")
+    return out
+
+
+def _close(a, b, dates):
+    scale = np.max(np.abs(b))
+    assert np.max(np.abs(a - b)) <= (1e-13 if dates <= 24 else 5e-13) * scale
+
+
+@pytest.mark.parametrize("n_paths", [1, 127, 128, 129, 152 * 128 + 1])
+def test_path_counts_at_tile_edges(engine, n_paths):
+    engine.set_market(_table_market(51))
+    engine.set_swap(Swap(n_periods=4))
+    cfg = RunConfig(n_paths=n_paths, n_steps=200, seed=5)
+    (v, x), (c, xc) = _both(engine, lambda: engine.run(cfg, "fp64"))
+    _close(x, xc, 4)
+    np.testing.assert_allclose(v.ee[:4], c.ee[:4], rtol=1e-12, atol=1e-13 * np.max(c.ee))
+    assert v.cva == pytest.approx(c.cva, rel=1e-12)
+
+
+@pytest.mark.parametrize("scheme", ["euler", "predictor_corrector"])
+@pytest.mark.parametrize("dates,dt", [(1, 0.01), (2, 0.01), (9, 0.01), (10, 0.02), (25, 0.02), (26, 0.02),
+                                      (33, 0.02), (34, 0.02), (60, 0.02), (20, 0.25), (34, 0.125), (60, 0.1),
+                                      (5, 0.00125)])
+def test_date_counts_and_strides(engine, scheme, dates, dt):
+    engine.set_scheme(scheme)
+    try:
+        engine.set_market(_table_market(61))
+        engine.set_swap(Swap(n_tenor=61, n_periods=dates))
+        cfg = RunConfig(n_paths=200, n_steps=dates * int(round(0.5 / dt)), dt=dt, seed=6)
+        (v, x), (c, xc) = _both(engine, lambda: engine.run(cfg, "fp64"))
+    finally:
+        engine.set_scheme("euler")
+    _close(x, xc, dates)
+    np.testing.assert_allclose(v.pfe, c.pfe, rtol=0, atol=5e-13 * np.max(np.abs(xc)))
+
+
+@pytest.mark.parametrize("dates", [20, 25, 26, 50])
+def test_external_normals_beyond_the_slices(engine, dates):
+    """FP64 normals, some paths scaled to 50 and 1e3 sigma (each path has a
+    scale of its own), one path with a NaN: its exposures are zero and every
+    other path equals the run without it."""
+    engine.set_market(_table_market(51))
+    engine.set_swap(Swap(n_periods=dates))
+    z = np.random.default_rng(dates).standard_normal((140, 25 * dates, 3))
+    z[3] *= 50.0
+    z[135, 30:] *= 1e3
+    run = lambda: engine.run_with_normals(z, 25 * dates, 0.02, "fp64")  # noqa: E731
+    (_, x), (_, xc) = _both(engine, run)
+    for p in range(140):  # the scaled paths on their own scale: their curves round at it
+        scale = np.max(np.abs(xc[:, p])) if p in (3, 135) else np.max(np.abs(np.delete(xc, (3, 135), axis=1)))
+        if np.isfinite(scale) and scale > 0:
+            tol = (1e-13 if dates <= 24 else 5e-13) * (1e3 if p in (3, 135) else 1.0)
+            assert np.max(np.abs(x[:, p] - xc[:, p])) <= tol * scale, p
+    z[17, 40, 1] = np.nan
+    engine.keep_exposures(True)
+    try:
+        run()
+        y = engine.exposures()
+    finally:
+        engine.keep_exposures(False)
+    assert np.all(y[:, 17] == 0.0)
+    keep = np.arange(140) != 17
+    np.testing.assert_array_equal(y[:, keep], x[:, keep])
