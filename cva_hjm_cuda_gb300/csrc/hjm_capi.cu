@@ -822,7 +822,7 @@ static hjm_status ensure_contract_table(hjm_ctx* ctx, const RunShape& sh, double
         HJM_CUDA(ctx, cudaStreamWaitEvent(s, ctx->resp_used, 0));
     HJM_CUDA(ctx, launch_contract_table(nt, c, sh.stride, sh.B, ctx->scheme == HJM_SCHEME_PREDICTOR_CORRECTOR, ext,
                                         sv, ctx->contract.p, s));
-    ctx->stat_launches += 1 + contract_windows(sh.B, sh.stride, ext, nullptr);
+    ctx->stat_launches += 2 + contract_windows(sh.B, sh.stride, ext, nullptr);
     k.nt = nt;
     k.stride = sh.stride;
     k.B = sh.B;

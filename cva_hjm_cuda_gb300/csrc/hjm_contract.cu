@@ -89,7 +89,7 @@ static_assert(kLevels * 2 * kContractMaxSlots <= a_col(false) && kLevels * 2 * k
 // bytes of one chunk of the B image: 3 k-tiles of 16 x (kLevels npad) halves
 __host__ __device__ constexpr size_t chunk_bytes(int npad) { return (size_t)3 * kLevels * npad * 32; }
 
-constexpr size_t kScaleBytes = 2 * kMaxTenor * sizeof(double);
+constexpr size_t kScaleBytes = 2 * kMaxTenor * sizeof(double);  // then as many bytes of maxima
 
 // A wait that runs out after this many cycles, about a second (every wait here
 // is for work in flight, so it would be a fault of the program), ends the
@@ -660,79 +660,138 @@ struct ContractLoadings {
     double sv[kFactors][kMaxTenor];
 };
 
-// R_jk(m) = (A^m S_k)[j] and its running sum for dates j = 2..B, m up to the
-// last lag any date reads, in FP64: one warp per factor, lane holding tenors
-// lane and lane + 32, neighbours by shuffles (the recursion is serial in m; a
-// warp-wide step needs no barrier).  resp[(k M + m)(B - 1) + j - 2]; scale
-// [date][2]: the power of two 2^(e - 8) that maps the date's largest response
-// into [2^7, 2^8).
-__global__ void __launch_bounds__(32 * kFactors)
-    contract_response_kernel(int nt, double c, int stride, int B, int pc, const __grid_constant__ ContractLoadings S,
-                             double* __restrict__ scale, double2* __restrict__ resp)
+// The step as a walk.  One step moves the curve by h[t] <- a0 h[t] + a1 h[t+1]
+// + a2 h[t+2] (Euler: 1 - c, c, 0; the predictor-corrector: 1 - c + c^2/2,
+// c - c^2, c^2/2) up to the last tenors, whose rows use the backward difference
+// d = h[L] - h[L-1].  That slope does not change over a step, so the rows are
+// the same walk on the curve extended beyond L along d, and with D_t the
+// loading's deviation from that line (zero from L - 1 on)
+//     (A^m S)[j] = S_L + (j - L + m c) d + sum_i f_m(i) D_{j+i},
+// f_m(i) the probability that m steps move i tenors.  Every lag is then
+// independent of the others: a few launches of thousands of threads instead of
+// a recursion over the lags, which is serial and bound by the FP64 pipe's
+// latency (2,450 lags of the 25y swap: 1.2 ms by one CTA; 40 us this way).
+struct WalkParams {
+    double a1, a2;          // r = a / a0 of the recurrence: see below
+    double log_hi, log_lo;  // log a0
+    double b1, b2, inv;     // a1 / (a1 + a2), a2 / (a1 + a2), 1 / (a1 + a2)
+    double rcp[kMaxTenor];  // 1 / (i + 1)
+};
+
+// weights[i M + m] = {f_m(i), G_m(i) = sum_{r <= m} f_r(i)}, i < n.  f_m are
+// the coefficients of p^m, p = a0 + a1 z + a2 z^2: from p (p^m)' = m p' p^m,
+//     (i + 1) a0 f(i+1) = (m - i) a1 f(i) + (2 m - i + 1) a2 f(i-1),
+// and G those of (p^{m+1} - 1) / (p - 1): G(i) = ([i = 0] - f_{m+1}(i)) / (a1 +
+// a2) + b1 G(i-1) + b2 G(i-2), weights that sum to one.  One thread per lag.
+__global__ void contract_weights_kernel(const __grid_constant__ WalkParams K, int M, int n, double2* __restrict__ weights)
 {
-    __shared__ double top_s[kFactors][2][kMaxTenor];
-    const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int L = nt - 1, M = (B - 1) * stride;
-    const double a0 = 1.0 - c + 0.5 * c * c, a1 = c - c * c, a2 = 0.5 * c * c;
-    const int t0 = lane, t1 = lane + 32;
-    double v0 = t0 < nt ? S.sv[k][t0] : 0.0, v1 = t1 < nt ? S.sv[k][t1] : 0.0;
-    double c0 = 0.0, c1 = 0.0, m0[2] = {0.0, 0.0}, m1[2] = {0.0, 0.0};
-    double2* row = resp + (size_t)k * M * (B - 1);
-    for (int m = 0; m < M; ++m, row += B - 1) {
-        c0 += v0;
-        c1 += v1;
-        if (t0 >= 2 && t0 <= B && m < (t0 - 1) * stride) {
-            row[t0 - 2] = make_double2(v0, c0);
-            m0[0] = fmax(m0[0], fabs(v0));
-            m0[1] = fmax(m0[1], fabs(c0));
-        }
-        if (t1 <= B && m < (t1 - 1) * stride) {
-            row[t1 - 2] = make_double2(v1, c1);
-            m1[0] = fmax(m1[0], fabs(v1));
-            m1[1] = fmax(m1[1], fabs(c1));
-        }
-        const double first1 = __shfl_sync(0xffffffffu, v1, 0), second1 = __shfl_sync(0xffffffffu, v1, 1);
-        double u0 = __shfl_down_sync(0xffffffffu, v0, 1), u1 = __shfl_down_sync(0xffffffffu, v1, 1);
-        if (lane == 31) u0 = first1;
-        const double d1 = __shfl_up_sync(0xffffffffu, v1, 1);  // (the last tenor lies in the upper half)
-        if (!pc) {
-            v0 += c * (u0 - v0);
-            v1 += t1 < L ? c * (u1 - v1) : (t1 == L ? c * (v1 - d1) : 0.0);
-        } else {
-            double w0 = __shfl_down_sync(0xffffffffu, v0, 2);
-            const double w1 = __shfl_down_sync(0xffffffffu, v1, 2);
-            if (lane == 30) w0 = first1;
-            if (lane == 31) w0 = second1;
-            v0 = a0 * v0 + a1 * u0 + a2 * w0;
-            if (t1 < L - 1)
-                v1 = a0 * v1 + a1 * u1 + a2 * w1;
-            else if (t1 == L - 1)
-                v1 += c * (u1 - v1);
-            else if (t1 == L)
-                v1 += c * (v1 - d1);
-        }
+    const int m = blockIdx.x * blockDim.x + threadIdx.x;
+    if (m >= M) return;
+    auto power = [&](double e) {  // a0^e: the exponent's rounding would cost e log a0 2^-53
+        const double x = e * K.log_hi;
+        return exp(x) * (1.0 + fma(e, K.log_lo, fma(e, K.log_hi, -x)));
+    };
+    const double md = m;
+    double f = power(md), f1 = 0.0, h = power(md + 1.0), h1 = 0.0, g1 = 0.0, g2 = 0.0;
+    for (int i = 0; i < n; ++i) {
+        const double g = fma((i == 0 ? 1.0 : 0.0) - h, K.inv, fma(K.b1, g1, K.b2 * g2));
+        weights[(size_t)i * M + m] = make_double2(f, g);
+        g2 = g1;
+        g1 = g;
+        const double di = i;
+        const double fn = fma((md - di) * K.a1, f, (2.0 * md - di + 1.0) * K.a2 * f1) * K.rcp[i];
+        const double hn = fma((md + 1.0 - di) * K.a1, h, (2.0 * md - di + 3.0) * K.a2 * h1) * K.rcp[i];
+        f1 = f;
+        f = fn;
+        h1 = h;
+        h = hn;
     }
-    for (int w = 0; w < 2; ++w) {
-        top_s[k][w][t0] = m0[w];
-        top_s[k][w][t1] = m1[w];
+}
+
+// R_jk(m) and its running sum for date j = blockIdx.y + 2 at every lag it reads
+// (m < (j - 1) stride): resp[(k (B - 1) + j - 2) M + m], and the largest
+// magnitude over lags and factors in top[2 j + {0 value, 1 sum}] (bits; cleared
+// before).
+__global__ void __launch_bounds__(128)
+    contract_response_kernel(int nt, double c, int stride, int B, const __grid_constant__ ContractLoadings S,
+                             const double2* __restrict__ weights, unsigned long long* __restrict__ top,
+                             double2* __restrict__ resp)
+{
+    __shared__ double dev_s[kFactors][kMaxTenor];
+    __shared__ double top_s[2][4];
+    const int L = nt - 1, M = (B - 1) * stride, j = blockIdx.y + 2, lags = (j - 1) * stride;
+    const int m0 = blockIdx.x * blockDim.x, m = m0 + threadIdx.x;
+    if (m0 >= lags) return;
+    for (int i = threadIdx.x; i < kFactors * nt; i += blockDim.x) {
+        const int k = i / nt, t = i % nt;
+        dev_s[k][t] = t < L - 1 ? S.sv[k][t] - (S.sv[k][L] + (double)(t - L) * (S.sv[k][L] - S.sv[k][L - 1])) : 0.0;
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < 2 * kMaxTenor; i += blockDim.x) {
-        const int j = i >> 1, w = i & 1;
-        const double top = fmax(top_s[0][w][j], fmax(top_s[1][w][j], top_s[2][w][j]));
-        // top <= 2^e, e = exponent + 1 (responses below 1e-280 count as zero)
-        scale[i] = (top > 1e-280 && top < 1e300) ? scalbn(1.0, ilogb(top) + 1 - kTopBits) : 1.0;
+    double best[2] = {0.0, 0.0};
+    if (m < lags) {
+        double v[kFactors], w[kFactors];
+        const double md = m;
+#pragma unroll
+        for (int k = 0; k < kFactors; ++k) {
+            const double d = S.sv[k][L] - S.sv[k][L - 1], at = fma((double)(j - L), d, S.sv[k][L]);
+            v[k] = fma(md * c, d, at);
+            w[k] = (md + 1.0) * fma(0.5 * md * c, d, at);
+        }
+        // the walk of this block's lags ends within ten standard deviations and a
+        // dozen tenors of its mean (1e-22 beyond)
+        const double mean = c * (double)min(m0 + (int)blockDim.x, lags);
+        const int n = min(L - 1 - j, (int)(mean + 10.0 * sqrt(mean)) + 12);
+        for (int i = 0; i < n; ++i) {
+            const double2 p = weights[(size_t)i * M + m];
+#pragma unroll
+            for (int k = 0; k < kFactors; ++k) {
+                const double x = dev_s[k][j + i];
+                v[k] = fma(p.x, x, v[k]);
+                w[k] = fma(p.y, x, w[k]);
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < kFactors; ++k) {
+            resp[((size_t)k * (B - 1) + (j - 2)) * M + m] = make_double2(v[k], w[k]);
+            best[0] = fmax(best[0], fabs(v[k]));
+            best[1] = fmax(best[1], fabs(w[k]));
+        }
     }
+    for (int o = 16; o > 0; o >>= 1) {
+        best[0] = fmax(best[0], __shfl_xor_sync(0xffffffffu, best[0], o));
+        best[1] = fmax(best[1], __shfl_xor_sync(0xffffffffu, best[1], o));
+    }
+    if ((threadIdx.x & 31) == 0) {
+        top_s[0][threadIdx.x >> 5] = best[0];
+        top_s[1][threadIdx.x >> 5] = best[1];
+    }
+    __syncthreads();
+    if (threadIdx.x < 2) {
+        const double* t = top_s[threadIdx.x];
+        const double x = fmax(fmax(t[0], t[1]), fmax(t[2], t[3]));
+        atomicMax(top + 2 * j + threadIdx.x, (unsigned long long)__double_as_longlong(x));
+    }
+}
+
+// The power of two that maps a date's largest response into [2^7, 2^8), as a
+// multiplier back (responses below 1e-280 count as zero)
+__device__ __forceinline__ double contract_scale(unsigned long long top)
+{
+    const double t = __longlong_as_double((long long)top);
+    return (t > 1e-280 && t < 1e300) ? scalbn(1.0, ilogb(t) + 1 - kTopBits) : 1.0;
 }
 
 // The image of one window: per chunk three k-tiles of 16 rows of the
 // contraction (value 3 i + k of the chunk: step i, factor k), per k-tile two
 // halves of 8, each holding the 4 npad rows n = slice npad + 2 slot + {0 value,
 // 1 sum} as consecutive 16-byte rows.
-__global__ void contract_image_kernel(int stride, int B, ContractWindow W, const double* __restrict__ scale,
-                                      const double2* __restrict__ resp, unsigned char* __restrict__ image)
+__global__ void contract_image_kernel(int stride, int B, ContractWindow W, const unsigned long long* __restrict__ top,
+                                      const double2* __restrict__ resp, double* __restrict__ scale,
+                                      unsigned char* __restrict__ image)
 {
     const int M = (B - 1) * stride;
+    if (blockIdx.x == 0)
+        for (int i = threadIdx.x; i < 2 * kMaxTenor; i += blockDim.x) scale[i] = contract_scale(top[i]);
     const int64_t per_chunk = 48 * (int64_t)W.npad;
     const int64_t total = per_chunk * W.chunks;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
@@ -744,8 +803,8 @@ __global__ void contract_image_kernel(int stride, int B, ContractWindow W, const
         if (slot < W.slots) {
             const int lag = (j - 1) * stride - 1 - step;
             if (lag >= 0) {
-                const double2 r = resp[((size_t)k * M + lag) * (B - 1) + (j - 2)];
-                x = ((col & 1) ? r.y : r.x) / scale[2 * j + (col & 1)];
+                const double2 r = resp[((size_t)k * (B - 1) + (j - 2)) * M + lag];
+                x = ((col & 1) ? r.y : r.x) / contract_scale(top[2 * j + (col & 1)]);
             }
         }
         unsigned char* out = image + (size_t)chunk * chunk_bytes(W.npad) +
@@ -794,7 +853,7 @@ int contract_windows(int n_blocks, int stride, bool ext, ContractWindow* w)
 {
     const int most = ext ? kContractExtSlots : kContractMaxSlots;
     int n = 0;
-    size_t image = align_up(kScaleBytes);
+    size_t image = align_up(2 * kScaleBytes);
     for (int hi = n_blocks; hi >= 1;) {
         const int lo = hi - 1 <= most ? 1 : hi - most + 1;
         ContractWindow x;
@@ -817,8 +876,9 @@ size_t contract_table_bytes(int stride, int n_blocks, bool ext)
     ContractWindow w[kMaxTenor];
     const int n = contract_windows(n_blocks, stride, ext, w);
     const ContractWindow& last = w[n - 1];
+    const size_t dates = std::max(n_blocks - 1, 1), lags = dates * stride;
     return last.image + align_up((size_t)last.chunks * chunk_bytes(last.npad)) +
-           sizeof(double2) * (size_t)kFactors * std::max(n_blocks - 1, 1) * stride * std::max(n_blocks - 1, 1);
+           sizeof(double2) * lags * (kFactors * dates + kMaxTenor);
 }
 
 cudaError_t launch_contract_table(int nt, double c, int stride, int n_blocks, bool pc, bool ext, const double* sv,
@@ -829,15 +889,34 @@ cudaError_t launch_contract_table(int nt, double c, int stride, int n_blocks, bo
     std::memcpy(S.sv, sv, sizeof(S.sv));
     ContractWindow w[kMaxTenor];
     const int n = contract_windows(n_blocks, stride, ext, w);
+    if (n_blocks == 1) return cudaSuccess;  // date 1 alone: nothing evolves
     double* scale = (double*)table;
+    unsigned long long* top = (unsigned long long*)((unsigned char*)table + kScaleBytes);
     double2* resp = (double2*)((unsigned char*)table + w[n - 1].image +
                                align_up((size_t)w[n - 1].chunks * chunk_bytes(w[n - 1].npad)));
-    contract_response_kernel<<<1, 32 * kFactors, 0, s>>>(nt, c, stride, n_blocks, pc ? 1 : 0, S, scale, resp);
+    const int M = (n_blocks - 1) * stride;
+    double2* weights = resp + (size_t)M * kFactors * (n_blocks - 1);
+    WalkParams K;
+    const double a0 = pc ? 1.0 - c + 0.5 * c * c : 1.0 - c, a1 = pc ? c - c * c : c, a2 = pc ? 0.5 * c * c : 0.0;
+    const long double cl = c, log_a0 = pc ? log1pl(-cl + 0.5L * cl * cl) : log1pl(-cl);
+    K.log_hi = (double)log_a0;
+    K.log_lo = (double)(log_a0 - (long double)K.log_hi);
+    K.a1 = a1 / a0;
+    K.a2 = a2 / a0;
+    K.b1 = a1 / (a1 + a2);
+    K.b2 = a2 / (a1 + a2);
+    K.inv = 1.0 / (a1 + a2);
+    for (int i = 0; i < kMaxTenor; ++i) K.rcp[i] = 1.0 / (double)(i + 1);
+    cudaError_t e = cudaMemsetAsync(top, 0, kScaleBytes, s);
+    if (e != cudaSuccess) return e;
+    contract_weights_kernel<<<(M + 63) / 64, 64, 0, s>>>(K, M, nt - 3, weights);
+    contract_response_kernel<<<dim3((M + 127) / 128, n_blocks - 1), 128, 0, s>>>(nt, c, stride, n_blocks, S, weights,
+                                                                                 top, resp);
     for (int i = 0; i < n; ++i) {
         if (w[i].chunks == 0) continue;
         const int64_t total = 48 * (int64_t)w[i].npad * w[i].chunks;
         contract_image_kernel<<<(unsigned)std::min<int64_t>((total + 255) / 256, 1216), 256, 0, s>>>(
-            stride, n_blocks, w[i], scale, resp, (unsigned char*)table + w[i].image);
+            stride, n_blocks, w[i], top, resp, scale, (unsigned char*)table + w[i].image);
     }
     return cudaGetLastError();
 }

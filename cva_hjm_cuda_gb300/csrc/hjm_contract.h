@@ -33,7 +33,7 @@ int contract_windows(int n_blocks, int stride, bool ext, ContractWindow* w);
 // they are cut from.
 size_t contract_table_bytes(int stride, int n_blocks, bool ext);
 
-// Builds the table on the stream (two launches) from the loadings sv
+// Builds the table on the stream (two launches and one per window) from the loadings sv
 // [kFactors][kMaxTenor] (sqrt(dt) sigma_k; the predictor-corrector's
 // N-projected ones): the impulse responses of the Euler or the three-point
 // step, sliced for the contraction.
