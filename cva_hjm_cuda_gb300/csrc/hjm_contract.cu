@@ -674,15 +674,16 @@ struct ContractLoadings {
 struct WalkParams {
     double a1, a2;          // r = a / a0 of the recurrence: see below
     double log_hi, log_lo;  // log a0
-    double b1, b2, inv;     // a1 / (a1 + a2), a2 / (a1 + a2), 1 / (a1 + a2)
+    double b2, inv;         // a2 / (a1 + a2), 1 / (a1 + a2)
     double rcp[kMaxTenor];  // 1 / (i + 1)
 };
 
 // weights[i M + m] = {f_m(i), G_m(i) = sum_{r <= m} f_r(i)}, i < n.  f_m are
 // the coefficients of p^m, p = a0 + a1 z + a2 z^2: from p (p^m)' = m p' p^m,
 //     (i + 1) a0 f(i+1) = (m - i) a1 f(i) + (2 m - i + 1) a2 f(i-1),
-// and G those of (p^{m+1} - 1) / (p - 1): G(i) = ([i = 0] - f_{m+1}(i)) / (a1 +
-// a2) + b1 G(i-1) + b2 G(i-2), weights that sum to one.  One thread per lag.
+// and G those of (p^{m+1} - 1) / (p - 1), whose partial sums telescope:
+//     (a1 + a2) G(i) + a2 G(i-1) = 1 - f_{m+1}(0) - .. - f_{m+1}(i),
+// so a rounding fades by a2 / (a1 + a2) a step.  One thread per lag.
 __global__ void contract_weights_kernel(const __grid_constant__ WalkParams K, int M, int n, double2* __restrict__ weights)
 {
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
@@ -692,12 +693,11 @@ __global__ void contract_weights_kernel(const __grid_constant__ WalkParams K, in
         return exp(x) * (1.0 + fma(e, K.log_lo, fma(e, K.log_hi, -x)));
     };
     const double md = m;
-    double f = power(md), f1 = 0.0, h = power(md + 1.0), h1 = 0.0, g1 = 0.0, g2 = 0.0;
+    double f = power(md), f1 = 0.0, h = power(md + 1.0), h1 = 0.0, g = 0.0, tail = 1.0;
     for (int i = 0; i < n; ++i) {
-        const double g = fma((i == 0 ? 1.0 : 0.0) - h, K.inv, fma(K.b1, g1, K.b2 * g2));
+        tail -= h;
+        g = fma(tail, K.inv, -(K.b2 * g));
         weights[(size_t)i * M + m] = make_double2(f, g);
-        g2 = g1;
-        g1 = g;
         const double di = i;
         const double fn = fma((md - di) * K.a1, f, (2.0 * md - di + 1.0) * K.a2 * f1) * K.rcp[i];
         const double hn = fma((md + 1.0 - di) * K.a1, h, (2.0 * md - di + 3.0) * K.a2 * h1) * K.rcp[i];
@@ -903,7 +903,6 @@ cudaError_t launch_contract_table(int nt, double c, int stride, int n_blocks, bo
     K.log_lo = (double)(log_a0 - (long double)K.log_hi);
     K.a1 = a1 / a0;
     K.a2 = a2 / a0;
-    K.b1 = a1 / (a1 + a2);
     K.b2 = a2 / (a1 + a2);
     K.inv = 1.0 / (a1 + a2);
     for (int i = 0; i < kMaxTenor; ++i) K.rcp[i] = 1.0 / (double)(i + 1);
