@@ -959,12 +959,12 @@ static hjm_status enqueue_impl(hjm_ctx* ctx, int64_t n_paths, int32_t n_steps, d
     const size_t esize = mixed ? 4 : 8;
 
     HJM_CUDA(ctx, ctx->partials.ensure(sizeof(double) * (size_t)n_ctas * R));
-    HJM_CUDA(ctx, ctx->sums.ensure(sizeof(double) * kMaxTenor * 4));
+    HJM_CUDA(ctx, ctx->sums.ensure(sizeof(double) * kSumsLen));
     HJM_CUDA(ctx, ctx->result.ensure(sizeof(double) * kResLen));
     if (store) HJM_CUDA(ctx, ctx->estore.ensure(esize * (size_t)n_dates * (size_t)ld));
     if (want_pfe) {
         HJM_CUDA(ctx, ctx->sel.ensure(sizeof(SelState) * kMaxTenor));
-        HJM_CUDA(ctx, ctx->hist.ensure(pfe_scratch_bytes()));
+        HJM_CUDA(ctx, ctx->hist.ensure(pfe_scratch_bytes(n_paths, n_dates, !mixed)));
     }
     cudaStream_t s = ctx->stream;
     ctx->have_result = false;
@@ -973,7 +973,7 @@ static hjm_status enqueue_impl(hjm_ctx* ctx, int64_t n_paths, int32_t n_steps, d
     FinalParams F;
     ctx->ev = ctx->ring[ctx->n_enqueued % hjm_ctx::kRing];
     ctx->n_enqueued++;
-    ctx->stat_launches = 3;  // path kernel, column reduction, finalisation
+    ctx->stat_launches = 2;  // path kernel, column reduction
     ctx->stat_h2d = (mixed ? sizeof(MixedParams) : sizeof(PathParams<double>)) + sizeof(FinalParams);
     ctx->stat_d2h = 0;
     HJM_CUDA(ctx, cudaEventRecord(ctx->ev[0], s));
@@ -1064,18 +1064,17 @@ static hjm_status enqueue_impl(hjm_ctx* ctx, int64_t n_paths, int32_t n_steps, d
         if (resp) HJM_CUDA(ctx, cudaEventRecord(ctx->resp_used, s));
     }
     HJM_CUDA(ctx, cudaEventRecord(ctx->ev[1], s));
-    HJM_CUDA(ctx, launch_reduce((const double*)ctx->partials.p, n_ctas, R, (double*)ctx->sums.p, F,
+    HJM_CUDA(ctx, launch_reduce((const double*)ctx->partials.p, n_ctas, R, (double*)ctx->sums.p, kSumsLen, F,
                                 (double*)ctx->result.p, s));
     HJM_CUDA(ctx, cudaEventRecord(ctx->ev[2], s));
     if (want_pfe) {
         const int64_t k = std::min<int64_t>(std::max<int64_t>((int64_t)std::ceil(pfe_q * (double)n_paths - 1e-7), 1),
                                             n_paths);
+        int launches = 0;
         HJM_CUDA(ctx, launch_pfe(ctx->estore.p, !mixed, ld, n_paths, n_dates, (uint64_t)(k - 1),
-                                 (SelState*)ctx->sel.p, ctx->hist.p, (double*)ctx->result.p, ctx->n_sms,
-                                 s));
-        // init, write, per 11-bit digit a histogram and a scan, and between
-        // digits the compaction and ranking (6 digits of FP64 keys, 3 of FP32)
-        ctx->stat_launches += 2 + (mixed ? 3 * 2 + 2 * 2 : 6 * 2 + 5 * 2);
+                                 (SelState*)ctx->sel.p, ctx->hist.p, (double*)ctx->result.p, ctx->n_sms, s,
+                                 &launches));
+        ctx->stat_launches += launches;
     }
     HJM_CUDA(ctx, cudaEventRecord(ctx->ev[3], s));
     {
@@ -1373,7 +1372,7 @@ hjm_status hjm_run_adjoint(hjm_ctx* ctx, int64_t n_paths, int32_t n_steps, doubl
     const int K = checkpoint_every;
     const int S = K > 0 ? (E + K - 1) / K : 0;
     HJM_CUDA(ctx, ctx->partials.ensure(sizeof(double) * (size_t)n_ctas * R));
-    HJM_CUDA(ctx, ctx->sums.ensure(sizeof(double) * kMaxTenor * 4));
+    HJM_CUDA(ctx, ctx->sums.ensure(sizeof(double) * kSumsLen));
     HJM_CUDA(ctx, ctx->result.ensure(sizeof(double) * kResLen));
     if (K > 0) {
         HJM_CUDA(ctx, ctx->ck_h.ensure(sizeof(float) * (size_t)S * (nt + 5) * (size_t)ld));
@@ -1410,11 +1409,11 @@ hjm_status hjm_run_adjoint(hjm_ctx* ctx, int64_t n_paths, int32_t n_steps, doubl
                                      K > 0 ? (float*)ctx->ck_h.p : nullptr, K > 0 ? (double*)ctx->ck_a.p : nullptr, s));
     }
     HJM_CUDA(ctx, cudaEventRecord(ctx->ev[1], s));
-    HJM_CUDA(ctx, launch_reduce((const double*)ctx->partials.p, n_ctas, R, (double*)ctx->sums.p, F,
+    HJM_CUDA(ctx, launch_reduce((const double*)ctx->partials.p, n_ctas, R, (double*)ctx->sums.p, kSumsLen, F,
                                 (double*)ctx->result.p, s));
     HJM_CUDA(ctx, cudaEventRecord(ctx->ev[2], s));
     HJM_CUDA(ctx, cudaEventRecord(ctx->ev[3], s));
-    ctx->stat_launches = 3;
+    ctx->stat_launches = 2;
     ctx->stat_h2d = (pc ? sizeof(PcParams<float>) : sizeof(AdjParams)) + sizeof(FinalParams);
     std::vector<double> res(kResLen), sums(R);
     HJM_CUDA(ctx, cudaMemcpyAsync(res.data(), ctx->result.p, sizeof(double) * kResLen, cudaMemcpyDeviceToHost, s));
@@ -1598,7 +1597,7 @@ hjm_status hjm_run_mlmc(hjm_ctx* ctx, int32_t n_levels, const int64_t* n_paths, 
         const int R = shf.B + 3;
         const int64_t n_ctas = (n_paths[l] + mlmc_cta() - 1) / mlmc_cta();
         HJM_CUDA(ctx, ctx->partials.ensure(sizeof(double) * (size_t)n_ctas * R));
-        HJM_CUDA(ctx, ctx->sums.ensure(sizeof(double) * kMaxTenor * 4));
+        HJM_CUDA(ctx, ctx->sums.ensure(sizeof(double) * kSumsLen));
         HJM_CUDA(ctx, ctx->result.ensure(sizeof(double) * kResLen));
         MlmcParams Q;
         MlmcPcParams Qp;
@@ -1625,7 +1624,7 @@ hjm_status hjm_run_mlmc(hjm_ctx* ctx, int32_t n_levels, const int64_t* n_paths, 
         else
             HJM_CUDA(ctx, launch_mlmc_level(nt, Q, use_poly_path(ctx), (double*)ctx->partials.p, s));
         HJM_CUDA(ctx, cudaEventRecord(ctx->ev[1], s));
-        HJM_CUDA(ctx, launch_reduce((const double*)ctx->partials.p, n_ctas, R, (double*)ctx->sums.p, F,
+        HJM_CUDA(ctx, launch_reduce((const double*)ctx->partials.p, n_ctas, R, (double*)ctx->sums.p, kSumsLen, F,
                                     (double*)ctx->result.p, s));
         HJM_CUDA(ctx, cudaEventRecord(ctx->ev[2], s));
         HJM_CUDA(ctx, cudaEventRecord(ctx->ev[3], s));

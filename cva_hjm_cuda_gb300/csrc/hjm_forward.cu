@@ -1,4 +1,4 @@
-// hjm_forward.cu -- fused Monte Carlo path kernel, reductions and PFE selection.
+// hjm_forward.cu -- fused Monte Carlo path kernel and reductions.
 //
 // One launch of path_kernel replaces the reference's whole GPU pipeline
 // (simulation_gpu.cu:956-1179): cuRAND normal buffer (:1057-1071), 2,500
@@ -594,11 +594,19 @@ void pack_mixed_params(int nt, const PathParams<float>& P, MixedParams& M)
 
 // ---------------------------------------------------------------------------
 // Deterministic column sums of the CTA partials (Neumaier-compensated FP64):
-// one CTA per column, fixed assignment of rows to threads, fixed tree order.
-// Replaces the cuBLAS gemv with a ones vector (simulation_gpu.cu:889-933) and
-// the host vAdd/saxpy (simulation_gpu.cu:941-951, 1157-1179).
+// blockIdx.x the column, blockIdx.y one of gridDim.y row ranges, fixed
+// assignment of rows to threads, fixed tree order.  Replaces the cuBLAS gemv with
+// a ones vector (simulation_gpu.cu:889-933) and the host vAdd/saxpy
+// (simulation_gpu.cu:941-951, 1157-1179).  The last CTA to finish (a counter in
+// the cleared result block) adds the ranges of each column and forms EE, CVA, its
+// standard error and dCVA/dhazard.  Bound: the FP64 pipe (18 cycles an
+// instruction and SM), so 256 threads a CTA (the tree's additions grow with
+// them: 25 us with 1,024) and up to six row ranges.  40 rows: 21 -> 16 us (two
+// launches before), 8,192 rows 38 -> 22 us, 32,768 rows 88 -> 33 us.
 // ---------------------------------------------------------------------------
 constexpr int kReduceThreads = 256;
+constexpr int kReduceRows = 1024;   // rows a range has at least
+constexpr int kReduceRanges = 6;    // a column's ranges (23 columns of the 10y swap: 138 CTAs)
 
 __device__ __forceinline__ void neumaier_add(double& s, double& comp, double x)
 {
@@ -607,244 +615,86 @@ __device__ __forceinline__ void neumaier_add(double& s, double& comp, double x)
     s = t;
 }
 
-__global__ void __launch_bounds__(kReduceThreads)
-    reduce_columns(const double* __restrict__ partials, int64_t n_rows, int R, double* __restrict__ sums)
+// The compensated sum of the warp's pairs, in every lane, in a fixed order
+__device__ __forceinline__ void neumaier_warp(double& s, double& comp)
 {
-    __shared__ double ss[kReduceThreads], cs[kReduceThreads];
-    const int col = blockIdx.x;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const double x = __shfl_down_sync(0xffffffffu, s, o), c = __shfl_down_sync(0xffffffffu, comp, o);
+        comp += c;
+        neumaier_add(s, comp, x);
+    }
+}
+
+__global__ void __launch_bounds__(kReduceThreads)
+    reduce_columns(const double* __restrict__ partials, int64_t n_rows, int R, double* __restrict__ sums,
+                   const __grid_constant__ FinalParams F, double* __restrict__ result)
+{
+    constexpr int kWarps = kReduceThreads / 32;
+    __shared__ double ss[kWarps], cs[kWarps];
+    __shared__ bool last_s;
+    const int col = blockIdx.x, t = threadIdx.x, lane = t & 31, warp = t >> 5, ranges = gridDim.y;
+    const int64_t per = (n_rows + ranges - 1) / ranges, begin = per * blockIdx.y, end = min(begin + per, n_rows);
     double s = 0.0, comp = 0.0;
-    for (int64_t r = threadIdx.x; r < n_rows; r += kReduceThreads) neumaier_add(s, comp, partials[(size_t)r * R + col]);
-    ss[threadIdx.x] = s;
-    cs[threadIdx.x] = comp;
+    for (int64_t r = begin + t; r < end; r += 4 * kReduceThreads) {
+        double v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int64_t q = r + u * kReduceThreads;
+            v[u] = q < end ? partials[(size_t)q * R + col] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) neumaier_add(s, comp, v[u]);
+    }
+    neumaier_warp(s, comp);
+    if (lane == 0) {
+        ss[warp] = s;
+        cs[warp] = comp;
+    }
     __syncthreads();
-    for (int w = kReduceThreads / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w) {
-            double a = ss[threadIdx.x], ca = cs[threadIdx.x] + cs[threadIdx.x + w];
-            neumaier_add(a, ca, ss[threadIdx.x + w]);
-            ss[threadIdx.x] = a;
-            cs[threadIdx.x] = ca;
+    if (t == 0) {
+        for (int w = 1; w < kWarps; ++w) {
+            comp += cs[w];
+            neumaier_add(s, comp, ss[w]);
+        }
+        sums[(size_t)(ranges > 1 ? blockIdx.y + 1 : 0) * R + col] = s + comp;
+        __threadfence();
+        last_s = atomicAdd(reinterpret_cast<uint32_t*>(result + kResCount), 1u) == gridDim.x * gridDim.y - 1;
+    }
+    __syncthreads();
+    if (!last_s) return;
+    __threadfence();
+    if (ranges > 1) {
+        for (int c = t; c < R; c += kReduceThreads) {
+            double a = 0.0, ca = 0.0;
+            for (int g = 1; g <= ranges; ++g) neumaier_add(a, ca, __ldcg(sums + (size_t)g * R + c));
+            sums[c] = a + ca;
         }
         __syncthreads();
     }
-    if (threadIdx.x == 0) sums[col] = ss[0] + cs[0];
-}
-
-// EE, CVA, its standard error and dCVA/dhazard from the column sums.
-__global__ void finalize_results(const double* __restrict__ sums, FinalParams F, double* __restrict__ result)
-{
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+    if (warp != 0) return;
+    auto sums_at = [&](int c) { return __ldcg(sums + c); };  // (written by this CTA or others)
     const int B = F.n_blocks;
     const double inv_n = 1.0 / (double)F.n_paths;
     double cva = 0.0, dcva = 0.0;
-    for (int j = 0; j < kMaxTenor; ++j) {
-        const double ee = (j <= B) ? sums[j] * inv_n : 0.0;
+#pragma unroll
+    for (int u = 0; u < kMaxTenor / 32; ++u) {
+        const int j = lane + 32 * u;
+        const double ee = (j <= B) ? sums_at(j) * inv_n : 0.0;
         result[kResEE + j] = ee;
-        cva += F.cvaw[j] * ee;
-        dcva += F.dcvaw[j] * ee;
+        cva = fma(F.cvaw[j], ee, cva);
+        dcva = fma(F.dcvaw[j], ee, dcva);
     }
-    const double s1 = sums[B + 1], s2 = sums[B + 2];
-    const double n = (double)F.n_paths;
-    const double var = (n > 1.0) ? fmax((s2 - s1 * s1 / n) / (n - 1.0), 0.0) : 0.0;
-    result[kResCVA] = cva;
-    result[kResCVAStderr] = sqrt(var / n);
-    result[kResDCVADHazard] = dcva;
-    result[kResCVAPathMean] = s1 * inv_n;
-}
-
-// ---------------------------------------------------------------------------
-// PFE: exact k-th smallest exposure of every date column by most-significant-
-// digit radix selection on the IEEE bit patterns (exposures are >= +0, so the
-// unsigned order of the bits is the numeric order).  11-bit digits; each pass
-// histograms the candidates that match the prefix found so far.  Once a
-// date's candidates number at most kPfeCap (two digits in, for a continuous
-// distribution: 1/2048 of an octave), one more pass copies them to a buffer
-// and one CTA ranks them in shared memory; the date's later passes exit at
-// once.  A date whose candidates stay many (ties: e.g. most exposures zero)
-// finishes by the global passes alone.  Three reads of the store instead of
-// eight (FP64) or four (FP32) with 8-bit digits.
-// ---------------------------------------------------------------------------
-constexpr int kPfeDigit = 11;
-constexpr int kPfeBins = 1 << kPfeDigit;
-
-template <typename K>
-__global__ void pfe_hist(const K* __restrict__ keys, int64_t ld, int64_t n, const SelState* __restrict__ st,
-                         uint32_t* __restrict__ hist, int shift, int bits)
-{
-    __shared__ uint32_t h[kPfeBins];
-    const int date = blockIdx.y;
-    if (st[date].stage != 0) return;  // compacted: ranked in shared memory
-    const int nb = 1 << bits;
-    for (int i = threadIdx.x; i < nb; i += blockDim.x) h[i] = 0;
-    __syncthreads();
-    const uint64_t prefix = st[date].prefix, mask = st[date].mask;
-    const K* col = keys + (size_t)date * (size_t)ld;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < n; base += stride) {
-        const int64_t i = base + threadIdx.x;
-        bool take = false;
-        uint32_t digit = 0;
-        if (i < n) {
-            const uint64_t k = (uint64_t)col[i];
-            take = (k & mask) == prefix;
-            digit = (uint32_t)(k >> shift) & (uint32_t)(nb - 1);
-        }
-        // warp-aggregated increments: one atomic per distinct digit per warp
-        const uint32_t active = __ballot_sync(0xffffffffu, take);
-        if (take) {
-            const uint32_t peers = __match_any_sync(active, digit);
-            if ((threadIdx.x & 31) == (__ffs(peers) - 1)) atomicAdd(&h[digit], (uint32_t)__popc(peers));
-        }
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < nb; i += blockDim.x)
-        if (h[i]) atomicAdd(&hist[(size_t)date * kPfeBins + i], h[i]);
-}
-
-// One CTA per date (256 threads): the digit whose cumulative count passes k,
-// by a block-wide prefix sum over the bins (8 per thread); the histogram is
-// cleared for the next pass.  A date left with at most kPfeCap candidates is
-// marked for compaction (stage 1).
-__global__ void __launch_bounds__(256) pfe_scan(SelState* __restrict__ st, uint32_t* __restrict__ hist, int shift,
-                                                int bits)
-{
-    __shared__ uint32_t wsum[8];
-    __shared__ int found;
-    const int date = blockIdx.x;
-    if (st[date].stage != 0) return;
-    const int nb = 1 << bits;
-    const int per = (nb + 255) / 256;  // bins per thread (8 at 11 bits)
-    uint32_t* hd = hist + (size_t)date * kPfeBins;
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    uint32_t mine = 0;
-    for (int b = 0; b < per; ++b) {
-        const int bin = t * per + b;
-        if (bin < nb) mine += hd[bin];
-    }
-    // exclusive prefix of the threads' sums
-    uint32_t incl = mine;
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += v;
-    }
-    if (lane == 31) wsum[warp] = incl;
-    if (t == 0) found = 0;
-    __syncthreads();
-    uint32_t before = incl - mine;
-    for (int w = 0; w < warp; ++w) before += wsum[w];
-    const uint64_t k = st[date].k;
-    if ((uint64_t)before <= k && k < (uint64_t)before + mine) {
-        uint64_t r = k - before;
-        int d = t * per;
-        for (;; ++d) {
-            const uint32_t c = hd[d];
-            if (r < c) break;
-            r -= c;
-        }
-        const uint32_t cnt = hd[d];
-        st[date].prefix |= (uint64_t)d << shift;
-        st[date].mask |= (uint64_t)(nb - 1) << shift;
-        st[date].k = r;
-        st[date].count = cnt;
-        if (cnt <= (uint32_t)kPfeCap && shift > 0) st[date].stage = 1;
-        found = 1;
-    }
-    __syncthreads();
-    for (int b = 0; b < per; ++b) {
-        const int bin = t * per + b;
-        if (bin < nb) hd[bin] = 0;
-    }
-}
-
-// Copies the candidates of the dates marked for compaction (stage 1) to their
-// buffers, warp-aggregated appends.
-template <typename K>
-__global__ void pfe_compact(const K* __restrict__ keys, int64_t ld, int64_t n, const SelState* __restrict__ st,
-                            uint64_t* __restrict__ buf, uint32_t* __restrict__ cnt)
-{
-    const int date = blockIdx.y;
-    if (st[date].stage != 1) return;
-    const uint64_t prefix = st[date].prefix, mask = st[date].mask;
-    const K* col = keys + (size_t)date * (size_t)ld;
-    uint64_t* out = buf + (size_t)date * kPfeCap;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    const int lane = threadIdx.x & 31;
-    for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < n; base += stride) {
-        const int64_t i = base + threadIdx.x;
-        uint64_t k = 0;
-        bool take = false;
-        if (i < n) {
-            k = (uint64_t)col[i];
-            take = (k & mask) == prefix;
-        }
-        const uint32_t ballot = __ballot_sync(0xffffffffu, take);
-        if (ballot) {
-            uint32_t at = 0;
-            if (lane == __ffs(ballot) - 1) at = atomicAdd(&cnt[date], (uint32_t)__popc(ballot));
-            at = __shfl_sync(0xffffffffu, at, __ffs(ballot) - 1);
-            if (take) {
-                const uint32_t pos = at + __popc(ballot & ((1u << lane) - 1u));
-                if (pos < (uint32_t)kPfeCap) out[pos] = k;  // (the scan counted them: at most kPfeCap)
-            }
-        }
-    }
-}
-
-// One CTA per compacted date: the candidate of rank k (ties by buffer
-// position, so exactly one has it) becomes the date's key; stage 2.
-__global__ void __launch_bounds__(256) pfe_finish(SelState* __restrict__ st, const uint64_t* __restrict__ buf,
-                                                  uint32_t* __restrict__ cnt)
-{
-    __shared__ uint64_t c_s[kPfeCap];
-    const int date = blockIdx.x;
-    if (st[date].stage != 1) return;
-    const uint32_t m = min(cnt[date], (uint32_t)kPfeCap);
-    for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) c_s[i] = buf[(size_t)date * kPfeCap + i];
-    __syncthreads();
-    const uint64_t k = st[date].k;
-    for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) {
-        const uint64_t v = c_s[i];
-        uint32_t rank = 0;
-        for (uint32_t j = 0; j < m; ++j) {
-            const uint64_t w = c_s[j];
-            rank += (w < v) || (w == v && j < i);
-        }
-        if (rank == k) st[date].prefix = v;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        st[date].mask = ~0ull;
-        st[date].k = 0;
-        st[date].stage = 2;
-        cnt[date] = 0;
-    }
-}
-
-template <typename K>
-__global__ void pfe_write(const SelState* __restrict__ st, int n_dates, double* __restrict__ result)
-{
-    const int j = threadIdx.x;
-    if (j < kMaxTenor) {
-        double v = 0.0;
-        if (j < n_dates) {
-            if (sizeof(K) == 8) {
-                v = __longlong_as_double((long long)st[j].prefix);
-            } else {
-                v = (double)__uint_as_float((uint32_t)st[j].prefix);
-            }
-        }
-        result[kResPFE + j] = v;
-    }
-}
-
-__global__ void pfe_init(SelState* __restrict__ st, int n_dates, uint64_t k0)
-{
-    const int j = threadIdx.x;
-    if (j < n_dates) {
-        st[j].prefix = 0;
-        st[j].mask = 0;
-        st[j].k = k0;
-        st[j].count = 0;
-        st[j].stage = 0;
+    cva = warp_sum(cva);
+    dcva = warp_sum(dcva);
+    if (lane == 0) {
+        const double s1 = sums_at(B + 1), s2 = sums_at(B + 2);
+        const double n = (double)F.n_paths;
+        const double var = (n > 1.0) ? fmax((s2 - s1 * s1 / n) / (n - 1.0), 0.0) : 0.0;
+        result[kResCVA] = cva;
+        result[kResCVAStderr] = sqrt(var / n);
+        result[kResDCVADHazard] = dcva;
+        result[kResCVAPathMean] = s1 * inv_n;
     }
 }
 
@@ -1071,54 +921,12 @@ int path_cta(bool mixed, int nt, int n_blocks, bool poly)
     return mixed ? mixed_cta(nt, n_blocks, poly) : kFp64Cta;
 }
 
-cudaError_t launch_reduce(const double* partials, int64_t n_rows, int R, double* sums, const FinalParams& F,
-                          double* result, cudaStream_t s)
+cudaError_t launch_reduce(const double* partials, int64_t n_rows, int R, double* sums, int64_t sums_len,
+                          const FinalParams& F, double* result, cudaStream_t s)
 {
-    reduce_columns<<<R, kReduceThreads, 0, s>>>(partials, n_rows, R, sums);
-    finalize_results<<<1, 32, 0, s>>>(sums, F, result);
-    return cudaGetLastError();
-}
-
-size_t pfe_scratch_bytes()
-{
-    return sizeof(uint32_t) * ((size_t)kPfeBins * kMaxTenor + kMaxTenor) + sizeof(uint64_t) * (size_t)kPfeCap * kMaxTenor;
-}
-
-cudaError_t launch_pfe(const void* estore, bool fp64_keys, int64_t ld, int64_t n_paths, int n_dates, uint64_t k0,
-                       SelState* st, void* scratch, double* result, int n_sms, cudaStream_t s)
-{
-    uint32_t* hist = (uint32_t*)scratch;
-    uint32_t* cnt = hist + (size_t)kPfeBins * kMaxTenor;
-    uint64_t* buf = (uint64_t*)(cnt + kMaxTenor);  // 8-byte aligned: kPfeBins * kMaxTenor + kMaxTenor is even
-    pfe_init<<<1, kMaxTenor, 0, s>>>(st, n_dates, k0);
-    cudaError_t e = cudaMemsetAsync(scratch, 0, sizeof(uint32_t) * ((size_t)kPfeBins * kMaxTenor + kMaxTenor), s);
-    if (e != cudaSuccess) return e;
-    int64_t gx = (n_paths + 1023) / 1024;
-    const int64_t cap = (int64_t)n_sms * 8;
-    if (gx > cap) gx = cap;
-    if (gx < 1) gx = 1;
-    const dim3 grid((unsigned)gx, (unsigned)n_dates);
-    const int total = fp64_keys ? 64 : 32;
-    for (int top = total; top > 0; top -= kPfeDigit) {
-        const int bits = top < kPfeDigit ? top : kPfeDigit;
-        const int shift = top - bits;
-        if (fp64_keys) {
-            pfe_hist<uint64_t><<<grid, 256, 0, s>>>((const uint64_t*)estore, ld, n_paths, st, hist, shift, bits);
-        } else {
-            pfe_hist<uint32_t><<<grid, 256, 0, s>>>((const uint32_t*)estore, ld, n_paths, st, hist, shift, bits);
-        }
-        pfe_scan<<<n_dates, 256, 0, s>>>(st, hist, shift, bits);
-        if (shift == 0) break;
-        if (fp64_keys)
-            pfe_compact<uint64_t><<<grid, 256, 0, s>>>((const uint64_t*)estore, ld, n_paths, st, buf, cnt);
-        else
-            pfe_compact<uint32_t><<<grid, 256, 0, s>>>((const uint32_t*)estore, ld, n_paths, st, buf, cnt);
-        pfe_finish<<<n_dates, 256, 0, s>>>(st, buf, cnt);
-    }
-    if (fp64_keys)
-        pfe_write<uint64_t><<<1, kMaxTenor, 0, s>>>(st, n_dates, result);
-    else
-        pfe_write<uint32_t><<<1, kMaxTenor, 0, s>>>(st, n_dates, result);
+    if (sums_len < R) return cudaErrorInvalidValue;
+    const int64_t ranges = std::max<int64_t>(1, std::min(std::min(n_rows / kReduceRows, (int64_t)kReduceRanges), sums_len / R - 1));
+    reduce_columns<<<dim3((unsigned)R, (unsigned)ranges), kReduceThreads, 0, s>>>(partials, n_rows, R, sums, F, result);
     return cudaGetLastError();
 }
 

@@ -21,6 +21,7 @@ constexpr int kResCVAStderr = kResCVA + 1;
 constexpr int kResDCVADHazard = kResCVA + 2;
 constexpr int kResCVAPathMean = kResCVA + 3;    // mean of per-path CVA contributions
 constexpr int kResErr = kResCVA + 4;         // nonzero: a wait of the contraction kernel ran out
+constexpr int kResCount = kResCVA + 5;       // columns reduced (uint32; cleared with the block)
 constexpr int kResLen = kResCVA + 8;
 
 struct FinalParams {
@@ -30,13 +31,12 @@ struct FinalParams {
     int n_blocks;
 };
 
+// PFE selection state of a date: its bracket (keys; -1 and the largest integer
+// when open) and the counts of keys at its ends, strictly inside and above
 struct SelState {
-    uint64_t prefix, mask, k;
-    uint32_t count;  // candidates matching the prefix after the last pass
-    uint32_t stage;  // 0: global passes; 1: to compact and rank; 2: done
+    int64_t lo, hi;
+    unsigned long long at_lo, inside, at_hi, above;
 };
-// Candidates of a date ranked in shared memory by the PFE selection.
-constexpr int kPfeCap = 2048;
 
 // Mixed-precision path kernel parameters: the FP32 parameter block plus the
 // volatility coefficients packed in tenor pairs {tenor p, tenor p + ceil(NT/2)}
@@ -110,13 +110,17 @@ size_t path_smem(int nt, int n_blocks, bool mixed);
 // FP64 64; mixed 128, or 64 with the compact sums (polynomial factors, many dates)
 int path_cta(bool mixed, int nt, int n_blocks, bool poly);
 
-cudaError_t launch_reduce(const double* partials, int64_t n_rows, int R, double* sums, const FinalParams& F,
-                          double* result, cudaStream_t s);
-// scratch: pfe_scratch_bytes() of device memory (histograms, counters,
-// candidate buffers).
-size_t pfe_scratch_bytes();
+// Column sums into sums[0 .. R) and the results (result cleared before on the
+// stream); sums_len doubles, more than R of them for row ranges of their own
+constexpr int64_t kSumsLen = 2048;
+cudaError_t launch_reduce(const double* partials, int64_t n_rows, int R, double* sums, int64_t sums_len,
+                          const FinalParams& F, double* result, cudaStream_t s);
+// The PFE selection (hjm_pfe.cu): result[kResPFE + date] = the key of rank k0 of
+// each date's column.  scratch: pfe_scratch_bytes() of device memory; *launches:
+// kernels enqueued.
+size_t pfe_scratch_bytes(int64_t n_paths, int n_dates, bool fp64_keys);
 cudaError_t launch_pfe(const void* estore, bool fp64_keys, int64_t ld, int64_t n_paths, int n_dates, uint64_t k0,
-                       SelState* st, void* scratch, double* result, int n_sms, cudaStream_t s);
+                       SelState* st, void* scratch, double* result, int n_sms, cudaStream_t s, int* launches);
 cudaError_t launch_dump_normals(int64_t n_paths, uint64_t path_offset, int n_steps, uint32_t k0, uint32_t k1,
                                 double* out, cudaStream_t s);
 cudaError_t launch_philox_words(int64_t n_paths, uint64_t path_offset, uint32_t step, uint32_t k0, uint32_t k1,
