@@ -24,8 +24,8 @@
 // deviations from the 2^24 up to which the accumulators add exactly; level 2's
 // rounding lies 2^-40 below the curve and is met once in 10^5, levels 3 and 4's
 // lies 2^-54 below.  Products of level 5 and above are dropped (2^-48).  After
-// 12 chunks the five accumulators are added, level by level, into double-FP32
-// running sums (Knuth's two-sum) and restart from zero.  Per-path exposures
+// 12 chunks the five accumulators become one 64-bit integer, added to the date's
+// running sum, and restart from zero.  Per-path exposures
 // then lie 1e-14 of their scale from the oracle (the convected all-FP64 step:
 // 5e-15; double-FP32 response sums on the FP32 pipe: 5e-14); with three slices
 // fewer bits (grids 2^-12 apart, four levels) it was 6e-13.
@@ -35,8 +35,8 @@
 //                paths 32 (w % 4) + lane and half the steps of every second chunk
 //                and stores the slices to the A operand in tensor memory
 //                (counter-based draws: 16 warps share 128 paths);
-//   warp 20      one lane: B operand tiles by bulk copy (TMA) into shared
-//                memory, tcgen05.mma, commits;
+//   warp 20      tcgen05.mma and commits, by one elected lane;
+//   warp 21      B operand tiles by bulk copy (TMA) into shared memory;
 //   warps 16-19  thread = path: accumulators to running sums, pricing of the
 //                dates in FP64, exposures, partial sums, exposure rows.
 // Accumulator columns are ordered [level][date slot]: the slices b0..b4 of a
@@ -47,17 +47,17 @@
 // What bounds it: instruction issue in the sixteen normal warps, ~180 issue
 // cycles per 32 path-steps (Philox's 18 wide multiplications take four each,
 // the packed slicing operations two).  The matrix instructions of the 10y
-// swap's 20 dates fill 1,008 of a chunk's ~3,100 cycles.  1,048,576 paths x
-// 1,000 steps, FP64, 10y swap: 5.15 ms against 12.9 ms for the same sums in
-// double-FP32 (a date costs no instructions per step any more); a table of any
-// shape 28.3 -> 5.3 ms; the reference driver's 25y call (its PCA table, 50
-// dates) 130 -> 19.7 ms.
+// swap's 20 dates fill 1,008 of a chunk's ~2,900 cycles.  1,048,576 paths x
+// 1,000 steps, FP64, 10y swap: 4.85 ms against 12.9 ms for the same sums in
+// double-FP32 (a date costs no instructions per step any more); the 25y swap
+// (50 dates) 17.7 ms against 92.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 
 #include "hjm_contract.h"
 #include "hjm_kernels.h"
@@ -73,8 +73,8 @@ constexpr int kSlices = 4;                // of a normal
 constexpr int kLevels = 5;                // of a response, and accumulators
 constexpr int kProducers = 16;           // warps
 constexpr int kEpilogueWarp = 16;        // first of four
-constexpr int kMmaWarp = 20;
-constexpr int kThreads = 32 * 21;
+constexpr int kMmaWarp = 20, kLoadWarp = 21;
+constexpr int kThreads = 32 * 22;
 constexpr int kAStages = 2, kBStages = 3;
 constexpr int kTmemCols = 512;
 // External FP64 normals take a fifth slice (what FP32 does not hold)
@@ -91,10 +91,12 @@ __host__ __device__ constexpr size_t chunk_bytes(int npad) { return (size_t)3 * 
 
 constexpr size_t kScaleBytes = 2 * kMaxTenor * sizeof(double);  // then as many bytes of maxima
 
-// A wait that runs out after this many cycles, about a second (every wait here
-// is for work in flight, so it would be a fault of the program), ends the
-// kernel with result[kResErr] set.
-constexpr long long kWaitCycles = 2000000000;
+// A wait that runs out, after a second or two (every wait here is for work in
+// flight, so it would be a fault of the program), ends the kernel with
+// result[kResErr] set.
+constexpr uint32_t kWaitNs = 1000000;
+constexpr int kWaitTries = 2000;
+constexpr int kSpinTries = 1 << 25;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -106,22 +108,43 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar)
 {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
+// SLEEP: a try sleeps in hardware until the barrier turns, up to kWaitNs (it
+// takes no issue slots, but wakes late); else it returns after the short
+// interval of the hardware's own.
+template <bool SLEEP>
 __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity)
 {
     uint32_t ok;
-    asm volatile(
-        "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
+    if constexpr (SLEEP)
+        asm volatile(
+            "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\nselp.u32 %0, 1, 0, p;\n}"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity), "r"(kWaitNs)
+            : "memory");
+    else
+        asm volatile(
+            "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity)
+            : "memory");
     return ok != 0;
 }
 // false when the wait ran out, here or in another warp (*abort_s)
+template <bool SLEEP>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_s)
 {
-    if (mbar_try(bar, parity)) return true;
-    for (const long long t0 = clock64(); clock64() - t0 < kWaitCycles && !*abort_s;)
-        if (mbar_try(bar, parity)) return true;
+    if (mbar_try<SLEEP>(bar, parity)) return true;
+    if constexpr (SLEEP) {
+        for (int i = 0; i < kWaitTries; ++i) {
+            if (*abort_s) return false;
+            if (mbar_try<true>(bar, parity)) return true;
+        }
+    } else {
+        for (int i = 0; i < kSpinTries; ++i) {
+            if (mbar_try<false>(bar, parity)) return true;
+            if ((i & 63) == 63 && *abort_s) return false;
+        }
+    }
     *abort_s = 1;
     return false;
 }
@@ -181,19 +204,20 @@ __device__ __forceinline__ void tmem_ld8(uint32_t addr, float* r)
     for (int i = 0; i < 8; ++i) r[i] = __uint_as_float(u[i]);
 }
 
-constexpr float kGrid = 98304.0f;      // 1.5 2^16: adding it rounds to multiples of 2^-7
+constexpr float kGrid = 12582912.0f;   // 1.5 2^23: adding it rounds to integers
+constexpr float kUnit = 128.0f;        // the first slice counts units of 2^-7
 constexpr float kShift = 1024.0f;      // 2^10 between slices
 constexpr int kTopBits = 8;            // the largest response of a date is scaled to at most 2^8
 
-// The four slices of two normals, negated (the epilogue's scale carries the
-// sign back): -a_s from the constant minus the rounded sum, so that no
-// instruction negates.  Packed FP32 pairs throughout; every step is exact
-// until the last conversion.
+// The four slices of two normals, negated (pricing carries the sign back): -a_s
+// from the constant minus the rounded sum, so that no instruction negates.
+// Packed FP32 pairs throughout; every step is exact until the last conversion.
 __device__ __forceinline__ void slice_pair(float2 v, uint32_t (&out)[kSlices])
 {
-    const float2 g = make_float2(kGrid, kGrid), m1 = make_float2(-1.0f, -1.0f), sh = make_float2(kShift, kShift);
-    float2 na = __ffma2_rn(__fadd2_rn(v, g), m1, g);
-    float2 d = __fadd2_rn(v, na);
+    const float2 g = make_float2(kGrid, kGrid), m1 = make_float2(-1.0f, -1.0f), sh = make_float2(kShift, kShift),
+                 un = make_float2(kUnit, kUnit);
+    float2 na = __ffma2_rn(__ffma2_rn(v, un, g), m1, g);
+    float2 d = __ffma2_rn(v, un, na);
 #pragma unroll
     for (int s = 0; s < kSlices - 1; ++s) {
         const __half2 h = __floats2half2_rn(na.x, na.y);
@@ -211,15 +235,12 @@ __device__ __forceinline__ void slice_pair(float2 v, uint32_t (&out)[kSlices])
 // the fourth leaves; values that FP32 holds give the slices above
 __device__ __forceinline__ void slice_pair(double x, double y, uint32_t (&out)[kSlices + 1])
 {
-    const double g = 52776558133248.0;  // 1.5 2^45: rounds to multiples of 2^-7
     const bool fx = (double)(float)x == x, fy = (double)(float)y == y;
+    x *= (double)kUnit;
+    y *= (double)kUnit;
 #pragma unroll
     for (int s = 0; s <= kSlices; ++s) {
-        double ax = x, ay = y;
-        if (s < kSlices - 1) {
-            ax = __dsub_rn(__dadd_rn(x, g), g);
-            ay = __dsub_rn(__dadd_rn(y, g), g);
-        }
+        const double ax = s < kSlices - 1 ? rint(x) : x, ay = s < kSlices - 1 ? rint(y) : y;
         __half2 h = __floats2half2_rn(-(float)ax, -(float)ay);
         if (s == kSlices) h = __halves2half2(fx ? __half(0.0f) : __low2half(h), fy ? __half(0.0f) : __high2half(h));
         out[s] = *reinterpret_cast<const uint32_t*>(&h);
@@ -264,17 +285,21 @@ __device__ __forceinline__ uint4 draw_words(const PathDraw& d, uint32_t step, co
 
 __device__ __forceinline__ float2 f2(float x, float y) { return make_float2(x, y); }
 
-// a - b as one packed FMA (a negated operand would take instructions of its own)
-__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, f2(-1.0f, -1.0f), a); }
-
-// {H, L} += a exactly up to 2^-48 of H: Knuth's two-sum into the high part
-__device__ __forceinline__ void pair_add(float2& H, float2& L, float2 a)
+// A group's five level sums (integers in FP32; the last two together rounded to
+// one) as one, in units of 2^-30: with the normals' 2^-7, 2^-37 of the response's
+constexpr double kSumUnit = 0x1p-37;
+__device__ __forceinline__ long long level_sum(float l0, float l1, float l2, float l3, float l4)
 {
-    const float2 s = __fadd2_rn(H, a);
-    const float2 bp = sub2(s, H);
-    const float2 ap = sub2(s, bp);
-    L = __fadd2_rn(L, __fadd2_rn(sub2(H, ap), sub2(a, bp)));
-    H = s;
+    return ((long long)__float2int_rn(l0) << 30) + ((long long)__float2int_rn(l1) << 20) +
+           ((long long)__float2int_rn(l2) << 10) + (long long)__float2int_rn(fmaf(l4, 0x1p-10f, l3));
+}
+// ... as FP64: each half in the significand of a power of two (the conversion
+// instruction is slow)
+__device__ __forceinline__ double sum_value(long long v)
+{
+    const double hi = __hiloint2double(0x45300000, (int)((uint32_t)(v >> 32) ^ 0x80000000u));  // 2^84 + 2^63 + hi 2^32
+    const double lo = __hiloint2double(0x43300000, (int)(uint32_t)v);                           // 2^52 + lo
+    return (hi - 0x1.00000801p+84) + lo;
 }
 
 __device__ __forceinline__ void epilogue_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
@@ -301,7 +326,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ __align__(8) uint64_t bars[2 * kAStages + 2 * kBStages + 3];
     __shared__ uint32_t tmem_s;
-    __shared__ int abort_flag;
+    __shared__ int abort_flag, stop_flag;
     __shared__ double red_s[8];
     volatile int* abort_s = &abort_flag;
 
@@ -309,7 +334,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int lo = W.lo, hi = W.hi, npad = W.npad, NC = W.chunks;
     const size_t cb = chunk_bytes(npad);
     unsigned char* b_s = smem;                                                       // [kBStages][cb]
-    float4* run_s = reinterpret_cast<float4*>(smem + kBStages * cb);                  // [npad / 2][128] {H x, H sum, L x, L sum}
+    longlong2* run_s = reinterpret_cast<longlong2*>(smem + kBStages * cb);            // [npad / 2][128] {value, sum}
     double* cf_s = reinterpret_cast<double*>(run_s + (size_t)(npad / 2) * kContractTile);  // [hi - lo + 3][128]
 
     const uint32_t a_full = smem_u32(bars), a_empty = a_full + 8 * kAStages, b_full = a_empty + 8 * kAStages,
@@ -397,7 +422,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                         }
                     }
                     if (half == 0) {
-                        ok = mbar_wait(a_empty + 8 * st, ph, abort_s);
+                        ok = mbar_wait<true>(a_empty + 8 * st, ph, abort_s);
                         ok = __all_sync(0xffffffffu, ok);
                         if (!ok) break;
                         tc_fence_after();
@@ -417,31 +442,11 @@ __global__ void __launch_bounds__(kThreads, 1)
             }
         }
     } else if (warp == kMmaWarp) {
-        // ---- B tiles and the matrix instructions: the warp waits as one, one
-        // elected lane issues
+        // ---- the matrix instructions: the warp waits as one, one elected lane issues
         const bool leader = elect_one();
         const uint32_t bs = smem_u32(b_s);
         const int64_t tiles = blockIdx.x < Q.n_tiles ? (Q.n_tiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
         const int64_t total = tiles * NC;
-        const unsigned char* image = table + W.image;
-        int64_t loaded = 0;
-        int load_c = 0, load_s = 0;  // the next load's chunk and stage
-        auto load = [&] {
-            const uint32_t bar = b_full + 8 * load_s;
-            if (leader) {
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"((uint32_t)cb)
-                             : "memory");
-                asm volatile(
-                    "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                        bs + (uint32_t)(load_s * cb)),
-                    "l"(image + (size_t)load_c * cb), "r"((uint32_t)cb), "r"(bar)
-                    : "memory");
-            }
-            ++loaded;
-            if (++load_c == NC) load_c = 0;
-            if (++load_s == kBStages) load_s = 0;
-        };
-        while (loaded < total && loaded < kBStages) load();
         bool ok = true;
         // a_s times the response slices b_0 .. b_{levels - 1 - s} gives the
         // levels s .. 4; beyond 256 columns b_4 takes an instruction of its own
@@ -452,15 +457,22 @@ __global__ void __launch_bounds__(kThreads, 1)
         const uint32_t idesc1 = tc_idesc(npad);
         const uint64_t desc0 = tc_smem_desc(bs, kLevels * npad * 16);
         const uint32_t kt_step = (uint32_t)(kLevels * npad * 32) >> 4, stage_step = (uint32_t)cb >> 4;
-        int c = 0, st = 0, sb = 0, fl = 0;          // chunk of the tile, A and B stages, chunk of the group
-        uint32_t a_ph = 0, b_ph = 0, d_ph = 1;      // parities
-        for (int64_t g = 0; g < total; ++g) {
+        // The loop is unrolled over the six combinations of an A and a B stage, so
+        // that their addresses and parities are constants or warp-uniform: the
+        // issuing warp shares one scheduler with four normal warps, which its
+        // instructions delay (and the barriers the other schedulers with them).
+        int c = 0, fl = 0;      // chunk of the tile, of the accumulator group
+        uint32_t ph = 0, d_ph = 1;
+        int64_t g = 0;
+        auto chunk = [&](auto iv) {
+            constexpr int i = decltype(iv)::value, st = i % kAStages, sb = i % kBStages;
             const bool first = fl == 0;
             const bool last = fl == kFlush - 1 || c == NC - 1;
-            ok = mbar_wait(a_full + 8 * st, a_ph, abort_s) && mbar_wait(b_full + 8 * sb, b_ph, abort_s) &&
-                 (!first || mbar_wait(d_empty, d_ph, abort_s));
+            ok = mbar_wait<false>(a_full + 8 * st, ph ^ (uint32_t)(i / kAStages & 1), abort_s) &&
+                 mbar_wait<false>(b_full + 8 * sb, (uint32_t)(i / kBStages & 1), abort_s) &&
+                 (!first || mbar_wait<false>(d_empty, d_ph, abort_s));
             ok = __all_sync(0xffffffffu, ok);
-            if (!ok) break;
+            if (!ok) return;
             tc_fence_after();
             if (leader) {
                 const uint64_t bd0 = desc0 + (uint64_t)(sb * stage_step);
@@ -480,49 +492,71 @@ __global__ void __launch_bounds__(kThreads, 1)
                 tc_commit(b_empty + 8 * sb);
                 if (last) tc_commit(d_full);
             }
-            // refill the stage of the chunk before (its instructions precede this chunk's)
-            if (g >= 1 && loaded < total) {
-                // that is stage load_s, in the phase before this chunk's if its ring wrapped
-                ok = mbar_wait(b_empty + 8 * load_s, sb == 0 ? b_ph ^ 1u : b_ph, abort_s);
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) break;
-                load();
-            }
             if (first) d_ph ^= 1u;
+            ++g;
             if (++fl == kFlush || c == NC - 1) fl = 0;
             if (++c == NC) c = 0;
-            if (++st == kAStages) {
-                st = 0;
-                a_ph ^= 1u;
-            }
-            if (++sb == kBStages) {
-                sb = 0;
-                b_ph ^= 1u;
+        };
+        static_assert(kAStages == 2 && kBStages == 3, "the unrolled period is six chunks");
+        while (ok && g < total) {
+            chunk(std::integral_constant<int, 0>{});
+            if (ok && g < total) chunk(std::integral_constant<int, 1>{});
+            if (ok && g < total) chunk(std::integral_constant<int, 2>{});
+            if (ok && g < total) chunk(std::integral_constant<int, 3>{});
+            if (ok && g < total) chunk(std::integral_constant<int, 4>{});
+            if (ok && g < total) chunk(std::integral_constant<int, 5>{});
+            ph ^= 1u;
+        }
+        if (!ok) {  // matrix instructions in flight end before the CTA does
+            if (leader) tc_commit(drain);
+            for (int i = 0; i < kWaitTries && !mbar_try<true>(drain, 0); ++i) {
             }
         }
-        if (!ok) {  // copies and matrix instructions in flight end before the CTA does
-            const long long t0 = clock64();
-            if (leader) tc_commit(drain);
-            while (!mbar_try(drain, 0) && clock64() - t0 < kWaitCycles) {
+        __syncwarp();
+    } else if (warp == kLoadWarp) {
+        // ---- B operand tiles by bulk copy
+        if (lane == 0) {
+            const uint32_t bs = smem_u32(b_s);
+            const int64_t tiles = blockIdx.x < Q.n_tiles ? (Q.n_tiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
+            const int64_t total = tiles * NC;
+            const unsigned char* image = table + W.image;
+            int c = 0, st = 0;
+            uint32_t ph = 1;
+            int64_t g = 0;
+            for (; g < total; ++g) {
+                if (!mbar_wait<true>(b_empty + 8 * st, ph, abort_s)) break;
+                const uint32_t bar = b_full + 8 * st;
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"((uint32_t)cb)
+                             : "memory");
+                asm volatile(
+                    "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                        bs + (uint32_t)(st * cb)),
+                    "l"(image + (size_t)c * cb), "r"((uint32_t)cb), "r"(bar)
+                    : "memory");
+                if (++c == NC) c = 0;
+                if (++st == kBStages) {
+                    st = 0;
+                    ph ^= 1u;
+                }
             }
-            for (int64_t i = loaded > kBStages ? loaded - kBStages : 0; i < loaded; ++i)
-                while (!mbar_try(b_full + 8 * (int)(i % kBStages), (uint32_t)((i / kBStages) & 1)) &&
-                       clock64() - t0 < 2 * kWaitCycles) {
+            // copies in flight land before the CTA ends (all have, unless it gave up)
+            for (int64_t i = g > kBStages ? g - kBStages : 0; i < g; ++i)
+                for (int w = 0; w < kWaitTries && !mbar_try<true>(b_full + 8 * (int)(i % kBStages),
+                                                                  (uint32_t)((i / kBStages) & 1)); ++w) {
                 }
         }
         __syncwarp();
     } else {
         // ---- running sums, pricing, exposures: thread = path
-        const int q = warp & 3, p = tid - 32 * kEpilogueWarp;
+        const int q = warp & 3, p = 32 * q + lane;
         const uint32_t d_addr = tmem + ((uint32_t)(32 * q) << 16);
         const double* scale = reinterpret_cast<const double*>(table);  // [date][2]
         const bool top = hi == P.n_blocks, bottom = lo == 1;
         const int B = P.n_blocks, R = B + 3;
-        const int first_date = lo > 2 ? lo : 2;
+        const int first_date = lo > 2 ? lo : 2;  // date 1 precedes any evolution
         double* e_s = cf_s + kContractTile;  // exposure row of date j: j - lo + 1 (the cash-flow row of date j + 1)
         int64_t grp = 0;
-        bool ok = true;
-        for (int64_t tile = blockIdx.x; ok && tile < Q.n_tiles; tile += gridDim.x) {
+        for (int64_t tile = blockIdx.x; tile < Q.n_tiles; tile += gridDim.x) {
             const int64_t base = tile * kContractTile, lp = base + p;
             const bool active = lp < P.n_paths;
             double rs = 1.0;
@@ -530,14 +564,14 @@ __global__ void __launch_bounds__(kThreads, 1)
             auto price = [&](int i) {
                 double x = P.psamp[i], a = P.psum[i];
                 if (i >= 2) {
-                    const float4 r = run_s[(size_t)(hi - i) * kContractTile + p];
+                    const longlong2 r = run_s[(size_t)(hi - i) * kContractTile + p];
                     double sx = __ldg(scale + 2 * i), sa = __ldg(scale + 2 * i + 1);
                     if constexpr (EXT) {
                         sx *= rs;
                         sa *= rs;
                     }
-                    x = fma(-(widen_f32(r.x) + widen_f32(r.z)), sx, x);  // (the slices are negated)
-                    a = fma(-(widen_f32(r.y) + widen_f32(r.w)), sa, a);
+                    x = fma(-sum_value(r.x), sx, x);  // (the slices are negated)
+                    a = fma(-sum_value(r.y), sa, a);
                 }
                 const double D = exp(-a * P.dt);
                 const double Lb = P.m * (exp(x * P.inv_m) - 1.0);
@@ -546,21 +580,19 @@ __global__ void __launch_bounds__(kThreads, 1)
             if (bottom) price(1);
             int next = first_date;  // the earliest date not priced yet
             for (int c = 0; c < NC; c += kFlush, ++grp) {
-                ok = mbar_wait(d_full, (uint32_t)(grp & 1), abort_s);
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) break;
+                const bool ok = mbar_wait<true>(d_full, (uint32_t)(grp & 1), abort_s);
+                if (!__all_sync(0xffffffffu, ok)) break;
                 tc_fence_after();
                 const int live = hi - next + 1;
-                // four slots at a time, padding included (its columns are zero): the
-                // four two-sum chains interleave
+                // four slots at a time, padding included (its columns are zero)
                 for (int r0 = 0; r0 < live; r0 += 4) {
                     float acc[kLevels][8];
 #pragma unroll
                     for (int s = 0; s < kLevels; ++s) tmem_ld8(d_addr + s * npad + 2 * r0, acc[s]);
-                    float4 cell[4];
+                    longlong2 cell[4];
 #pragma unroll
                     for (int u = 0; u < 4; ++u)
-                        cell[u] = c ? run_s[(size_t)(r0 + u) * kContractTile + p] : make_float4(0.f, 0.f, 0.f, 0.f);
+                        cell[u] = c ? run_s[(size_t)(r0 + u) * kContractTile + p] : make_longlong2(0, 0);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                     if (r0 + 4 >= live) {  // the accumulators are read: the next group may start
                         tc_fence_before();
@@ -569,26 +601,23 @@ __global__ void __launch_bounds__(kThreads, 1)
                     }
 #pragma unroll
                     for (int u = 0; u < 4; ++u) {
-                        float2 H = f2(cell[u].x, cell[u].y), L = f2(cell[u].z, cell[u].w);
-                        pair_add(H, L, f2(acc[0][2 * u], acc[0][2 * u + 1]));
-                        pair_add(H, L, __fmul2_rn(f2(acc[1][2 * u], acc[1][2 * u + 1]), f2(0x1p-10f, 0x1p-10f)));
-                        pair_add(H, L, __fmul2_rn(f2(acc[2][2 * u], acc[2][2 * u + 1]), f2(0x1p-20f, 0x1p-20f)));
-                        L = __ffma2_rn(f2(acc[3][2 * u], acc[3][2 * u + 1]), f2(0x1p-30f, 0x1p-30f), L);
-                        L = __ffma2_rn(f2(acc[4][2 * u], acc[4][2 * u + 1]), f2(0x1p-40f, 0x1p-40f), L);
-                        const float2 sum = __fadd2_rn(H, L);
-                        L = __fadd2_rn(L, sub2(H, sum));
-                        H = sum;
-                        run_s[(size_t)(r0 + u) * kContractTile + p] = make_float4(H.x, H.y, L.x, L.y);
+                        cell[u].x += level_sum(acc[0][2 * u], acc[1][2 * u], acc[2][2 * u], acc[3][2 * u], acc[4][2 * u]);
+                        cell[u].y += level_sum(acc[0][2 * u + 1], acc[1][2 * u + 1], acc[2][2 * u + 1],
+                                               acc[3][2 * u + 1], acc[4][2 * u + 1]);
+                        run_s[(size_t)(r0 + u) * kContractTile + p] = cell[u];
                     }
                 }
                 // the dates whose last step this group held
                 const int done = kChunk * min(c + kFlush, NC);
                 for (; next <= hi && (next - 1) * P.stride <= done; ++next) price(next);
             }
-            if (!ok) break;
-
+            // (a wait that ran out ends all four warps at the same tile)
+            if (p == 0) stop_flag = *abort_s;
+            epilogue_sync();
+            if (stop_flag) break;
             // exposures E_j = max(sum_{i > j} cf_i, 0) of dates lo - 1 .. hi - 1
             // (and E_B = 0 for the latest window), the later dates' cash flows in carry
+            const int j0 = lo - 1, j1 = top ? B : hi - 1;
             double v = 0.0, cva_c = 0.0;
             if (!top && active) {
                 v = carry[lp];
@@ -606,9 +635,15 @@ __global__ void __launch_bounds__(kThreads, 1)
                 carry[lp] = v;
                 carry[P.n_paths + lp] = cva_c;
             }
+            if (bottom) {
+                const double s1 = warp_sum(cva_c), s2 = warp_sum(cva_c * cva_c);
+                if (lane == 0) {
+                    red_s[q] = s1;
+                    red_s[4 + q] = s2;
+                }
+            }
             if (P.store_exposures) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             epilogue_sync();
-            const int j0 = lo - 1, j1 = top ? B : hi - 1;
             for (int j = j0 + q; j <= j1; j += 4) {
                 double sum = 0.0;
 #pragma unroll
@@ -616,12 +651,9 @@ __global__ void __launch_bounds__(kThreads, 1)
                 sum = warp_sum(sum);
                 if (lane == 0) partials[(size_t)tile * R + j] = sum;
             }
-            if (bottom) {
-                const double s1 = warp_sum(cva_c), s2 = warp_sum(cva_c * cva_c);
-                if (lane == 0) {
-                    red_s[q] = s1;
-                    red_s[4 + q] = s2;
-                }
+            if (p == 127 && bottom) {
+                partials[(size_t)tile * R + B + 1] = (red_s[0] + red_s[1]) + (red_s[2] + red_s[3]);
+                partials[(size_t)tile * R + B + 2] = (red_s[4] + red_s[5]) + (red_s[6] + red_s[7]);
             }
             if (p == 0 && P.store_exposures) {
                 const int64_t cnt = (P.n_paths - base < kContractTile) ? (P.n_paths - base) : kContractTile;
@@ -635,11 +667,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 asm volatile("cp.async.bulk.commit_group;" ::: "memory");
                 asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
             }
-            epilogue_sync();
-            if (p == 0 && bottom) {
-                partials[(size_t)tile * R + B + 1] = (red_s[0] + red_s[1]) + (red_s[2] + red_s[3]);
-                partials[(size_t)tile * R + B + 2] = (red_s[4] + red_s[5]) + (red_s[6] + red_s[7]);
-            }
+            epilogue_sync();  // (the rows are read: the next tile may price)
         }
         if (p == 0 && P.store_exposures) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     }
@@ -791,7 +819,8 @@ __global__ void contract_image_kernel(int stride, int B, ContractWindow W, const
 {
     const int M = (B - 1) * stride;
     if (blockIdx.x == 0)
-        for (int i = threadIdx.x; i < 2 * kMaxTenor; i += blockDim.x) scale[i] = contract_scale(top[i]);
+        for (int i = threadIdx.x; i < 2 * kMaxTenor; i += blockDim.x)
+            scale[i] = contract_scale(top[i]) * kSumUnit;
     const int64_t per_chunk = 48 * (int64_t)W.npad;
     const int64_t total = per_chunk * W.chunks;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
@@ -824,15 +853,20 @@ __global__ void contract_ext_scale_kernel(const double* __restrict__ raw, int64_
     const int lane = threadIdx.x & 31;
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
     for (int64_t p = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; p < n_paths; p += warps) {
-        int e = 0;  // exponents of finite values only: a non-finite normal spoils its own path and no other
+        int e = 0;
+        bool finite = true;  // a non-finite normal makes its own path's scale, and so its curve, a NaN
         for (int64_t i = lane; i < per_path; i += 32) {
             const uint32_t x = ((uint32_t)(__double_as_longlong(raw[p * per_path + i]) >> 52)) & 0x7ffu;
-            if (x < 0x7ffu) e = max(e, (int)x - 1023 - 2);
+            if (x < 0x7ffu)
+                e = max(e, (int)x - 1023 - 2);
+            else
+                finite = false;
         }
         e = __reduce_max_sync(0xffffffffu, e);
+        finite = __all_sync(0xffffffffu, finite);
         if (lane == 0) {
             out[2 * p] = scalbn(1.0, -e);
-            out[2 * p + 1] = scalbn(1.0, e);
+            out[2 * p + 1] = finite ? scalbn(1.0, e) : __longlong_as_double(0x7ff8000000000000ll);
         }
     }
 }
@@ -841,7 +875,7 @@ size_t align_up(size_t x) { return (x + 255) & ~(size_t)255; }
 
 size_t contract_smem(const ContractWindow& W)
 {
-    const size_t need = kBStages * chunk_bytes(W.npad) + sizeof(float4) * (size_t)(W.npad / 2) * kContractTile +
+    const size_t need = kBStages * chunk_bytes(W.npad) + sizeof(longlong2) * (size_t)(W.npad / 2) * kContractTile +
                         sizeof(double) * (size_t)(W.hi - W.lo + 3) * kContractTile;
     // more than half an SM's shared memory: one CTA per SM, which takes all of its tensor memory
     return std::max<size_t>(need, 120 * 1024);

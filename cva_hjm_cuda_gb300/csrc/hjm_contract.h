@@ -41,7 +41,8 @@ cudaError_t launch_contract_table(int nt, double c, int stride, int n_blocks, bo
                                   void* table, cudaStream_t s);
 
 // Row scales of external normals [path][step][3]: out[2 p] = 2^-e, out[2 p +
-// 1] = 2^e with e >= 0 the least that brings every |normal| of path p below 8.
+// 1] = 2^e with e >= 0 the least that brings every |normal| of path p below 8
+// (NaN for a path with a non-finite normal).
 cudaError_t launch_contract_ext_scale(const double* raw, int64_t n_paths, int n_steps, double* out, cudaStream_t s);
 
 // The valuation: one launch per window (carry [2][n_paths] doubles when there
