@@ -106,17 +106,17 @@ struct hjm_ctx {
     bool keep_exposures = false;
 
     // device buffers
-    DevBuf partials, sums, result, estore, sel, hist, ext, ext_raw, wide, scratch, ck_h, ck_a, contract, carry,
+    DevBuf partials, sums, result, estore, sel, hist, ext, ext_raw, wide, scratch, ck_h, ck_a, contract, split, carry,
         mresp;
     MemBudget budget;
     hjm_ctx()
     {
         for (DevBuf* b : buffers()) b->budget = &budget;
     }
-    std::array<DevBuf*, 15> buffers()
+    std::array<DevBuf*, 16> buffers()
     {
         return {&partials, &sums, &result, &estore, &sel, &hist, &ext, &ext_raw, &wide, &scratch, &ck_h, &ck_a,
-                &contract, &carry, &mresp};
+                &contract, &split, &carry, &mresp};
     }
     // the tables in contract and mresp hold the run shapes of their keys;
     // resp_used is recorded after the last kernel that reads one
@@ -871,9 +871,12 @@ static hjm_status enqueue_contract(hjm_ctx* ctx, const RunShape& sh, double dt, 
     }
     const double* ext_scale =
         ext_dev ? ext_dev + (size_t)P.n_paths * (size_t)sh.B * (size_t)sh.stride * kFactors : nullptr;
+    const size_t split = contract_sums_bytes(P.n_paths, sh.B, sh.stride, ctx->n_sms, ext_dev != nullptr);
+    if (split) HJM_CUDA(ctx, ctx->split.ensure(split));
     int launches = 0;
     HJM_CUDA(ctx, launch_path_contract(ctx->nt, P, ctx->contract.p, ext_dev, ext_scale, (double*)ctx->partials.p,
-                                       estore, carry, (double*)ctx->result.p, ctx->n_sms, s, &launches));
+                                       estore, carry, split ? (longlong2*)ctx->split.p : nullptr,
+                                       (double*)ctx->result.p, ctx->n_sms, s, &launches));
     ctx->stat_launches += launches - 1;
     return HJM_OK;
 }
@@ -974,7 +977,8 @@ static hjm_status enqueue_impl(hjm_ctx* ctx, int64_t n_paths, int32_t n_steps, d
     const int cta = !mixed && use_response_form(ctx) ? kContractTile
                     : mresp_ns                       ? kCta
                              : (pc ? pc_cta() : path_cta(mixed, ctx->nt, sh.B, use_poly_path(ctx) || mixed_cubic));
-    const int64_t n_ctas = (n_paths + cta - 1) / cta;
+    const int64_t n_ctas = !mixed && use_response_form(ctx) ? contract_rows(n_paths, sh.B, sh.stride, ctx->n_sms)
+                                                            : (n_paths + cta - 1) / cta;
     const int64_t ld = (n_paths + 3) / 4 * 4;
     const size_t esize = mixed ? 4 : 8;
 

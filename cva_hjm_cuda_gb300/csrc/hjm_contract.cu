@@ -306,12 +306,61 @@ __device__ __forceinline__ void epilogue_sync() { asm volatile("bar.sync 1, 128;
 
 }  // namespace
 
-// The launch's constants besides the path parameters.
+// The launch's constants besides the path parameters.  Whole tiles [0, n_tiles)
+// go to the CTAs in turn; in a split launch the accumulator groups of tiles
+// [tile0, tile0 + n_tiles) are dealt to the CTAs in equal runs, and each CTA adds
+// its groups' sums of a tile to sums [n_tiles][npad / 2][128], which
+// contract_price_kernel then prices.
 struct ContractParams {
     PathParams<double> P;
     ContractWindow W;
-    int64_t n_tiles;
+    int64_t tile0, n_tiles;
+    longlong2* sums;  // null: whole tiles
 };
+
+// Chunks [begin, end) of a tile's accumulator groups
+__host__ __device__ constexpr int group_chunk(int64_t group, int chunks)
+{
+    return group * kFlush < chunks ? (int)group * kFlush : chunks;
+}
+__host__ __device__ constexpr int tile_groups(int chunks) { return (chunks + kFlush - 1) / kFlush; }
+
+// What a CTA works through: chunk c0 of tile first on, `chunks` chunks, tiles
+// `step` apart
+struct ContractRun {
+    int64_t first, step, chunks;
+    int c0;
+};
+__device__ __forceinline__ ContractRun contract_run(const ContractParams& Q)
+{
+    const int NC = Q.W.chunks;
+    ContractRun r;
+    if (!Q.sums) {
+        r.first = blockIdx.x;
+        r.step = gridDim.x;
+        r.chunks = (blockIdx.x < Q.n_tiles ? (Q.n_tiles - 1 - blockIdx.x) / gridDim.x + 1 : 0) * NC;
+        r.c0 = 0;
+        return r;
+    }
+    const int G = tile_groups(NC);
+    const int64_t units = Q.n_tiles * G, u0 = units * blockIdx.x / gridDim.x, u1 = units * (blockIdx.x + 1) / gridDim.x;
+    r.first = Q.tile0 + u0 / G;
+    r.step = 1;
+    r.c0 = group_chunk(u0 % G, NC);
+    r.chunks = (u1 / G - u0 / G) * NC + group_chunk(u1 % G, NC) - r.c0;
+    return r;
+}
+
+// The cash flow of date i from its running sums v (times the scales sx, sa; the
+// slices are negated)
+__device__ __forceinline__ double contract_cash_flow(const PathParams<double>& P, int i, longlong2 v, double sx,
+                                                     double sa)
+{
+    const double x = fma(-sum_value(v.x), sx, P.psamp[i]), a = fma(-sum_value(v.y), sa, P.psum[i]);
+    const double D = exp(-a * P.dt);
+    const double Lb = P.m * (exp(x * P.inv_m) - 1.0);
+    return D * (P.payA[i] * Lb - P.payB[i]);
+}
 
 template <bool EXT>
 __global__ void __launch_bounds__(kThreads, 1)
@@ -364,6 +413,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_s;
+    const ContractRun run = contract_run(Q);
 
     if (warp < kProducers) {
         // ---- normals -> A slices in tensor memory.  Two groups of 8 warps take
@@ -374,18 +424,17 @@ __global__ void __launch_bounds__(kThreads, 1)
         const uint32_t a_addr = tmem + ((uint32_t)(32 * q) << 16) + kACol + st * kAStageCols + 12 * sub;
         const int n_last = P.n_blocks * P.stride - 1;
         uint32_t ph = 1;
-        bool ok = NC > 0;
-        int c = st;
-        int64_t tile = blockIdx.x;
-        while (ok) {
-            for (; c >= NC; c -= NC) tile += gridDim.x;
-            if (tile >= Q.n_tiles) break;
+        bool ok = true;
+        int c = run.c0 + st;
+        int64_t tile = run.first, left = (run.chunks - st + kAStages - 1) / kAStages;  // this group's chunks
+        while (ok && left > 0) {
+            for (; c >= NC; c -= NC) tile += run.step;
             const int64_t lp = tile * kContractTile + 32 * q + lane;
             const PathDraw pd = path_draw(P.path_offset + (uint64_t)lp, P.rk0, P.rk1);
             const int64_t lpc = lp < P.n_paths ? lp : 0;
             double xs = 1.0;
             if constexpr (EXT) xs = __ldg(ext_scale + 2 * lpc);
-            for (; c < NC; c += kAStages, ph ^= 1u) {
+            for (; c < NC && left > 0; c += kAStages, ph ^= 1u, --left) {
 #pragma unroll 1
                 for (int half = 0; half < 2; ++half) {
                     const int n0 = P.stride + kChunk * c + 8 * sub + 4 * half;
@@ -445,8 +494,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         // ---- the matrix instructions: the warp waits as one, one elected lane issues
         const bool leader = elect_one();
         const uint32_t bs = smem_u32(b_s);
-        const int64_t tiles = blockIdx.x < Q.n_tiles ? (Q.n_tiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
-        const int64_t total = tiles * NC;
+        const int64_t total = run.chunks;
         bool ok = true;
         // a_s times the response slices b_0 .. b_{levels - 1 - s} gives the
         // levels s .. 4; beyond 256 columns b_4 takes an instruction of its own
@@ -461,7 +509,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         // that their addresses and parities are constants or warp-uniform: the
         // issuing warp shares one scheduler with four normal warps, which its
         // instructions delay (and the barriers the other schedulers with them).
-        int c = 0, fl = 0;      // chunk of the tile, of the accumulator group
+        int c = run.c0, fl = 0;  // chunk of the tile, of the accumulator group
         uint32_t ph = 0, d_ph = 1;
         int64_t g = 0;
         auto chunk = [&](auto iv) {
@@ -517,10 +565,9 @@ __global__ void __launch_bounds__(kThreads, 1)
         // ---- B operand tiles by bulk copy
         if (lane == 0) {
             const uint32_t bs = smem_u32(b_s);
-            const int64_t tiles = blockIdx.x < Q.n_tiles ? (Q.n_tiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
-            const int64_t total = tiles * NC;
+            const int64_t total = run.chunks;
             const unsigned char* image = table + W.image;
-            int c = 0, st = 0;
+            int c = run.c0, st = 0;
             uint32_t ph = 1;
             int64_t g = 0;
             for (; g < total; ++g) {
@@ -556,118 +603,150 @@ __global__ void __launch_bounds__(kThreads, 1)
         const int first_date = lo > 2 ? lo : 2;  // date 1 precedes any evolution
         double* e_s = cf_s + kContractTile;  // exposure row of date j: j - lo + 1 (the cash-flow row of date j + 1)
         int64_t grp = 0;
-        for (int64_t tile = blockIdx.x; tile < Q.n_tiles; tile += gridDim.x) {
-            const int64_t base = tile * kContractTile, lp = base + p;
-            const bool active = lp < P.n_paths;
-            double rs = 1.0;
-            if constexpr (EXT) rs = __ldg(ext_scale + 2 * (active ? lp : 0) + 1);
-            auto price = [&](int i) {
-                double x = P.psamp[i], a = P.psum[i];
-                if (i >= 2) {
-                    const longlong2 r = run_s[(size_t)(hi - i) * kContractTile + p];
-                    double sx = __ldg(scale + 2 * i), sa = __ldg(scale + 2 * i + 1);
-                    if constexpr (EXT) {
-                        sx *= rs;
-                        sa *= rs;
+        // waits for an accumulator group and adds it to the running sums of the live
+        // slots (fresh: the first of them), four slots at a time, padding included
+        // (its columns are zero); false if the wait ran out
+        auto drain_group = [&](bool fresh, int live) {
+            const bool ok = mbar_wait<true>(d_full, (uint32_t)(grp & 1), abort_s);
+            if (!__all_sync(0xffffffffu, ok)) return false;
+            ++grp;
+            tc_fence_after();
+            for (int r0 = 0; r0 < live; r0 += 4) {
+                float acc[kLevels][8];
+#pragma unroll
+                for (int s = 0; s < kLevels; ++s) tmem_ld8(d_addr + s * npad + 2 * r0, acc[s]);
+                longlong2 cell[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    cell[u] = fresh ? make_longlong2(0, 0) : run_s[(size_t)(r0 + u) * kContractTile + p];
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                if (r0 + 4 >= live) {  // the accumulators are read: the next group may start
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(d_empty);
+                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    cell[u].x += level_sum(acc[0][2 * u], acc[1][2 * u], acc[2][2 * u], acc[3][2 * u], acc[4][2 * u]);
+                    cell[u].y += level_sum(acc[0][2 * u + 1], acc[1][2 * u + 1], acc[2][2 * u + 1], acc[3][2 * u + 1],
+                                           acc[4][2 * u + 1]);
+                    run_s[(size_t)(r0 + u) * kContractTile + p] = cell[u];
+                }
+            }
+            return true;
+        };
+        if (Q.sums) {  // ---- split tiles: this CTA's groups of each, to the tile's sums
+            int64_t left = run.chunks, tile = run.first;
+            for (int c = run.c0; left > 0; c = 0, ++tile) {
+                const int end = (int)min((int64_t)NC, c + left);
+                left -= end - c;
+                int next = first_date;
+                auto skip_to = [&](int chunk) {  // dates sampled before the chunk
+                    while ((next - 1) * P.stride <= kChunk * chunk) ++next;
+                };
+                skip_to(c);
+                const int live0 = hi - next + 1;
+                bool ok = true;
+                for (int b = c; b < end && ok; b += kFlush) {
+                    skip_to(b);
+                    ok = drain_group(b == c, hi - next + 1);
+                }
+                if (!ok) break;
+                unsigned long long* to = reinterpret_cast<unsigned long long*>(
+                    Q.sums + (size_t)(tile - Q.tile0) * (npad / 2) * kContractTile);
+                for (int r = 0; r < live0; ++r) {
+                    const size_t at = (size_t)r * kContractTile + p;
+                    const longlong2 v = run_s[at];
+                    atomicAdd(to + 2 * at, (unsigned long long)v.x);
+                    atomicAdd(to + 2 * at + 1, (unsigned long long)v.y);
+                }
+            }
+        } else {
+            for (int64_t tile = blockIdx.x; tile < Q.n_tiles; tile += gridDim.x) {
+                const int64_t base = tile * kContractTile, lp = base + p;
+                const bool active = lp < P.n_paths;
+                double rs = 1.0;
+                if constexpr (EXT) rs = __ldg(ext_scale + 2 * (active ? lp : 0) + 1);
+                auto price = [&](int i) {
+                    double sx = 0.0, sa = 0.0;
+                    longlong2 v = make_longlong2(0, 0);
+                    if (i >= 2) {
+                        v = run_s[(size_t)(hi - i) * kContractTile + p];
+                        sx = __ldg(scale + 2 * i);
+                        sa = __ldg(scale + 2 * i + 1);
+                        if constexpr (EXT) {
+                            sx *= rs;
+                            sa *= rs;
+                        }
                     }
-                    x = fma(-sum_value(r.x), sx, x);  // (the slices are negated)
-                    a = fma(-sum_value(r.y), sa, a);
+                    cf_s[(size_t)(i - lo + 1) * kContractTile + p] = contract_cash_flow(P, i, v, sx, sa);
+                };
+                if (bottom) price(1);
+                int next = first_date;  // the earliest date not priced yet
+                for (int c = 0; c < NC; c += kFlush) {
+                    if (!drain_group(c == 0, hi - next + 1)) break;
+                    // the dates whose last step this group held
+                    const int done = kChunk * min(c + kFlush, NC);
+                    for (; next <= hi && (next - 1) * P.stride <= done; ++next) price(next);
                 }
-                const double D = exp(-a * P.dt);
-                const double Lb = P.m * (exp(x * P.inv_m) - 1.0);
-                cf_s[(size_t)(i - lo + 1) * kContractTile + p] = D * (P.payA[i] * Lb - P.payB[i]);
-            };
-            if (bottom) price(1);
-            int next = first_date;  // the earliest date not priced yet
-            for (int c = 0; c < NC; c += kFlush, ++grp) {
-                const bool ok = mbar_wait<true>(d_full, (uint32_t)(grp & 1), abort_s);
-                if (!__all_sync(0xffffffffu, ok)) break;
-                tc_fence_after();
-                const int live = hi - next + 1;
-                // four slots at a time, padding included (its columns are zero)
-                for (int r0 = 0; r0 < live; r0 += 4) {
-                    float acc[kLevels][8];
-#pragma unroll
-                    for (int s = 0; s < kLevels; ++s) tmem_ld8(d_addr + s * npad + 2 * r0, acc[s]);
-                    longlong2 cell[4];
-#pragma unroll
-                    for (int u = 0; u < 4; ++u)
-                        cell[u] = c ? run_s[(size_t)(r0 + u) * kContractTile + p] : make_longlong2(0, 0);
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    if (r0 + 4 >= live) {  // the accumulators are read: the next group may start
-                        tc_fence_before();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(d_empty);
+                // (a wait that ran out ends all four warps at the same tile)
+                if (p == 0) stop_flag = *abort_s;
+                epilogue_sync();
+                if (stop_flag) break;
+                // exposures E_j = max(sum_{i > j} cf_i, 0) of dates lo - 1 .. hi - 1
+                // (and E_B = 0 for the latest window), the later dates' cash flows in carry
+                const int j0 = lo - 1, j1 = top ? B : hi - 1;
+                double v = 0.0, cva_c = 0.0;
+                if (!top && active) {
+                    v = carry[lp];
+                    cva_c = carry[P.n_paths + lp];
+                }
+                if (top) e_s[(size_t)(B - lo + 1) * kContractTile + p] = 0.0;
+                for (int j = hi - 1; j >= lo - 1; --j) {
+                    v += cf_s[(size_t)(j - lo + 2) * kContractTile + p];
+                    double e = (v > 0.0) ? v : 0.0;
+                    if (!active) e = 0.0;
+                    e_s[(size_t)(j - lo + 1) * kContractTile + p] = e;
+                    cva_c = fma(P.cvaw[j], e, cva_c);
+                }
+                if (!bottom && active) {
+                    carry[lp] = v;
+                    carry[P.n_paths + lp] = cva_c;
+                }
+                if (bottom) {
+                    const double s1 = warp_sum(cva_c), s2 = warp_sum(cva_c * cva_c);
+                    if (lane == 0) {
+                        red_s[q] = s1;
+                        red_s[4 + q] = s2;
                     }
+                }
+                if (P.store_exposures) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                epilogue_sync();
+                for (int j = j0 + q; j <= j1; j += 4) {
+                    double sum = 0.0;
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        cell[u].x += level_sum(acc[0][2 * u], acc[1][2 * u], acc[2][2 * u], acc[3][2 * u], acc[4][2 * u]);
-                        cell[u].y += level_sum(acc[0][2 * u + 1], acc[1][2 * u + 1], acc[2][2 * u + 1],
-                                               acc[3][2 * u + 1], acc[4][2 * u + 1]);
-                        run_s[(size_t)(r0 + u) * kContractTile + p] = cell[u];
+                    for (int u = 0; u < 4; ++u) sum += e_s[(size_t)(j - lo + 1) * kContractTile + lane + 32 * u];
+                    sum = warp_sum(sum);
+                    if (lane == 0) partials[(size_t)tile * R + j] = sum;
+                }
+                if (p == 127 && bottom) {
+                    partials[(size_t)tile * R + B + 1] = (red_s[0] + red_s[1]) + (red_s[2] + red_s[3]);
+                    partials[(size_t)tile * R + B + 2] = (red_s[4] + red_s[5]) + (red_s[6] + red_s[7]);
+                }
+                if (p == 0 && P.store_exposures) {
+                    const int64_t cnt = (P.n_paths - base < kContractTile) ? (P.n_paths - base) : kContractTile;
+                    const uint32_t bytes = (uint32_t)(((cnt + 1) / 2) * 2 * sizeof(double));
+                    for (int j = j0; j <= j1; ++j) {
+                        double* dst = estore + (size_t)j * (size_t)P.ld + (size_t)base;
+                        asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst),
+                                     "r"(smem_u32(e_s + (size_t)(j - lo + 1) * kContractTile)), "r"(bytes)
+                                     : "memory");
                     }
+                    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                    asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
                 }
-                // the dates whose last step this group held
-                const int done = kChunk * min(c + kFlush, NC);
-                for (; next <= hi && (next - 1) * P.stride <= done; ++next) price(next);
+                epilogue_sync();  // (the rows are read: the next tile may price)
             }
-            // (a wait that ran out ends all four warps at the same tile)
-            if (p == 0) stop_flag = *abort_s;
-            epilogue_sync();
-            if (stop_flag) break;
-            // exposures E_j = max(sum_{i > j} cf_i, 0) of dates lo - 1 .. hi - 1
-            // (and E_B = 0 for the latest window), the later dates' cash flows in carry
-            const int j0 = lo - 1, j1 = top ? B : hi - 1;
-            double v = 0.0, cva_c = 0.0;
-            if (!top && active) {
-                v = carry[lp];
-                cva_c = carry[P.n_paths + lp];
-            }
-            if (top) e_s[(size_t)(B - lo + 1) * kContractTile + p] = 0.0;
-            for (int j = hi - 1; j >= lo - 1; --j) {
-                v += cf_s[(size_t)(j - lo + 2) * kContractTile + p];
-                double e = (v > 0.0) ? v : 0.0;
-                if (!active) e = 0.0;
-                e_s[(size_t)(j - lo + 1) * kContractTile + p] = e;
-                cva_c = fma(P.cvaw[j], e, cva_c);
-            }
-            if (!bottom && active) {
-                carry[lp] = v;
-                carry[P.n_paths + lp] = cva_c;
-            }
-            if (bottom) {
-                const double s1 = warp_sum(cva_c), s2 = warp_sum(cva_c * cva_c);
-                if (lane == 0) {
-                    red_s[q] = s1;
-                    red_s[4 + q] = s2;
-                }
-            }
-            if (P.store_exposures) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            epilogue_sync();
-            for (int j = j0 + q; j <= j1; j += 4) {
-                double sum = 0.0;
-#pragma unroll
-                for (int u = 0; u < 4; ++u) sum += e_s[(size_t)(j - lo + 1) * kContractTile + lane + 32 * u];
-                sum = warp_sum(sum);
-                if (lane == 0) partials[(size_t)tile * R + j] = sum;
-            }
-            if (p == 127 && bottom) {
-                partials[(size_t)tile * R + B + 1] = (red_s[0] + red_s[1]) + (red_s[2] + red_s[3]);
-                partials[(size_t)tile * R + B + 2] = (red_s[4] + red_s[5]) + (red_s[6] + red_s[7]);
-            }
-            if (p == 0 && P.store_exposures) {
-                const int64_t cnt = (P.n_paths - base < kContractTile) ? (P.n_paths - base) : kContractTile;
-                const uint32_t bytes = (uint32_t)(((cnt + 1) / 2) * 2 * sizeof(double));
-                for (int j = j0; j <= j1; ++j) {
-                    double* dst = estore + (size_t)j * (size_t)P.ld + (size_t)base;
-                    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst),
-                                 "r"(smem_u32(e_s + (size_t)(j - lo + 1) * kContractTile)), "r"(bytes)
-                                 : "memory");
-                }
-                asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-                asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-            }
-            epilogue_sync();  // (the rows are read: the next tile may price)
         }
         if (p == 0 && P.store_exposures) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     }
@@ -677,6 +756,79 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (tid == 0 && abort_flag) result[kResErr] = 1.0;
     if (warp == kMmaWarp)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(kTmemCols) : "memory");
+}
+
+// Prices the split tiles from their sums: a CTA takes 32 paths (lane = path),
+// its four warps every fourth date, so that few paths still reach many SMs' FP64
+// pipes (18 cycles an instruction and SM, ~45 per date and path).  Partial-sum
+// rows and exposure rows as the path kernel's, one row per 32 paths from row0.
+template <bool EXT>
+__global__ void __launch_bounds__(128)
+    contract_price_kernel(const __grid_constant__ ContractParams Q, const double* __restrict__ scale,
+                          const double* __restrict__ ext_scale, int64_t row0, double* __restrict__ partials,
+                          double* __restrict__ estore, double* __restrict__ carry)
+{
+    const PathParams<double>& P = Q.P;
+    const int lo = Q.W.lo, hi = Q.W.hi, B = P.n_blocks, R = B + 3;
+    const bool top = hi == B, bottom = lo == 1;
+    __shared__ double cf_s[kContractMaxSlots + 4][32];  // row i - lo + 1: date i, then its exposures one row up
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int in_tile = (int)(blockIdx.x & 3) * 32 + lane;
+    const int64_t tile = Q.tile0 + blockIdx.x / 4, lp = tile * kContractTile + in_tile;
+    const bool active = lp < P.n_paths;
+    const longlong2* sums = Q.sums + (size_t)(blockIdx.x / 4) * (Q.W.npad / 2) * kContractTile + in_tile;
+    double rs = 1.0;
+    if constexpr (EXT) rs = __ldg(ext_scale + 2 * (active ? lp : 0) + 1);
+    for (int i = lo + warp; i <= hi; i += 4) {
+        double sx = 0.0, sa = 0.0;
+        longlong2 v = make_longlong2(0, 0);
+        if (i >= 2) {
+            v = sums[(size_t)(hi - i) * kContractTile];
+            sx = __ldg(scale + 2 * i);
+            sa = __ldg(scale + 2 * i + 1);
+            if constexpr (EXT) {
+                sx *= rs;
+                sa *= rs;
+            }
+        }
+        cf_s[i - lo + 1][lane] = contract_cash_flow(P, i, v, sx, sa);
+    }
+    __syncthreads();
+    double(*e_s)[32] = cf_s + 1;  // exposure row of date j: j - lo + 1
+    if (warp == 0) {
+        double v = 0.0, cva_c = 0.0;
+        if (!top && active) {
+            v = carry[lp];
+            cva_c = carry[P.n_paths + lp];
+        }
+        if (top) e_s[B - lo + 1][lane] = 0.0;
+        for (int j = hi - 1; j >= lo - 1; --j) {
+            v += cf_s[j - lo + 2][lane];
+            double e = (v > 0.0) ? v : 0.0;
+            if (!active) e = 0.0;
+            e_s[j - lo + 1][lane] = e;
+            cva_c = fma(P.cvaw[j], e, cva_c);
+        }
+        if (!bottom && active) {
+            carry[lp] = v;
+            carry[P.n_paths + lp] = cva_c;
+        }
+        if (bottom) {
+            const double s1 = warp_sum(cva_c), s2 = warp_sum(cva_c * cva_c);
+            if (lane == 0) {
+                partials[(size_t)(row0 + blockIdx.x) * R + B + 1] = s1;
+                partials[(size_t)(row0 + blockIdx.x) * R + B + 2] = s2;
+            }
+        }
+    }
+    __syncthreads();
+    const int j1 = top ? B : hi - 1;
+    for (int j = lo - 1 + warp; j <= j1; j += 4) {
+        const double e = e_s[j - lo + 1][lane];
+        const double sum = warp_sum(e);
+        if (lane == 0) partials[(size_t)(row0 + blockIdx.x) * R + j] = sum;
+        if (P.store_exposures && active) estore[(size_t)j * (size_t)P.ld + (size_t)lp] = e;
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -961,9 +1113,37 @@ cudaError_t launch_contract_ext_scale(const double* raw, int64_t n_paths, int n_
     return cudaGetLastError();
 }
 
+// Tiles whose steps are split over all SMs: those left over after the whole
+// waves, when dealing their groups costs less than a wave of whole tiles.  Decided
+// on the whole run's groups, so every window (and an external-normals run's other
+// windows) splits the same paths.  Two groups' time covers the second launch and
+// the pricing kernel.  FP64 calls: 128 paths 10y 189 -> 124 us, 5,000 paths 185 ->
+// 151 us, 5,000 paths 25y 471 -> 296 us, 100,003 paths 30y 2.73 -> 2.46 ms.
+static int64_t split_tiles(int64_t n_paths, int n_blocks, int stride, int n_sms)
+{
+    const int64_t tiles = (n_paths + kContractTile - 1) / kContractTile, rest = tiles % n_sms;
+    const int G = tile_groups(((n_blocks - 1) * stride + kChunk - 1) / kChunk);
+    return rest > 0 && (rest * G + n_sms - 1) / n_sms + 2 <= G ? rest : 0;
+}
+
+int64_t contract_rows(int64_t n_paths, int n_blocks, int stride, int n_sms)
+{
+    const int64_t split = split_tiles(n_paths, n_blocks, stride, n_sms);
+    return (n_paths + kContractTile - 1) / kContractTile + 3 * split;
+}
+
+size_t contract_sums_bytes(int64_t n_paths, int n_blocks, int stride, int n_sms, bool ext)
+{
+    ContractWindow w[kMaxTenor];
+    const int n = contract_windows(n_blocks, stride, ext, w);
+    int npad = 0;
+    for (int i = 0; i < n; ++i) npad = std::max(npad, w[i].npad);
+    return sizeof(longlong2) * (size_t)split_tiles(n_paths, n_blocks, stride, n_sms) * (npad / 2) * kContractTile;
+}
+
 cudaError_t launch_path_contract(int nt, const PathParams<double>& P, const void* table, const double* ext,
                                  const double* ext_scale, double* partials, double* estore, double* carry,
-                                 double* result, int n_sms, cudaStream_t s, int* launches)
+                                 longlong2* sums, double* result, int n_sms, cudaStream_t s, int* launches)
 {
     if (!path_tenor_supported(nt) || P.n_blocks < 1 || P.n_blocks >= nt || P.stride < 1 || (ext && !ext_scale))
         return cudaErrorInvalidValue;
@@ -971,20 +1151,44 @@ cudaError_t launch_path_contract(int nt, const PathParams<double>& P, const void
     const int n = contract_windows(P.n_blocks, P.stride, ext != nullptr, w);
     if (n > 1 && !carry) return cudaErrorInvalidValue;
     auto kernel = ext ? path_kernel_contract<true> : path_kernel_contract<false>;
+    auto price = ext ? contract_price_kernel<true> : contract_price_kernel<false>;
     ContractParams Q;
     Q.P = P;
-    Q.n_tiles = (P.n_paths + kContractTile - 1) / kContractTile;
+    const int64_t tiles = (P.n_paths + kContractTile - 1) / kContractTile;
+    const int64_t split = sums ? split_tiles(P.n_paths, P.n_blocks, P.stride, n_sms) : 0, whole = tiles - split;
+    int count = 0;
     for (int i = 0; i < n; ++i) {
         Q.W = w[i];
         const size_t smem = contract_smem(w[i]);
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
-        kernel<<<(unsigned)std::min<int64_t>(Q.n_tiles, n_sms), kThreads, smem, s>>>(
-            Q, (const unsigned char*)table, ext, ext_scale, partials, estore, carry, result);
+        if (whole > 0) {
+            Q.tile0 = 0;
+            Q.n_tiles = whole;
+            Q.sums = nullptr;
+            kernel<<<(unsigned)std::min<int64_t>(whole, n_sms), kThreads, smem, s>>>(
+                Q, (const unsigned char*)table, ext, ext_scale, partials, estore, carry, result);
+            ++count;
+        }
+        if (split > 0) {
+            Q.tile0 = whole;
+            Q.n_tiles = split;
+            Q.sums = sums;
+            const int64_t groups = split * tile_groups(w[i].chunks);
+            if (groups > 0) {
+                e = cudaMemsetAsync(sums, 0, sizeof(longlong2) * (size_t)split * (w[i].npad / 2) * kContractTile, s);
+                if (e != cudaSuccess) return e;
+                kernel<<<(unsigned)std::min<int64_t>(groups, n_sms), kThreads, smem, s>>>(
+                    Q, (const unsigned char*)table, ext, ext_scale, partials, estore, carry, result);
+                ++count;
+            }
+            price<<<(unsigned)(4 * split), 128, 0, s>>>(Q, (const double*)table, ext_scale, whole, partials, estore, carry);
+            ++count;
+        }
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
-    if (launches) *launches = n;
+    if (launches) *launches = count;
     return cudaSuccess;
 }
 

@@ -45,13 +45,19 @@ cudaError_t launch_contract_table(int nt, double c, int stride, int n_blocks, bo
 // (NaN for a path with a non-finite normal).
 cudaError_t launch_contract_ext_scale(const double* raw, int64_t n_paths, int n_steps, double* out, cudaStream_t s);
 
-// The valuation: one launch per window (carry [2][n_paths] doubles when there
-// is more than one).  partials: one row of n_blocks + 3 doubles per tile of
-// kContractTile paths.  ext: external normals [step][3][path] with their row
-// scales, or null for the generator.  result[kResErr] is set if a wait in the
-// kernel ran out.
+// Partial-sum rows of a run: one per tile of kContractTile paths, four for a tile
+// whose steps are split over the SMs (the tiles after the last whole wave, where
+// that pays); the split tiles' sums take contract_sums_bytes (0: none).
+int64_t contract_rows(int64_t n_paths, int n_blocks, int stride, int n_sms);
+size_t contract_sums_bytes(int64_t n_paths, int n_blocks, int stride, int n_sms, bool ext);
+
+// The valuation: per window a launch over the whole tiles and one over the split
+// ones with their pricing (carry [2][n_paths] doubles when there is more than one
+// window).  partials: contract_rows rows of n_blocks + 3 doubles.  ext: external
+// normals [step][3][path] with their row scales, or null for the generator.
+// result[kResErr] is set if a wait in the kernel ran out.
 cudaError_t launch_path_contract(int nt, const PathParams<double>& P, const void* table, const double* ext,
                                  const double* ext_scale, double* partials, double* estore, double* carry,
-                                 double* result, int n_sms, cudaStream_t s, int* launches);
+                                 longlong2* sums, double* result, int n_sms, cudaStream_t s, int* launches);
 
 }  // namespace hjm

@@ -98,3 +98,16 @@ def test_external_normals_beyond_the_slices(engine, dates):
     assert np.all(y[:, 17] == 0.0)
     keep = np.arange(140) != 17
     np.testing.assert_array_equal(y[:, keep], x[:, keep])
+
+
+@pytest.mark.parametrize("n_paths,dates", [(152 * 128 + 129, 20), (40 * 128 - 5, 50), (3 * 152 * 128 + 700, 34)])
+def test_whole_waves_and_split_tiles(engine, n_paths, dates):
+    """Tiles beyond the last whole wave of 152 have their steps split over the
+    SMs: they must join the whole tiles' paths, exposures and partial sums."""
+    engine.set_market(_table_market(51))
+    engine.set_swap(Swap(n_periods=dates))
+    cfg = RunConfig(n_paths=n_paths, n_steps=25 * dates, dt=0.02, seed=12)
+    (v, x), (c, xc) = _both(engine, lambda: engine.run(cfg, "fp64"))
+    _close(x, xc, dates)
+    np.testing.assert_allclose(v.ee[:dates], c.ee[:dates], rtol=1e-12, atol=1e-13 * np.max(c.ee))
+    assert v.cva == pytest.approx(c.cva, rel=1e-12) and v.cva_stderr == pytest.approx(c.cva_stderr, rel=1e-9)
