@@ -46,6 +46,8 @@
 // nothing is recomputed.
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include <cstdint>
 
 #include "hjm_device.cuh"
@@ -754,7 +756,8 @@ constexpr int adj_resp_min_ctas(int ns) { return ns <= 8 ? 11 : 8; }
 
 template <int NS>
 __global__ void __launch_bounds__(kAdjCta, adj_resp_min_ctas(NS))
-    adjoint_kernel_resp(const __grid_constant__ MixedParams M, const float4* __restrict__ resp,
+    adjoint_kernel_resp(const __grid_constant__ MixedParams M, const RespLive live,
+                        const float4* __restrict__ resp,
                         double* __restrict__ partials)
 {
     constexpr int C = kAdjCta;
@@ -799,8 +802,9 @@ __global__ void __launch_bounds__(kAdjCta, adj_resp_min_ctas(NS))
     const int n_last = n_steps - 1;
     float q0, q1, q2;
     draw_phi<float, false>(nullptr, gpath, lp, P.n_paths, min(stride, n_last), P.rk0, P.rk1, q0, q1, q2);
-    for (int b = 1; b < B; ++b) {
-        float sS = 0.f, sU = 0.f, sW = 0.f;
+    float sS, sU, sW;
+    auto steps = [&](auto live_c, int b) {  // (as path_kernel_mixed_resp's)
+        constexpr int LIVE = decltype(live_c)::value;
         const float4* row = resp + (size_t)b * stride * (NS / 2);
 #pragma unroll 5  // (a divisor of 50 steps per block: 8.66 ms against 8.77 by 2 at 1M paths)
         for (int s = 0; s < stride; ++s) {
@@ -810,7 +814,7 @@ __global__ void __launch_bounds__(kAdjCta, adj_resp_min_ctas(NS))
             const float2 w2 = make_float2(W, W);
             const float4* rr = row + (size_t)s * (NS / 2);
 #pragma unroll
-            for (int u = 0; u < NS / 2; ++u) {
+            for (int u = 0; u < LIVE / 2; ++u) {
                 const float4 e = __ldg(rr + u);
                 A[2 * u] = __ffma2_rn(make_float2(e.x, e.y), w2, A[2 * u]);
                 A[2 * u + 1] = __ffma2_rn(make_float2(e.z, e.w), w2, A[2 * u + 1]);
@@ -827,6 +831,15 @@ __global__ void __launch_bounds__(kAdjCta, adj_resp_min_ctas(NS))
             sU += U;
             sW += W;
         }
+    };
+    for (int b = 1; b < B; ++b) {
+        sS = sU = sW = 0.f;
+        if (b < live.half)
+            steps(std::integral_constant<int, NS>(), b);
+        else if (b < live.none)
+            steps(std::integral_constant<int, NS / 2>(), b);
+        else
+            steps(std::integral_constant<int, 0>(), b);
         zS += (double)sS;
         zU += (double)sU;
         zW += (double)sW;
@@ -975,7 +988,7 @@ __global__ void __launch_bounds__(kAdjCta, adj_resp_min_ctas(NS))
 
 size_t adjoint_resp_smem(int n_blocks) { return adj_resp_layout(n_blocks, 3 * n_blocks + 12).total; }
 
-cudaError_t launch_adjoint_resp(const AdjParams& A, int ns, const float4* table, double* partials, cudaStream_t s)
+cudaError_t launch_adjoint_resp(const AdjParams& A, int ns, const RespLive& live, const float4* table, double* partials, cudaStream_t s)
 {
     if (ns != 8 && ns != 16) return cudaErrorInvalidValue;
     const int B = A.M.P.n_blocks;
@@ -985,7 +998,7 @@ cudaError_t launch_adjoint_resp(const AdjParams& A, int ns, const float4* table,
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     const int64_t grid = (A.M.P.n_paths + kAdjCta - 1) / kAdjCta;
-    k<<<(unsigned)grid, kAdjCta, smem, s>>>(A.M, table, partials);
+    k<<<(unsigned)grid, kAdjCta, smem, s>>>(A.M, live, table, partials);
     return cudaGetLastError();
 }
 

@@ -130,6 +130,7 @@ struct hjm_ctx {
         bool valid = false, on_device = false, pc = false;
         int nt = 0, stride = 0, B = 0, ns = 0;
         double c = 0, dtau = 0;
+        RespLive live = {};
     } mresp_key;
     cudaEvent_t resp_used = nullptr;
 
@@ -920,7 +921,7 @@ static int mresp_run_slots(hjm_ctx* ctx, const RunShape& sh, double dt, bool pc 
     hjm_ctx::MrespKey& k = ctx->mresp_key;
     if (!(k.valid && k.pc == pc && k.nt == ctx->nt && k.stride == sh.stride && k.B == sh.B && k.c == c &&
           k.dtau == ctx->dtau)) {
-        k.ns = mresp_slots(ctx->nt, c, ctx->dtau, sh.stride, sh.B, pc);
+        k.ns = mresp_slots(ctx->nt, c, ctx->dtau, sh.stride, sh.B, pc, &k.live);
         k.pc = pc;
         k.nt = ctx->nt;
         k.stride = sh.stride;
@@ -1027,7 +1028,7 @@ static hjm_status enqueue_impl(hjm_ctx* ctx, int64_t n_paths, int32_t n_steps, d
             M.k2f = Q.k2p;
             st = ensure_mresp_table(ctx, s);
             if (st != HJM_OK) return st;
-            HJM_CUDA(ctx, launch_path_mixed_resp(M, mresp_ns, false, (const float4*)ctx->mresp.p, ext_dev,
+            HJM_CUDA(ctx, launch_path_mixed_resp(M, mresp_ns, ctx->mresp_key.live, false, (const float4*)ctx->mresp.p, ext_dev,
                                                  (double*)ctx->partials.p, store ? (float*)ctx->estore.p : nullptr,
                                                  s));
             HJM_CUDA(ctx, cudaEventRecord(ctx->resp_used, s));
@@ -1063,7 +1064,7 @@ static hjm_status enqueue_impl(hjm_ctx* ctx, int64_t n_paths, int32_t n_steps, d
         if (mresp_ns) {
             st = ensure_mresp_table(ctx, s);
             if (st != HJM_OK) return st;
-            HJM_CUDA(ctx, launch_path_mixed_resp(M, mresp_ns, mixed_cubic, (const float4*)ctx->mresp.p, ext_dev,
+            HJM_CUDA(ctx, launch_path_mixed_resp(M, mresp_ns, ctx->mresp_key.live, mixed_cubic, (const float4*)ctx->mresp.p, ext_dev,
                                                  (double*)ctx->partials.p, store ? (float*)ctx->estore.p : nullptr,
                                                  s));
             HJM_CUDA(ctx, cudaEventRecord(ctx->resp_used, s));
@@ -1426,7 +1427,7 @@ hjm_status hjm_run_adjoint(hjm_ctx* ctx, int64_t n_paths, int32_t n_steps, doubl
     } else if (adj_ns) {
         st = ensure_mresp_table(ctx, s);
         if (st != HJM_OK) return st;
-        HJM_CUDA(ctx, launch_adjoint_resp(A, adj_ns, (const float4*)ctx->mresp.p, (double*)ctx->partials.p, s));
+        HJM_CUDA(ctx, launch_adjoint_resp(A, adj_ns, ctx->mresp_key.live, (const float4*)ctx->mresp.p, (double*)ctx->partials.p, s));
         HJM_CUDA(ctx, cudaEventRecord(ctx->resp_used, s));
     } else {
         HJM_CUDA(ctx, launch_adjoint(nt, A, use_poly_path(ctx), (double*)ctx->partials.p,

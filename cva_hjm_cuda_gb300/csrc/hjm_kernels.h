@@ -96,14 +96,19 @@ void pack_mixed_params(int nt, const PathParams<float>& P, MixedParams& M);
 // kernel with the N-projected loadings aS, aU, aW as the coefficients of 1,
 // T, T^2 and k2f = (c + c^2) dtau^2; not for a run whose last date samples
 // the last tenor)
-int mresp_slots(int nt, double c, double dtau, int stride, int n_blocks, bool pc = false);
+// Per block the slots still counting: from block `half` on only the first half
+// of the slots, from block `none` on no slot (mresp_slots counts them).
+struct RespLive {
+    int half, none;
+};
+int mresp_slots(int nt, double c, double dtau, int stride, int n_blocks, bool pc, RespLive* live);
 size_t mresp_table_elems(int stride, int n_blocks, int ns);
 cudaError_t launch_mresp_table(int nt, double c, double dtau, int stride, int n_blocks, int ns, bool pc,
                                float4* table, cudaStream_t s);
 size_t mresp_smem_bytes(int n_blocks);
 // paths per CTA: kCta, as launch_path_mixed's table form (path_cta)
-cudaError_t launch_path_mixed_resp(const MixedParams& M, int ns, bool cub, const float4* table, const double* ext,
-                                   double* partials, float* estore, cudaStream_t s);
+cudaError_t launch_path_mixed_resp(const MixedParams& M, int ns, const RespLive& live, bool cub,
+                                   const float4* table, const double* ext, double* partials, float* estore, cudaStream_t s);
 bool path_tenor_supported(int nt);
 size_t path_smem(int nt, int n_blocks, bool mixed);
 // paths per CTA of the Euler path kernel of a run (one partial-sum row each):
@@ -189,7 +194,7 @@ cudaError_t launch_adjoint(int nt, const AdjParams& A, bool poly, double* partia
 // kept): the mixed response form's forward pass and table (mresp_slots'
 // ns slots), the same partial-sum columns as launch_adjoint
 size_t adjoint_resp_smem(int n_blocks);
-cudaError_t launch_adjoint_resp(const AdjParams& A, int ns, const float4* table, double* partials, cudaStream_t s);
+cudaError_t launch_adjoint_resp(const AdjParams& A, int ns, const RespLive& live, const float4* table, double* partials, cudaStream_t s);
 // the predictor-corrector adjoint (sampled states kept; same partial-sum columns
 // as launch_adjoint, the coefficient columns gather phi_k (M0, M1, M2 + gL g[L]))
 size_t adjoint_pc_smem(int nt, int n_blocks);

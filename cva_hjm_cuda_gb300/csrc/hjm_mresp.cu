@@ -26,6 +26,14 @@
 // this kernel, the others (the 25y and 30y runs: 38 and 44 slots) the
 // convected form.
 //
+// A response that counts needs a lag long enough to cross from the last tenor
+// to the date's, so a slot counts only up to a block well before its date (the
+// 10y swap's eight slots, dates 20 to 13, up to blocks 12, 10, 9, 7, 6, 4, 3
+// and 1 of 19; 52 of 152 slot-blocks).  A block's steps run with all, the
+// first half or none of the slots (RespLive, by the same 2^-30 line): 7.98 ->
+// 7.31 ms at 2M paths on the 10y swap, of which the generator alone is 6.0;
+// all or none: 7.45.
+//
 // The predictor-corrector step runs the same kernel: its parts advance by
 // the same update with the N-projected loadings and (c + c^2) dtau^2, and its
 // remainder, driven at L - 1 and L by the old and the new W, has per old W
@@ -37,6 +45,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 
 #include "hjm_epilogue.cuh"
 #include "hjm_kernels.h"
@@ -46,8 +55,10 @@ namespace hjm {
 namespace {
 
 // CTAs per SM of the response kernel with ns slots: the registers' bound
-// (8 slots in 80 registers, 6 CTAs; 16 spill below 128 registers, 4 CTAs)
-constexpr int mresp_min_ctas(int ns) { return ns <= 8 ? 6 : 4; }
+// (8 slots without spills in 102 registers, 5 CTAs: 7.30 ms at 2M paths on the
+// 10y swap against 7.43 with 6 CTAs of 80 registers and 7.39 with 4; external
+// normals, which wait for memory, keep 6; 16 slots spill below 128 registers)
+constexpr int mresp_min_ctas(int ns, bool ext) { return ns > 8 ? 4 : (ext ? 6 : 5); }
 
 }  // namespace
 
@@ -55,8 +66,9 @@ constexpr int mresp_min_ctas(int ns) { return ns <= 8 ? 6 : 4; }
 // date slots (8 or 16), slot r holding date B - r.  resp: rows b stride + s of
 // NS / 2 float4, each two {kappa G, kappa CG} pairs (mresp_table_kernel).
 template <bool EXT, bool CUB, int NS>
-__global__ void __launch_bounds__(kCta, mresp_min_ctas(NS))
-    path_kernel_mixed_resp(const __grid_constant__ MixedParams M, const float4* __restrict__ resp,
+__global__ void __launch_bounds__(kCta, mresp_min_ctas(NS, EXT))
+    path_kernel_mixed_resp(const __grid_constant__ MixedParams M, const RespLive live,
+                           const float4* __restrict__ resp,
                            const double* __restrict__ ext, double* __restrict__ partials,
                            float* __restrict__ estore)
 {
@@ -103,13 +115,16 @@ __global__ void __launch_bounds__(kCta, mresp_min_ctas(NS))
     const int64_t lpc = active ? lp : 0;
     float q0, q1, q2;
     draw_phi<float, EXT>(ext, gpath, lpc, P.n_paths, min(P.stride, n_last), P.rk0, P.rk1, q0, q1, q2);
-    for (int b = 1; b < B; ++b) {
-        float sS = 0.f, sU = 0.f, sW = 0.f, sX = 0.f;
+    float sS, sU, sW, sX;
+    // the steps of block b with the first LIVE slots' responses
+    auto steps = [&](auto live_c, int b) {
+        constexpr int LIVE = decltype(live_c)::value;
         const float4* row = resp + (size_t)b * P.stride * (NS / 2);
         // unrolled by 5 (a divisor of 50 steps per block; the generator's
-        // draws of five steps in flight): 15.65 ms at 4M paths on the 10y
-        // swap, against 15.77 by 4 and 16.67 by 2; the cubic, 16-slot and
-        // external-normals variants spill beyond 2
+        // draws of five steps in flight): 7.31 ms at 2M paths on the 10y swap,
+        // against 7.40 by 4 and 7.61 by 2; by 10, or with more than three
+        // bodies, the loops outgrow the instruction cache (8.1 to 9.2 ms).
+        // The cubic, 16-slot and external-normals variants spill beyond 2
 #pragma unroll((EXT || CUB || NS > 8) ? 2 : 5)
         for (int s = 0; s < P.stride; ++s) {
             const int n = b * P.stride + s;
@@ -120,7 +135,7 @@ __global__ void __launch_bounds__(kCta, mresp_min_ctas(NS))
             const float2 w2 = make_float2(w, w);
             const float4* rr = row + (size_t)s * (NS / 2);
 #pragma unroll
-            for (int u = 0; u < NS / 2; ++u) {
+            for (int u = 0; u < LIVE / 2; ++u) {
                 const float4 e = __ldg(rr + u);
                 A[2 * u] = __ffma2_rn(make_float2(e.x, e.y), w2, A[2 * u]);
                 A[2 * u + 1] = __ffma2_rn(make_float2(e.z, e.w), w2, A[2 * u + 1]);
@@ -145,6 +160,15 @@ __global__ void __launch_bounds__(kCta, mresp_min_ctas(NS))
             sU += U;
             sW += W;
         }
+    };
+    for (int b = 1; b < B; ++b) {
+        sS = sU = sW = sX = 0.f;
+        if (b < live.half)
+            steps(std::integral_constant<int, NS>(), b);
+        else if (b < live.none)
+            steps(std::integral_constant<int, NS / 2>(), b);
+        else
+            steps(std::integral_constant<int, 0>(), b);
         zS += (double)sS;
         zU += (double)sU;
         zW += (double)sW;
@@ -172,7 +196,7 @@ static void pc_sources(double c, double dtau, double& w0, double& w1, double& w2
     w2 = -c * d2;
 }
 
-int mresp_slots(int nt, double c, double dtau, int stride, int n_blocks, bool pc)
+int mresp_slots(int nt, double c, double dtau, int stride, int n_blocks, bool pc, RespLive* live)
 {
     const int B = n_blocks, L = nt - 1;
     if (nt < 3 || nt > kMaxTenor || B < 1 || B >= nt || stride < 1 || !(c > 0.0 && c < 1.0)) return 0;
@@ -196,6 +220,7 @@ int mresp_slots(int nt, double c, double dtau, int stride, int n_blocks, bool pc
     v[L] = 1.0;
     if (pc) u[L - 1] = 1.0;
     int need = 0;
+    int last[kMaxTenor] = {};  // per slot, the last block that counts
     for (int m = 0; m <= M + (pc ? 1 : 0); ++m) {
         for (int t = 0; t < nt; ++t) {
             cum[t] += v[t];
@@ -203,12 +228,16 @@ int mresp_slots(int nt, double c, double dtau, int stride, int n_blocks, bool pc
         }
         const int l = pc ? m - 1 : m;  // the lag this iteration completes
         if (l >= 0)
-            for (int j = 2; j < B + 1 - need; ++j) {
+            for (int j = 2; j <= B; ++j) {
                 // date j reads lags up to K_j - stride = (j - 1) stride - 1
                 if (l > (j - 1) * stride - 1) continue;
                 const double h = pc ? (hp[j] + w2 * v[j]) / kap : v[j];
                 const double ch = pc ? (chp[j] + w2 * cum[j]) / kap : cum[j];
-                if (std::fabs(h) >= thr || std::fabs(ch) >= thr * (double)(j * stride)) need = B - j + 1;
+                if (std::fabs(h) >= thr || std::fabs(ch) >= thr * (double)(j * stride)) {
+                    const int r = B - j, b = (j * stride - 1 - l) / stride;  // slot r counts in block b
+                    need = std::max(need, r + 1);
+                    last[r] = std::max(last[r], b);
+                }
             }
         if (pc) {
             for (int t = 0; t < nt; ++t) {
@@ -230,7 +259,15 @@ int mresp_slots(int nt, double c, double dtau, int stride, int n_blocks, bool pc
         }
         for (int t = 0; t < nt; ++t) v[t] = vn[t];
     }
-    return need <= 8 ? 8 : (need <= 16 ? 16 : 0);
+    const int ns = need <= 8 ? 8 : (need <= 16 ? 16 : 0);
+    if (live) {
+        live->half = live->none = 1;
+        for (int r = 0; r < ns; ++r) {
+            if (r >= ns / 2) live->half = std::max(live->half, last[r] + 1);
+            live->none = std::max(live->none, last[r] + 1);
+        }
+    }
+    return ns;
 }
 
 size_t mresp_table_elems(int stride, int n_blocks, int ns) { return (size_t)n_blocks * stride * (ns / 2); }
@@ -333,7 +370,7 @@ cudaError_t launch_mresp_table(int nt, double c, double dtau, int stride, int n_
 namespace {
 
 template <bool EXT, bool CUB>
-cudaError_t launch_mresp_t(const MixedParams& M, int ns, const float4* table, const double* ext, double* partials,
+cudaError_t launch_mresp_t(const MixedParams& M, int ns, const RespLive& live, const float4* table, const double* ext, double* partials,
                            float* estore, cudaStream_t s)
 {
     auto k = ns == 8 ? path_kernel_mixed_resp<EXT, CUB, 8> : path_kernel_mixed_resp<EXT, CUB, 16>;
@@ -341,21 +378,21 @@ cudaError_t launch_mresp_t(const MixedParams& M, int ns, const float4* table, co
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     const int64_t grid = (M.P.n_paths + kCta - 1) / kCta;
-    k<<<(unsigned)grid, kCta, smem, s>>>(M, table, ext, partials, estore);
+    k<<<(unsigned)grid, kCta, smem, s>>>(M, live, table, ext, partials, estore);
     return cudaGetLastError();
 }
 
 }  // namespace
 
-cudaError_t launch_path_mixed_resp(const MixedParams& M, int ns, bool cub, const float4* table, const double* ext,
-                                   double* partials, float* estore, cudaStream_t s)
+cudaError_t launch_path_mixed_resp(const MixedParams& M, int ns, const RespLive& live, bool cub,
+                                   const float4* table, const double* ext, double* partials, float* estore, cudaStream_t s)
 {
     if (ns != 8 && ns != 16) return cudaErrorInvalidValue;
     if (M.P.n_blocks < 1 || M.P.n_blocks >= kMaxTenor || M.P.stride < 1) return cudaErrorInvalidValue;
-    if (ext) return cub ? launch_mresp_t<true, true>(M, ns, table, ext, partials, estore, s)
-                        : launch_mresp_t<true, false>(M, ns, table, ext, partials, estore, s);
-    return cub ? launch_mresp_t<false, true>(M, ns, table, ext, partials, estore, s)
-               : launch_mresp_t<false, false>(M, ns, table, ext, partials, estore, s);
+    if (ext) return cub ? launch_mresp_t<true, true>(M, ns, live, table, ext, partials, estore, s)
+                        : launch_mresp_t<true, false>(M, ns, live, table, ext, partials, estore, s);
+    return cub ? launch_mresp_t<false, true>(M, ns, live, table, ext, partials, estore, s)
+               : launch_mresp_t<false, false>(M, ns, live, table, ext, partials, estore, s);
 }
 
 }  // namespace hjm

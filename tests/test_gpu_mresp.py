@@ -92,6 +92,23 @@ def test_mixed_response_external_normals_equal_generator(engine):
     assert v.cva == w.cva
 
 
+@pytest.mark.parametrize("dt,n_periods,n_tenor", [(0.02, 20, 51), (0.05, 22, 51), (0.01, 17, 51), (0.01, 12, 51),
+                                                  (0.01, 20, 61), (0.25, 12, 51)])
+def test_mixed_response_live_slots(engine, dt, n_periods, n_tenor):
+    """The blocks in which all, the first half or none of the slots still count
+    lie elsewhere for each of these runs (blocks of 50, 25, 10 and 2 steps; 8
+    and 16 slots; runs that no response reaches).  A response left out is below
+    2^-30 of the remainder's source, 1e-6 of it over 1,000 steps, and the
+    source is at most 2.5e-3 of W: FORM_TOL holds as for the others."""
+    engine.set_market(Market(n_tenor=n_tenor))
+    engine.set_swap(Swap(n_tenor=n_tenor, n_periods=n_periods))
+    cfg = RunConfig(n_paths=2_001, n_steps=round(n_periods * 0.5 / dt), dt=dt, seed=6)
+    (vr, xr, fr), (vc, xc, fc) = _both_forms(engine, cfg, pfe=False)
+    assert (fr, fc) == ("response", "convect")
+    assert np.max(np.abs(xr - xc)) <= FORM_TOL * np.max(np.abs(xc))
+    assert abs(vr.cva - vc.cva) <= FORM_TOL * vc.cva
+
+
 @pytest.mark.parametrize("n_steps", [50, 100, 150])
 def test_mixed_response_shortest_runs(engine, n_steps):
     """One to three dates (one date: no evolution; the look-ahead draw stays
