@@ -713,292 +713,299 @@ cudaError_t launch_adjoint_pc(int nt, const PcParams<float>& Q, bool poly, doubl
 
 // ---------------------------------------------------------------------------
 // The adjoint in the response form (Euler step, quadratic factors, the sampled
-// states kept: checkpoint_every = 0).  The forward pass is the mixed
-// valuation's response form (path_kernel_mixed_resp, hjm_mresp.cu: the parts
-// S, U, W as FP32 scalars, the remainder as FP32 impulse-response sums in NS
-// date slots, the same operations in the same order, so the path's cash
-// flows are the valuation's); it keeps each date's sampled forward and
-// discount factor.  The reverse sweep needs the per-tenor adjoint only for its
-// last tenor, the remainder's coupling to W in the moment recursion
-// (adjoint_kernel above): the adjoint of hc after step n at the last tenor is
-//     g_n[L] = sum_j xbar_j G_j(n_j - n) + abar_j CG_j(n_j - n),
-// G_j(m) = (A^m e_L)[j], CG_j its running sum, over the dates j still ahead
-// of step n -- the forward table's own entries, so with the slot dates' seeds
-// {xbar_j, abar_j} in registers the sweep's kappa g_n[L] is one packed FMA
-// per slot (table row n) instead of the transposed convection of every tenor.
-// Dates whose responses never count (no slot) contribute below 2^-30 of
-// kappa per seed, as in the valuation.
-// Shared memory: the cash flows (then the exposures, one row up) share their
-// region with the sweep's coefficient sums, which start after the seeds have
-// read the exposures (17.1 KB per CTA at 20 dates: 12 CTAs per SM, as the
-// registers allow, instead of 10 with separate regions).
+// states kept: checkpoint_every = 0), in one pass over the steps.  The forward
+// values are the mixed valuation's response form (path_kernel_mixed_resp,
+// hjm_mresp.cu: the parts S, U, W as FP32 scalars, the remainder as FP32
+// impulse-response sums in NS date slots, the same operations in the same
+// order, so the path's cash flows are the valuation's).
+//
+// A date's sampled forward x_i and discount sum a_i are linear in the loadings
+// a_kd of factor k on T^d, so their derivatives run along with the path
+// instead of a reverse sweep that draws every normal a second time.  With
+//     r0 = sum phi_k,  r1 = sum r0,  r2 = sum r1,  r3 = sum r2
+// (each step adds the values before it) and t the date's tenor,
+//     dx/da_k0 = r0
+//     dx/da_k1 = t r0 + k1 r1                                (k1 = c dtau)
+//     dx/da_k2 = t^2 r0 + (2 k1 t + k2) r1 + 2 k1^2 r2 + Y_kx   (k2 = c dtau^2)
+// and the discount sum's are the same with r0 + r1, r1 + r2, r2 + r3 and Y_ky
+// in place of r0, r1, r2 and Y_kx: the parts' update rules with a unit
+// loading.  Y_k = sum_n {kappa G_j, kappa CG_j}(n) r0(n) is the remainder's
+// response to W = r0: the table row and the slots of A, once per factor.
+// The twelve sums of a date go to memory (a part of sens per CTA, rewritten
+// tile by tile, 71 MB for 20 dates: it stays in the second-level cache) until
+// the seeds {xbar_i, abar_i}, which need the exposures of the whole path,
+// weigh them.
+//
+// Bounds: the generator (115 of ~165 issue cycles per 32 path-steps), then the
+// packed FMAs of Y.  10y swap, 1M paths: 8.35 ms -> 5.75 ms against the
+// two-pass form; 12y (16 slots), 512k paths: 6.37 -> 4.83 ms; 5,000 paths: 0.58 ->
+// 0.38 ms.  Eight CTAs per SM with the widest loop unrolled by 2: by 5 its
+// three bodies outgrow the instruction cache (6.15 ms); seven CTAs leave one
+// scheduler a warp more (6.69), six take 5.85.  Slots dropped by quarters
+// instead of halves: 5.77 ms.
 struct AdjRespLayout {
-    size_t cf, cb, xs, ds, red, total;
+    size_t cf, xs, ds, red, total;
 };
 
 __host__ __device__ inline AdjRespLayout adj_resp_layout(int B, int R)
 {
     AdjRespLayout L;
     const size_t rows = (size_t)B + 1;
-    const size_t cf = (rows + 1) * kAdjCta * 4, cb = (size_t)9 * kAdjCta * 8;
-    L.cf = L.cb = 0;
-    L.xs = align128(cf > cb ? cf : cb);
+    L.cf = 0;
+    L.xs = align128((rows + 1) * kAdjCta * 4);
     L.ds = align128(L.xs + rows * kAdjCta * 4);
     L.red = align128(L.ds + rows * kAdjCta * 4);
     L.total = align128(L.red + (size_t)(kAdjCta / 32) * R * 8);
     return L;
 }
 
-// CTAs per SM the launch bounds ask for (8 slots: at 11 the compiler keeps
-// 80 registers without spills, so 12 CTAs are resident, as the shared
-// memory allows; asked for 12 it spills; 16 slots in 128 registers, 8)
-constexpr int adj_resp_min_ctas(int ns) { return ns <= 8 ? 11 : 8; }
+// CTAs per SM: four warps per scheduler with 8 slots (128 registers), two with
+// 16 (255 registers; five CTAs spill, 6.8 ms at 512k paths of the 12y swap)
+constexpr int adj_resp_ctas(int ns) { return ns <= 8 ? 8 : 4; }
 
 template <int NS>
-__global__ void __launch_bounds__(kAdjCta, adj_resp_min_ctas(NS))
+__global__ void __launch_bounds__(kAdjCta, adj_resp_ctas(NS))
     adjoint_kernel_resp(const __grid_constant__ MixedParams M, const RespLive live,
-                        const float4* __restrict__ resp,
-                        double* __restrict__ partials)
+                        const float4* __restrict__ resp, float4* __restrict__ sens, double* __restrict__ partials,
+                        int64_t n_tiles)
 {
     constexpr int C = kAdjCta;
     const PathParams<float>& P = M.P;
     extern __shared__ __align__(128) unsigned char smem[];
     const int tid = threadIdx.x;
+    const int warp = tid >> 5, lane = tid & 31;
     const int B = P.n_blocks;
     const int R = 3 * B + 12;
     const AdjRespLayout Ly = adj_resp_layout(B, R);
     float* cf_s = reinterpret_cast<float*>(smem + Ly.cf);  // [B+2][C]: cash flows, then exposures one row up
+    float* e_s = cf_s + C;
     float* xs_s = reinterpret_cast<float*>(smem + Ly.xs);  // [B+1][C]: x_i, then xbar_i
     float* ds_s = reinterpret_cast<float*>(smem + Ly.ds);  // [B+1][C]: D_i, then abar_i
-    double* cb_s = reinterpret_cast<double*>(smem + Ly.cb);  // [9][C], the sweep's (over cf_s)
-    double* red_s = reinterpret_cast<double*>(smem + Ly.red);
-
-    const int64_t lp = (int64_t)blockIdx.x * C + tid;
-    const bool active = lp < P.n_paths;
-    const uint64_t gpath = P.path_offset + (uint64_t)lp;
+    double* red_s = reinterpret_cast<double*>(smem + Ly.red);  // [warp][R]
+    float4* sens_p = sens + (size_t)blockIdx.x * (B - 1) * kFactors * C + tid;  // [date - 2][factor][C]
     const int stride = P.stride;
-    const int n_steps = B * stride;
+    const int n_last = B * stride - 1;
 
-    // ---------------------------------------------------------------- forward
-    float2 A[NS];  // {hc at date j's tenor, its running sum}, slot B - j
+    for (int64_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+        const int64_t lp = tile * C + tid;
+        const bool active = lp < P.n_paths;
+        const uint64_t gpath = P.path_offset + (uint64_t)lp;
+
+        float2 A[NS];            // {hc at date j's tenor, its running sum}, slot B - j
+        float2 Y[kFactors][NS];  // the same per unit of factor k's loading of T^2
 #pragma unroll
-    for (int r = 0; r < NS; ++r) A[r] = make_float2(0.f, 0.f);
-    float S = 0.f, U = 0.f, W = 0.f;
-    double zS = 0.0, zU = 0.0, zW = 0.0;
-    auto price = [&](int i, float2 rc) {
-        const float ti = P.tau[i];
-        const float pv = fmaf(ti, fmaf(ti, W, U), S);
-        const double xv = P.psamp[i] + (double)(rc.x + pv);
-        const double td = (double)ti;
-        const double a = P.psum[i] + (double)rc.y + fma(td, fma(td, zW, zU), zS);
-        const float D = expf((float)(-a * P.dt));
-        const float mm = (float)P.m;
-        const float L = mm * expm1f((float)xv / mm);
-        cf_s[i * C + tid] = D * ((float)P.payA[i] * L - (float)P.payB[i]);
-        xs_s[i * C + tid] = (float)xv;
-        ds_s[i * C + tid] = D;
-    };
-    price(1, make_float2(0.f, 0.f));
-    const int n_last = n_steps - 1;
-    float q0, q1, q2;
-    draw_phi<float, false>(nullptr, gpath, lp, P.n_paths, min(stride, n_last), P.rk0, P.rk1, q0, q1, q2);
-    float sS, sU, sW;
-    auto steps = [&](auto live_c, int b) {  // (as path_kernel_mixed_resp's)
-        constexpr int LIVE = decltype(live_c)::value;
-        const float4* row = resp + (size_t)b * stride * (NS / 2);
-#pragma unroll 5  // (a divisor of 50 steps per block: 8.66 ms against 8.77 by 2 at 1M paths)
-        for (int s = 0; s < stride; ++s) {
-            const int n = b * stride + s;
-            const float phi0 = q0, phi1 = q1, phi2 = q2;
-            draw_phi<float, false>(nullptr, gpath, lp, P.n_paths, min(n + 1, n_last), P.rk0, P.rk1, q0, q1, q2);
-            const float2 w2 = make_float2(W, W);
-            const float4* rr = row + (size_t)s * (NS / 2);
+        for (int r = 0; r < NS; ++r) {
+            A[r] = make_float2(0.f, 0.f);
 #pragma unroll
-            for (int u = 0; u < LIVE / 2; ++u) {
-                const float4 e = __ldg(rr + u);
-                A[2 * u] = __ffma2_rn(make_float2(e.x, e.y), w2, A[2 * u]);
-                A[2 * u + 1] = __ffma2_rn(make_float2(e.z, e.w), w2, A[2 * u + 1]);
+            for (int k = 0; k < kFactors; ++k) Y[k][r] = make_float2(0.f, 0.f);
+        }
+        float r0[kFactors] = {}, r1[kFactors] = {}, r2[kFactors] = {}, r3[kFactors] = {};
+        float S = 0.f, U = 0.f, W = 0.f;
+        double zS = 0.0, zU = 0.0, zW = 0.0;
+        auto price = [&](int i, float2 rc) {
+            const float ti = P.tau[i];
+            const float pv = fmaf(ti, fmaf(ti, W, U), S);
+            const double xv = P.psamp[i] + (double)(rc.x + pv);
+            const double td = (double)ti;
+            const double a = P.psum[i] + (double)rc.y + fma(td, fma(td, zW, zU), zS);
+            const float D = expf((float)(-a * P.dt));
+            const float mm = (float)P.m;
+            const float L = mm * expm1f((float)xv / mm);
+            cf_s[i * C + tid] = D * ((float)P.payA[i] * L - (float)P.payB[i]);
+            xs_s[i * C + tid] = (float)xv;
+            ds_s[i * C + tid] = D;
+        };
+        price(1, make_float2(0.f, 0.f));
+        float q0, q1, q2;
+        draw_phi<float, false>(nullptr, gpath, lp, P.n_paths, min(stride, n_last), P.rk0, P.rk1, q0, q1, q2);
+        float sS, sU, sW;
+        auto steps = [&](auto live_c, int b) {  // (the values as path_kernel_mixed_resp's)
+            constexpr int LIVE = decltype(live_c)::value;
+            const float4* row = resp + (size_t)b * stride * (NS / 2);
+#pragma unroll(NS == 8 && LIVE == NS ? 2 : 5)
+            for (int s = 0; s < stride; ++s) {
+                const int n = b * stride + s;
+                const float phi0 = q0, phi1 = q1, phi2 = q2;
+                draw_phi<float, false>(nullptr, gpath, lp, P.n_paths, min(n + 1, n_last), P.rk0, P.rk1, q0, q1, q2);
+                const float2 w2 = make_float2(W, W);
+                const float4* rr = row + (size_t)s * (NS / 2);
+#pragma unroll
+                for (int u = 0; u < LIVE / 2; ++u) {
+                    const float4 e = __ldg(rr + u);
+                    const float2 e0 = make_float2(e.x, e.y), e1 = make_float2(e.z, e.w);
+                    A[2 * u] = __ffma2_rn(e0, w2, A[2 * u]);
+                    A[2 * u + 1] = __ffma2_rn(e1, w2, A[2 * u + 1]);
+#pragma unroll
+                    for (int k = 0; k < kFactors; ++k) {
+                        const float2 p2 = make_float2(r0[k], r0[k]);
+                        Y[k][2 * u] = __ffma2_rn(e0, p2, Y[k][2 * u]);
+                        Y[k][2 * u + 1] = __ffma2_rn(e1, p2, Y[k][2 * u + 1]);
+                    }
+                }
+                float Sn = fmaf(M.svcf[0][0], phi0, fmaf(M.k2f, W, fmaf(M.k1f, U, S)));
+                Sn = fmaf(M.svcf[2][0], phi2, fmaf(M.svcf[1][0], phi1, Sn));
+                float Un = fmaf(M.svcf[1][1], phi1, fmaf(M.svcf[0][1], phi0, fmaf(2.0f * M.k1f, W, U)));
+                Un = fmaf(M.svcf[2][1], phi2, Un);
+                const float Wn = fmaf(M.svcf[2][2], phi2, fmaf(M.svcf[1][2], phi1, fmaf(M.svcf[0][2], phi0, W)));
+                S = Sn;
+                U = Un;
+                W = Wn;
+                sS += S;
+                sU += U;
+                sW += W;
+                const float ph[kFactors] = {phi0, phi1, phi2};
+#pragma unroll
+                for (int k = 0; k < kFactors; ++k) {
+                    r3[k] += r2[k];
+                    r2[k] += r1[k];
+                    r1[k] += r0[k];
+                    r0[k] += ph[k];
+                }
             }
-            float Sn = fmaf(M.svcf[0][0], phi0, fmaf(M.k2f, W, fmaf(M.k1f, U, S)));
-            Sn = fmaf(M.svcf[2][0], phi2, fmaf(M.svcf[1][0], phi1, Sn));
-            float Un = fmaf(M.svcf[1][1], phi1, fmaf(M.svcf[0][1], phi0, fmaf(2.0f * M.k1f, W, U)));
-            Un = fmaf(M.svcf[2][1], phi2, Un);
-            const float Wn = fmaf(M.svcf[2][2], phi2, fmaf(M.svcf[1][2], phi1, fmaf(M.svcf[0][2], phi0, W)));
-            S = Sn;
-            U = Un;
-            W = Wn;
-            sS += S;
-            sU += U;
-            sW += W;
-        }
-    };
-    for (int b = 1; b < B; ++b) {
-        sS = sU = sW = 0.f;
-        if (b < live.half)
-            steps(std::integral_constant<int, NS>(), b);
-        else if (b < live.none)
-            steps(std::integral_constant<int, NS / 2>(), b);
-        else
-            steps(std::integral_constant<int, 0>(), b);
-        zS += (double)sS;
-        zU += (double)sU;
-        zW += (double)sW;
-        const int r = B - (b + 1);
-        price(b + 1, r < NS ? select_reg<NS, float2>(A, r) : make_float2(0.f, 0.f));
-    }
-
-    // exposures, the path's CVA contribution, the CTA's EE and CVA partial sums
-    float* e_s = cf_s + C;
-    double v = 0.0, cva_c = 0.0;
-    e_s[B * C + tid] = 0.f;
-    for (int j = B - 1; j >= 0; --j) {
-        v += (double)cf_s[(j + 1) * C + tid];
-        double e = (v > 0.0) ? v : 0.0;
-        if (!active) e = 0.0;
-        e_s[j * C + tid] = (float)e;
-        cva_c = fma(P.cvaw[j], e, cva_c);
-    }
-    __syncthreads();
-    const int warp = tid >> 5, lane = tid & 31;
-    for (int j = warp; j <= B; j += C / 32) {
-        double sum = 0.0;
+        };
+        for (int b = 1; b < B; ++b) {
+            sS = sU = sW = 0.f;
+            if (b < live.half)
+                steps(std::integral_constant<int, NS>(), b);
+            else if (b < live.none)
+                steps(std::integral_constant<int, NS / 2>(), b);
+            else
+                steps(std::integral_constant<int, 0>(), b);
+            zS += (double)sS;
+            zU += (double)sU;
+            zW += (double)sW;
+            const int r = B - (b + 1);
+            price(b + 1, r < NS ? select_reg<NS, float2>(A, r) : make_float2(0.f, 0.f));
 #pragma unroll
-        for (int q = 0; q < C / 32; ++q) sum += (double)e_s[j * C + lane + 32 * q];
-        sum = warp_sum(sum);
-        if (lane == 0) partials[(size_t)blockIdx.x * R + j] = sum;
-    }
-    {
-        const double s1 = warp_sum(cva_c), s2 = warp_sum(cva_c * cva_c);
-        if (lane == 0) {
-            red_s[warp] = s1;
-            red_s[C / 32 + warp] = s2;
+            for (int k = 0; k < kFactors; ++k)
+                sens_p[((size_t)(b - 1) * kFactors + k) * C] = make_float4(r0[k], r1[k], r2[k], r3[k]);
         }
-    }
-    __syncthreads();
-    if (tid == 0) {
-        double s1 = 0.0, s2 = 0.0;
-        for (int w = 0; w < C / 32; ++w) {
-            s1 += red_s[w];
-            s2 += red_s[C / 32 + w];
-        }
-        partials[(size_t)blockIdx.x * R + B + 1] = s1;
-        partials[(size_t)blockIdx.x * R + B + 2] = s2;
-    }
-    __syncthreads();  // (red_s is reused by the final reduction)
 
-    // per-date seeds from cfbar_i = sum_{j<i} w_j [E_j > 0]
-    {
+        // exposures, the path's CVA contribution, the tile's EE and CVA partial sums
+        double v = 0.0, cva_c = 0.0;
+        e_s[B * C + tid] = 0.f;
+        for (int j = B - 1; j >= 0; --j) {
+            v += (double)cf_s[(j + 1) * C + tid];
+            double e = (v > 0.0) ? v : 0.0;
+            if (!active) e = 0.0;
+            e_s[j * C + tid] = (float)e;
+            cva_c = fma(P.cvaw[j], e, cva_c);
+        }
+        __syncthreads();
+        double* out = partials + (size_t)tile * R;
+        for (int j = warp; j <= B; j += C / 32) {
+            double sum = 0.0;
+#pragma unroll
+            for (int q = 0; q < C / 32; ++q) sum += (double)e_s[j * C + lane + 32 * q];
+            sum = warp_sum(sum);
+            if (lane == 0) out[j] = sum;
+        }
+        {
+            const double s1 = warp_sum(cva_c), s2 = warp_sum(cva_c * cva_c);
+            if (lane == 0) {
+                red_s[warp * R + B + 1] = s1;
+                red_s[warp * R + B + 2] = s2;
+            }
+        }
+
+        // per-date seeds from cfbar_i = sum_{j<i} w_j [E_j > 0], and the
+        // coefficients' sums in FP32 pairs (hi + lo)
+        float hi[3 * kFactors] = {}, lo[3 * kFactors] = {};
+        auto add = [&](int q, float val) {
+            const float t = hi[q] + val, z = t - hi[q];
+            lo[q] += (hi[q] - (t - z)) + (val - z);
+            hi[q] = t;
+        };
         float cfbar = 0.f;
         for (int i = 1; i <= B; ++i) {
             const int j = i - 1;
             if (e_s[j * C + tid] > 0.f) cfbar += (float)P.cvaw[j];
             if (!active) cfbar = 0.f;
-            float xbar, abar;
-            date_seeds(P, i, (double)xs_s[i * C + tid], ds_s[i * C + tid], cfbar, xbar, abar);
-            xs_s[i * C + tid] = xbar;
-            ds_s[i * C + tid] = abar;
-        }
-    }
-
-    // ---------------------------------------------------------------- reverse
-    __syncthreads();  // (cb_s overlays the exposures that the seeds just read)
-    for (int q = 0; q < 9; ++q) cb_s[q * C + tid] = 0.0;
-    float2 sd[NS];  // {xbar_j, abar_j} of slot r's date j = B - r once the sweep reaches it
+            float xb, ab;
+            date_seeds(P, i, (double)xs_s[i * C + tid], ds_s[i * C + tid], cfbar, xb, ab);
+            xs_s[i * C + tid] = xb;
+            ds_s[i * C + tid] = ab;
+            if (i == 1) continue;
+            const float ti = P.tau[i];
+            const float t2 = ti * ti, t1 = fmaf(2.f * M.k1f, ti, M.k2f), t0 = 2.f * M.k1f * M.k1f;
 #pragma unroll
-    for (int r = 0; r < NS; ++r) sd[r] = make_float2(0.f, 0.f);
-    float M0 = 0.f, M1 = 0.f, M2 = 0.f, I0 = 0.f, I1 = 0.f, I2 = 0.f;
-    const float dtau = (float)(1.0 / P.m);
-    const float k1 = P.c * dtau, k2 = P.c * dtau * dtau;
-    float r0, r1, r2;
-    draw_phi<float, false>(nullptr, gpath, lp, P.n_paths, n_steps - 1, P.rk0, P.rk1, r0, r1, r2);
-    for (int i = B; i >= 2; --i) {
-        {
-            const float xb = xs_s[i * C + tid], ab = ds_s[i * C + tid];
-            const int rs = B - i;
-#pragma unroll
-            for (int r = 0; r < NS; ++r)
-                if (r == rs) sd[r] = make_float2(xb, ab);
-            const float ti = dtau * (float)i;
-            I0 += ab;
-            I1 = fmaf(ab, ti, I1);
-            I2 = fmaf(ab, ti * ti, I2);
-            M0 += xb;
-            M1 = fmaf(xb, ti, M1);
-            M2 = fmaf(xb, ti * ti, M2);
-        }
-        float cbb[9];
-#pragma unroll
-        for (int q = 0; q < 9; ++q) cbb[q] = 0.f;
-#pragma unroll 2
-        for (int n = i * stride - 1; n >= (i - 1) * stride; --n) {
-            M0 += I0;
-            M1 += I1;
-            M2 += I2;
-            const float phi0 = r0, phi1 = r1, phi2 = r2;
-            draw_phi<float, false>(nullptr, gpath, lp, P.n_paths, max(n - 1, stride), P.rk0, P.rk1, r0, r1, r2);
-            cbb[0] = fmaf(phi0, M0, cbb[0]);
-            cbb[1] = fmaf(phi0, M1, cbb[1]);
-            cbb[2] = fmaf(phi0, M2, cbb[2]);
-            cbb[3] = fmaf(phi1, M0, cbb[3]);
-            cbb[4] = fmaf(phi1, M1, cbb[4]);
-            cbb[5] = fmaf(phi1, M2, cbb[5]);
-            cbb[6] = fmaf(phi2, M0, cbb[6]);
-            cbb[7] = fmaf(phi2, M1, cbb[7]);
-            cbb[8] = fmaf(phi2, M2, cbb[8]);
-            // kappa g_n[L] from the slot dates' seeds and table row n
-            float2 kg = make_float2(0.f, 0.f);
-            const float4* rr = resp + (size_t)n * (NS / 2);
-#pragma unroll
-            for (int u = 0; u < NS / 2; ++u) {
-                const float4 e = __ldg(rr + u);
-                kg = __ffma2_rn(make_float2(e.x, e.y), sd[2 * u], kg);
-                kg = __ffma2_rn(make_float2(e.z, e.w), sd[2 * u + 1], kg);
+            for (int k = 0; k < kFactors; ++k) {
+                const float4 m = sens_p[((size_t)(i - 2) * kFactors + k) * C];
+                const float v0 = fmaf(xb, m.x, ab * (m.x + m.y));
+                const float v1 = fmaf(xb, m.y, ab * (m.y + m.z));
+                const float v2 = fmaf(xb, m.z, ab * (m.z + m.w));
+                add(3 * k, v0);
+                add(3 * k + 1, fmaf(ti, v0, M.k1f * v1));
+                add(3 * k + 2, fmaf(t2, v0, fmaf(t1, v1, t0 * v2)));
             }
-            M2 = fmaf(k2, M0, fmaf(2.f * k1, M1, M2)) + (kg.x + kg.y);
-            M1 = fmaf(k1, M0, M1);
+        }
+        // the remainder's share of the T^2 loadings
+        {
+            float c2[kFactors] = {};
+#pragma unroll
+            for (int r = 0; r < NS; ++r) {
+                const int j = B - r;
+                if (j >= 2) {
+                    const float xb = xs_s[j * C + tid], ab = ds_s[j * C + tid];
+#pragma unroll
+                    for (int k = 0; k < kFactors; ++k) c2[k] = fmaf(xb, Y[k][r].x, fmaf(ab, Y[k][r].y, c2[k]));
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < kFactors; ++k) add(3 * k + 2, c2[k]);
+        }
+
+        // columns as adjoint_kernel's: [0..B] EE, B+1/B+2 CVA stats, E xbar_i,
+        // E abar_i (i = 1..B), the 9 coefficient columns
+        const int cx = B + 3, ca = 2 * B + 3, cc = 3 * B + 3;
+        for (int i = 1; i <= B; ++i) {
+            const double sx = warp_sum((double)xs_s[i * C + tid]);
+            const double sa = warp_sum((double)ds_s[i * C + tid]);
+            if (lane == 0) {
+                red_s[warp * R + cx + i - 1] = sx;
+                red_s[warp * R + ca + i - 1] = sa;
+            }
         }
 #pragma unroll
-        for (int q = 0; q < 9; ++q) cb_s[q * C + tid] += (double)cbb[q];
-    }
-
-    // ---------------------------------------------------------------- CTA reduction
-    // columns as adjoint_kernel's: [0..B] EE, B+1/B+2 CVA stats, E xbar_i,
-    // E abar_i (i = 1..B), the 9 coefficient columns
-    const int cx = B + 3, ca = 2 * B + 3, cc = 3 * B + 3;
-    double* wred = red_s;  // [warp][R]
-    for (int i = 1; i <= B; ++i) {
-        const double sx_ = warp_sum(active ? (double)xs_s[i * C + tid] : 0.0);
-        const double sa_ = warp_sum(active ? (double)ds_s[i * C + tid] : 0.0);
-        if (lane == 0) {
-            wred[warp * R + cx + i - 1] = sx_;
-            wred[warp * R + ca + i - 1] = sa_;
+        for (int q = 0; q < 3 * kFactors; ++q) {
+            const double sum = warp_sum((double)hi[q] + (double)lo[q]);
+            if (lane == 0) red_s[warp * R + cc + q] = sum;
         }
-    }
-    for (int q = 0; q < 9; ++q) {
-        const double sum = warp_sum(active ? cb_s[q * C + tid] : 0.0);
-        if (lane == 0) wred[warp * R + cc + q] = sum;
-    }
-    __syncthreads();
-    for (int col = cx + tid; col < R; col += C) {
-        double sum = 0.0;
-        for (int w = 0; w < C / 32; ++w) sum += wred[w * R + col];
-        partials[(size_t)blockIdx.x * R + col] = sum;
+        __syncthreads();
+        for (int col = B + 1 + tid; col < R; col += C) {
+            double sum = 0.0;
+            for (int w = 0; w < C / 32; ++w) sum += red_s[w * R + col];
+            out[col] = sum;
+        }
+        __syncthreads();  // (the next tile writes the rows and sums just read)
     }
 }
 
 size_t adjoint_resp_smem(int n_blocks) { return adj_resp_layout(n_blocks, 3 * n_blocks + 12).total; }
 
-cudaError_t launch_adjoint_resp(const AdjParams& A, int ns, const RespLive& live, const float4* table, double* partials, cudaStream_t s)
+int adjoint_resp_grid(int64_t n_paths, int ns, int n_sms)
+{
+    const int64_t tiles = (n_paths + kAdjCta - 1) / kAdjCta, most = (int64_t)n_sms * adj_resp_ctas(ns);
+    return (int)(tiles < most ? tiles : most);
+}
+
+size_t adjoint_resp_sens_bytes(int n_blocks, int grid)
+{
+    return sizeof(float4) * kFactors * kAdjCta * (size_t)(n_blocks - 1) * (size_t)grid;
+}
+
+cudaError_t launch_adjoint_resp(const AdjParams& A, int ns, const RespLive& live, const float4* table, float4* sens,
+                                int grid, double* partials, cudaStream_t s)
 {
     if (ns != 8 && ns != 16) return cudaErrorInvalidValue;
     const int B = A.M.P.n_blocks;
-    if (B < 1 || B >= kMaxTenor || A.M.P.stride < 1) return cudaErrorInvalidValue;
+    if (B < 1 || B >= kMaxTenor || A.M.P.stride < 1 || grid < 1) return cudaErrorInvalidValue;
     auto k = ns == 8 ? adjoint_kernel_resp<8> : adjoint_kernel_resp<16>;
     const size_t smem = adjoint_resp_smem(B);
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    const int64_t grid = (A.M.P.n_paths + kAdjCta - 1) / kAdjCta;
-    k<<<(unsigned)grid, kAdjCta, smem, s>>>(A.M, live, table, partials);
+    const int64_t tiles = (A.M.P.n_paths + kAdjCta - 1) / kAdjCta;
+    k<<<(unsigned)grid, kAdjCta, smem, s>>>(A.M, live, table, sens, partials, tiles);
     return cudaGetLastError();
 }
 

@@ -107,16 +107,16 @@ struct hjm_ctx {
 
     // device buffers
     DevBuf partials, sums, result, estore, sel, hist, ext, ext_raw, wide, scratch, ck_h, ck_a, contract, split, carry,
-        mresp;
+        mresp, sens;
     MemBudget budget;
     hjm_ctx()
     {
         for (DevBuf* b : buffers()) b->budget = &budget;
     }
-    std::array<DevBuf*, 16> buffers()
+    std::array<DevBuf*, 17> buffers()
     {
         return {&partials, &sums, &result, &estore, &sel, &hist, &ext, &ext_raw, &wide, &scratch, &ck_h, &ck_a,
-                &contract, &split, &carry, &mresp};
+                &contract, &split, &carry, &mresp, &sens};
     }
     // the tables in contract and mresp hold the run shapes of their keys;
     // resp_used is recorded after the last kernel that reads one
@@ -1384,7 +1384,7 @@ hjm_status hjm_run_adjoint(hjm_ctx* ctx, int64_t n_paths, int32_t n_steps, doubl
     const int R = adjoint_columns(nt, B);
     // quadratic factors under the Euler step with the sampled states kept:
     // the response form's adjoint where the valuation's response form fits
-    const int adj_ns = (!pc && checkpoint_every == 0 && use_poly_path(ctx) && ctx->remainder != HJM_REMAINDER_CONVECT)
+    int adj_ns = (!pc && checkpoint_every == 0 && use_poly_path(ctx) && ctx->remainder != HJM_REMAINDER_CONVECT)
                            ? mresp_run_slots(ctx, sh, dt)
                            : 0;
     const size_t smem = pc ? adjoint_pc_smem(nt, B)
@@ -1422,12 +1422,24 @@ hjm_status hjm_run_adjoint(hjm_ctx* ctx, int64_t n_paths, int32_t n_steps, doubl
     ctx->n_enqueued++;
     HJM_CUDA(ctx, cudaMemsetAsync(ctx->result.p, 0, sizeof(double) * kResLen, s));
     HJM_CUDA(ctx, cudaEventRecord(ctx->ev[0], s));
+    // the response form's sums at the dates, one part per CTA: fewer CTAs where
+    // the memory does not allow more, the convected form where not even one fits
+    int grid = 0;
+    if (adj_ns) {
+        st = ensure_mresp_table(ctx, s);
+        if (st != HJM_OK) return st;
+        grid = adjoint_resp_grid(n_paths, adj_ns, ctx->n_sms);
+        while (grid > 0 && ctx->sens.ensure(adjoint_resp_sens_bytes(B, grid)) != cudaSuccess) {
+            cudaGetLastError();
+            grid /= 2;
+        }
+        if (grid == 0) adj_ns = 0;
+    }
     if (pc) {
         HJM_CUDA(ctx, launch_adjoint_pc(nt, Qp, use_poly_path(ctx), (double*)ctx->partials.p, s));
     } else if (adj_ns) {
-        st = ensure_mresp_table(ctx, s);
-        if (st != HJM_OK) return st;
-        HJM_CUDA(ctx, launch_adjoint_resp(A, adj_ns, ctx->mresp_key.live, (const float4*)ctx->mresp.p, (double*)ctx->partials.p, s));
+        HJM_CUDA(ctx, launch_adjoint_resp(A, adj_ns, ctx->mresp_key.live, (const float4*)ctx->mresp.p,
+                                          (float4*)ctx->sens.p, grid, (double*)ctx->partials.p, s));
         HJM_CUDA(ctx, cudaEventRecord(ctx->resp_used, s));
     } else {
         HJM_CUDA(ctx, launch_adjoint(nt, A, use_poly_path(ctx), (double*)ctx->partials.p,

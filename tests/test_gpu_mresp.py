@@ -212,3 +212,45 @@ def test_pc_mixed_response_vs_convected_and_oracle(engine):
         assert engine.remainder_form() == "convect"
     finally:
         engine.set_scheme("euler")
+
+
+@pytest.mark.parametrize("dt,n_periods,n_tenor,n_paths", [(0.02, 20, 51, 100_001), (0.01, 24, 51, 45_013), (0.25, 12, 51, 777),
+                                                          (0.01, 1, 51, 100), (0.01, 2, 51, 65), (0.01, 17, 61, 40_000)])
+def test_response_adjoint_shapes(engine, dt, n_periods, n_tenor, n_paths):
+    """The one-pass adjoint where its loops end: more tiles than CTAs and a
+    ragged last tile, 8 and 16 slots, blocks of 2 steps, one and two dates, runs
+    that few or no responses reach; against the convected sweep with the
+    tolerances of the comparison above.  Memory for one CTA's sums only gives
+    the same results bit for bit (each tile is summed by itself)."""
+    from cva_hjm_cuda_gb300.engine import HJMEngine
+    from cva_hjm_cuda_gb300.market import DEFAULT_VOL_COEFFS, nelson_siegel_curve, tenor_grid
+
+    cfg = RunConfig(n_paths=n_paths, n_steps=round(n_periods * 0.5 / dt), dt=dt, seed=17)
+    names = ("dcva_dspot", "dcva_ddrift", "dcva_dvolcoef")
+
+    def run(eng, form):
+        eng.set_market_poly(n_tenor, 0.5, nelson_siegel_curve(tenor_grid(n_tenor, 0.5)), DEFAULT_VOL_COEFFS)
+        eng.set_swap(Swap(n_tenor=n_tenor, n_periods=n_periods))
+        eng.set_remainder_form(form)
+        try:
+            return eng.run_adjoint(cfg, checkpoint_every=0)
+        finally:
+            eng.set_remainder_form("auto")
+
+    a, c = run(engine, "auto"), run(engine, "convect")
+    assert abs(a.cva - c.cva) <= 1e-6 * c.cva
+    for name in names:
+        ga, gc = np.ravel(getattr(a, name)), np.ravel(getattr(c, name))
+        if name == "dcva_dvolcoef":
+            w = np.array([25.0 ** (q % 3) for q in range(9)])
+            ga, gc = ga / w, gc / w
+        np.testing.assert_allclose(ga, gc, rtol=0, atol=1e-4 * np.max(np.abs(gc)), err_msg=name)
+    if n_periods == 20:
+        with HJMEngine(0) as eng:
+            run(eng, "convect")  # (the buffers every form holds)
+            eng.run(RunConfig(n_paths=64, n_steps=cfg.n_steps, dt=dt), "mixed", pfe=False)  # and the table
+            eng.set_memory_limit(eng.memory_in_use() + 3 * 16 * 64 * (n_periods - 1) * 3)
+            b = run(eng, "auto")
+        assert b.cva == a.cva
+        for name in names:
+            np.testing.assert_array_equal(getattr(b, name), getattr(a, name))
