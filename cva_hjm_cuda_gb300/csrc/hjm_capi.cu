@@ -1382,13 +1382,15 @@ hjm_status hjm_run_adjoint(hjm_ctx* ctx, int64_t n_paths, int32_t n_steps, doubl
                     "volatility-coefficient sensitivities need a polynomial market (hjm_set_market_poly)");
     const int nt = ctx->nt, B = sh.B;
     const int R = adjoint_columns(nt, B);
-    // quadratic factors under the Euler step with the sampled states kept:
-    // the response form's adjoint where the valuation's response form fits
-    int adj_ns = (!pc && checkpoint_every == 0 && use_poly_path(ctx) && ctx->remainder != HJM_REMAINDER_CONVECT)
-                           ? mresp_run_slots(ctx, sh, dt)
-                           : 0;
+    // quadratic factors under the Euler step: the one-pass adjoint where the
+    // dates the remainder reaches fit its slots, with the response form's
+    // values, or the convected form's where checkpoints are asked for (which
+    // it then has no use for)
+    int adj_ns = (!pc && use_poly_path(ctx) && ctx->remainder != HJM_REMAINDER_CONVECT) ? mresp_run_slots(ctx, sh, dt)
+                                                                                        : 0;
+    const int conv_nt = checkpoint_every > 0 ? nt : 0;
     const size_t smem = pc ? adjoint_pc_smem(nt, B)
-                           : (adj_ns ? adjoint_resp_smem(B) : adjoint_smem(nt, B, checkpoint_every > 0));
+                           : (adj_ns ? adjoint_resp_smem(B, conv_nt) : adjoint_smem(nt, B, checkpoint_every > 0));
     if (smem > 227 * 1024) return fail(ctx, HJM_ERR_UNSUPPORTED, "adjoint shared memory %zu B exceeds 227 KB", smem);
     HJM_CUDA(ctx, cudaSetDevice(ctx->device));
     const int64_t n_ctas = (n_paths + adjoint_cta() - 1) / adjoint_cta();
@@ -1399,10 +1401,6 @@ hjm_status hjm_run_adjoint(hjm_ctx* ctx, int64_t n_paths, int32_t n_steps, doubl
     HJM_CUDA(ctx, ctx->partials.ensure(sizeof(double) * (size_t)n_ctas * R));
     HJM_CUDA(ctx, ctx->sums.ensure(sizeof(double) * kSumsLen));
     HJM_CUDA(ctx, ctx->result.ensure(sizeof(double) * kResLen));
-    if (K > 0) {
-        HJM_CUDA(ctx, ctx->ck_h.ensure(sizeof(float) * (size_t)S * (nt + 5) * (size_t)ld));
-        HJM_CUDA(ctx, ctx->ck_a.ensure(sizeof(double) * (size_t)S * (size_t)ld));
-    }
     AdjParams A;
     PcParams<float> Qp;
     FinalParams F;
@@ -1422,23 +1420,27 @@ hjm_status hjm_run_adjoint(hjm_ctx* ctx, int64_t n_paths, int32_t n_steps, doubl
     ctx->n_enqueued++;
     HJM_CUDA(ctx, cudaMemsetAsync(ctx->result.p, 0, sizeof(double) * kResLen, s));
     HJM_CUDA(ctx, cudaEventRecord(ctx->ev[0], s));
-    // the response form's sums at the dates, one part per CTA: fewer CTAs where
-    // the memory does not allow more, the convected form where not even one fits
+    // the one-pass form's sums at the dates, one part per CTA: fewer CTAs where
+    // the memory does not allow more, the reverse sweep where not even one fits
     int grid = 0;
     if (adj_ns) {
         st = ensure_mresp_table(ctx, s);
         if (st != HJM_OK) return st;
-        grid = adjoint_resp_grid(n_paths, adj_ns, ctx->n_sms);
+        grid = adjoint_resp_grid(n_paths, adj_ns, conv_nt, ctx->n_sms);
         while (grid > 0 && ctx->sens.ensure(adjoint_resp_sens_bytes(B, grid)) != cudaSuccess) {
             cudaGetLastError();
             grid /= 2;
         }
         if (grid == 0) adj_ns = 0;
     }
+    if (K > 0 && !adj_ns) {
+        HJM_CUDA(ctx, ctx->ck_h.ensure(sizeof(float) * (size_t)S * (nt + 5) * (size_t)ld));
+        HJM_CUDA(ctx, ctx->ck_a.ensure(sizeof(double) * (size_t)S * (size_t)ld));
+    }
     if (pc) {
         HJM_CUDA(ctx, launch_adjoint_pc(nt, Qp, use_poly_path(ctx), (double*)ctx->partials.p, s));
     } else if (adj_ns) {
-        HJM_CUDA(ctx, launch_adjoint_resp(A, adj_ns, ctx->mresp_key.live, (const float4*)ctx->mresp.p,
+        HJM_CUDA(ctx, launch_adjoint_resp(A, adj_ns, conv_nt, ctx->mresp_key.live, (const float4*)ctx->mresp.p,
                                           (float4*)ctx->sens.p, grid, (double*)ctx->partials.p, s));
         HJM_CUDA(ctx, cudaEventRecord(ctx->resp_used, s));
     } else {
@@ -1521,7 +1523,7 @@ hjm_status hjm_run_adjoint(hjm_ctx* ctx, int64_t n_paths, int32_t n_steps, doubl
     r.nt = nt;
     r.precision = HJM_PRECISION_MIXED;
     r.vol_form = use_poly_path(ctx) ? vol_form_code(ctx) : 0;  // a cubic market runs the table step here
-    r.remainder = adj_ns ? 2 : 1;
+    r.remainder = adj_ns && !conv_nt ? 2 : 1;
     r.scheme = ctx->scheme;
     r.ckpt = K;
     r.dt = dt;

@@ -193,12 +193,13 @@ cudaError_t launch_adjoint(int nt, const AdjParams& A, bool poly, double* partia
 // the adjoint in the response form (Euler, quadratic factors, sampled states
 // kept): the mixed response form's forward pass and table (mresp_slots'
 // ns slots), the same partial-sum columns as launch_adjoint
-size_t adjoint_resp_smem(int n_blocks);
+size_t adjoint_resp_smem(int n_blocks, int conv_nt);
 // (paths as a grid of CTAs over the tiles, each with its own part of sens)
-int adjoint_resp_grid(int64_t n_paths, int ns, int n_sms);
+// conv_nt: with the convected form's values on that many tenors, 0: the response form's
+int adjoint_resp_grid(int64_t n_paths, int ns, int conv_nt, int n_sms);
 size_t adjoint_resp_sens_bytes(int n_blocks, int grid);
-cudaError_t launch_adjoint_resp(const AdjParams& A, int ns, const RespLive& live, const float4* table, float4* sens,
-                                int grid, double* partials, cudaStream_t s);
+cudaError_t launch_adjoint_resp(const AdjParams& A, int ns, int conv_nt, const RespLive& live, const float4* table,
+                                float4* sens, int grid, double* partials, cudaStream_t s);
 // the predictor-corrector adjoint (sampled states kept; same partial-sum columns
 // as launch_adjoint, the coefficient columns gather phi_k (M0, M1, M2 + gL g[L]))
 size_t adjoint_pc_smem(int nt, int n_blocks);

@@ -82,6 +82,34 @@ def test_checkpoint_mode_matches_seed_mode(engine):
                                    atol=1e-4 * np.max(np.abs(a.dcva_dvolcoef)))
 
 
+@pytest.mark.parametrize("n_periods,n_tenor,n_paths,k", [(20, 51, 60_001, 16), (24, 51, 41_111, 50), (17, 61, 5_000, 1),
+                                                         (30, 61, 33_000, 32), (2, 51, 63, 32)])
+def test_checkpointed_adjoint_without_sweep(engine, n_periods, n_tenor, n_paths, k):
+    """The one-pass adjoint on the convected values (checkpoints asked for, 8
+    and 16 slots, 51 and 61 tenors, more tiles than CTAs, a ragged last tile)
+    against the convected sweep with and without checkpoints: CVA bit for bit,
+    the sensitivities as two FP32 orderings of the same sums (1e-4 of the
+    group's largest)."""
+    spot = nelson_siegel_curve(tenor_grid(n_tenor, 0.5))
+    engine.set_market_poly(n_tenor, 0.5, spot, DEFAULT_VOL_COEFFS)
+    engine.set_swap(Swap(n_tenor=n_tenor, n_periods=n_periods))
+    cfg = RunConfig(n_paths=n_paths, n_steps=50 * n_periods, seed=3)
+    engine.set_remainder_form("convect")
+    try:
+        sweeps = [engine.run_adjoint(cfg, checkpoint_every=e) for e in (0, k)]
+    finally:
+        engine.set_remainder_form("auto")
+    a = engine.run_adjoint(cfg, checkpoint_every=k)
+    for c in sweeps:
+        assert (a.cva, a.cva_stderr, a.dcva_dhazard) == (c.cva, c.cva_stderr, c.dcva_dhazard)
+        for name in ("dcva_dspot", "dcva_ddrift", "dcva_dvolcoef"):
+            ga, gc = np.ravel(getattr(a, name)), np.ravel(getattr(c, name))
+            if name == "dcva_dvolcoef":  # in units of a volatility change at T = 25y
+                w = np.array([25.0 ** (q % 3) for q in range(9)])
+                ga, gc = ga / w, gc / w
+            np.testing.assert_allclose(ga, gc, rtol=0, atol=1e-4 * np.max(np.abs(gc)), err_msg=name)
+
+
 def _fd_fp64(engine, cfg, spot, coef, hazard, which, idx, h):
     def val(sp, cf, hz):
         _poly(engine, sp, cf)
