@@ -147,7 +147,10 @@ __device__ __forceinline__ void pair_add(float2 (&v)[PairGrid<NT>::H], int i, fl
 template <int NT>
 constexpr int adj_min_ctas() { return NT > 56 ? 4 : 6; }
 
-template <int NT, bool CKPT, bool POLY>
+// WIN: the values of the long convected runs (path_kernel_mixed_conv: POLY,
+// discount sums by LongSums; the curve is stepped whole, which leaves the
+// window's tenors as they are)
+template <int NT, bool CKPT, bool POLY, bool WIN>
 __global__ void __launch_bounds__(kAdjCta, adj_min_ctas<NT>())
     adjoint_kernel(const __grid_constant__ AdjParams A, double* __restrict__ partials, float* __restrict__ ck_h,
                    double* __restrict__ ck_a)
@@ -179,14 +182,26 @@ __global__ void __launch_bounds__(kAdjCta, adj_min_ctas<NT>())
 
     // ---------------------------------------------------------------- forward
     // The same arithmetic as path_kernel_mixed, plus what the sweep needs.
+    static_assert(!WIN || POLY, "the windows are the polynomial form's");
+    constexpr int W1 = conv_window(NT, 0), W2 = conv_window(NT, 1);
     MixedPath<NT, POLY> x;
     x.reset();
+    LongSums<NT, false> z;
+    z.reset();
     for (int i = 0; i < rows; ++i) acc_s[i * kCtaA + tid] = 0.0;
     for (int t = 0; t <= B + 1; ++t) hs_s[t * kCtaA + tid] = 0.f;
 
     auto sample = [&](int i) {
-        const double xv = P.psamp[i] + (double)x.value(P, i);
-        const double a = P.psum[i] + acc_s[i * kCtaA + tid];
+        float value = 0.f;
+        double sum = 0.0;
+        if constexpr (WIN) {
+            if (i > 1) z.template read<1>(x, P, z.start, i, value, sum);
+        } else {
+            value = x.value(P, i);
+            sum = acc_s[i * kCtaA + tid];
+        }
+        const double xv = P.psamp[i] + (double)value;
+        const double a = P.psum[i] + sum;
         const float D = expf((float)(-a * P.dt));
         const float mm = (float)P.m;
         const float L = mm * expm1f((float)xv / mm);
@@ -201,6 +216,12 @@ __global__ void __launch_bounds__(kAdjCta, adj_min_ctas<NT>())
     // part), then S, U, W and the scales g, ig: the recomputation restarts from
     // the forward pass's own state and repeats its arithmetic
     constexpr int kCkRows = NT + 5;
+    // the curve at the window's start
+    auto anchor = [&](const MixedPath<NT, POLY>& y) {
+        return z.start == W2   ? pair_tenor<NT>(y.h, W2)
+               : z.start == W1 ? pair_tenor<NT>(y.h, W1)
+                               : pair_tenor<NT>(y.h, 1);
+    };
     sample(1);
     int ck = 0, ck_next = stride;  // next checkpoint: before step ck_next
     const int n_last = n_steps - 1;
@@ -209,6 +230,10 @@ __global__ void __launch_bounds__(kAdjCta, adj_min_ctas<NT>())
     for (int b = 1; b < B; ++b) {
         BlockSums bs;
         bs.reset();
+        if constexpr (WIN) {
+            const int w = window_start<NT>(M, b);
+            if (w != z.start) z.move(x, P, w);
+        }
         x.begin_block(P, b);
         for (int s = 0; s < stride; ++s) {
             const int n = b * stride + s;
@@ -221,11 +246,19 @@ __global__ void __launch_bounds__(kAdjCta, adj_min_ctas<NT>())
                 // only a segment that holds a date's sampling step (the block's
                 // last step) is ever restarted by the seed pass
                 const bool needed = (b + 1) * stride - 1 < n + K;
+                // (WIN: of the window's start and the parts; the recomputation
+                // adds the date's difference from the start)
                 double part = 0.0;
-                if (needed && s > 0)
-                    block_sums_up<NT, POLY>(x, hs_s, tid, kCtaA, P, bs, inext, [&](int t, float Ht) {
-                        if (t == inext) part = as_f64(Ht);
-                    });
+                if constexpr (WIN) {
+                    part = z.zR + z.parts((double)P.tau[inext]) + as_f64(bs.H1) +
+                           as_f64(bs.poly<false>(P.tau[inext]));
+                } else {
+                    if (needed && s > 0)
+                        block_sums_up<NT, POLY>(x, hs_s, tid, kCtaA, P, bs, inext, [&](int t, float Ht) {
+                            if (t == inext) part = as_f64(Ht);
+                        });
+                    part += acc_s[inext * kCtaA + tid];
+                }
                 if (needed && active) {
 #pragma unroll
                     for (int t = 0; t < NT; ++t) ck_h[((size_t)ck * kCkRows + t) * ld + lp] = pair_tenor<NT>(x.h, t);
@@ -234,21 +267,28 @@ __global__ void __launch_bounds__(kAdjCta, adj_min_ctas<NT>())
                     ck_h[((size_t)ck * kCkRows + NT + 2) * ld + lp] = x.W;
                     ck_h[((size_t)ck * kCkRows + NT + 3) * ld + lp] = x.g;
                     ck_h[((size_t)ck * kCkRows + NT + 4) * ld + lp] = x.ig;
-                    ck_a[(size_t)ck * ld + lp] = acc_s[inext * kCtaA + tid] + part;
+                    ck_a[(size_t)ck * ld + lp] = part;
                 }
                 ++ck;
             }
             const float phi0 = q0, phi1 = q1, phi2 = q2;
             draw_phi<float, false>(nullptr, gpath, lp, P.n_paths, min(n + 1, n_last), P.rk0, P.rk1, q0, q1, q2);
             x.step(M, phi0, phi1, phi2);
-            bs.add(x, phi0, phi1, phi2);
+            if constexpr (WIN)
+                bs.add_at(x, anchor(x));
+            else
+                bs.add(x, phi0, phi1, phi2);
         }
-        block_sums_up<NT, POLY>(x, hs_s, tid, kCtaA, P, bs, B, [&](int t, float Ht) {
-            if (t > b) acc_s[t * kCtaA + tid] += as_f64(Ht);
-        });
+        if constexpr (WIN) {
+            z.fold(bs.H1, bs.sS, bs.sU, bs.sW, 0.f);
+        } else {
+            block_sums_up<NT, POLY>(x, hs_s, tid, kCtaA, P, bs, B, [&](int t, float Ht) {
+                if (t > b) acc_s[t * kCtaA + tid] += as_f64(Ht);
+            });
 #pragma unroll
-        for (int t = 1; t < NT; ++t)
-            if (t <= B + 1) hs_s[t * kCtaA + tid] = x.rem(t);
+            for (int t = 1; t < NT; ++t)
+                if (t <= B + 1) hs_s[t * kCtaA + tid] = x.rem(t);
+        }
         sample(b + 1);
     }
 
@@ -336,9 +376,13 @@ __global__ void __launch_bounds__(kAdjCta, adj_min_ctas<NT>())
                 xr.W = active ? ck_h[(base + NT + 2) * ld + lp] : 0.f;
                 xr.g = active ? ck_h[(base + NT + 3) * ld + lp] : 1.f;
                 xr.ig = active ? ck_h[(base + NT + 4) * ld + lp] : 1.f;
+                if constexpr (WIN) {
+                    z.start = window_start<NT>(M, i - 1);
+                } else {
 #pragma unroll
-                for (int t = 1; t < NT; ++t)
-                    if (t <= B + 1) hs_s[t * kCtaA + tid] = xr.rem(t);
+                    for (int t = 1; t < NT; ++t)
+                        if (t <= B + 1) hs_s[t * kCtaA + tid] = xr.rem(t);
+                }
                 const double a0 = active ? ck_a[(size_t)sg * ld + lp] : 0.0;
                 BlockSums bs;
                 bs.reset();
@@ -348,12 +392,21 @@ __global__ void __launch_bounds__(kAdjCta, adj_min_ctas<NT>())
                     const float phi0 = r0, phi1 = r1, phi2 = r2;
                     draw_phi<float, false>(nullptr, gpath, lp, P.n_paths, min(n + 1, ni), P.rk0, P.rk1, r0, r1, r2);
                     xr.step(M, phi0, phi1, phi2);
-                    bs.add(xr, phi0, phi1, phi2);
+                    if constexpr (WIN)
+                        bs.add_at(xr, anchor(xr));
+                    else
+                        bs.add(xr, phi0, phi1, phi2);
                 }
                 double part = 0.0;
-                block_sums_up<NT, POLY>(xr, hs_s, tid, kCtaA, P, bs, i, [&](int t, float Ht) {
-                    if (t == i) part = as_f64(Ht);
-                });
+                if constexpr (WIN) {
+                    float v;
+                    part = as_f64(bs.H1) + as_f64(z.template climb<1>(xr, P, z.start, i, v)) +
+                           as_f64(bs.poly<false>(P.tau[i]));
+                } else {
+                    block_sums_up<NT, POLY>(xr, hs_s, tid, kCtaA, P, bs, i, [&](int t, float Ht) {
+                        if (t == i) part = as_f64(Ht);
+                    });
+                }
                 const double xv = P.psamp[i] + (double)xr.value(P, i);
                 const double a = P.psum[i] + a0 + part;
                 const float D = expf((float)(-a * P.dt));
@@ -1188,11 +1241,11 @@ int adjoint_columns(int nt, int n_blocks)
 
 int adjoint_cta() { return kAdjCta; }
 
-template <int NT, bool CKPT, bool POLY>
+template <int NT, bool CKPT, bool POLY, bool WIN>
 static cudaError_t launch_adj_t(const AdjParams& A, double* partials, float* ck_h, double* ck_a, cudaStream_t s)
 {
     const size_t smem = adjoint_smem(NT, A.M.P.n_blocks, CKPT);
-    auto k = adjoint_kernel<NT, CKPT, POLY>;
+    auto k = adjoint_kernel<NT, CKPT, POLY, WIN>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     const int64_t grid = (A.M.P.n_paths + kAdjCta - 1) / kAdjCta;
@@ -1205,10 +1258,13 @@ static cudaError_t launch_adj_nt(const AdjParams& A, bool poly, double* partials
                                  cudaStream_t s)
 {
     const bool ck = A.ckpt_every > 0;
-    if (poly) return ck ? launch_adj_t<NT, true, true>(A, partials, ck_h, ck_a, s)
-                        : launch_adj_t<NT, false, true>(A, partials, ck_h, ck_a, s);
-    return ck ? launch_adj_t<NT, true, false>(A, partials, ck_h, ck_a, s)
-              : launch_adj_t<NT, false, false>(A, partials, ck_h, ck_a, s);
+    if (mixed_windowed(NT, A.M.P.n_blocks, poly))
+        return ck ? launch_adj_t<NT, true, true, true>(A, partials, ck_h, ck_a, s)
+                  : launch_adj_t<NT, false, true, true>(A, partials, ck_h, ck_a, s);
+    if (poly) return ck ? launch_adj_t<NT, true, true, false>(A, partials, ck_h, ck_a, s)
+                        : launch_adj_t<NT, false, true, false>(A, partials, ck_h, ck_a, s);
+    return ck ? launch_adj_t<NT, true, false, false>(A, partials, ck_h, ck_a, s)
+              : launch_adj_t<NT, false, false, false>(A, partials, ck_h, ck_a, s);
 }
 
 cudaError_t launch_adjoint(int nt, const AdjParams& A, bool poly, double* partials, float* ck_h, double* ck_a,

@@ -1070,6 +1070,8 @@ static hjm_status enqueue_impl(hjm_ctx* ctx, int64_t n_paths, int32_t n_steps, d
             HJM_CUDA(ctx, cudaEventRecord(ctx->resp_used, s));
             resp = true;
         } else {
+            if (use_response_form(ctx) && (use_poly_path(ctx) || mixed_cubic))
+                std::copy(ctx->mresp_key.live.win, ctx->mresp_key.live.win + 2, M.win);
             HJM_CUDA(ctx, launch_path_mixed(ctx->nt, M, use_poly_path(ctx), ext_dev, (double*)ctx->partials.p,
                                             store ? (float*)ctx->estore.p : nullptr, s, mixed_cubic));
         }
@@ -1444,6 +1446,8 @@ hjm_status hjm_run_adjoint(hjm_ctx* ctx, int64_t n_paths, int32_t n_steps, doubl
                                           (float4*)ctx->sens.p, grid, (double*)ctx->partials.p, s));
         HJM_CUDA(ctx, cudaEventRecord(ctx->resp_used, s));
     } else {
+        if (use_response_form(ctx) && use_poly_path(ctx))
+            std::copy(ctx->mresp_key.live.win, ctx->mresp_key.live.win + 2, A.M.win);
         HJM_CUDA(ctx, launch_adjoint(nt, A, use_poly_path(ctx), (double*)ctx->partials.p,
                                      K > 0 ? (float*)ctx->ck_h.p : nullptr, K > 0 ? (double*)ctx->ck_a.p : nullptr, s));
     }

@@ -446,35 +446,25 @@ __global__ void __launch_bounds__(kMaxTenor)
 // Shared memory per thread: acc (B+1) FP64 discount sums, whose slot i holds
 // date i's cash flow once tenor i is sampled; hs (B+2) FP32 curve at the block
 // start, reused for the exposure tile at the end.
-// CMP (polynomial factors, many dates): acc holds FP32 instead, the sums of the
-// convected remainder only (its block sums in FP32, as folded into FP64
-// otherwise; the remainder is a small fraction of the curve), and the FP64
-// running sums of the scalar parts S, U, W stay in registers, so that the
-// shared memory of a CTA (the occupancy limit with 60 dates) shrinks by a third.
 // Occupancy: 512 threads per SM by the registers (<= 128 per thread; 112 with
 // polynomial factors, 4 CTAs of 128).  Capped at 96 registers (5 CTAs, 20
 // warps) the polynomial form does not spill but ran slower (20.8 ms against
-// 20.5 at 4,194,304 paths); the compact sums' 64-thread CTAs are bounded by
-// shared memory first (7 per SM for the netting set).
-template <int NT, bool EXT, bool POLY, bool CMP, int C, bool CUB = false>
+// 20.5 at 4,194,304 paths).
+template <int NT, bool EXT, bool POLY, int C, bool CUB = false>
 __global__ void __launch_bounds__(C, 512 / C)
     path_kernel_mixed(const __grid_constant__ MixedParams M, const double* __restrict__ ext,
                       double* __restrict__ partials, float* __restrict__ estore)
 {
-    static_assert(!CMP || POLY, "the compact sums need the polynomial parts");
     static_assert(!CUB || POLY, "the cubic part extends the polynomial form");
-    using Acc = typename std::conditional<CMP, float, double>::type;
     const PathParams<float>& P = M.P;
     extern __shared__ __align__(128) unsigned char smem[];
     const int tid = threadIdx.x;
     const int B = P.n_blocks;
     const int rows = B + 1;
-    constexpr size_t ka = sizeof(Acc);
-    Acc* acc_s = reinterpret_cast<Acc*>(smem);                                // [B+1][C]
-    float* hs_s = reinterpret_cast<float*>(smem + (size_t)rows * C * ka);  // [B+2][C]
+    double* acc_s = reinterpret_cast<double*>(smem);                      // [B+1][C]
+    float* hs_s = reinterpret_cast<float*>(smem + (size_t)rows * C * 8);  // [B+2][C]
     double* red_s = reinterpret_cast<double*>(
-        smem + (((size_t)rows * C * ka + (size_t)(rows + 1) * C * 4 + 7) & ~(size_t)7));
-    double zS = 0.0, zU = 0.0, zW = 0.0, zX = 0.0;  // CMP: FP64 running sums of the parts over the evolved steps
+        smem + (((size_t)rows * C * 8 + (size_t)(rows + 1) * C * 4 + 7) & ~(size_t)7));
 
     const int64_t cta_base = (int64_t)blockIdx.x * C;
     const int64_t lp = cta_base + tid;
@@ -483,21 +473,17 @@ __global__ void __launch_bounds__(C, 512 / C)
 
     MixedPath<NT, POLY, CUB> x;
     x.reset();
-    for (int i = 0; i < rows; ++i) acc_s[i * C + tid] = Acc(0);
+    for (int i = 0; i < rows; ++i) acc_s[i * C + tid] = 0.0;
     for (int t = 0; t <= B + 1; ++t) hs_s[t * C + tid] = 0.f;
 
     auto sample = [&](int i) {
         const double xv = P.psamp[i] + (double)x.value(P, i);
-        double a = P.psum[i] + as_f64(acc_s[i * C + tid]);
-        if constexpr (CMP) {
-            const double ti = (double)P.tau[i];
-            a += CUB ? fma(ti, fma(ti, fma(ti, zX, zW), zU), zS) : fma(ti, fma(ti, zW, zU), zS);
-        }
+        const double a = P.psum[i] + acc_s[i * C + tid];
         const float D = expf((float)(-a * P.dt));
         const float mm = (float)P.m;
         const float L = mm * expm1f((float)xv / mm);
         const float cf = D * ((float)P.payA[i] * L - (float)P.payB[i]);
-        acc_s[i * C + tid] = (Acc)cf;  // cash flow of date i
+        acc_s[i * C + tid] = (double)cf;  // cash flow of date i
     };
 
     sample(1);
@@ -519,21 +505,10 @@ __global__ void __launch_bounds__(C, 512 / C)
             x.step(M, phi0, phi1, phi2);
             bs.add(x, phi0, phi1, phi2);
         }
-        // block sums of tenors 2 .. B; fold (b, B] into FP64 (CMP: the
-        // remainder's in FP32, the parts' into their FP64 running sums)
-        if constexpr (CMP) {
-            recover_sums_up<NT>(x.h, hs_s, tid, C, P, x.g, 0.f, 0.f, 0.f, bs.H1, B, [&](int t, float Ht) {
-                if (t > b) acc_s[t * C + tid] += Ht;
-            });
-            zS += as_f64(bs.sS);
-            zU += as_f64(bs.sU);
-            zW += as_f64(bs.sW);
-            if constexpr (CUB) zX += as_f64(bs.sX);
-        } else {
-            block_sums_up<NT, POLY>(x, hs_s, tid, C, P, bs, B, [&](int t, float Ht) {
-                if (t > b) acc_s[t * C + tid] += as_f64(Ht);
-            });
-        }
+        // block sums of tenors 2 .. B; fold (b, B] into FP64
+        block_sums_up<NT, POLY>(x, hs_s, tid, C, P, bs, B, [&](int t, float Ht) {
+            if (t > b) acc_s[t * C + tid] += as_f64(Ht);
+        });
         // the block-end curve (POLY: its convected part) is the next block's start
 #pragma unroll
         for (int t = 1; t < NT; ++t)
@@ -541,38 +516,124 @@ __global__ void __launch_bounds__(C, 512 / C)
         sample(b + 1);
     }
 
-    mixed_epilogue<Acc, C>(P, acc_s, hs_s, red_s, partials, estore, cta_base, active);
+    mixed_epilogue<double, C>(P, acc_s, hs_s, red_s, partials, estore, cta_base, active);
 }
 
-__host__ __device__ inline size_t mixed_smem_bytes(int nt, int n_blocks, bool cmp = false, int cta = kCta)
+// The convected form of long runs (polynomial factors, many dates) on the
+// tenors that matter.  In block b (from step b stride on) the remainder
+// * holds nothing that counts below the tenor its source has reached (2^-46 per
+//   unit of the source, MixedParams::win; at 2^-30 the netting set's CVA moves
+//   by 2e-8, and the windows would be only half a tenor narrower), and
+// * is read by no later date at or below tenor b: information moves down the
+//   tenors only,
+// so a block convects tenors S0 .. L, S0 the largest window start (thirds of
+// the tenors) at or below either bound: 28 of 51 tenors on average on the 25y
+// swap.  The discount sums telescope (LongSums): no per-tenor sums and no
+// block starts in shared memory, 0.25 KB per path at 60 dates instead of 0.5, so
+// the registers bound the occupancy (16 warps per SM instead of 14).
+// 512k paths: 25y quadratic 7.15 -> 5.95 ms, 25y cubic 7.66 -> 6.23, the
+// 61-tenor netting set 9.61 -> 7.39 (with the windows alone 6.54 and 9.53).
+// Steps unrolled by 2: 7.0 ms by 1 on the cubic run, 6.6 by 3.
+template <int NT, bool EXT, bool CUB>
+__global__ void __launch_bounds__(kCta, 512 / kCta)
+    path_kernel_mixed_conv(const __grid_constant__ MixedParams M, const double* __restrict__ ext,
+                           double* __restrict__ partials, float* __restrict__ estore)
+{
+    constexpr int C = kCta;
+    const PathParams<float>& P = M.P;
+    extern __shared__ __align__(128) unsigned char smem[];
+    const int tid = threadIdx.x;
+    const int B = P.n_blocks;
+    float* cf_s = reinterpret_cast<float*>(smem);  // [B+2][C]: cash flows, then exposures one row up
+    double* red_s = reinterpret_cast<double*>(smem + (size_t)(B + 2) * C * sizeof(float));
+
+    const int64_t cta_base = (int64_t)blockIdx.x * C;
+    const int64_t lp = cta_base + tid;
+    const bool active = lp < P.n_paths;
+    const uint64_t gpath = P.path_offset + (uint64_t)lp;
+
+    MixedPath<NT, true, CUB> x;
+    x.reset();
+    LongSums<NT, CUB> z;
+    z.reset();
+    auto price = [&](int i, float value, double sum) {
+        const double xv = P.psamp[i] + (double)value;
+        const double a = P.psum[i] + sum;
+        const float D = expf((float)(-a * P.dt));
+        const float mm = (float)P.m;
+        const float L = mm * expm1f((float)xv / mm);
+        cf_s[i * C + tid] = D * ((float)P.payA[i] * L - (float)P.payB[i]);
+    };
+    price(1, 0.f, 0.0);
+    // normals drawn one step ahead, so that the generator's dependent chain
+    // overlaps the curve update (the last step redraws itself, unused)
+    const int n_last = B * P.stride - 1;
+    const int64_t lpc = active ? lp : 0;
+    float q0, q1, q2;
+    draw_phi<float, EXT>(ext, gpath, lpc, P.n_paths, min(P.stride, n_last), P.rk0, P.rk1, q0, q1, q2);
+    auto block = [&](auto s0_c, int b) {
+        constexpr int S0 = decltype(s0_c)::value;
+        float sR = 0.f, sS = 0.f, sU = 0.f, sW = 0.f, sX = 0.f;
+        x.begin_block(P, b);
+#pragma unroll 2
+        for (int s = 0; s < P.stride; ++s) {
+            const int n = b * P.stride + s;
+            const float phi0 = q0, phi1 = q1, phi2 = q2;
+            draw_phi<float, EXT>(ext, gpath, lpc, P.n_paths, min(n + 1, n_last), P.rk0, P.rk1, q0, q1, q2);
+            x.template step<S0>(M, phi0, phi1, phi2);
+            sR = fmaf(x.g, pair_tenor<NT>(x.h, S0), sR);
+            sS += x.S;
+            sU += x.U;
+            sW += x.W;
+            if constexpr (CUB) sX += x.X;
+        }
+        z.fold(sR, sS, sU, sW, sX);
+        float value;
+        double sum;
+        z.template read<S0>(x, P, S0, b + 1, value, sum);
+        price(b + 1, value, sum);
+    };
+    constexpr int W1 = conv_window(NT, 0), W2 = conv_window(NT, 1);
+    for (int b = 1; b < B; ++b) {
+        const int w = window_start<NT>(M, b);
+        if (w != z.start) z.move(x, P, w);
+        if (w == W2)
+            block(std::integral_constant<int, W2>(), b);
+        else if (w == W1)
+            block(std::integral_constant<int, W1>(), b);
+        else
+            block(std::integral_constant<int, 1>(), b);
+    }
+    mixed_epilogue<float, C>(P, cf_s, cf_s + C, red_s, partials, estore, cta_base, active);
+}
+
+__host__ __device__ inline size_t mixed_smem_bytes(int nt, int n_blocks, int cta = kCta)
 {
     (void)nt;
     const size_t rows = (size_t)n_blocks + 1;
-    const size_t head = rows * cta * (cmp ? 4 : 8) + (rows + 1) * cta * 4;
+    const size_t head = rows * cta * 8 + (rows + 1) * cta * 4;
     return ((head + 7) & ~(size_t)7) + 2 * (cta / 32) * 8;
 }
 
-// The compact sums when the FP64 ones would hold a CTA's shared memory above a
-// quarter of the SM's (fewer than the 4 CTAs the registers allow)
-inline bool mixed_compact(int nt, int n_blocks, bool poly)
+// The windowed form where the general kernel's shared memory (FP64 sums and
+// block starts per tenor) leaves fewer than the 4 CTAs that the registers
+// allow: 37 dates and more.  Shorter convected runs keep the kernel whose
+// values the adjoint's sweeps repeat bit for bit.
+bool mixed_windowed(int nt, int n_blocks, bool poly)
 {
-    return poly && mixed_smem_bytes(nt, n_blocks, false) > (size_t)228 * 1024 / 4;
+    return poly && mixed_smem_bytes(nt, n_blocks) > (size_t)228 * 1024 / 4;
 }
 
-// Paths per CTA of the mixed kernel.  With the compact sums shared memory
-// bounds the occupancy (~0.5 KB per path with 60 dates), and 64-thread CTAs
-// pack an SM more finely: 7 of them (14 warps) where 3 of 128 threads fit
-// (12 warps) for the 61-tenor netting set (36.5 ms from 37.1); a 25y swap on
-// 51 tenors keeps 16 warps either way.  Otherwise the registers bound it,
-// whatever the CTA size.
-// The table step keeps FP64 sums per tenor (no compact form without the
-// parts), so with many dates its shared memory binds the same way (25y on 51
-// tenors: 79 KB per CTA of 128, 2 per SM; 5 of 64, 10 warps instead of 8).
-constexpr int kMixedCompactCta = 64;
+// Paths per CTA of the mixed kernel.  The table step keeps FP64 sums per tenor,
+// so with many dates its shared memory bounds the occupancy and 64-thread CTAs
+// pack an SM more finely (25y on 51 tenors: 79 KB per CTA of 128, 2 per SM; 5
+// of 64, 10 warps instead of 8).  Otherwise the registers bound it, whatever
+// the CTA size.
+constexpr int kMixedSmallCta = 64;
 inline int mixed_cta(int nt, int n_blocks, bool poly)
 {
-    if (mixed_compact(nt, n_blocks, poly)) return kMixedCompactCta;
-    return mixed_smem_bytes(nt, n_blocks, false) > (size_t)228 * 1024 / 4 ? kMixedCompactCta : kCta;
+    if (mixed_windowed(nt, n_blocks, poly)) return kCta;
+    return mixed_smem_bytes(nt, n_blocks) > (size_t)228 * 1024 / 4 ? kMixedSmallCta : kCta;
 }
 
 void pack_mixed_params(int nt, const PathParams<float>& P, MixedParams& M)
@@ -873,14 +934,16 @@ template <int NT, bool EXT, bool POLY, bool CUB = false>
 static cudaError_t launch_mixed_t(const MixedParams& M, const double* ext, double* partials, float* estore,
                                   cudaStream_t s)
 {
-    const bool cmp = mixed_compact(NT, M.P.n_blocks, POLY);
     const int cta = mixed_cta(NT, M.P.n_blocks, POLY);
-    const size_t smem = mixed_smem_bytes(NT, M.P.n_blocks, cmp, cta);
-    auto k = path_kernel_mixed<NT, EXT, POLY, false, kCta, CUB>;
+    size_t smem = mixed_smem_bytes(NT, M.P.n_blocks, cta);
+    auto k = path_kernel_mixed<NT, EXT, POLY, kCta, CUB>;
     if constexpr (POLY) {
-        if (cmp) k = path_kernel_mixed<NT, EXT, true, true, kMixedCompactCta, CUB>;
+        if (mixed_windowed(NT, M.P.n_blocks, POLY)) {
+            k = path_kernel_mixed_conv<NT, EXT, CUB>;
+            smem = mresp_smem_bytes(M.P.n_blocks);  // (cash flows only, as the response form)
+        }
     } else {
-        if (cta == kMixedCompactCta) k = path_kernel_mixed<NT, EXT, false, false, kMixedCompactCta>;
+        if (cta == kMixedSmallCta) k = path_kernel_mixed<NT, EXT, false, kMixedSmallCta>;
     }
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;

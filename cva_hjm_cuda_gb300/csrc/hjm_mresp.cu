@@ -199,6 +199,7 @@ static void pc_sources(double c, double dtau, double& w0, double& w1, double& w2
 int mresp_slots(int nt, double c, double dtau, int stride, int n_blocks, bool pc, RespLive* live)
 {
     const int B = n_blocks, L = nt - 1;
+    if (live) *live = {};
     if (nt < 3 || nt > kMaxTenor || B < 1 || B >= nt || stride < 1 || !(c > 0.0 && c < 1.0)) return 0;
     // (the predictor-corrector's date at the last tenor takes a lag -1 term
     // this kernel leaves out)
@@ -220,13 +221,16 @@ int mresp_slots(int nt, double c, double dtau, int stride, int n_blocks, bool pc
     v[L] = 1.0;
     if (pc) u[L - 1] = 1.0;
     int need = 0;
-    int last[kMaxTenor] = {};  // per slot, the last block that counts
+    int last[kMaxTenor] = {};   // per slot, the last block that counts
+    int first[kMaxTenor] = {};  // per tenor, the first block in which a response reaches 2^-46 (0: none)
     for (int m = 0; m <= M + (pc ? 1 : 0); ++m) {
         for (int t = 0; t < nt; ++t) {
             cum[t] += v[t];
             cu[t] += u[t];
         }
         const int l = pc ? m - 1 : m;  // the lag this iteration completes
+        for (int t = 1; !pc && t < nt; ++t)
+            if (first[t] == 0 && std::fabs(v[t]) >= std::ldexp(1.0, -46)) first[t] = l / stride + 1;
         if (l >= 0)
             for (int j = 2; j <= B; ++j) {
                 // date j reads lags up to K_j - stride = (j - 1) stride - 1
@@ -265,6 +269,11 @@ int mresp_slots(int nt, double c, double dtau, int stride, int n_blocks, bool pc
         for (int r = 0; r < ns; ++r) {
             if (r >= ns / 2) live->half = std::max(live->half, last[r] + 1);
             live->none = std::max(live->none, last[r] + 1);
+        }
+        for (int i = 0; !pc && i < 2; ++i) {
+            live->win[i] = B;
+            for (int t = 1; t < conv_window(nt, i); ++t)
+                if (first[t]) live->win[i] = std::min(live->win[i], first[t]);
         }
     }
     return ns;

@@ -111,7 +111,9 @@ __device__ __forceinline__ void recover_sums_up(const float2 (&h)[PairGrid<NT>::
 // The growth-scaled convection of the packed curve (polynomial volatility:
 // the noise lives in the scalar parts S, U, W), with the last-tenor source
 // src already scaled by (1 + rr)^(n'+1): one packed FMA per pair of tenors.
-template <int NT>
+// S0 > 0: tenors S0 .. L only (a pair with one tenor below takes a scalar FMA,
+// half a packed one's issue).
+template <int NT, int S0 = 0>
 __device__ __forceinline__ void convect_pairs(float2 (&h)[PairGrid<NT>::H], const MixedParams& M, float src)
 {
     constexpr int H = PairGrid<NT>::H, L = PairGrid<NT>::L;
@@ -120,10 +122,12 @@ __device__ __forceinline__ void convect_pairs(float2 (&h)[PairGrid<NT>::H], cons
 #pragma unroll
     for (int p = 0; p < H; ++p) {
         const int q = H + p;
-        if (p + 1 < H && q < L) {
+        if (p >= S0 && p + 1 < H && q < L) {
             hn[p] = __ffma2_rn(M.rp, h[p + 1], h[p]);
         } else {
-            hn[p].x = fmaf(rr, (p + 1 < H) ? h[p + 1].x : h[0].y, h[p].x);
+            hn[p] = h[p];
+            if (p >= S0) hn[p].x = fmaf(rr, (p + 1 < H) ? h[p + 1].x : h[0].y, h[p].x);
+            if (q < S0) continue;
             if (q < L)
                 hn[p].y = fmaf(rr, h[p + 1].y, h[p].y);
             else if (q == L)
@@ -167,11 +171,13 @@ struct MixedPath {
         g = P.gblk[b];
         ig = POLY ? P.m2k2 * P.igblk[b] : P.igblk[b];
     }
+    // S0 (POLY): tenors S0 .. L of the remainder only
+    template <int S0 = 0>
     __device__ __forceinline__ void step(const MixedParams& M, float phi0, float phi1, float phi2)
     {
         ig *= M.P.ip;
         if constexpr (POLY) {
-            convect_pairs<NT>(h, M, ig * (CUB ? fmaf(M.src3f, X, W) : W));
+            convect_pairs<NT, S0>(h, M, ig * (CUB ? fmaf(M.src3f, X, W) : W));
             // the noise projection folded into the updates (old U, W, X on the right)
             float Sn = fmaf(M.svcf[0][0], phi0, fmaf(M.k2f, W, fmaf(M.k1f, U, S)));
             if constexpr (CUB) Sn = fmaf(M.k3f, X, Sn);
@@ -228,6 +234,16 @@ struct BlockSums {
         }
         H1 = fmaf(x.g, x.h[1].x, H1);
     }
+    // (polynomial factors) with the curve's value `at` (unscaled) as the anchor
+    template <int NT, bool CUB>
+    __device__ __forceinline__ void add_at(const MixedPath<NT, true, CUB>& x, float at)
+    {
+        sS += x.S;
+        sU += x.U;
+        sW += x.W;
+        if constexpr (CUB) sX += x.X;
+        H1 = fmaf(x.g, at, H1);
+    }
     // the block sums of the polynomial part at basis coordinate t
     template <bool CUB>
     __device__ __forceinline__ float poly(float t) const
@@ -251,6 +267,85 @@ __device__ __forceinline__ void block_sums_up(const MixedPath<NT, POLY, CUB>& x,
         recover_sums_up<NT>(x.h, hs_s, tid, cta, P, x.g, bs.F0, bs.F1, bs.F2, bs.H1, tmax, fold);
     }
 }
+
+// The start of the window of tenors that block b of a long convected run needs
+// (polynomial factors): the remainder has not reached below it (MixedParams::win)
+// or no later date reads below it.
+template <int NT>
+__device__ __forceinline__ int window_start(const MixedParams& M, int b)
+{
+    constexpr int W1 = conv_window(NT, 0), W2 = conv_window(NT, 1);
+    return b < M.win[1] || b + 1 >= W2 ? W2 : b < M.win[0] || b + 1 >= W1 ? W1 : 1;
+}
+
+// Running sums over all steps of a long convected run.  The convected
+// remainder starts at zero and moves by hc' = A hc (+ the source at L), so the
+// running sum R[t] of tenor t over the steps' results telescopes along the
+// tenors:
+//     R[t+1] = R[t] + (A hc)[t] / c,   hc the curve as it is now,
+// and a date's sum follows from that of one tenor, the window's start, and
+// the curve: no per-tenor sums are kept.
+template <int NT, bool CUB>
+struct LongSums {
+    double zR, zS, zU, zW, zX;  // of the remainder at tenor start, of the parts
+    int start;
+
+    __device__ __forceinline__ void reset()
+    {
+        zR = zS = zU = zW = zX = 0.0;
+        start = 1;
+    }
+    // hc at tenor `to` (in v) and R[to] - R[from], over the tenors S0 .. L
+    template <int S0>
+    __device__ __forceinline__ float climb(const MixedPath<NT, true, CUB>& x, const PathParams<float>& P, int from,
+                                           int to, float& v) const
+    {
+        float run = 0.f, v0 = 0.f;
+        v = 0.f;
+#pragma unroll
+        for (int t = S0; t < NT; ++t) {
+            const float ht = pair_tenor<NT>(x.h, t);
+            if (t >= from && t < to) run += ht;
+            if (t == from) v0 = ht;
+            if (t == to) v = ht;
+        }
+        v *= x.g;
+        return (float)P.inv_c * fmaf(P.c, v, x.g * fmaf(-P.c, v0, run));
+    }
+    // the window starts at tenor w from here on: up along the curve, down to
+    // a tenor that has held nothing yet
+    __device__ __forceinline__ void move(const MixedPath<NT, true, CUB>& x, const PathParams<float>& P, int w)
+    {
+        float v;
+        zR = w > start ? zR + as_f64(climb<1>(x, P, start, w, v)) : 0.0;
+        start = w;
+    }
+    __device__ __forceinline__ void fold(float sR, float sS, float sU, float sW, float sX)
+    {
+        zR += as_f64(sR);
+        zS += as_f64(sS);
+        zU += as_f64(sU);
+        zW += as_f64(sW);
+        if constexpr (CUB) zX += as_f64(sX);
+    }
+    // the parts' running sums at basis coordinate t
+    __device__ __forceinline__ double parts(double t) const
+    {
+        return CUB ? fma(t, fma(t, fma(t, zX, zW), zU), zS) : fma(t, fma(t, zW, zU), zS);
+    }
+    // date i's sampled value (without its FP64 part) and discount sum, from
+    // the window's start
+    template <int S0>
+    __device__ __forceinline__ void read(const MixedPath<NT, true, CUB>& x, const PathParams<float>& P, int from,
+                                         int i, float& value, double& sum) const
+    {
+        const float t = P.tau[i];
+        float v;
+        const float up = climb<S0>(x, P, from, i, v);
+        value = v + x.poly(t);
+        sum = (i < from ? 0.0 : zR + as_f64(up)) + parts((double)t);
+    }
+};
 
 // One growth-scaled reverse step on the packed adjoint state.  The adjoint
 // obeys g <- A^T (g + inj) with A^T, per tenor (L the last tenor):

@@ -321,6 +321,7 @@ hjm_status hjm_run_static(void* cuda_stream, int32_t n_tenor, double dtau, const
             STATIC_CUDA(launch_mresp_table(n_tenor, dt / dtau, dtau, (int)stride, B, mresp_ns, false, table, s));
             STATIC_CUDA(launch_path_mixed_resp(M, mresp_ns, live, cub, table, nullptr, partials, nullptr, s));
         } else {
+            std::copy(live.win, live.win + 2, M.win);
             STATIC_CUDA(launch_path_mixed(n_tenor, M, poly, nullptr, partials, nullptr, s, cub));
         }
     } else {

@@ -141,6 +141,34 @@ def test_mixed_response_long_runs_convect(engine):
     np.testing.assert_allclose(v.ee[:50], ee_o[:50], rtol=MIXED_RTOL, atol=MIXED_RTOL * np.max(ee_o))
 
 
+@pytest.mark.parametrize("dt,n_periods,n_tenor,cubic", [(0.01, 36, 51, False), (0.01, 38, 51, False), (0.02, 50, 51, True),
+                                                        (0.05, 47, 61, False), (0.25, 50, 51, False), (0.1, 60, 61, False)])
+def test_mixed_long_runs_windows(engine, dt, n_periods, n_tenor, cubic):
+    """Convected runs about the size from which they convect a window of the
+    tenors only (36 and 38 dates), with the windows reached early and late
+    (blocks of 50 to 2 steps), both tenor grids, the cubic form, a ragged path
+    count and the last date at the last tenor: per-path exposures against the
+    oracle to the mixed tolerance, and against the form without the early
+    windows (a response left out is below 2^-46 of the source) to FP32's
+    rounding of another starting tenor, as the two forms above; external
+    normals give the generator's run bit for bit."""
+    mk = _own_market() if cubic else Market(n_tenor=n_tenor)
+    sw = Swap(n_tenor=n_tenor, n_periods=n_periods)
+    engine.set_market(mk)
+    engine.set_swap(sw)
+    cfg = RunConfig(n_paths=1_003, n_steps=round(n_periods * 0.5 / dt), dt=dt, seed=12)
+    (va, xa, fa), (vc, xc, fc) = _both_forms(engine, cfg, pfe=False)
+    assert (fa, fc) == ("convect", "convect")
+    scale = np.max(np.abs(xa))
+    assert np.max(np.abs(xa - xc)) <= FORM_TOL * scale
+    assert abs(va.cva - vc.cva) <= FORM_TOL * abs(vc.cva)
+    normals = engine.dump_normals(cfg.n_paths, cfg.n_steps, cfg.seed)
+    e = engine.run_with_normals(normals, cfg.n_steps, cfg.dt, "mixed")
+    np.testing.assert_array_equal(e.ee, va.ee)
+    xo = O.exposure_paths(mk, sw, cfg.n_steps, cfg.dt, normals)[:, : n_periods + 1].T
+    assert np.max(np.abs(xa - xo)) <= MIXED_RTOL * scale
+
+
 def test_mixed_response_path_ranges_compose(engine):
     """Paths are independent: a run over [0, n) equals, in EE sums, the runs
     over its two halves (path_offset), and a ragged count runs its tail CTA."""
