@@ -20,7 +20,6 @@
 
 #include "../../include/hjm_cva.h"
 #include "hjm_contract.h"
-#include "hjm_eresp.h"
 #include "hjm_kernels.h"
 
 using namespace hjm;
@@ -836,11 +835,7 @@ static hjm_status ensure_contract_table(hjm_ctx* ctx, const RunShape& sh, double
         k.ext == ext && k.sv == key)
         return HJM_OK;
     k.valid = false;
-    const size_t bytes = contract_table_bytes(sh.stride, sh.B, ext);
-    if (bytes > ctx->contract.bytes)
-        HJM_CUDA(ctx, ctx->contract.ensure(bytes));  // cudaFree waits for the device
-    else
-        HJM_CUDA(ctx, cudaStreamWaitEvent(s, ctx->resp_used, 0));
+    HJM_CUDA(ctx, cudaStreamWaitEvent(s, ctx->resp_used, 0));
     HJM_CUDA(ctx, launch_contract_table(nt, c, sh.stride, sh.B, ctx->scheme == HJM_SCHEME_PREDICTOR_CORRECTOR, ext,
                                         sv, ctx->contract.p, s));
     ctx->stat_launches += 2 + contract_windows(sh.B, sh.stride, ext, nullptr);
@@ -855,29 +850,40 @@ static hjm_status ensure_contract_table(hjm_ctx* ctx, const RunShape& sh, double
     return HJM_OK;
 }
 
+static bool try_ensure(DevBuf& b, size_t bytes)
+{
+    if (b.ensure(bytes) == cudaSuccess) return true;
+    cudaGetLastError();
+    return false;
+}
+
+// Room for the contraction's table and the carry of a windowed run.
+static bool contract_room(hjm_ctx* ctx, const RunShape& sh, int64_t n_paths, bool ext)
+{
+    const size_t bytes = contract_table_bytes(sh.stride, sh.B, ext);
+    if (bytes > ctx->contract.bytes) {
+        ctx->contract_key.valid = false;  // (growing drops the table it held)
+        if (!try_ensure(ctx->contract, bytes)) return false;
+    }
+    return contract_windows(sh.B, sh.stride, ext, nullptr) <= 1 ||
+           try_ensure(ctx->carry, sizeof(double) * 2 * (size_t)n_paths);
+}
+
 // An FP64 valuation in the response form (hjm_contract.cu): the operand table
-// of the market's loadings, the carry of a windowed run, one launch per
-// window.  P: the scheme's parameters (the predictor-corrector's N-projected
+// of the market's loadings (contract_room made room for it and the carry), the
+// launches of its windows.  P: the scheme's parameters (the predictor-corrector's N-projected
 // loadings and deterministic curve).  ext_dev: external normals with their row
 // scales behind them (hjm_run_with_normals), or null.
 static hjm_status enqueue_contract(hjm_ctx* ctx, const RunShape& sh, double dt, const PathParams<double>& P,
-                                   const double* ext_dev, double* estore, cudaStream_t s)
+                                   const double* ext_dev, double* estore, longlong2* split, cudaStream_t s)
 {
     hjm_status st = ensure_contract_table(ctx, sh, dt, &P.sv[0][0], ext_dev != nullptr, s);
     if (st != HJM_OK) return st;
-    double* carry = nullptr;
-    if (contract_windows(sh.B, sh.stride, ext_dev != nullptr, nullptr) > 1) {
-        HJM_CUDA(ctx, ctx->carry.ensure(sizeof(double) * 2 * (size_t)P.n_paths));
-        carry = (double*)ctx->carry.p;
-    }
     const double* ext_scale =
         ext_dev ? ext_dev + (size_t)P.n_paths * (size_t)sh.B * (size_t)sh.stride * kFactors : nullptr;
-    const size_t split = contract_sums_bytes(P.n_paths, sh.B, sh.stride, ctx->n_sms, ext_dev != nullptr);
-    if (split) HJM_CUDA(ctx, ctx->split.ensure(split));
     int launches = 0;
     HJM_CUDA(ctx, launch_path_contract(ctx->nt, P, ctx->contract.p, ext_dev, ext_scale, (double*)ctx->partials.p,
-                                       estore, carry, split ? (longlong2*)ctx->split.p : nullptr,
-                                       (double*)ctx->result.p, ctx->n_sms, s, &launches));
+                                       estore, (double*)ctx->carry.p, split, (double*)ctx->result.p, ctx->n_sms, s, &launches));
     ctx->stat_launches += launches - 1;
     return HJM_OK;
 }
@@ -898,7 +904,7 @@ __attribute__((visibility("hidden"))) void mixed_cubic_params(int nt, double dta
 {
     const double c = dt / dtau, sq = std::sqrt(dt);
     const double TL = dtau * (nt - 1);
-    const double tau0 = eresp_window_centre(dtau, 1, n_blocks);
+    const double tau0 = 0.5 * dtau * (double)(1 + n_blocks);
     const double dl = tau0 - TL;  // sum_e a_e (T - T_L)^e = sum_d a'_d (T - tau0)^d
     for (int k = 0; k < kFactors; ++k) {
         const double* a = cubic + 4 * k;
@@ -975,11 +981,12 @@ static hjm_status enqueue_impl(hjm_ctx* ctx, int64_t n_paths, int32_t n_steps, d
                           use_response_form(ctx))
                              ? mresp_run_slots(ctx, sh, dt, pc)
                              : 0;
-    const int cta = !mixed && use_response_form(ctx) ? kContractTile
-                    : mresp_ns                       ? kCta
+    // partial rows: the contraction's, else one per CTA of the convected kernels
+    bool contract = !mixed && use_response_form(ctx);
+    const int cta = mresp_ns ? kCta
                              : (pc ? pc_cta() : path_cta(mixed, ctx->nt, sh.B, use_poly_path(ctx) || mixed_cubic));
-    const int64_t n_ctas = !mixed && use_response_form(ctx) ? contract_rows(n_paths, sh.B, sh.stride, ctx->n_sms)
-                                                            : (n_paths + cta - 1) / cta;
+    int64_t n_ctas =
+        contract ? contract_rows(n_paths, sh.B, sh.stride, ctx->n_sms, false) : (n_paths + cta - 1) / cta;
     const int64_t ld = (n_paths + 3) / 4 * 4;
     const size_t esize = mixed ? 4 : 8;
 
@@ -990,6 +997,22 @@ static hjm_status enqueue_impl(hjm_ctx* ctx, int64_t n_paths, int32_t n_steps, d
     if (want_pfe) {
         HJM_CUDA(ctx, ctx->sel.ensure(sizeof(SelState) * kMaxTenor));
         HJM_CUDA(ctx, ctx->hist.ensure(pfe_scratch_bytes(n_paths, n_dates, !mixed)));
+    }
+    // what the contraction needs besides: its table and carry, without which
+    // the run convects, and its split tiles' sums, without which they run whole
+    longlong2* split = nullptr;
+    if (contract && !contract_room(ctx, sh, n_paths, ext_dev != nullptr)) {
+        contract = false;
+        n_ctas = (n_paths + cta - 1) / cta;
+        HJM_CUDA(ctx, ctx->partials.ensure(sizeof(double) * (size_t)n_ctas * R));
+    }
+    if (contract) {
+        const size_t bytes = contract_sums_bytes(n_paths, sh.B, sh.stride, ctx->n_sms, ext_dev != nullptr);
+        const int64_t rows = contract_rows(n_paths, sh.B, sh.stride, ctx->n_sms);
+        if (bytes && try_ensure(ctx->split, bytes) && try_ensure(ctx->partials, sizeof(double) * (size_t)rows * R)) {
+            split = (longlong2*)ctx->split.p;
+            n_ctas = rows;
+        }
     }
     cudaStream_t s = ctx->stream;
     ctx->have_result = false;
@@ -1043,9 +1066,9 @@ static hjm_status enqueue_impl(hjm_ctx* ctx, int64_t n_paths, int32_t n_steps, d
         PcParams<double> Q;
         fill_pc<double>(ctx, sh, dt, P, Q);
         ctx->stat_h2d = sizeof(Q) + sizeof(FinalParams);
-        resp = use_response_form(ctx);
+        resp = contract;
         if (resp) {
-            st = enqueue_contract(ctx, sh, dt, Q.P, ext_dev, store ? (double*)ctx->estore.p : nullptr, s);
+            st = enqueue_contract(ctx, sh, dt, Q.P, ext_dev, store ? (double*)ctx->estore.p : nullptr, split, s);
             if (st != HJM_OK) return st;
         } else {
             HJM_CUDA(ctx, launch_path_pc(ctx->nt, Q, use_poly_path(ctx), ext_dev, (double*)ctx->partials.p,
@@ -1078,9 +1101,9 @@ static hjm_status enqueue_impl(hjm_ctx* ctx, int64_t n_paths, int32_t n_steps, d
     } else {
         PathParams<double> P;
         fill_params<double>(ctx, sh, n_paths, dt, seed, path_offset, hazard, recovery, ld, store, P, F);
-        resp = use_response_form(ctx);
+        resp = contract;
         if (resp) {
-            st = enqueue_contract(ctx, sh, dt, P, ext_dev, store ? (double*)ctx->estore.p : nullptr, s);
+            st = enqueue_contract(ctx, sh, dt, P, ext_dev, store ? (double*)ctx->estore.p : nullptr, split, s);
             if (st != HJM_OK) return st;
             if (use_cubic_path(ctx)) run_form = vol_form_code(ctx);
         } else {
@@ -1429,10 +1452,7 @@ hjm_status hjm_run_adjoint(hjm_ctx* ctx, int64_t n_paths, int32_t n_steps, doubl
         st = ensure_mresp_table(ctx, s);
         if (st != HJM_OK) return st;
         grid = adjoint_resp_grid(n_paths, adj_ns, conv_nt, ctx->n_sms);
-        while (grid > 0 && ctx->sens.ensure(adjoint_resp_sens_bytes(B, grid)) != cudaSuccess) {
-            cudaGetLastError();
-            grid /= 2;
-        }
+        while (grid > 0 && !try_ensure(ctx->sens, adjoint_resp_sens_bytes(B, grid))) grid /= 2;
         if (grid == 0) adj_ns = 0;
     }
     if (K > 0 && !adj_ns) {

@@ -61,7 +61,6 @@
 
 #include "hjm_contract.h"
 #include "hjm_kernels.h"
-#include "hjm_resp.cuh"
 
 namespace hjm {
 
@@ -72,7 +71,6 @@ constexpr int kFlush = 12;               // chunks per accumulator group
 constexpr int kSlices = 4;                // of a normal
 constexpr int kLevels = 5;                // of a response, and accumulators
 constexpr int kProducers = 16;           // warps
-constexpr int kEpilogueWarp = 16;        // first of four
 constexpr int kMmaWarp = 20, kLoadWarp = 21;
 constexpr int kThreads = 32 * 22;
 constexpr int kAStages = 2, kBStages = 3;
@@ -1126,9 +1124,9 @@ static int64_t split_tiles(int64_t n_paths, int n_blocks, int stride, int n_sms)
     return rest > 0 && (rest * G + n_sms - 1) / n_sms + 2 <= G ? rest : 0;
 }
 
-int64_t contract_rows(int64_t n_paths, int n_blocks, int stride, int n_sms)
+int64_t contract_rows(int64_t n_paths, int n_blocks, int stride, int n_sms, bool with_split)
 {
-    const int64_t split = split_tiles(n_paths, n_blocks, stride, n_sms);
+    const int64_t split = with_split ? split_tiles(n_paths, n_blocks, stride, n_sms) : 0;
     return (n_paths + kContractTile - 1) / kContractTile + 3 * split;
 }
 

@@ -47,8 +47,9 @@ cudaError_t launch_contract_ext_scale(const double* raw, int64_t n_paths, int n_
 
 // Partial-sum rows of a run: one per tile of kContractTile paths, four for a tile
 // whose steps are split over the SMs (the tiles after the last whole wave, where
-// that pays); the split tiles' sums take contract_sums_bytes (0: none).
-int64_t contract_rows(int64_t n_paths, int n_blocks, int stride, int n_sms);
+// that pays); the split tiles' sums take contract_sums_bytes (0: none).  Without
+// room for them (split = false, sums = null) every tile runs whole.
+int64_t contract_rows(int64_t n_paths, int n_blocks, int stride, int n_sms, bool split = true);
 size_t contract_sums_bytes(int64_t n_paths, int n_blocks, int stride, int n_sms, bool ext);
 
 // The valuation: per window a launch over the whole tiles and one over the split

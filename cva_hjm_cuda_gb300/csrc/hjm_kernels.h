@@ -69,24 +69,9 @@ constexpr int kFormPolyTri = 2;  // ... with factor k of degree <= k
 
 // The convected FP64 path kernel.  poly: the volatility factors are
 // polynomials of degree <= 2 in T (PathParams::svc), else the table step.
-// (The response forms of the Euler step are in hjm_eresp.h.)
+// (The response form is in hjm_contract.h.)
 cudaError_t launch_path_fp64(int nt, const PathParams<double>& P, bool poly, const double* ext, double* partials,
                              double* estore, cudaStream_t s);
-int response_max_dates();
-// The response form of the volatility-table step (FP64 accuracy, either
-// scheme: the table carries the scheme): vresp from launch_response_table_vol
-// with the kernel's loadings sv [kFactors][kMaxTenor] (PathParams::sv); one
-// launch per window of at most max_slots dates (16, or 24 for one launch up
-// to 24 dates; vresp_windows of them), carry [2][n_paths] doubles when there
-// is more than one; *launches: kernels enqueued.
-cudaError_t launch_path_fp64_vresp(int nt, const PathParams<double>& P, const float4* vresp, const double* ext,
-                                   double* partials, double* estore, double* carry, cudaStream_t s,
-                                   int* launches = nullptr, int max_slots = 16);
-int vresp_windows(int n_blocks, int max_slots = 16);
-int vresp_row(int n_blocks);                                // slots per table row
-size_t response_table_vol_elems(int stride, int n_blocks);  // float4 entries
-cudaError_t launch_response_table_vol(int nt, double c, int stride, int n_blocks, bool pc, const double* sv,
-                                      float4* vresp, cudaStream_t s);
 // cub: the cubic polynomial form (MixedParams::svcx, k3f, src3f; P.tau the
 // tenors minus the basis centre), which implies poly
 cudaError_t launch_path_mixed(int nt, const MixedParams& M, bool poly, const double* ext, double* partials,
@@ -163,8 +148,8 @@ struct PcParams {
     T wL1, wL, gL;         // sources: -c^2 dtau^2 W at L-1; -(2c + c^2) dtau^2 W - c dtau^2 gamma at L
 };
 
-// The predictor-corrector's convected kernels (the FP64 response form of its
-// decomposition runs in hjm_eresp.cu)
+// The predictor-corrector's convected kernels (its FP64 response form runs in
+// hjm_contract.cu)
 cudaError_t launch_path_pc(int nt, const PcParams<double>& Q, bool poly, const double* ext, double* partials,
                            double* estore, cudaStream_t s);
 cudaError_t launch_path_pc(int nt, const PcParams<float>& Q, bool poly, const double* ext, double* partials,

@@ -10,8 +10,8 @@
 // stride - 1, with its running sum for the discount, so per date still to be
 // sampled the kernel keeps those two numbers and adds per step
 //     {kappa G_j(lag), kappa CG_j(lag)} w,   lag = K_j - n,
-// G_j(m) = (A^m e_L)[j] and CG_j its running sum (the FP64 response form's
-// algebra, hjm_eresp.cu, here in FP32 sums).  The convected form moves every
+// G_j(m) = (A^m e_L)[j] and CG_j its running sum (of the
+// remainder alone, in FP32 sums).  The convected form moves every
 // tenor of hc per step (one packed FMA per two tenors, 26 at 51 tenors); the
 // responses reach only the dates near the last tenor: on the 10y swap (20
 // dates on 51 tenors, c = 0.02) no response of dates 2 to 12 ever reaches
@@ -208,7 +208,7 @@ int mresp_slots(int nt, double c, double dtau, int stride, int n_blocks, bool pc
     const int M = (B - 1) * stride - 1;  // the longest lag read
     // Euler: G = A^m e_L.  Predictor-corrector: H(l) = w0 G1(l) + w1 G2(l) +
     // w2 G2(l + 1) per unit kappa, G1, G2 the three-point step's responses to
-    // e_{L-1}, e_L (the tables' recursions, eresp_table_pc_kernel)
+    // e_{L-1}, e_L (the tables' recursions, mresp_table_pc_kernel)
     double w0 = 0.0, w1 = 0.0, w2 = 0.0, kap = 1.0;
     if (pc) {
         pc_sources(c, dtau, w0, w1, w2);
@@ -314,8 +314,8 @@ __global__ void __launch_bounds__(kMaxTenor)
 
 // The predictor-corrector's table in the same layout: per old W at lag l,
 // {H(l), CH(l)} with H(l) = w0 G1(l) + w1 G2(l) + w2 G2(l + 1) (W_new of one
-// step is W_old of the next) and CH likewise from the running sums, the
-// recursions of eresp_table_pc_kernel (hjm_eresp.cu) rounded to FP32.
+// step is W_old of the next) and CH likewise from the running sums, FP64
+// recursions rounded to FP32.
 __global__ void __launch_bounds__(kMaxTenor)
     mresp_table_pc_kernel(int nt, double c, int stride, int B, int ns, double w0, double w1, double w2,
                           float4* __restrict__ table)

@@ -35,7 +35,6 @@
 #include "hjm_epilogue.cuh"
 #include "hjm_kernels.h"
 #include "hjm_pc.cuh"
-#include "hjm_resp.cuh"
 
 namespace hjm {
 

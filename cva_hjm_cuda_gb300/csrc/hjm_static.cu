@@ -18,19 +18,12 @@
 // cudaGetSymbolAddress, with that device current, and passes it to the same
 // path and reduction kernels that hjm_run launches.
 //
-// A volatility table whose factors are quadratics in T (the synthetic
-// factors of the configured workloads) runs the polynomial decomposition in
-// both precisions, as hjm_run does.  FP64 runs take a response form whenever
-// its table fits a second static array (4 MB; recomputed on the device at
-// every call) and one launch covers the run's dates (hjm_run takes a response
-// form for every FP64 valuation, in as many windows as it needs, each after
-// the last with a carry): with polynomial factors the decomposition's
-// remainder in double-FP32 impulse-response sums, else the whole stochastic
-// curve as double-FP32 sums of the three factors' responses (12x the
-// convected table step on the 10y swap).  Other FP64 runs take the convected
-// step (decomposed or table).  Mixed precision with polynomial factors takes
-// the FP32 response form where hjm_run does (its table, also rebuilt at every
-// call, in the same static array), else the convected pairs.
+// FP64 runs take the contraction (hjm_contract.cu) as hjm_run does, whenever
+// its operand table (rebuilt on the device at every call), the carry between
+// windows and the split tiles' sums fit a second static array (48 MB); the
+// others the convected step (quadratic factors decomposed, else the table).
+// Mixed precision with polynomial factors takes the FP32 response form where
+// hjm_run does (its table in the same array), else the convected pairs.
 //
 // Limits: at most HJM_STATIC_MAX_PATHS paths per call; EE and CVA only (the
 // per-path exposure store a PFE needs would not fit a modest static buffer).
@@ -48,7 +41,7 @@
 #include <string>
 
 #include "../../include/hjm_cva.h"
-#include "hjm_eresp.h"
+#include "hjm_contract.h"
 #include "hjm_kernels.h"
 
 using namespace hjm;
@@ -69,7 +62,7 @@ constexpr size_t kPartialsDoubles = (size_t)kStaticCtas * kStaticCols;
 constexpr size_t kSumsOffset = kPartialsDoubles;        // 2 * kMaxTenor doubles
 constexpr size_t kResultOffset = kSumsOffset + 2 * kMaxTenor;
 constexpr size_t kScratchDoubles = kResultOffset + kResLen;
-constexpr size_t kStaticRespEntries = (size_t)1 << 18;  // double2: 4 MB of response table
+constexpr size_t kStaticRespBytes = (size_t)48 << 20;
 constexpr int kMaxDevices = 64;
 
 std::mutex g_static_mu;
@@ -92,10 +85,10 @@ hjm_status static_fail(hjm_status st, const char* fmt, ...)
 // The scratch: 8.4 MB of FP64 per device (HJM_STATIC_MAX_PATHS / 64 CTA rows
 // of 64 partial sums, plus column sums and the result block).
 static __device__ __align__(256) double g_hjm_static_scratch[kScratchDoubles];
-// ... and 4 MB for the FP64 response table (the float4 entries of either
-// response form, in a double2 array for its 16-byte alignment).
-static __device__ __align__(256) double2 g_hjm_static_resp[kStaticRespEntries];
-static_assert(sizeof(float4) == sizeof(double2), "both response tables use 16-byte entries");
+// ... and 48 MB for a response form's table (FP64: also the carry between
+// windows, 16 MB at HJM_STATIC_MAX_PATHS, and the split tiles' sums, 10 MB).
+// The 25y run at dt = 0.01 takes 41 MB at most, the 10y run down to dt = 0.001.
+static __device__ __align__(256) double2 g_hjm_static_resp[kStaticRespBytes / sizeof(double2)];
 
 #define STATIC_CUDA(call)                                                                          \
     do {                                                                                           \
@@ -267,9 +260,26 @@ hjm_status hjm_run_static(void* cuda_stream, int32_t n_tenor, double dtau, const
     RespLive live = {};
     const int mresp_ns =
         (precision == HJM_PRECISION_MIXED && (poly || cub)) ? mresp_slots(n_tenor, dt / dtau, dtau, (int)stride, B, false, &live) : 0;
-    const bool mresp = mresp_ns > 0 && mresp_table_elems((int)stride, B, mresp_ns) <= kStaticRespEntries;
+    const bool mresp =
+        mresp_ns > 0 && sizeof(float4) * mresp_table_elems((int)stride, B, mresp_ns) <= kStaticRespBytes;
+    // FP64: the contraction where its table, the carry of several windows and
+    // the split tiles' sums fit the static array
+    int n_sms = 0;
+    const size_t align = 256;
+    size_t carry_at = 0, split_at = 0;
+    bool contract = false;
+    if (precision == HJM_PRECISION_FP64) {
+        int dev = 0;
+        STATIC_CUDA(cudaGetDevice(&dev));
+        STATIC_CUDA(cudaDeviceGetAttribute(&n_sms, cudaDevAttrMultiProcessorCount, dev));
+        carry_at = (contract_table_bytes((int)stride, B, false) + align - 1) / align * align;
+        const bool windows = contract_windows(B, (int)stride, false, nullptr) > 1;
+        split_at = carry_at + (windows ? (sizeof(double) * 2 * (size_t)n_paths + align - 1) / align * align : 0);
+        contract = split_at + contract_sums_bytes(n_paths, B, (int)stride, n_sms, false) <= kStaticRespBytes;
+    }
     const int cta = mresp ? kCta : path_cta(precision == HJM_PRECISION_MIXED, n_tenor, B, poly || cub);
-    const int64_t n_ctas = (n_paths + cta - 1) / cta;
+    const int64_t n_ctas =
+        contract ? contract_rows(n_paths, B, (int)stride, n_sms) : (n_paths + cta - 1) / cta;
     if (R > kStaticCols || n_ctas > kStaticCtas)
         return static_fail(HJM_ERR_INVALID_ARGUMENT, "run exceeds the static scratch");
 
@@ -331,36 +341,12 @@ hjm_status hjm_run_static(void* cuda_stream, int32_t n_tenor, double dtau, const
         if (poly)
             for (int k = 0; k < kFactors; ++k)
                 for (int d = 0; d < 3; ++d) P.svc[k][d] = sq * coef[k * 3 + d];
-        const size_t entries = response_table_vol_elems((int)stride, B);
-        const int nres = cub ? eresp_residual_factors(resid, vol_host, n_tenor) : 0;
-        const int first = (poly || cub) ? eresp_first_active_date(n_tenor, dt / dtau, (int)stride, B, nres) : 2;
-        if ((poly || cub) && eresp_windows(B, first, nullptr, nullptr, nullptr, eresp_window_dates(nres)) == 1 &&
-            eresp_table_elems((int)stride, B, cub ? 4 : 3, nres, 1) <= kStaticRespEntries) {
-            // the decomposition's response form in one window: its table (FP32
-            // pairs, 16 bytes per entry) in the static array
-            EulerRespFrame fr;
-            int degs;
-            eresp_make_frame(dt, dtau, n_tenor, P.svc, cub ? cubic : nullptr, cdegs, eresp_window_centre(dtau, 1, B), fr,
-                             degs);
-            for (int i = 0; i < HJM_N_FACTOR * n_tenor; ++i) resid[i] *= sq;
-            float4* table = reinterpret_cast<float4*>(resp_table);
-            STATIC_CUDA(launch_eresp_tables(n_tenor, dt / dtau, dtau, (int)stride, B, &fr, 1, cub ? resid : nullptr, nres,
-                                            false, table, s));
-            EulerRespParams E;
-            std::memset(&E, 0, sizeof(E));
-            E.P = P;
-            E.frame = block_frame_n(fr.n, (int)stride);
-            E.row = eresp_row(B);
-            E.renorm = (cub || B > kRespSlots + 1) ? 1 : 0;  // as hjm_run
-            STATIC_CUDA(launch_path_fp64_eresp(E, &fr, degs, nres, table, first, nullptr, partials, nullptr, nullptr, s,
-                                               nullptr));
-        } else if (B >= 2 && B <= response_max_dates() && entries <= kStaticRespEntries) {
-            // the response form: its table (zero outside the live entries) into the static array
-            STATIC_CUDA(cudaMemsetAsync(resp_table, 0, sizeof(float4) * entries, s));
-            float4* vtable = reinterpret_cast<float4*>(resp_table);
-            STATIC_CUDA(launch_response_table_vol(n_tenor, dt / dtau, (int)stride, B, false, &P.sv[0][0], vtable, s));
-            // one launch of 24 slots (the static scratch holds no carry)
-            STATIC_CUDA(launch_path_fp64_vresp(n_tenor, P, vtable, nullptr, partials, nullptr, nullptr, s, nullptr, 24));
+        if (contract) {
+            unsigned char* area = reinterpret_cast<unsigned char*>(resp_table);
+            STATIC_CUDA(launch_contract_table(n_tenor, dt / dtau, (int)stride, B, false, false, &P.sv[0][0], area, s));
+            STATIC_CUDA(launch_path_contract(n_tenor, P, area, nullptr, nullptr, partials, nullptr,
+                                             reinterpret_cast<double*>(area + carry_at),
+                                             reinterpret_cast<longlong2*>(area + split_at), result, n_sms, s, nullptr));
         } else {
             STATIC_CUDA(launch_path_fp64(n_tenor, P, poly, nullptr, partials, nullptr, s));
         }
@@ -369,6 +355,7 @@ hjm_status hjm_run_static(void* cuda_stream, int32_t n_tenor, double dtau, const
     double res[kResLen];
     STATIC_CUDA(cudaMemcpyAsync(res, result, sizeof(res), cudaMemcpyDeviceToHost, s));
     STATIC_CUDA(cudaStreamSynchronize(s));
+    if (res[kResErr] != 0.0) return static_fail(HJM_ERR_CUDA, "a wait inside the path kernel ran out");
     for (int j = 0; j < n_tenor; ++j) ee_out[j] = res[kResEE + j];
     cva_out[HJM_CVA_VALUE] = res[kResCVA];
     cva_out[HJM_CVA_STDERR] = res[kResCVAStderr];

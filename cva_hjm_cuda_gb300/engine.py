@@ -122,9 +122,9 @@ class HJMEngine:
         """Transport form of the remainder: "convect" (the remainder, or with a
         table of any shape the whole stochastic curve, over the live tenors
         every step), "response" (impulse-response sums at the sampled tenors:
-        FP64 valuations in double-FP32, in windows of dates; mixed precision
-        and its adjoint without checkpoints in FP32 where the dates the
-        remainder reaches fit 16 slots) or "auto" (the response form where it
+        FP64 valuations, an exact contraction on the tensor cores; mixed
+        precision and its adjoint without checkpoints in FP32 where the dates
+        the remainder reaches fit 16 slots) or "auto" (the response form where it
         applies)."""
         self._check(self.lib.hjm_ctx_set_remainder_form(self.ctx, {"auto": 0, "convect": 1, "response": 2}[form]))
 

@@ -125,36 +125,31 @@ hjm_status hjm_ctx_set_scheme(hjm_ctx* ctx, int32_t scheme);
 hjm_status hjm_ctx_set_vol_decomposition(hjm_ctx* ctx, int32_t enable);
 hjm_status hjm_ctx_vol_decomposition(hjm_ctx* ctx, int32_t* active);
 
-/* Transport form of the remainder.  The pricing reads the stochastic curve only at each
- * date's own tenor.  With the polynomial decomposition the remainder, driven
- * only at the last tenor (the last two for the predictor-corrector), is either
- * convected over the live tenors every step (HJM_REMAINDER_CONVECT) or carried,
- * for each date still to be sampled, as its value and running sum in impulse
- * responses of the convection (HJM_REMAINDER_RESPONSE: one double-FP32 term
- * per such date per step, on the FP32 pipe; the remainder is ~1e-5 of the
- * curve; the polynomial parts S, U, W then advance as double-FP32 sums in a
- * moving frame, with FP64 only at the sampled dates).  With a volatility
- * table of any shape (no decomposition) the whole stochastic curve is either
- * convected with the noise injected at every tenor (four FP64 FMAs per live
- * tenor per step), or carried in the response form as double-FP32 sums of
- * the three factors' impulse responses (three terms per date per step).
- * Every response form takes any number of dates: a run with more than
- * HJM_RESPONSE_MAX_DATES is priced in windows of at most that many dates, one
- * launch each, the later windows passing each path's later cash flows to the
- * earlier ones.  HJM_REMAINDER_AUTO (default) takes the response form for
- * every FP64 valuation.  Both time schemes; the forms agree to rounding
- * (per-path exposures within ~1e-13 of the exposure scale).  Mixed precision
- * with the decomposition carries the remainder as FP32
+/* Transport form of the stochastic curve.  The pricing reads it only at each
+ * date's own tenor.  HJM_REMAINDER_CONVECT moves it over the tenors every step:
+ * with the polynomial decomposition the remainder, driven only at the last
+ * tenor (the last two for the predictor-corrector), else the whole curve with
+ * the noise injected at every tenor.  HJM_REMAINDER_RESPONSE carries, for each
+ * date, its value and running sum in impulse responses of the convection.
+ * FP64: for any market and either scheme the sums over steps and factors of
+ * normal times response are a contraction, which the tensor cores run exactly
+ * on 10-bit slices of both (per-path exposures within ~1e-14 of the exposure
+ * scale of the exact sums); any number of dates, in launches of at most 32
+ * (external normals: 24).  AUTO (default) takes it for every FP64 valuation
+ * whose tables the memory limit allows.
+ * Mixed precision with the decomposition carries the remainder as FP32
  * impulse-response sums (one packed FMA per date per step) when the dates
  * whose responses ever reach 2^-30 of the source fit 16 slots (the 10y swap's
  * 20 dates on 51 tenors: 8), else convects it in FP32 pairs (the 25y swap,
- * the 30y netting set); the two agree to FP32 rounding (~1e-7 of the
+ * the 30y netting set), from 37 dates on only over the tenors that it has
+ * reached and a later date reads; the two agree to FP32 rounding (~1e-7 of the
  * exposure scale).  AUTO and RESPONSE take it where it fits, under either
  * scheme (the predictor-corrector's only when its last date does not sample
  * the last tenor), and in hjm_run_adjoint without checkpoints (Euler); the
  * adjoint with checkpoints, the predictor-corrector's adjoint and MLMC's
  * coupled levels convect.  The report names the form a valuation ran
- * ("remainder"). */
+ * ("remainder").  HJM_RESPONSE_MAX_DATES: dates that one launch holds in
+ * every response form. */
 #define HJM_REMAINDER_AUTO 0
 #define HJM_REMAINDER_CONVECT 1
 #define HJM_REMAINDER_RESPONSE 2
@@ -312,9 +307,9 @@ hjm_status hjm_run_adjoint(hjm_ctx* ctx, int64_t n_paths, int32_t n_steps, doubl
  * stream) and the call is synchronous: it waits for cuda_stream and returns
  * when ee_out [n_tenor] and cva_out [HJM_CVA_OUT_LEN] hold the results.  Its
  * device memory is two fixed static arrays that each GPU loading the library
- * keeps until exit: 8.4 MB of scratch and 4 MB for a response form's table
- * (FP64, or mixed precision's), about 12.4 MB in all; it calls no cudaMalloc, cudaFree or allocating
- * library routine.  Limits: at most
+ * keeps until exit: 8.4 MB of scratch and 48 MB for a response form's table
+ * (FP64: also the sums that its launches pass on), 57 MB in all; it calls no
+ * cudaMalloc, cudaFree or allocating library routine.  Limits: at most
  * HJM_STATIC_MAX_PATHS paths per call (larger runs fail with
  * HJM_ERR_INVALID_ARGUMENT), EE and CVA only (no PFE).  The first call on a
  * device looks up the scratch address (cudaGetSymbolAddress): make that first

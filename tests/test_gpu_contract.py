@@ -111,3 +111,53 @@ def test_whole_waves_and_split_tiles(engine, n_paths, dates):
     _close(x, xc, dates)
     np.testing.assert_allclose(v.ee[:dates], c.ee[:dates], rtol=1e-12, atol=1e-13 * np.max(c.ee))
     assert v.cva == pytest.approx(c.cva, rel=1e-12) and v.cva_stderr == pytest.approx(c.cva_stderr, rel=1e-9)
+
+
+def test_memory_cap_runs_whole_tiles_or_convects():
+    """Under a memory cap that leaves no room for the table the run convects, as
+    if asked to; with the table but without the split tiles' sums it runs its
+    tiles whole (the same integer sums per path, other partial rows)."""
+    from cva_hjm_cuda_gb300.engine import HJMEngine
+
+    cfg = RunConfig(n_paths=5000, seed=3)
+    with HJMEngine(0) as eng:
+        eng.set_market(Market())
+        eng.set_swap(Swap())
+        eng.set_remainder_form("convect")
+        c = eng.run(cfg, "fp64", pfe=False)
+        eng.set_remainder_form("auto")
+        eng.set_memory_limit(eng.memory_in_use())
+        v = eng.run(cfg, "fp64", pfe=False)
+        assert eng.remainder_form() == "convect"
+        np.testing.assert_array_equal(v.ee, c.ee)
+        eng.set_memory_limit(0)
+        eng.run(RunConfig(n_paths=152 * 128, seed=3), "fp64", pfe=False)  # (one whole wave: nothing split)
+        eng.set_memory_limit(eng.memory_in_use())
+        w = eng.run(cfg, "fp64", pfe=False)
+        assert eng.remainder_form() == "response"
+        eng.set_memory_limit(0)
+        s = eng.run(cfg, "fp64", pfe=False)
+    np.testing.assert_allclose(w.ee, s.ee, rtol=1e-13, atol=0)
+    assert w.cva == pytest.approx(s.cva, rel=1e-13) and w.cva == pytest.approx(c.cva, rel=1e-12)
+
+
+@pytest.mark.parametrize("n_tenor,dates,n_paths", [(51, 50, 3000), (61, 60, 20_001), (51, 33, 152 * 128)])
+def test_static_entry_in_windows(n_tenor, dates, n_paths):
+    """The allocation-free entry with one and several windows, split tiles and
+    none, equals the context's run (1e-13: the same integer sums)."""
+    from test_zz_no_alloc import _run_static
+
+    from cva_hjm_cuda_gb300 import _lib
+    from cva_hjm_cuda_gb300.engine import HJMEngine
+
+    mk, sw = _table_market(n_tenor), Swap(n_tenor=n_tenor, n_periods=dates)
+    cfg = RunConfig(n_paths=n_paths, n_steps=25 * dates, dt=0.02, seed=4)
+    with HJMEngine(0) as eng:
+        eng.set_market(mk)
+        eng.set_swap(sw)
+        ref = eng.run(cfg, "fp64", pfe=False)
+    lib = _lib.load()
+    st, ee, cva = _run_static(lib, mk, sw, cfg, "fp64")
+    assert st == 0, lib.hjm_last_error(None)
+    np.testing.assert_allclose(ee, ref.ee, rtol=1e-13, atol=0)
+    assert cva[0] == pytest.approx(ref.cva, rel=1e-13)
