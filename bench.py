@@ -97,8 +97,9 @@ def algorithmic_flops_per_path(n_tenor: int, n_steps: int, stride: int, form: st
     ADD or MUL issues like an FMA, so the fraction is a lower bound on the
     FP64 pipe's use (ncu's pipe utilisation is the direct measure).
 
-    ``remainder="response"`` (FP64): polynomial forms, the FP64 pipe forms the
-    parts and their running sums from the moving-frame sums only at the
+    ``remainder="response"`` (the double-FP32 response form, which the
+    contraction replaced: ``contraction_flops_per_path``): polynomial forms, the
+    FP64 pipe forms the parts and their running sums from the moving-frame sums only at the
     sampled dates (41 flops per date: widening the six sums (6), x = M^a y
     (6), Z += Q(a) y - v (15), the two quadratics at the date's tenor (11) and
     the re-anchoring's rests (3)); the per-step work runs in double-FP32 on the
@@ -230,56 +231,32 @@ def mixed_response_flops_per_path(n_tenor: int, n_steps: int, stride: int, form:
 
 
 def adjoint_response_flops_per_path(n_tenor: int, n_steps: int, stride: int, form: str = "poly_tri") -> int:
-    """FP32 flops per path of the response form's adjoint
-    (adjoint_kernel_resp): its forward pass, the mixed response form's count
-    (``mixed_response_flops_per_path``), and per reverse step the discount
-    seeds into the three moments (3 ADD), the nine coefficient products (9
-    FMA), the moments' step (3 FMA + 1 ADD) and one packed FMA (4 flops) per
-    slot for the remainder's last-tenor adjoint."""
+    """FP32 flops per path of the one-pass adjoint (adjoint_kernel_resp): the
+    mixed response form's count (``mixed_response_flops_per_path``), and per
+    step four running sums per factor (12 ADD) and one packed FMA per factor
+    (12 flops) for each slot of a date still to be sampled."""
     B = n_steps // stride
     ns = mixed_response_slots(n_tenor, n_steps, stride)
-    reverse = (B - 1) * stride * (3 + 18 + 7 + 4 * ns)
-    return mixed_response_flops_per_path(n_tenor, n_steps, stride, form) + reverse
+    sens = sum(stride * (12 + 12 * min(ns, B - b)) for b in range(1, B))
+    return mixed_response_flops_per_path(n_tenor, n_steps, stride, form) + sens
 
 
-def eresp_windows(n_blocks: int, dates: int = 24) -> list[tuple[int, int]]:
-    """The Euler response form's windows of dates, latest first (eresp_windows,
-    every date from 2 on active: ``dates`` of them per window)."""
-    out, h = [], n_blocks
-    while h >= 1:
-        lo = h - dates + 1
-        if lo <= 2:
-            lo = 1
-        out.append((lo, h))
-        h = lo - 1
-    return out
-
-
-def cubic_fp32_flops_per_path(n_tenor: int, n_steps: int, stride: int, nres: int = 2) -> int:
-    """FP32 flops per path of the Euler response form with cubic factors (factor 1
-    constant, factors 2 and 3 cubic) and a residual table, counted as
-    response_fp32_flops_per_path counts the quadratic form: per window, per
-    evolved step up to its last date, each live date slot of the window in
-    groups of four (the residual reaches every tenor, so every date still to be
-    sampled is active): the residual's packed FMAs (4 flops per residual
-    factor) and the renormalisation every fourth step (6 flops / 4), and in the
-    groups that reach the remainder's own prefix (``response_active_prefix``;
-    the first two groups always) its double-FP32 term (30 flops); the parts'
-    moving frame, 9 terms of 26 flops, 4 renormalisations of 6, and the source
-    w = y_W + sigma y_X in double-FP32 (14 flops)."""
-    B = n_steps // stride
-    pre_w = response_active_prefix(n_tenor, n_steps, stride)
-    total = 0
-    for lo, hi in eresp_windows(B, 16):  # with a residual table the windows hold 16 dates
-        roff, nslot = B - hi, hi - max(lo, 2) + 1
-        for b in range(1, hi):
-            live = sum(1 for j in range(max(lo, 2), hi + 1) if j > b)
-            groups = (live + 3) // 4
-            for s_ in range(stride):
-                n_w = min(max(int(pre_w[b * stride + s_]) - roff, 0), nslot)
-                w_groups = min(groups, max(2, (n_w + 3) // 4))
-                total += 4 * groups * (4 * nres + 1.5) + 4 * w_groups * 30 + 9 * 26 + 4 * 6 + 14
-    return int(total)
+def contraction_flops_per_path(n_steps: int, stride: int) -> int:
+    """Tensor-core flops per path of the FP64 contraction (path_kernel_contract)
+    as its instructions run them: windows of at most 32 dates, latest first,
+    each over the steps up to its last date in chunks of 16 (48 normals), per
+    chunk the 14 products of normal slice i and response slice j with i + j <=
+    4 and i <= 3 over the window's columns (value and running sum per date,
+    padded to 16)."""
+    total, hi = 0, n_steps // stride
+    while hi >= 1:
+        lo = 1 if hi - 1 <= 32 else hi - 31
+        slots = max(hi - max(lo, 2) + 1, 0)
+        npad = max((2 * slots + 15) // 16 * 16, 16)
+        chunks = ((hi - 1) * stride + 15) // 16
+        total += chunks * 48 * 14 * npad * 2
+        hi = lo - 1
+    return total
 
 
 class ClockSampler:
@@ -580,57 +557,41 @@ def run_ours(args) -> None:
                                f"{prec}-{n_paths}")
     side = None
     bound = "fp64_pipe" if prec == "fp64" else "fp32_pipe"
-    if prec == "fp64" and remainder == "response" and form == "cubic_resid":
-        flops = cubic_fp32_flops_per_path(mk.n_tenor, n_steps, stride) * n_paths
+    if prec == "fp64" and remainder == "response" and not is_adjoint:
+        # the contraction on the tensor cores; what bounds the kernel is the
+        # issue of the normals beside it (Philox, Box-Muller, slices), whose
+        # share of the pipes the committed ncu capture gives
+        flops = contraction_flops_per_path(n_steps, stride) * n_paths
         achieved = flops / (path_ms * 1e-3) / 1e12
-        peak = extras.get("measured_fma_peak_tflops", {}).get("fp32")
-        bound = "fp32_pipe (double-FP32)"
-        fma_busy = profiled_value("fma_pipe_cycles_active", f"{args.workload}-{n_paths}")
-        side = {"pipe": "fp64 (parts at the sampled dates)", "note": "see the headline workload"}
-    elif prec == "fp64" and remainder == "response" and form == "table":
-        # the table step's response sums, double-FP32 on the FP32 pipe
-        flops = table_response_fp32_flops_per_path(mk.n_tenor, n_steps, stride) * n_paths
-        achieved = flops / (path_ms * 1e-3) / 1e12
-        peak = extras.get("measured_fma_peak_tflops", {}).get("fp32")
-        bound = "fp32_pipe (double-FP32)"
-    elif prec == "fp64" and remainder == "response" and form != "table" and not is_adjoint:
-        # the per-step work is double-FP32 on the FP32 pipe: that is the
-        # roofline; the FP64 pipe only forms the parts at the sampled dates
-        side = {"pipe": "fp64 (parts at the sampled dates)", "algorithmic_flops_per_launch": flops,
-                "achieved": achieved, "peak": peak, "frac": (achieved / peak) if peak else None}
-        flops = response_fp32_flops_per_path(mk.n_tenor, n_steps, stride, form) * n_paths
-        achieved = flops / (path_ms * 1e-3) / 1e12
-        peak = extras.get("measured_fma_peak_tflops", {}).get("fp32")
-        bound = "fp32_pipe (double-FP32)"
-        # the FMA pipe's busy fraction from the committed ncu capture: the
-        # double-FP32 terms are mostly adds, which occupy it as FMAs do
-        fma_busy = profiled_value("fma_pipe_cycles_active", f"{prec}-{n_paths}")
+        peak = _measured_peak("bf16_tflops")
+        bound = "tensor (exact FP16 slices; issue of the normals binds first)"
+        side = {name: profiled_value(name, "fp64-contract") for name in
+                ("alu_pipe_cycles_active", "fma_pipe_cycles_active", "issue_active", "fp64_pipe_cycles_active",
+                 "tensor_pipe_cycles_active")}
     roofline = {"bound": bound, "achieved": achieved, "peak": peak,
                 "unit": "TFLOP/s", "frac": (achieved / peak) if peak else None, "traffic": traffic,
                 "kernel": (f"adjoint_kernel_resp<{mixed_response_slots(mk.n_tenor, n_steps, stride)}>"
                            if is_adjoint and remainder == "response" else
+                           f"adjoint_kernel_conv<{mixed_response_slots(mk.n_tenor, n_steps, stride)},{mk.n_tenor}>"
+                           if is_adjoint and mixed_response_slots(mk.n_tenor, n_steps, stride) else
                            f"adjoint_kernel<{mk.n_tenor},ckpt,{form}>" if is_adjoint else
-                           "path_kernel_fp64_eresp<philox,degs(0,3,3),residual2>"
-                           if prec == "fp64" and remainder == "response" and form == "cubic_resid" else
-                           f"path_kernel_fp64_vresp<{mk.n_tenor},philox>"
-                           if prec == "fp64" and remainder == "response" and form == "table" else
-                           "path_kernel_fp64_eresp<philox,degs(0,1,2)>"
-                           if prec == "fp64" and remainder == "response" else
+                           "path_kernel_contract<philox>" if prec == "fp64" and remainder == "response" else
                            f"path_kernel_fp64<{mk.n_tenor},philox,{form}>" if prec == "fp64" else
                            f"path_kernel_mixed_resp<philox,{form},{mixed_response_slots(mk.n_tenor, n_steps, stride)}>"
                            if remainder == "response" else
+                           f"path_kernel_mixed_conv<{mk.n_tenor},philox,{form}>" if n_steps // stride >= 37 else
                            f"path_kernel_mixed<{mk.n_tenor},philox,{form}>"),
                 "algorithmic_flops_per_launch": flops, "avg_launch_ms": path_ms,
-                "peak_source": "measured live by bench.py (FMA microkernel, this GPU)",
-                "hbm_peak_gbs_measured": _measured_hbm(),
+                "peak_source": ("measured cuBLAS bf16 burst of this GPU type" if bound.startswith("tensor") else
+                                "measured live by bench.py (FMA microkernel, this GPU)"),
+                "hbm_peak_gbs_measured": _measured_peak("hbm_gbs"),
                 # the reference's Euler step, 11 flops per tenor per path-step,
                 # at this run's rate (the kernel runs an exact reformulation
                 # with far fewer operations; not a roofline of this kernel)
                 "reference_equivalent_tflops": 11 * mk.n_tenor * world * n_paths * n_steps * args.steps
                 / elapsed / 1e12 if not is_adjoint else None}
     if side:
-        roofline["fp64_side"] = side
-        roofline["fma_pipe_cycles_active_ncu"] = fma_busy
+        roofline["pipes_ncu_percent"] = side
 
     if not args.no_extras and prec == "fp64":
         if remainder == "response":
@@ -675,15 +636,12 @@ def run_ours(args) -> None:
                                 "quadratic factors (detected in the volatility table): decomposed step" if vol_form_poly
                                 else "volatility table: generic step"),
                    "remainder": remainder,
-                   "arithmetic": (("FP64 deterministic curve, parts at the sampled dates, pricing, discounting "
-                                   "and reductions; per step the stochastic parts S, U, W (moving frame) and the "
-                                   "remainder's response sums in double-FP32 (48-bit) on the FP32 pipe: a path's "
-                                   "exposures within ~2e-13 of the exposure scale of the all-FP64 step "
-                                   "(fp64_convected_form), EE and CVA within 1e-10 of the FP64 oracle"
-                                   if form != "table" else
-                                   "FP64 deterministic curve, pricing, discounting and reductions; per step the "
-                                   "three factors' impulse-response sums (value and running sum per date) in "
-                                   "double-FP32 (48-bit) on the FP32 pipe")
+                   "arithmetic": ("FP64 deterministic curve, pricing, discounting and reductions; the stochastic "
+                                  "curve at the dates and its running sums as an exact contraction on the tensor "
+                                  "cores: FP32 normals in four FP16 slices of 10 bits (the fourth 11), FP64 "
+                                  "responses in five, level sums in FP32 accumulators that add exactly, 64-bit "
+                                  "integer running sums: a path's exposures within 1e-14 of the exposure scale of "
+                                  "the exact sums, EE and CVA within 1e-10 of the FP64 oracle"
                                   if remainder == "response" and prec == "fp64" else None),
                    "path_step": ("one Euler step of one path's whole tenor curve, the reference's unit; the "
                                  "response form computes the same values by exact algebra without evolving every "
@@ -735,10 +693,10 @@ def fp32_roofline(kernel: str, flops_per_launch: float, launch_ms: float, peak32
     return out
 
 
-def _measured_hbm():
+def _measured_peak(name: str):
     f = ROOT / "MEASURED_PEAKS.json"
     try:
-        return json.loads(f.read_text()).get("hbm_gbs")
+        return json.loads(f.read_text()).get(name)
     except (OSError, ValueError):
         return None
 
@@ -930,12 +888,12 @@ def generic_step_run(eng, mk, sw, args, flush, stride, peak64, peak32) -> dict:
             res = eng.fetch()
             form = eng.remainder_form() if prec == "fp64" else "convect"
             fl = algorithmic_flops_per_path(mk.n_tenor, N_STEPS, stride, "table", form) * n
-            if form == "response":  # the double-FP32 response sums, on the FP32 pipe
-                fl, peak = table_response_fp32_flops_per_path(mk.n_tenor, N_STEPS, stride) * n, peak32
+            if form == "response":  # the contraction on the tensor cores
+                fl, peak = contraction_flops_per_path(N_STEPS, stride) * n, _measured_peak("bf16_tflops")
             out[prec] = {"n_paths": n, "remainder": form,
                          "path_steps_per_s": n * N_STEPS / (step_ms * 1e-3), "device_ms_per_step": step_ms,
                          "path_kernel_ms": kern_ms, "achieved_tflops": fl / (kern_ms * 1e-3) / 1e12,
-                         "frac_of_measured_fma_peak": (fl / (kern_ms * 1e-3) / 1e12 / peak) if peak else None,
+                         "frac_of_measured_peak": (fl / (kern_ms * 1e-3) / 1e12 / peak) if peak else None,
                          "cva": res.cva}
     finally:
         eng.vol_decomposition(True)
