@@ -1012,6 +1012,8 @@ static hjm_status enqueue_impl(hjm_ctx* ctx, int64_t n_paths, int32_t n_steps, d
         if (bytes && try_ensure(ctx->split, bytes) && try_ensure(ctx->partials, sizeof(double) * (size_t)rows * R)) {
             split = (longlong2*)ctx->split.p;
             n_ctas = rows;
+        } else {  // (a refused growth may have dropped the smaller buffer)
+            HJM_CUDA(ctx, ctx->partials.ensure(sizeof(double) * (size_t)n_ctas * R));
         }
     }
     cudaStream_t s = ctx->stream;

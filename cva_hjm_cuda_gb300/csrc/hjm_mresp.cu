@@ -204,7 +204,7 @@ int mresp_slots(int nt, double c, double dtau, int stride, int n_blocks, bool pc
     // (the predictor-corrector's date at the last tenor takes a lag -1 term
     // this kernel leaves out)
     if (pc && B == L) return 0;
-    const double thr = std::ldexp(1.0, -30);
+    const double thr = std::ldexp(1.0, -30), reach = std::ldexp(1.0, -46);
     const int M = (B - 1) * stride - 1;  // the longest lag read
     // Euler: G = A^m e_L.  Predictor-corrector: H(l) = w0 G1(l) + w1 G2(l) +
     // w2 G2(l + 1) per unit kappa, G1, G2 the three-point step's responses to
@@ -230,7 +230,7 @@ int mresp_slots(int nt, double c, double dtau, int stride, int n_blocks, bool pc
         }
         const int l = pc ? m - 1 : m;  // the lag this iteration completes
         for (int t = 1; !pc && t < nt; ++t)
-            if (first[t] == 0 && std::fabs(v[t]) >= std::ldexp(1.0, -46)) first[t] = l / stride + 1;
+            if (first[t] == 0 && std::fabs(v[t]) >= reach) first[t] = l / stride + 1;
         if (l >= 0)
             for (int j = 2; j <= B; ++j) {
                 // date j reads lags up to K_j - stride = (j - 1) stride - 1
