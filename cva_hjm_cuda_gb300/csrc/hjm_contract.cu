@@ -61,6 +61,7 @@
 
 #include "hjm_contract.h"
 #include "hjm_kernels.h"
+#include "hjm_walk.cuh"
 
 namespace hjm {
 
@@ -838,40 +839,18 @@ struct ContractLoadings {
     double sv[kFactors][kMaxTenor];
 };
 
-// The step as a walk.  One step moves the curve by h[t] <- a0 h[t] + a1 h[t+1]
-// + a2 h[t+2] (Euler: 1 - c, c, 0; the predictor-corrector: 1 - c + c^2/2,
-// c - c^2, c^2/2) up to the last tenors, whose rows use the backward difference
-// d = h[L] - h[L-1].  That slope does not change over a step, so the rows are
-// the same walk on the curve extended beyond L along d, and with D_t the
-// loading's deviation from that line (zero from L - 1 on)
-//     (A^m S)[j] = S_L + (j - L + m c) d + sum_i f_m(i) D_{j+i},
-// f_m(i) the probability that m steps move i tenors.  Every lag is then
-// independent of the others: a few launches of thousands of threads instead of
-// a recursion over the lags, which is serial and bound by the FP64 pipe's
-// latency (2,450 lags of the 25y swap: 1.2 ms by one CTA; 40 us this way).
-struct WalkParams {
-    double a1, a2;          // r = a / a0 of the recurrence: see below
-    double log_hi, log_lo;  // log a0
-    double b2, inv;         // a2 / (a1 + a2), 1 / (a1 + a2)
-    double rcp[kMaxTenor];  // 1 / (i + 1)
-};
-
 // weights[i M + m] = {f_m(i), G_m(i) = sum_{r <= m} f_r(i)}, i < n.  f_m are
 // the coefficients of p^m, p = a0 + a1 z + a2 z^2: from p (p^m)' = m p' p^m,
 //     (i + 1) a0 f(i+1) = (m - i) a1 f(i) + (2 m - i + 1) a2 f(i-1),
 // and G those of (p^{m+1} - 1) / (p - 1), whose partial sums telescope:
 //     (a1 + a2) G(i) + a2 G(i-1) = 1 - f_{m+1}(0) - .. - f_{m+1}(i),
-// so a rounding fades by a2 / (a1 + a2) a step.  One thread per lag.
+// so a rounding fades by a2 / (a1 + a2) a step.  One thread per lag (hjm_walk.cuh).
 __global__ void contract_weights_kernel(const __grid_constant__ WalkParams K, int M, int n, double2* __restrict__ weights)
 {
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= M) return;
-    auto power = [&](double e) {  // a0^e: the exponent's rounding would cost e log a0 2^-53
-        const double x = e * K.log_hi;
-        return exp(x) * (1.0 + fma(e, K.log_lo, fma(e, K.log_hi, -x)));
-    };
     const double md = m;
-    double f = power(md), f1 = 0.0, h = power(md + 1.0), h1 = 0.0, g = 0.0, tail = 1.0;
+    double f = walk_power(K, md), f1 = 0.0, h = walk_power(K, md + 1.0), h1 = 0.0, g = 0.0, tail = 1.0;
     for (int i = 0; i < n; ++i) {
         tail -= h;
         g = fma(tail, K.inv, -(K.b2 * g));
@@ -1080,16 +1059,7 @@ cudaError_t launch_contract_table(int nt, double c, int stride, int n_blocks, bo
                                align_up((size_t)w[n - 1].chunks * chunk_bytes(w[n - 1].npad)));
     const int M = (n_blocks - 1) * stride;
     double2* weights = resp + (size_t)M * kFactors * (n_blocks - 1);
-    WalkParams K;
-    const double a0 = pc ? 1.0 - c + 0.5 * c * c : 1.0 - c, a1 = pc ? c - c * c : c, a2 = pc ? 0.5 * c * c : 0.0;
-    const long double cl = c, log_a0 = pc ? log1pl(-cl + 0.5L * cl * cl) : log1pl(-cl);
-    K.log_hi = (double)log_a0;
-    K.log_lo = (double)(log_a0 - (long double)K.log_hi);
-    K.a1 = a1 / a0;
-    K.a2 = a2 / a0;
-    K.b2 = a2 / (a1 + a2);
-    K.inv = 1.0 / (a1 + a2);
-    for (int i = 0; i < kMaxTenor; ++i) K.rcp[i] = 1.0 / (double)(i + 1);
+    const WalkParams K = walk_params(c, pc);
     cudaError_t e = cudaMemsetAsync(top, 0, kScaleBytes, s);
     if (e != cudaSuccess) return e;
     contract_weights_kernel<<<(M + 63) / 64, 64, 0, s>>>(K, M, nt - 3, weights);

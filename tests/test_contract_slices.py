@@ -121,3 +121,55 @@ def test_walk_form_of_the_responses(pc, c, M):
             v = _advance(v, np.longdouble(c), pc)
         for j in range(2, 51):
             assert np.max(np.abs(R[:, j] - want[:, j])) <= 48 * 4 * 2.0**-53 * np.max(np.abs(want[:, j]))
+
+
+def _ramp_responses(nt, c, m, j, pc):
+    """mresp_table_kernel's tail sums: G2, CG2 (responses to e_L), G1, CG1 (to
+    e_{L-1}) and G2 a lag on, of date j at lag m."""
+    a0, a1, a2 = (1 - c + 0.5 * c * c, c - c * c, 0.5 * c * c) if pc else (1 - c, c, 0.0)
+    r1, r2, inv, b2 = a1 / a0, a2 / a0, 1 / (a1 + a2), a2 / (a1 + a2)
+    mean = c * (m + 1.0)
+    n = min(128, int(mean + 10.0 * np.sqrt(mean)) + 12)
+    f, h = np.zeros(n), np.zeros(n)
+    f[0], h[0] = np.exp(m * np.log1p(a0 - 1)), np.exp((m + 1) * np.log1p(a0 - 1))
+    for i in range(n - 1):
+        f[i + 1] = ((m - i) * r1 * f[i] + (2 * m - i + 1) * r2 * (f[i - 1] if i else 0.0)) / (i + 1)
+        h[i + 1] = ((m + 1 - i) * r1 * h[i] + (2 * m - i + 3) * r2 * (h[i - 1] if i else 0.0)) / (i + 1)
+    q = nt - 1 - j
+    i = np.arange(n)
+    up = np.maximum(i - q + 1, 0)
+    tail = np.append(np.cumsum(h[::-1])[::-1][1:], 0.0)
+    g = np.zeros(n)
+    for k in range(n):
+        g[k] = tail[k] * inv - (b2 * g[k - 1] if k else 0.0)
+    down = np.where(i >= q - 1, q - i, 0)
+    return (up * f)[::-1].sum(), (up * g).sum(), (down * f)[::-1].sum(), (down * g).sum(), (up * h)[::-1].sum()
+
+
+@pytest.mark.parametrize("nt,c,stride,B,pc", [(51, 0.02, 50, 20, False), (51, 0.02, 50, 24, True), (61, 0.04, 25, 30, True),
+                                              (51, 0.5, 2, 28, False), (35, 0.1, 10, 34, False), (35, 0.5, 2, 33, True)])
+def test_walk_tails_equal_the_recursion_over_the_lags(nt, c, stride, B, pc):
+    """The mixed response table's closed form against the step's recursion in
+    extended precision: entries that count (2^-30 and more) to FP32's rounding,
+    smaller ones to 2^-54, half of that rounding at 2^-30."""
+    L = nt - 1
+    a0, a1, a2 = 1 - c + 0.5 * c * c, c - c * c, 0.5 * c * c
+    M = (B - 1) * stride
+    hist = np.zeros((2, M + 1, nt), dtype=np.longdouble)
+    v = np.zeros((2, nt), dtype=np.longdouble)
+    v[0, L] = v[1, L - 1] = 1
+    for m in range(M + 1):
+        hist[:, m] = v
+        w = v.copy()
+        w[:, :L] += c * (v[:, 1:] - v[:, :L])
+        if pc:
+            w[:, : L - 1] = a0 * v[:, : L - 1] + a1 * v[:, 1:L] + a2 * v[:, 2:]
+        w[:, L] = v[:, L] + c * (v[:, L] - v[:, L - 1])
+        v = w
+    cum = np.cumsum(hist, axis=1)
+    for j in sorted({2, B // 2, B - 1, B}):
+        for m in sorted({0, 1, stride, (j - 1) * stride // 2, (j - 1) * stride - 1}):
+            got = _ramp_responses(nt, c, m, j, pc)
+            want = [hist[0, m, j], cum[0, m, j], hist[1, m, j], cum[1, m, j], hist[0, m + 1, j]]
+            for x, y in list(zip(got, want))[: 5 if pc else 2]:
+                assert abs(x - float(y)) <= max(2.0 ** -24 * abs(float(y)), 2.0 ** -54), (j, m, x, y)
