@@ -579,8 +579,8 @@ def run_ours(args) -> None:
                            f"path_kernel_fp64<{mk.n_tenor},philox,{form}>" if prec == "fp64" else
                            f"path_kernel_mixed_resp<philox,{form},{mixed_response_slots(mk.n_tenor, n_steps, stride)}>"
                            if remainder == "response" else
-                           f"path_kernel_mixed_conv<{mk.n_tenor},philox,{form}>" if n_steps // stride >= 37 else
-                           f"path_kernel_mixed<{mk.n_tenor},philox,{form}>"),
+                           f"path_kernel_mixed<{mk.n_tenor},philox>" if form == "table" else
+                           f"path_kernel_mixed_conv<{mk.n_tenor},philox,{form}>"),
                 "algorithmic_flops_per_launch": flops, "avg_launch_ms": path_ms,
                 "peak_source": ("measured cuBLAS bf16 burst of this GPU type" if bound.startswith("tensor") else
                                 "measured live by bench.py (FMA microkernel, this GPU)"),
@@ -844,7 +844,7 @@ def mixed_vs_fp64(eng, mk, sw, args, stream, flush, fp64_value, peak32=None) -> 
         kname = f"path_kernel_mixed_resp<philox,{form},{mixed_response_slots(mk.n_tenor, N_STEPS, stride)}>"
     else:
         flops = algorithmic_flops_per_path(mk.n_tenor, N_STEPS, stride, form, "convect") * n
-        kname = f"path_kernel_mixed<{mk.n_tenor},philox,{form}>"
+        kname = f"path_kernel_mixed_conv<{mk.n_tenor},philox,{form}>"
     return {
         "value": value, "unit": UNIT, "n_paths": n, "ms_per_step": 1e3 * el / args.steps,
         "path_kernel_ms": kern_ms, "remainder": engine_form,
@@ -1134,7 +1134,7 @@ def netting_set_run(eng, args, flush, peak32=None) -> dict:
     return {"n_paths": n, "n_steps": steps, "n_tenor": 61, "n_swaps": len(ns), "dates": steps // 50,
             "valuation_ms": val_ms, "path_steps_per_s": n * steps / (val_ms * 1e-3),
             "path_kernel_ms": kern_ms,
-            "roofline": fp32_roofline("path_kernel_mixed<61,philox,poly_tri,compact>", flops, kern_ms, peak32,
+            "roofline": fp32_roofline("path_kernel_mixed_conv<61,philox,poly_tri>", flops, kern_ms, peak32,
                                       f"mixed-{n}"),
             "cva": v.cva, "cva_stderr": v.cva_stderr,
             "adjoint_ms_checkpoint_32": adj_ms, "adjoint_cost_in_valuations": adj_ms / val_ms,

@@ -128,10 +128,9 @@ __device__ __forceinline__ void pair_add(float2 (&v)[PairGrid<NT>::H], int i, fl
 template <int NT>
 constexpr int adj_min_ctas() { return NT > 56 ? 4 : 6; }
 
-// WIN: the values of the long convected runs (path_kernel_mixed_conv: POLY,
-// discount sums by LongSums; the curve is stepped whole, which leaves the
-// window's tenors as they are)
-template <int NT, bool CKPT, bool POLY, bool WIN>
+// POLY: the values of path_kernel_mixed_conv (discount sums by LongSums; the
+// curve is stepped whole, which leaves the window's tenors as they are)
+template <int NT, bool CKPT, bool POLY>
 __global__ void __launch_bounds__(kAdjCta, adj_min_ctas<NT>())
     adjoint_kernel(const __grid_constant__ AdjParams A, double* __restrict__ partials, float* __restrict__ ck_h,
                    double* __restrict__ ck_a)
@@ -163,7 +162,6 @@ __global__ void __launch_bounds__(kAdjCta, adj_min_ctas<NT>())
 
     // ---------------------------------------------------------------- forward
     // The same arithmetic as path_kernel_mixed, plus what the sweep needs.
-    static_assert(!WIN || POLY, "the windows are the polynomial form's");
     constexpr int W1 = conv_window(NT, 0), W2 = conv_window(NT, 1);
     MixedPath<NT, POLY> x;
     x.reset();
@@ -175,7 +173,7 @@ __global__ void __launch_bounds__(kAdjCta, adj_min_ctas<NT>())
     auto sample = [&](int i) {
         float value = 0.f;
         double sum = 0.0;
-        if constexpr (WIN) {
+        if constexpr (POLY) {
             if (i > 1) z.template read<1>(x, P, z.start, i, value, sum);
         } else {
             value = x.value(P, i);
@@ -211,7 +209,7 @@ __global__ void __launch_bounds__(kAdjCta, adj_min_ctas<NT>())
     for (int b = 1; b < B; ++b) {
         BlockSums bs;
         bs.reset();
-        if constexpr (WIN) {
+        if constexpr (POLY) {
             const int w = window_start<NT>(M, b);
             if (w != z.start) z.move(x, P, w);
         }
@@ -227,10 +225,10 @@ __global__ void __launch_bounds__(kAdjCta, adj_min_ctas<NT>())
                 // only a segment that holds a date's sampling step (the block's
                 // last step) is ever restarted by the seed pass
                 const bool needed = (b + 1) * stride - 1 < n + K;
-                // (WIN: of the window's start and the parts; the recomputation
+                // (POLY: of the window's start and the parts; the recomputation
                 // adds the date's difference from the start)
                 double part = 0.0;
-                if constexpr (WIN) {
+                if constexpr (POLY) {
                     part = z.zR + z.parts((double)P.tau[inext]) + as_f64(bs.H1) +
                            as_f64(bs.poly<false>(P.tau[inext]));
                 } else {
@@ -255,12 +253,12 @@ __global__ void __launch_bounds__(kAdjCta, adj_min_ctas<NT>())
             const float phi0 = q0, phi1 = q1, phi2 = q2;
             draw_phi<float, false>(nullptr, gpath, lp, P.n_paths, min(n + 1, n_last), P.rk0, P.rk1, q0, q1, q2);
             x.step(M, phi0, phi1, phi2);
-            if constexpr (WIN)
+            if constexpr (POLY)
                 bs.add_at(x, anchor(x));
             else
                 bs.add(x, phi0, phi1, phi2);
         }
-        if constexpr (WIN) {
+        if constexpr (POLY) {
             z.fold(bs.H1, bs.sS, bs.sU, bs.sW, 0.f);
         } else {
             block_sums_up<NT, POLY>(x, hs_s, tid, kCtaA, P, bs, B, [&](int t, float Ht) {
@@ -357,7 +355,7 @@ __global__ void __launch_bounds__(kAdjCta, adj_min_ctas<NT>())
                 xr.W = active ? ck_h[(base + NT + 2) * ld + lp] : 0.f;
                 xr.g = active ? ck_h[(base + NT + 3) * ld + lp] : 1.f;
                 xr.ig = active ? ck_h[(base + NT + 4) * ld + lp] : 1.f;
-                if constexpr (WIN) {
+                if constexpr (POLY) {
                     z.start = window_start<NT>(M, i - 1);
                 } else {
 #pragma unroll
@@ -373,13 +371,13 @@ __global__ void __launch_bounds__(kAdjCta, adj_min_ctas<NT>())
                     const float phi0 = r0, phi1 = r1, phi2 = r2;
                     draw_phi<float, false>(nullptr, gpath, lp, P.n_paths, min(n + 1, ni), P.rk0, P.rk1, r0, r1, r2);
                     xr.step(M, phi0, phi1, phi2);
-                    if constexpr (WIN)
+                    if constexpr (POLY)
                         bs.add_at(xr, anchor(xr));
                     else
                         bs.add(xr, phi0, phi1, phi2);
                 }
                 double part = 0.0;
-                if constexpr (WIN) {
+                if constexpr (POLY) {
                     float v;
                     part = as_f64(bs.H1) + as_f64(z.template climb<1>(xr, P, z.start, i, v)) +
                            as_f64(bs.poly<false>(P.tau[i]));
@@ -761,11 +759,11 @@ int adjoint_columns(int nt, int n_blocks)
 
 int adjoint_cta() { return kAdjCta; }
 
-template <int NT, bool CKPT, bool POLY, bool WIN>
+template <int NT, bool CKPT, bool POLY>
 static cudaError_t launch_adj_t(const AdjParams& A, double* partials, float* ck_h, double* ck_a, cudaStream_t s)
 {
     const size_t smem = adjoint_smem(NT, A.M.P.n_blocks, CKPT);
-    auto k = adjoint_kernel<NT, CKPT, POLY, WIN>;
+    auto k = adjoint_kernel<NT, CKPT, POLY>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     const int64_t grid = (A.M.P.n_paths + kAdjCta - 1) / kAdjCta;
@@ -778,13 +776,10 @@ static cudaError_t launch_adj_nt(const AdjParams& A, bool poly, double* partials
                                  cudaStream_t s)
 {
     const bool ck = A.ckpt_every > 0;
-    if (mixed_windowed(NT, A.M.P.n_blocks, poly))
-        return ck ? launch_adj_t<NT, true, true, true>(A, partials, ck_h, ck_a, s)
-                  : launch_adj_t<NT, false, true, true>(A, partials, ck_h, ck_a, s);
-    if (poly) return ck ? launch_adj_t<NT, true, true, false>(A, partials, ck_h, ck_a, s)
-                        : launch_adj_t<NT, false, true, false>(A, partials, ck_h, ck_a, s);
-    return ck ? launch_adj_t<NT, true, false, false>(A, partials, ck_h, ck_a, s)
-              : launch_adj_t<NT, false, false, false>(A, partials, ck_h, ck_a, s);
+    if (poly) return ck ? launch_adj_t<NT, true, true>(A, partials, ck_h, ck_a, s)
+                        : launch_adj_t<NT, false, true>(A, partials, ck_h, ck_a, s);
+    return ck ? launch_adj_t<NT, true, false>(A, partials, ck_h, ck_a, s)
+              : launch_adj_t<NT, false, false>(A, partials, ck_h, ck_a, s);
 }
 
 cudaError_t launch_adjoint(int nt, const AdjParams& A, bool poly, double* partials, float* ck_h, double* ck_a,

@@ -108,8 +108,8 @@ struct PathSens {
 // A tile's end, for both forward forms: exposures (cash flows cf, rows 1..B of
 // kAdjCta columns; e_s may lie one row above a float cf), EE and CVA sums,
 // seeds, the coefficients' sums and the partial row `out`.
-template <int NS, typename CF>
-__device__ __forceinline__ void adjoint_tile_end(const MixedParams& M, const CF* cf_s, float* e_s, float* xs_s,
+template <int NS>
+__device__ __forceinline__ void adjoint_tile_end(const MixedParams& M, const float* cf_s, float* e_s, float* xs_s,
                                                  float* ds_s, double* red_s, const float4* sens_p,
                                                  const PathSens<NS>& sn, bool active, double* __restrict__ out)
 {
@@ -321,32 +321,16 @@ __global__ void __launch_bounds__(kAdjCta, adj_resp_ctas(NS))
 }
 
 // The same for the convected form (checkpoint_every > 0 where the dates the
-// remainder reaches fit the slots): the values are path_kernel_mixed's, tenor
-// by tenor, the derivatives as above, so no state is kept and no normal drawn
-// twice.  Shared memory per thread: FP64 discount sums (then cash flows), the
-// curve at the block start (then exposures), x_i (xbar_i), D_i (abar_i).
-struct AdjConvLayout {
-    size_t acc, hs, xs, ds, red, total;
-};
-
-__host__ __device__ inline AdjConvLayout adj_conv_layout(int B, int R)
-{
-    AdjConvLayout L;
-    const size_t rows = (size_t)B + 1;
-    L.acc = 0;
-    L.hs = align128(rows * 8 * kAdjCta);
-    L.xs = align128(L.hs + (rows + 1) * kAdjCta * 4);
-    L.ds = align128(L.xs + rows * kAdjCta * 4);
-    L.red = align128(L.ds + rows * kAdjCta * 4);
-    L.total = align128(L.red + (size_t)(kAdjCta / 32) * R * 8);
-    return L;
-}
-
+// remainder reaches fit the slots): the values are path_kernel_mixed_conv's
+// (stepped whole, which leaves the window's tenors as they are), the derivatives
+// as above, so no state is kept and no normal drawn twice.
+//
 // Checkpoints every 32 steps on the 10y swap, 256k paths: 4.45 ms with the
-// state written, the segments recomputed and the sweep -> 2.06 ms (of which
-// the convected valuation is 1.5); 12y (16 slots) 3.07 ms.  Whole warps per
+// state written, the segments recomputed and the sweep -> 2.00 ms (of which
+// the convected valuation is 1.3); 12y (16 slots) 3.01 ms.  Whole warps per
 // scheduler: 6 CTAs with 8 slots (168 registers; 7 take 2.96 ms, 4 2.42),
-// 4 with 16 or with 61 tenors; steps unrolled by 2 (by 1 2.18, by 5 2.20).
+// 4 with 16 or with 61 tenors; steps unrolled by 2 (by 1 2.18, by 5 2.20).  The
+// window's start as a constant of the loop: selected per step 2.16 ms.
 constexpr int adj_conv_ctas(int ns, int nt) { return ns <= 8 && nt <= 56 ? 6 : 4; }
 
 template <int NS, int NT>
@@ -356,17 +340,19 @@ __global__ void __launch_bounds__(kAdjCta, adj_conv_ctas(NS, NT))
                         int64_t n_tiles)
 {
     constexpr int C = kAdjCta;
+    constexpr int W1 = conv_window(NT, 0), W2 = conv_window(NT, 1);
     const PathParams<float>& P = M.P;
     extern __shared__ __align__(128) unsigned char smem[];
     const int tid = threadIdx.x;
     const int B = P.n_blocks;
     const int R = 3 * B + 12;
-    const AdjConvLayout Ly = adj_conv_layout(B, R);
-    double* acc_s = reinterpret_cast<double*>(smem + Ly.acc);
-    float* hs_s = reinterpret_cast<float*>(smem + Ly.hs);
+    const AdjRespLayout Ly = adj_resp_layout(B, R);
+    float* cf_s = reinterpret_cast<float*>(smem + Ly.cf);
     float* xs_s = reinterpret_cast<float*>(smem + Ly.xs);
     float* ds_s = reinterpret_cast<float*>(smem + Ly.ds);
     double* red_s = reinterpret_cast<double*>(smem + Ly.red);
+    // (in shared memory: read and written once a block)
+    LongSums<NT, false>& z = reinterpret_cast<LongSums<NT, false>*>(smem + align128(Ly.total))[tid];
     float4* sens_p = sens + (size_t)blockIdx.x * (B - 1) * kFactors * C + tid;
     const int stride = P.stride;
     const int n_last = B * stride - 1;
@@ -379,24 +365,25 @@ __global__ void __launch_bounds__(kAdjCta, adj_conv_ctas(NS, NT))
         x.reset();
         PathSens<NS> sn;
         sn.reset();
-        for (int i = 0; i <= B; ++i) acc_s[i * C + tid] = 0.0;
-        for (int t = 0; t <= B + 1; ++t) hs_s[t * C + tid] = 0.f;
-        auto sample = [&](int i) {
-            const double xv = P.psamp[i] + (double)x.value(P, i);
-            const double a = P.psum[i] + acc_s[i * C + tid];
+        z.reset();
+        auto price = [&](int i, float value, double sum) {
+            const double xv = P.psamp[i] + (double)value;
+            const double a = P.psum[i] + sum;
             const float D = expf((float)(-a * P.dt));
             const float mm = (float)P.m;
             const float L = mm * expm1f((float)xv / mm);
-            acc_s[i * C + tid] = (double)(D * ((float)P.payA[i] * L - (float)P.payB[i]));
+            cf_s[i * C + tid] = D * ((float)P.payA[i] * L - (float)P.payB[i]);
             xs_s[i * C + tid] = (float)xv;
             ds_s[i * C + tid] = D;
         };
-        sample(1);
+        price(1, 0.f, 0.0);
         float q0, q1, q2;
         draw_phi<float, false>(nullptr, gpath, lp, P.n_paths, min(stride, n_last), P.rk0, P.rk1, q0, q1, q2);
         BlockSums bs;
-        auto steps = [&](auto live_c, int b) {
-            constexpr int LIVE = decltype(live_c)::value;
+        // block b with the first LIVE slots' responses, on the tenors from S0 (0:
+        // on all, the window's start w selected)
+        auto steps = [&](auto live_c, auto s0_c, int b, int w) {
+            constexpr int LIVE = decltype(live_c)::value, S0 = decltype(s0_c)::value;
             const float4* row = resp + (size_t)b * stride * (NS / 2);
 #pragma unroll 2
             for (int s = 0; s < stride; ++s) {
@@ -410,39 +397,53 @@ __global__ void __launch_bounds__(kAdjCta, adj_conv_ctas(NS, NT))
                     sn.respond(u, make_float2(e.x, e.y), make_float2(e.z, e.w));
                 }
                 sn.advance(phi0, phi1, phi2);
-                x.step(M, phi0, phi1, phi2);
-                bs.add(x, phi0, phi1, phi2);
+                x.template step<S0>(M, phi0, phi1, phi2);
+                bs.add_at(x, S0        ? pair_tenor<NT>(x.h, S0)
+                             : w == W2 ? pair_tenor<NT>(x.h, W2)
+                                       : pair_tenor<NT>(x.h, W1));
             }
         };
         for (int b = 1; b < B; ++b) {
             bs.reset();
+            const int w = window_start<NT>(M, b);
+            if (w != z.start) z.move(x, P, w);
             x.begin_block(P, b);
-            if (b < live.half)
-                steps(std::integral_constant<int, NS>(), b);
+            using std::integral_constant;
+            const integral_constant<int, NS> all;
+            const integral_constant<int, NS / 2> half;
+            const integral_constant<int, 0> none;
+            const integral_constant<int, 1> whole;
+            if (b < live.none && w > 1)
+                steps(all, none, b, w);
+            else if (b < live.half)
+                steps(all, whole, b, w);
             else if (b < live.none)
-                steps(std::integral_constant<int, NS / 2>(), b);
+                steps(half, whole, b, w);
+            else if (w == 1)
+                steps(none, whole, b, w);
+            else if (w == W1)
+                steps(none, integral_constant<int, W1>(), b, w);
             else
-                steps(std::integral_constant<int, 0>(), b);
-            block_sums_up<NT, true>(x, hs_s, tid, C, P, bs, B, [&](int t, float Ht) {
-                if (t > b) acc_s[t * C + tid] += as_f64(Ht);
-            });
-#pragma unroll
-            for (int t = 1; t < NT; ++t)
-                if (t <= B + 1) hs_s[t * C + tid] = x.rem(t);
-            sample(b + 1);
+                steps(none, integral_constant<int, W2>(), b, w);
+            z.fold(bs.H1, bs.sS, bs.sU, bs.sW, 0.f);
+            float value;
+            double sum;
+            z.template read<1>(x, P, z.start, b + 1, value, sum);
+            price(b + 1, value, sum);
             sn.store(sens_p, b);
         }
-        adjoint_tile_end<NS>(M, acc_s, hs_s, xs_s, ds_s, red_s, sens_p, sn, active, partials + (size_t)tile * R);
+        adjoint_tile_end<NS>(M, cf_s, cf_s + C, xs_s, ds_s, red_s, sens_p, sn, active, partials + (size_t)tile * R);
         __syncthreads();  // (the next tile writes the rows and sums just read)
     }
 }
 
-// conv_nt: the tenors of the convected forward form, 0 for the response form
+// (the convected form's running sums behind the layout)
 size_t adjoint_resp_smem(int n_blocks, int conv_nt)
 {
-    const int R = 3 * n_blocks + 12;
-    return conv_nt ? adj_conv_layout(n_blocks, R).total : adj_resp_layout(n_blocks, R).total;
+    return adj_resp_layout(n_blocks, 3 * n_blocks + 12).total + (conv_nt ? sizeof(LongSums<51, false>) * kAdjCta : 0);
 }
+
+// conv_nt: the tenors of the convected forward form, 0 for the response form
 
 int adjoint_resp_grid(int64_t n_paths, int ns, int conv_nt, int n_sms)
 {

@@ -259,16 +259,12 @@ __global__ void __launch_bounds__(kFp64Cta, 4)
 // Shared memory per thread: acc (B+1) FP64 discount sums, whose slot i holds
 // date i's cash flow once tenor i is sampled; hs (B+2) FP32 curve at the block
 // start, reused for the exposure tile at the end.
-// Occupancy: 512 threads per SM by the registers (<= 128 per thread; 112 with
-// polynomial factors, 4 CTAs of 128).  Capped at 96 registers (5 CTAs, 20
-// warps) the polynomial form does not spill but ran slower (20.8 ms against
-// 20.5 at 4,194,304 paths).
-template <int NT, bool EXT, bool POLY, int C, bool CUB = false>
+// Occupancy: 512 threads per SM by the registers (<= 128 per thread).
+template <int NT, bool EXT, int C>
 __global__ void __launch_bounds__(C, 512 / C)
     path_kernel_mixed(const __grid_constant__ MixedParams M, const double* __restrict__ ext,
                       double* __restrict__ partials, float* __restrict__ estore)
 {
-    static_assert(!CUB || POLY, "the cubic part extends the polynomial form");
     const PathParams<float>& P = M.P;
     extern __shared__ __align__(128) unsigned char smem[];
     const int tid = threadIdx.x;
@@ -284,7 +280,7 @@ __global__ void __launch_bounds__(C, 512 / C)
     const bool active = lp < P.n_paths;
     const uint64_t gpath = P.path_offset + (uint64_t)lp;
 
-    MixedPath<NT, POLY, CUB> x;
+    MixedPath<NT, false> x;
     x.reset();
     for (int i = 0; i < rows; ++i) acc_s[i * C + tid] = 0.0;
     for (int t = 0; t <= B + 1; ++t) hs_s[t * C + tid] = 0.f;
@@ -310,7 +306,6 @@ __global__ void __launch_bounds__(C, 512 / C)
         BlockSums bs;
         bs.reset();
         x.begin_block(P, b);
-#pragma unroll(POLY ? 2 : 1)  // ping-pong the normals drawn ahead instead of copying them
         for (int s = 0; s < P.stride; ++s) {
             const int n = b * P.stride + s;
             const float phi0 = q0, phi1 = q1, phi2 = q2;
@@ -319,10 +314,10 @@ __global__ void __launch_bounds__(C, 512 / C)
             bs.add(x, phi0, phi1, phi2);
         }
         // block sums of tenors 2 .. B; fold (b, B] into FP64
-        block_sums_up<NT, POLY>(x, hs_s, tid, C, P, bs, B, [&](int t, float Ht) {
+        block_sums_up<NT, false>(x, hs_s, tid, C, P, bs, B, [&](int t, float Ht) {
             if (t > b) acc_s[t * C + tid] += as_f64(Ht);
         });
-        // the block-end curve (POLY: its convected part) is the next block's start
+        // the block-end curve is the next block's start
 #pragma unroll
         for (int t = 1; t < NT; ++t)
             if (t <= B + 1) hs_s[t * C + tid] = x.rem(t);
@@ -332,11 +327,11 @@ __global__ void __launch_bounds__(C, 512 / C)
     mixed_epilogue<double, C>(P, acc_s, hs_s, red_s, partials, estore, cta_base, active);
 }
 
-// The convected form of long runs (polynomial factors, many dates) on the
-// tenors that matter.  In block b (from step b stride on) the remainder
+// The convected form of the polynomial factors on the tenors that matter.  In
+// block b (from step b stride on) the remainder
 // * holds nothing that counts below the tenor its source has reached (2^-46 per
-//   unit of the source, MixedParams::win; at 2^-30 the netting set's CVA moves
-//   by 2e-8, and the windows would be only half a tenor narrower), and
+//   unit of the source, MixedParams::win; 2^-30 would make the windows only half
+//   a tenor narrower), and
 // * is read by no later date at or below tenor b: information moves down the
 //   tenors only,
 // so a block convects tenors S0 .. L, S0 the largest window start (thirds of
@@ -345,14 +340,17 @@ __global__ void __launch_bounds__(C, 512 / C)
 // block starts in shared memory, 0.25 KB per path at 60 dates instead of 0.5, so
 // the registers bound the occupancy (16 warps per SM instead of 14).
 // 512k paths: 25y quadratic 7.15 -> 5.95 ms, 25y cubic 7.66 -> 6.23, the
-// 61-tenor netting set 9.61 -> 7.39 (with the windows alone 6.54 and 9.53).
+// 61-tenor netting set 9.61 -> 7.39 (with the windows alone 6.54 and 9.53); 15y at
+// 256k paths 2.14 -> 1.94, the 10y swap convected 1.37 -> 1.30.
 // Steps unrolled by 2: 7.0 ms by 1 on the cubic run, 6.6 by 3.
+// CTAs of 64 paths, as the adjoint's (the same partial sums; 128 run as fast).
+constexpr int kConvCta = 64;
 template <int NT, bool EXT, bool CUB>
-__global__ void __launch_bounds__(kCta, 512 / kCta)
+__global__ void __launch_bounds__(kConvCta, 512 / kConvCta)
     path_kernel_mixed_conv(const __grid_constant__ MixedParams M, const double* __restrict__ ext,
                            double* __restrict__ partials, float* __restrict__ estore)
 {
-    constexpr int C = kCta;
+    constexpr int C = kConvCta;
     const PathParams<float>& P = M.P;
     extern __shared__ __align__(128) unsigned char smem[];
     const int tid = threadIdx.x;
@@ -428,16 +426,12 @@ __host__ __device__ inline size_t mixed_smem_bytes(int nt, int n_blocks, int cta
     return ((head + 7) & ~(size_t)7) + 2 * (cta / 32) * 8;
 }
 
-// The windowed form where the general kernel's shared memory (FP64 sums and
-// block starts per tenor) leaves fewer than the 4 CTAs that the registers
-// allow: 37 dates and more.  Shorter convected runs keep the kernel whose
-// values the adjoint's sweeps repeat bit for bit.
-bool mixed_windowed(int nt, int n_blocks, bool poly)
+inline size_t conv_smem_bytes(int n_blocks)  // path_kernel_mixed_conv
 {
-    return poly && mixed_smem_bytes(nt, n_blocks) > (size_t)228 * 1024 / 4;
+    return (size_t)(n_blocks + 2) * kConvCta * sizeof(float) + 2 * (kConvCta / 32) * 8;
 }
 
-// Paths per CTA of the mixed kernel.  The table step keeps FP64 sums per tenor,
+// Paths per CTA of the mixed kernels.  The table step keeps FP64 sums per tenor,
 // so with many dates its shared memory bounds the occupancy and 64-thread CTAs
 // pack an SM more finely (25y on 51 tenors: 79 KB per CTA of 128, 2 per SM; 5
 // of 64, 10 warps instead of 8).  Otherwise the registers bound it, whatever
@@ -445,7 +439,7 @@ bool mixed_windowed(int nt, int n_blocks, bool poly)
 constexpr int kMixedSmallCta = 64;
 inline int mixed_cta(int nt, int n_blocks, bool poly)
 {
-    if (mixed_windowed(nt, n_blocks, poly)) return kCta;
+    if (poly) return kConvCta;
     return mixed_smem_bytes(nt, n_blocks) > (size_t)228 * 1024 / 4 ? kMixedSmallCta : kCta;
 }
 
@@ -662,21 +656,16 @@ cudaError_t launch_path_fp64(int nt, const PathParams<double>& P, bool poly, con
     return cudaErrorInvalidValue;
 }
 
-template <int NT, bool EXT, bool POLY, bool CUB = false>
-static cudaError_t launch_mixed_t(const MixedParams& M, const double* ext, double* partials, float* estore,
-                                  cudaStream_t s)
+template <int NT, bool EXT>
+static cudaError_t launch_mixed_t(const MixedParams& M, bool poly, bool cub, const double* ext, double* partials,
+                                  float* estore, cudaStream_t s)
 {
-    const int cta = mixed_cta(NT, M.P.n_blocks, POLY);
-    size_t smem = mixed_smem_bytes(NT, M.P.n_blocks, cta);
-    auto k = path_kernel_mixed<NT, EXT, POLY, kCta, CUB>;
-    if constexpr (POLY) {
-        if (mixed_windowed(NT, M.P.n_blocks, POLY)) {
-            k = path_kernel_mixed_conv<NT, EXT, CUB>;
-            smem = mresp_smem_bytes(M.P.n_blocks);  // (cash flows only, as the response form)
-        }
-    } else {
-        if (cta == kMixedSmallCta) k = path_kernel_mixed<NT, EXT, false, kMixedSmallCta>;
-    }
+    const int B = M.P.n_blocks, cta = mixed_cta(NT, B, poly);
+    auto k = cub    ? path_kernel_mixed_conv<NT, EXT, true>
+             : poly ? path_kernel_mixed_conv<NT, EXT, false>
+             : cta == kMixedSmallCta ? path_kernel_mixed<NT, EXT, kMixedSmallCta>
+                                     : path_kernel_mixed<NT, EXT, kCta>;
+    const size_t smem = poly ? conv_smem_bytes(B) : mixed_smem_bytes(NT, B, cta);
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     const int64_t grid = (M.P.n_paths + cta - 1) / cta;
@@ -688,12 +677,8 @@ template <int NT>
 static cudaError_t launch_mixed_nt(const MixedParams& M, bool poly, bool cub, const double* ext, double* partials,
                                    float* estore, cudaStream_t s)
 {
-    if (cub) return ext ? launch_mixed_t<NT, true, true, true>(M, ext, partials, estore, s)
-                        : launch_mixed_t<NT, false, true, true>(M, ext, partials, estore, s);
-    if (ext) return poly ? launch_mixed_t<NT, true, true>(M, ext, partials, estore, s)
-                         : launch_mixed_t<NT, true, false>(M, ext, partials, estore, s);
-    return poly ? launch_mixed_t<NT, false, true>(M, ext, partials, estore, s)
-                : launch_mixed_t<NT, false, false>(M, ext, partials, estore, s);
+    return ext ? launch_mixed_t<NT, true>(M, poly, cub, ext, partials, estore, s)
+               : launch_mixed_t<NT, false>(M, poly, cub, ext, partials, estore, s);
 }
 
 cudaError_t launch_path_mixed(int nt, const MixedParams& M, bool poly, const double* ext, double* partials,

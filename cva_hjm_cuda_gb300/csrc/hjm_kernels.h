@@ -52,11 +52,11 @@ struct MixedParams {
     float svcx[kFactors];
     float k3f;       // c dtau^3
     float src3f;     // 3 (T_L - centre): the cubic's share of the remainder's source
-    int win[2];      // the long convected runs' windows: before block win[i] the remainder holds
+    int win[2];      // the convected runs' windows: before block win[i] the remainder holds
                      // nothing that counts below tenor conv_window(nt, i)
 };
 
-// The long convected runs' windows of the remainder: thirds of the tenors (with
+// The convected runs' windows of the remainder: thirds of the tenors (with
 // quarters the loops' four bodies outgrow the instruction cache: 6.39 ms at
 // 512k paths of the cubic 25y run against 6.23; halves 6.40).
 __host__ __device__ constexpr int conv_window(int nt, int i) { return (i + 1) * nt / 3; }
@@ -106,9 +106,7 @@ cudaError_t launch_path_mixed_resp(const MixedParams& M, int ns, const RespLive&
 bool path_tenor_supported(int nt);
 size_t path_smem(int nt, int n_blocks, bool mixed);
 // paths per CTA of the Euler path kernel of a run (one partial-sum row each):
-// FP64 64; mixed 128, or 64 with the compact sums (polynomial factors, many dates)
-// the long convected runs, on windows of the tenors (polynomial factors)
-bool mixed_windowed(int nt, int n_blocks, bool poly);
+// FP64 64; mixed 64 with polynomial factors, else 128, or 64 with many dates
 int path_cta(bool mixed, int nt, int n_blocks, bool poly);
 
 // Column sums into sums[0 .. R) and the results (result cleared before on the

@@ -268,7 +268,7 @@ __device__ __forceinline__ void block_sums_up(const MixedPath<NT, POLY, CUB>& x,
     }
 }
 
-// The start of the window of tenors that block b of a long convected run needs
+// The start of the window of tenors that block b of a convected run needs
 // (polynomial factors): the remainder has not reached below it (MixedParams::win)
 // or no later date reads below it.
 template <int NT>
@@ -278,7 +278,7 @@ __device__ __forceinline__ int window_start(const MixedParams& M, int b)
     return b < M.win[1] || b + 1 >= W2 ? W2 : b < M.win[0] || b + 1 >= W1 ? W1 : 1;
 }
 
-// Running sums over all steps of a long convected run.  The convected
+// Running sums over all steps of a convected run.  The convected
 // remainder starts at zero and moves by hc' = A hc (+ the source at L), so the
 // running sum R[t] of tenor t over the steps' results telescopes along the
 // tenors:

@@ -140,9 +140,8 @@ hjm_status hjm_ctx_vol_decomposition(hjm_ctx* ctx, int32_t* active);
  * Mixed precision with the decomposition carries the remainder as FP32
  * impulse-response sums (one packed FMA per date per step) when the dates
  * whose responses ever reach 2^-30 of the source fit 16 slots (the 10y swap's
- * 20 dates on 51 tenors: 8), else convects it in FP32 pairs (the 25y swap,
- * the 30y netting set), from 37 dates on only over the tenors that it has
- * reached and a later date reads; the two agree to FP32 rounding (~1e-7 of the
+ * 20 dates on 51 tenors: 8), else convects it in FP32 over the tenors
+ * that it has reached and a later date reads (the 25y swap, the 30y netting set); the two agree to FP32 rounding (~1e-7 of the
  * exposure scale).  AUTO and RESPONSE take it where it fits, under either
  * scheme (the predictor-corrector's only when its last date does not sample
  * the last tenor), and in hjm_run_adjoint without checkpoints (Euler); the
