@@ -831,14 +831,14 @@ static hjm_status ensure_contract_table(hjm_ctx* ctx, const RunShape& sh, double
         for (int t = 0; t < nt; ++t) key[(size_t)k * nt + t] = sv[k * kMaxTenor + t];
     hjm_ctx::ContractKey& k = ctx->contract_key;
     if (!ctx->resp_used) HJM_CUDA(ctx, cudaEventCreateWithFlags(&ctx->resp_used, cudaEventDisableTiming));
-    if (k.valid && k.nt == nt && k.stride == sh.stride && k.B == sh.B && k.c == c && k.scheme == ctx->scheme &&
-        k.ext == ext && k.sv == key)
-        return HJM_OK;
+    const bool same_shape = k.valid && k.nt == nt && k.stride == sh.stride && k.B == sh.B && k.c == c &&
+                            k.scheme == ctx->scheme && k.ext == ext;
+    if (same_shape && k.sv == key) return HJM_OK;
     k.valid = false;
     HJM_CUDA(ctx, cudaStreamWaitEvent(s, ctx->resp_used, 0));
     HJM_CUDA(ctx, launch_contract_table(nt, c, sh.stride, sh.B, ctx->scheme == HJM_SCHEME_PREDICTOR_CORRECTOR, ext,
-                                        sv, ctx->contract.p, s));
-    ctx->stat_launches += 2 + contract_windows(sh.B, sh.stride, ext, nullptr);
+                                        sv, same_shape, ctx->contract.p, s));
+    ctx->stat_launches += (same_shape ? 1 : 2) + contract_windows(sh.B, sh.stride, ext, nullptr);
     k.nt = nt;
     k.stride = sh.stride;
     k.B = sh.B;

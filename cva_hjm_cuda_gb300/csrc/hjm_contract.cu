@@ -757,12 +757,15 @@ __global__ void __launch_bounds__(kThreads, 1)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(kTmemCols) : "memory");
 }
 
-// Prices the split tiles from their sums: a CTA takes 32 paths (lane = path),
-// its four warps every fourth date, so that few paths still reach many SMs' FP64
-// pipes (18 cycles an instruction and SM, ~45 per date and path).  Partial-sum
-// rows and exposure rows as the path kernel's, one row per 32 paths from row0.
+// Prices the split tiles from their sums: a CTA takes 32 paths (lane = path), its
+// warps every kPriceWarps-th date: a date is ~45 FP64 instructions in a chain,
+// bound by their latency until many warps share an SM's pipe (18 cycles an
+// instruction).  A 128-path call of the 10y run 125 -> 117 us against four
+// warps; sixteen the same.  Partial-sum rows and exposure rows as the path
+// kernel's, one row per 32 paths from row0.
+constexpr int kPriceWarps = 8;
 template <bool EXT>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(32 * kPriceWarps)
     contract_price_kernel(const __grid_constant__ ContractParams Q, const double* __restrict__ scale,
                           const double* __restrict__ ext_scale, int64_t row0, double* __restrict__ partials,
                           double* __restrict__ estore, double* __restrict__ carry)
@@ -778,7 +781,7 @@ __global__ void __launch_bounds__(128)
     const longlong2* sums = Q.sums + (size_t)(blockIdx.x / 4) * (Q.W.npad / 2) * kContractTile + in_tile;
     double rs = 1.0;
     if constexpr (EXT) rs = __ldg(ext_scale + 2 * (active ? lp : 0) + 1);
-    for (int i = lo + warp; i <= hi; i += 4) {
+    for (int i = lo + warp; i <= hi; i += kPriceWarps) {
         double sx = 0.0, sa = 0.0;
         longlong2 v = make_longlong2(0, 0);
         if (i >= 2) {
@@ -822,7 +825,7 @@ __global__ void __launch_bounds__(128)
     }
     __syncthreads();
     const int j1 = top ? B : hi - 1;
-    for (int j = lo - 1 + warp; j <= j1; j += 4) {
+    for (int j = lo - 1 + warp; j <= j1; j += kPriceWarps) {
         const double e = e_s[j - lo + 1][lane];
         const double sum = warp_sum(e);
         if (lane == 0) partials[(size_t)(row0 + blockIdx.x) * R + j] = sum;
@@ -1049,7 +1052,7 @@ size_t contract_table_bytes(int stride, int n_blocks, bool ext)
 }
 
 cudaError_t launch_contract_table(int nt, double c, int stride, int n_blocks, bool pc, bool ext, const double* sv,
-                                  void* table, cudaStream_t s)
+                                  bool same_shape, void* table, cudaStream_t s)
 {
     if (nt < 35 || nt > kMaxTenor || n_blocks < 1 || n_blocks >= nt || stride < 1) return cudaErrorInvalidValue;
     ContractLoadings S;
@@ -1066,7 +1069,7 @@ cudaError_t launch_contract_table(int nt, double c, int stride, int n_blocks, bo
     const WalkParams K = walk_params(c, pc);
     cudaError_t e = cudaMemsetAsync(top, 0, kScaleBytes, s);
     if (e != cudaSuccess) return e;
-    contract_weights_kernel<<<(M + 63) / 64, 64, 0, s>>>(K, M, nt - 3, weights);
+    if (!same_shape) contract_weights_kernel<<<(M + 63) / 64, 64, 0, s>>>(K, M, nt - 3, weights);
     contract_response_kernel<<<dim3((M + 127) / 128, n_blocks - 1), 128, 0, s>>>(nt, c, stride, n_blocks, S, weights,
                                                                                  top, resp);
     for (int i = 0; i < n; ++i) {
@@ -1154,7 +1157,7 @@ cudaError_t launch_path_contract(int nt, const PathParams<double>& P, const void
                     Q, (const unsigned char*)table, ext, ext_scale, partials, estore, carry, result);
                 ++count;
             }
-            price<<<(unsigned)(4 * split), 128, 0, s>>>(Q, (const double*)table, ext_scale, whole, partials, estore, carry);
+            price<<<(unsigned)(4 * split), 32 * kPriceWarps, 0, s>>>(Q, (const double*)table, ext_scale, whole, partials, estore, carry);
             ++count;
         }
         e = cudaGetLastError();

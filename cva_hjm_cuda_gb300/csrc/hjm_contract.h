@@ -36,9 +36,11 @@ size_t contract_table_bytes(int stride, int n_blocks, bool ext);
 // Builds the table on the stream (two launches and one per window) from the loadings sv
 // [kFactors][kMaxTenor] (sqrt(dt) sigma_k; the predictor-corrector's
 // N-projected ones): the impulse responses of the Euler or the three-point
-// step, sliced for the contraction.
+// step, sliced for the contraction.  same_shape: the table holds that of the same
+// run shape and scheme with other loadings, whose walk weights serve again (one
+// launch and 34 us less, whatever the shape: serial FP64 latency).
 cudaError_t launch_contract_table(int nt, double c, int stride, int n_blocks, bool pc, bool ext, const double* sv,
-                                  void* table, cudaStream_t s);
+                                  bool same_shape, void* table, cudaStream_t s);
 
 // Row scales of external normals [path][step][3]: out[2 p] = 2^-e, out[2 p +
 // 1] = 2^e with e >= 0 the least that brings every |normal| of path p below 8

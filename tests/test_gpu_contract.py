@@ -161,3 +161,34 @@ def test_static_entry_in_windows(n_tenor, dates, n_paths):
     assert st == 0, lib.hjm_last_error(None)
     np.testing.assert_allclose(ee, ref.ee, rtol=1e-13, atol=0)
     assert cva[0] == pytest.approx(ref.cva, rel=1e-13)
+
+
+def test_table_of_another_market_in_the_same_shape():
+    """A market change keeps the run shape's walk weights in the table: the
+    second market's results equal a new context's bit for bit, also after a run
+    of another shape and scheme in between."""
+    from cva_hjm_cuda_gb300.engine import HJMEngine
+
+    cfg = RunConfig(n_paths=500, n_steps=26 * 25, dt=0.02, seed=9)
+    sw = Swap(n_periods=26)
+
+    def run(eng, mk):
+        eng.set_market(mk)
+        eng.set_swap(sw)
+        return eng.run(cfg, "fp64", pfe=False)
+
+    with HJMEngine(0) as fresh:
+        want = run(fresh, _table_market(51))
+    with HJMEngine(0) as eng:
+        run(eng, Market())
+        got = [run(eng, _table_market(51))]
+        eng.set_scheme("predictor_corrector")
+        run(eng, Market())
+        eng.set_scheme("euler")
+        eng.set_swap(Swap(n_periods=4))
+        eng.run(RunConfig(n_paths=100, n_steps=100, dt=0.02), "fp64", pfe=False)
+        run(eng, Market())
+        got.append(run(eng, _table_market(51)))
+    for v in got:
+        np.testing.assert_array_equal(v.ee, want.ee)
+        assert v.cva == want.cva
