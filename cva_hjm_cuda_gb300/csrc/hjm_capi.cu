@@ -872,15 +872,19 @@ static bool contract_room(hjm_ctx* ctx, const RunShape& sh, int64_t n_paths, boo
 // An FP64 valuation in the response form (hjm_contract.cu): the operand table
 // of the market's loadings (contract_room made room for it and the carry), the
 // launches of its windows.  P: the scheme's parameters (the predictor-corrector's N-projected
-// loadings and deterministic curve).  ext_dev: external normals with their row
-// scales behind them (hjm_run_with_normals), or null.
+// loadings and deterministic curve).  ext_dev: external normals, with room for
+// their row scales behind them (hjm_run_with_normals), or null.
 static hjm_status enqueue_contract(hjm_ctx* ctx, const RunShape& sh, double dt, const PathParams<double>& P,
                                    const double* ext_dev, double* estore, longlong2* split, cudaStream_t s)
 {
     hjm_status st = ensure_contract_table(ctx, sh, dt, &P.sv[0][0], ext_dev != nullptr, s);
     if (st != HJM_OK) return st;
-    const double* ext_scale =
-        ext_dev ? ext_dev + (size_t)P.n_paths * (size_t)sh.B * (size_t)sh.stride * kFactors : nullptr;
+    double* ext_scale = nullptr;
+    if (ext_dev) {
+        ext_scale = (double*)ctx->ext.p + (size_t)P.n_paths * (size_t)sh.B * (size_t)sh.stride * kFactors;
+        HJM_CUDA(ctx, launch_contract_ext_scale((const double*)ctx->ext_raw.p, P.n_paths, sh.B * sh.stride, sh.stride,
+                                                ext_scale, s));
+    }
     int launches = 0;
     HJM_CUDA(ctx, launch_path_contract(ctx->nt, P, ctx->contract.p, ext_dev, ext_scale, (double*)ctx->partials.p,
                                        estore, (double*)ctx->carry.p, split, (double*)ctx->result.p, ctx->n_sms, s, &launches));
@@ -1228,8 +1232,6 @@ hjm_status hjm_run_with_normals(hjm_ctx* ctx, int64_t n_paths, int32_t n_steps, 
                                   ctx->stream));
     HJM_CUDA(ctx, launch_transpose_normals((const double*)ctx->ext_raw.p, n_paths, n_steps, (double*)ctx->ext.p,
                                            ctx->stream));
-    HJM_CUDA(ctx, launch_contract_ext_scale((const double*)ctx->ext_raw.p, n_paths, n_steps,
-                                            (double*)ctx->ext.p + count, ctx->stream));
     const double q = pfe_out ? pfe_quantile : 0.0;
     hjm_status st = enqueue_impl(ctx, n_paths, n_steps, dt, 0, 0, precision, hazard_rate, recovery, q,
                                  (const double*)ctx->ext.p);

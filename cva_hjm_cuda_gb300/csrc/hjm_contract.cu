@@ -983,15 +983,17 @@ __global__ void contract_image_kernel(int stride, int B, ContractWindow W, const
     }
 }
 
-__global__ void contract_ext_scale_kernel(const double* __restrict__ raw, int64_t n_paths, int64_t per_path,
-                                          double* __restrict__ out)
+// (values first .. per_path - 1 of a path: the steps before them are not drawn
+// upon, so nothing that a caller leaves there may set a scale)
+__global__ void contract_ext_scale_kernel(const double* __restrict__ raw, int64_t n_paths, int64_t first,
+                                          int64_t per_path, double* __restrict__ out)
 {
     const int lane = threadIdx.x & 31;
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
     for (int64_t p = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; p < n_paths; p += warps) {
         int e = 0;
         bool finite = true;  // a non-finite normal makes its own path's scale, and so its curve, a NaN
-        for (int64_t i = lane; i < per_path; i += 32) {
+        for (int64_t i = first + lane; i < per_path; i += 32) {
             const uint32_t x = ((uint32_t)(__double_as_longlong(raw[p * per_path + i]) >> 52)) & 0x7ffu;
             if (x < 0x7ffu)
                 e = max(e, (int)x - 1023 - 2);
@@ -1081,10 +1083,12 @@ cudaError_t launch_contract_table(int nt, double c, int stride, int n_blocks, bo
     return cudaGetLastError();
 }
 
-cudaError_t launch_contract_ext_scale(const double* raw, int64_t n_paths, int n_steps, double* out, cudaStream_t s)
+cudaError_t launch_contract_ext_scale(const double* raw, int64_t n_paths, int n_steps, int stride, double* out,
+                                      cudaStream_t s)
 {
     const int64_t blocks = std::min<int64_t>((n_paths + 7) / 8, 4096);
-    contract_ext_scale_kernel<<<(unsigned)blocks, 256, 0, s>>>(raw, n_paths, (int64_t)n_steps * 3, out);
+    contract_ext_scale_kernel<<<(unsigned)blocks, 256, 0, s>>>(raw, n_paths, (int64_t)stride * 3,
+                                                               (int64_t)n_steps * 3, out);
     return cudaGetLastError();
 }
 

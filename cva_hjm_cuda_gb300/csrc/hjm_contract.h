@@ -42,10 +42,12 @@ size_t contract_table_bytes(int stride, int n_blocks, bool ext);
 cudaError_t launch_contract_table(int nt, double c, int stride, int n_blocks, bool pc, bool ext, const double* sv,
                                   bool same_shape, void* table, cudaStream_t s);
 
-// Row scales of external normals [path][step][3]: out[2 p] = 2^-e, out[2 p +
+// Row scales of external normals [path][step][3], of the evolved steps (from
+// `stride` on; the first block holds the curve): out[2 p] = 2^-e, out[2 p +
 // 1] = 2^e with e >= 0 the least that brings every |normal| of path p below 8
 // (NaN for a path with a non-finite normal).
-cudaError_t launch_contract_ext_scale(const double* raw, int64_t n_paths, int n_steps, double* out, cudaStream_t s);
+cudaError_t launch_contract_ext_scale(const double* raw, int64_t n_paths, int n_steps, int stride, double* out,
+                                      cudaStream_t s);
 
 // Partial-sum rows of a run: one per tile of kContractTile paths, four for a tile
 // whose steps are split over the SMs (the tiles after the last whole wave, where
