@@ -735,7 +735,7 @@ static cudaError_t launch_adj_pc_t(const PcParams<float>& Q, double* partials, c
 {
     const size_t smem = adjoint_pc_smem(NT, Q.P.n_blocks);
     auto k = adjoint_kernel_pc<NT, POLY>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_dynamic_smem(k);
     if (e != cudaSuccess) return e;
     const int64_t grid = (Q.P.n_paths + kPcCta - 1) / kPcCta;
     k<<<(unsigned)grid, kPcCta, smem, s>>>(Q, partials);
@@ -764,7 +764,7 @@ static cudaError_t launch_adj_t(const AdjParams& A, double* partials, float* ck_
 {
     const size_t smem = adjoint_smem(NT, A.M.P.n_blocks, CKPT);
     auto k = adjoint_kernel<NT, CKPT, POLY>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_dynamic_smem(k);
     if (e != cudaSuccess) return e;
     const int64_t grid = (A.M.P.n_paths + kAdjCta - 1) / kAdjCta;
     k<<<(unsigned)grid, kAdjCta, smem, s>>>(A, partials, ck_h, ck_a);

@@ -467,7 +467,7 @@ cudaError_t launch_adjoint_resp(const AdjParams& A, int ns, int conv_nt, const R
     if (conv_nt == 61) k = ns == 8 ? adjoint_kernel_conv<8, 61> : adjoint_kernel_conv<16, 61>;
     if (!k) return cudaErrorInvalidValue;
     const size_t smem = adjoint_resp_smem(B, conv_nt);
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_dynamic_smem(k);
     if (e != cudaSuccess) return e;
     const int64_t tiles = (A.M.P.n_paths + kAdjCta - 1) / kAdjCta;
     k<<<(unsigned)grid, kAdjCta, smem, s>>>(A.M, live, table, sens, partials, tiles);

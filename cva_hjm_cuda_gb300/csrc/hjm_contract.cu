@@ -1011,13 +1011,15 @@ __global__ void contract_ext_scale_kernel(const double* __restrict__ raw, int64_
 
 size_t align_up(size_t x) { return (x + 255) & ~(size_t)255; }
 
-size_t contract_smem(const ContractWindow& W)
+constexpr size_t contract_smem(int npad, int dates)
 {
-    const size_t need = kBStages * chunk_bytes(W.npad) + sizeof(longlong2) * (size_t)(W.npad / 2) * kContractTile +
-                        sizeof(double) * (size_t)(W.hi - W.lo + 3) * kContractTile;
+    const size_t need = kBStages * chunk_bytes(npad) + sizeof(longlong2) * (size_t)(npad / 2) * kContractTile +
+                        sizeof(double) * (size_t)(dates + 2) * kContractTile;
     // more than half an SM's shared memory: one CTA per SM, which takes all of its tensor memory
     return std::max<size_t>(need, 120 * 1024);
 }
+// the largest window: kContractMaxSlots dates and date 1
+constexpr size_t kContractSmemMost = contract_smem(2 * kContractMaxSlots, kContractMaxSlots + 1);
 
 }  // namespace
 
@@ -1131,6 +1133,8 @@ cudaError_t launch_path_contract(int nt, const PathParams<double>& P, const void
     if (n > 1 && !carry) return cudaErrorInvalidValue;
     auto kernel = ext ? path_kernel_contract<true> : path_kernel_contract<false>;
     auto price = ext ? contract_price_kernel<true> : contract_price_kernel<false>;
+    const cudaError_t allowed = allow_dynamic_smem(kernel, kContractSmemMost);
+    if (allowed != cudaSuccess) return allowed;
     ContractParams Q;
     Q.P = P;
     const int64_t tiles = (P.n_paths + kContractTile - 1) / kContractTile;
@@ -1138,9 +1142,8 @@ cudaError_t launch_path_contract(int nt, const PathParams<double>& P, const void
     int count = 0;
     for (int i = 0; i < n; ++i) {
         Q.W = w[i];
-        const size_t smem = contract_smem(w[i]);
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
+        const size_t smem = contract_smem(w[i].npad, w[i].hi - w[i].lo + 1);
+        cudaError_t e;
         if (whole > 0) {
             Q.tile0 = 0;
             Q.n_tiles = whole;

@@ -628,7 +628,7 @@ static cudaError_t launch_fp64_t(const PathParams<double>& P, const double* ext,
 {
     const size_t smem = path_smem_bytes(NT, P.n_blocks, false);
     auto k = path_kernel_fp64<NT, EXT, FORM>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_dynamic_smem(k);
     if (e != cudaSuccess) return e;
     const int64_t grid = (P.n_paths + kFp64Cta - 1) / kFp64Cta;
     k<<<(unsigned)grid, kFp64Cta, smem, s>>>(P, ext, partials, estore);
@@ -666,7 +666,7 @@ static cudaError_t launch_mixed_t(const MixedParams& M, bool poly, bool cub, con
              : cta == kMixedSmallCta ? path_kernel_mixed<NT, EXT, kMixedSmallCta>
                                      : path_kernel_mixed<NT, EXT, kCta>;
     const size_t smem = poly ? conv_smem_bytes(B) : mixed_smem_bytes(NT, B, cta);
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_dynamic_smem(k);
     if (e != cudaSuccess) return e;
     const int64_t grid = (M.P.n_paths + cta - 1) / cta;
     k<<<(unsigned)grid, cta, smem, s>>>(M, ext, partials, estore);

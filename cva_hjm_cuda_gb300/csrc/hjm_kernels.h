@@ -24,6 +24,16 @@ constexpr int kResErr = kResCVA + 4;         // nonzero: a wait of the contracti
 constexpr int kResCount = kResCVA + 5;       // columns reduced (uint32; cleared with the block)
 constexpr int kResLen = kResCVA + 8;
 
+// Lets a kernel without static shared memory take up to all of an SM's: one
+// limit per kernel whatever the run's size, because it belongs to the kernel and
+// the device, not to the launch (a smaller run on another thread's context would
+// lower it between this thread's setting and its launch).
+template <typename K>
+cudaError_t allow_dynamic_smem(K kernel, size_t most = 227 * 1024)
+{
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+}
+
 struct FinalParams {
     double cvaw[kMaxTenor];    // CVA weights per date
     double dcvaw[kMaxTenor];   // d(weights)/d(hazard)

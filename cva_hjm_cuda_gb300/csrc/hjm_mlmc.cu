@@ -169,7 +169,7 @@ static cudaError_t launch_mlmc_t(const MlmcParams& Q, double* partials, cudaStre
 {
     const size_t smem = mlmc_smem_bytes(Q.fine.P.n_blocks);
     auto k = mlmc_level_kernel<NT, POLY>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_dynamic_smem(k);
     if (e != cudaSuccess) return e;
     const int64_t grid = (Q.fine.P.n_paths + kMlCta - 1) / kMlCta;
     k<<<(unsigned)grid, kMlCta, smem, s>>>(Q, partials);
@@ -307,7 +307,7 @@ static cudaError_t launch_mlmc_pc_t(const MlmcPcParams& Q, double* partials, cud
 {
     const size_t smem = mlmc_pc_smem_bytes(NT, Q.fine.P.n_blocks);
     auto k = mlmc_level_kernel_pc<NT, POLY>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_dynamic_smem(k);
     if (e != cudaSuccess) return e;
     const int64_t grid = (Q.fine.P.n_paths + kMlCta - 1) / kMlCta;
     k<<<(unsigned)grid, kMlCta, smem, s>>>(Q, partials);

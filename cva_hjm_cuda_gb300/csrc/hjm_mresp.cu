@@ -382,7 +382,7 @@ cudaError_t launch_mresp_t(const MixedParams& M, int ns, const RespLive& live, c
 {
     auto k = ns == 8 ? path_kernel_mixed_resp<EXT, CUB, 8> : path_kernel_mixed_resp<EXT, CUB, 16>;
     const size_t smem = mresp_smem_bytes(M.P.n_blocks);
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_dynamic_smem(k);
     if (e != cudaSuccess) return e;
     const int64_t grid = (M.P.n_paths + kCta - 1) / kCta;
     k<<<(unsigned)grid, kCta, smem, s>>>(M, live, table, ext, partials, estore);

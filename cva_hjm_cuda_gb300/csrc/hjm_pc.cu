@@ -159,7 +159,7 @@ static cudaError_t launch_pc_t(const PcParams<T>& Q, const double* ext, double* 
 {
     const size_t smem = pc_smem_bytes(NT, Q.P.n_blocks, sizeof(T));
     auto k = path_kernel_pc<NT, T, EXT, POLY>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_dynamic_smem(k);
     if (e != cudaSuccess) return e;
     const int64_t grid = (Q.P.n_paths + kPcCta - 1) / kPcCta;
     k<<<(unsigned)grid, kPcCta, smem, s>>>(Q, ext, partials, estore);

@@ -322,8 +322,7 @@ cudaError_t select_t(const K* keys, int64_t ld, int64_t n, int n_dates, uint64_t
 {
     if (fits_column(n, sizeof(K))) {
         const size_t smem = (size_t)n * sizeof(K);
-        cudaError_t e = cudaFuncSetAttribute(pfe_column<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)kColumnBytes);
+        cudaError_t e = allow_dynamic_smem(pfe_column<K>, kColumnBytes);
         if (e != cudaSuccess) return e;
         pfe_column<K><<<n_dates, kThreads, smem, s>>>(keys, ld, (int)n, n_dates, k, result);
         *launches = 1;
@@ -336,7 +335,7 @@ cudaError_t select_t(const K* keys, int64_t ld, int64_t n, int n_dates, uint64_t
     const double mid = q * m, half = 6.0 * std::sqrt((double)m * q * (1.0 - q)) + 8.0;
     const int r0 = (int)std::floor(mid - half), r1 = (int)std::ceil(mid + half);
     const size_t smem = (size_t)m * sizeof(K);
-    cudaError_t e = cudaFuncSetAttribute(pfe_bracket<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_dynamic_smem(pfe_bracket<K>, kSample * sizeof(K));
     if (e != cudaSuccess) return e;
     pfe_bracket<K><<<n_dates, kThreads, smem, s>>>(keys, ld, step, m, r0, r1, st);
     // eight CTAs per SM over all dates, each with at least a few thousand keys
