@@ -872,22 +872,16 @@ static bool contract_room(hjm_ctx* ctx, const RunShape& sh, int64_t n_paths, boo
 // An FP64 valuation in the response form (hjm_contract.cu): the operand table
 // of the market's loadings (contract_room made room for it and the carry), the
 // launches of its windows.  P: the scheme's parameters (the predictor-corrector's N-projected
-// loadings and deterministic curve).  ext_dev: external normals, with room for
-// their row scales behind them (hjm_run_with_normals), or null.
+// loadings and deterministic curve).  ext_dev: external normals
+// (launch_contract_ext), or null.
 static hjm_status enqueue_contract(hjm_ctx* ctx, const RunShape& sh, double dt, const PathParams<double>& P,
                                    const double* ext_dev, double* estore, longlong2* split, cudaStream_t s)
 {
     hjm_status st = ensure_contract_table(ctx, sh, dt, &P.sv[0][0], ext_dev != nullptr, s);
     if (st != HJM_OK) return st;
-    double* ext_scale = nullptr;
-    if (ext_dev) {
-        ext_scale = (double*)ctx->ext.p + (size_t)P.n_paths * (size_t)sh.B * (size_t)sh.stride * kFactors;
-        HJM_CUDA(ctx, launch_contract_ext_scale((const double*)ctx->ext_raw.p, P.n_paths, sh.B * sh.stride, sh.stride,
-                                                ext_scale, s));
-    }
     int launches = 0;
-    HJM_CUDA(ctx, launch_path_contract(ctx->nt, P, ctx->contract.p, ext_dev, ext_scale, (double*)ctx->partials.p,
-                                       estore, (double*)ctx->carry.p, split, (double*)ctx->result.p, ctx->n_sms, s, &launches));
+    HJM_CUDA(ctx, launch_path_contract(ctx->nt, P, ctx->contract.p, ext_dev, (double*)ctx->partials.p, estore,
+                                       (double*)ctx->carry.p, split, (double*)ctx->result.p, ctx->n_sms, s, &launches));
     ctx->stat_launches += launches - 1;
     return HJM_OK;
 }
@@ -965,7 +959,7 @@ static hjm_status ensure_mresp_table(hjm_ctx* ctx, cudaStream_t s)
 
 static hjm_status enqueue_impl(hjm_ctx* ctx, int64_t n_paths, int32_t n_steps, double dt, uint64_t seed,
                                uint64_t path_offset, int32_t precision, double hazard, double recovery, double pfe_q,
-                               const double* ext_dev)
+                               const double* ext_raw)
 {
     RunShape sh;
     hjm_status st = check_run(ctx, n_paths, n_steps, dt, precision, hazard, recovery, pfe_q, sh);
@@ -1005,13 +999,13 @@ static hjm_status enqueue_impl(hjm_ctx* ctx, int64_t n_paths, int32_t n_steps, d
     // what the contraction needs besides: its table and carry, without which
     // the run convects, and its split tiles' sums, without which they run whole
     longlong2* split = nullptr;
-    if (contract && !contract_room(ctx, sh, n_paths, ext_dev != nullptr)) {
+    if (contract && !contract_room(ctx, sh, n_paths, ext_raw != nullptr)) {
         contract = false;
         n_ctas = (n_paths + cta - 1) / cta;
         HJM_CUDA(ctx, ctx->partials.ensure(sizeof(double) * (size_t)n_ctas * R));
     }
     if (contract) {
-        const size_t bytes = contract_sums_bytes(n_paths, sh.B, sh.stride, ctx->n_sms, ext_dev != nullptr);
+        const size_t bytes = contract_sums_bytes(n_paths, sh.B, sh.stride, ctx->n_sms, ext_raw != nullptr);
         const int64_t rows = contract_rows(n_paths, sh.B, sh.stride, ctx->n_sms);
         if (bytes && try_ensure(ctx->split, bytes) && try_ensure(ctx->partials, sizeof(double) * (size_t)rows * R)) {
             split = (longlong2*)ctx->split.p;
@@ -1021,13 +1015,19 @@ static hjm_status enqueue_impl(hjm_ctx* ctx, int64_t n_paths, int32_t n_steps, d
         }
     }
     cudaStream_t s = ctx->stream;
+    // external normals (on the device in the caller's order) in the form's own
+    const double* ext_dev = ext_raw ? (const double*)ctx->ext.p : nullptr;
+    if (ext_raw && contract)
+        HJM_CUDA(ctx, launch_contract_ext(ext_raw, n_paths, sh.B, sh.stride, ctx->ext.p, s));
+    else if (ext_raw)
+        HJM_CUDA(ctx, launch_transpose_normals(ext_raw, n_paths, n_steps, (double*)ctx->ext.p, s));
     ctx->have_result = false;
     HJM_CUDA(ctx, cudaMemsetAsync(ctx->result.p, 0, sizeof(double) * kResLen, s));
 
     FinalParams F;
     ctx->ev = ctx->ring[ctx->n_enqueued % hjm_ctx::kRing];
     ctx->n_enqueued++;
-    ctx->stat_launches = 2;  // path kernel, column reduction
+    ctx->stat_launches = 2 + (ext_raw ? (contract ? 2 : 1) : 0);  // path kernel, column reduction; the normals' order
     ctx->stat_h2d = (mixed ? sizeof(MixedParams) : sizeof(PathParams<double>)) + sizeof(FinalParams);
     ctx->stat_d2h = 0;
     HJM_CUDA(ctx, cudaEventRecord(ctx->ev[0], s));
@@ -1227,16 +1227,13 @@ hjm_status hjm_run_with_normals(hjm_ctx* ctx, int64_t n_paths, int32_t n_steps, 
     if (count > ((size_t)1 << 33)) return fail(ctx, HJM_ERR_INVALID_ARGUMENT, "normals buffer too large");
     HJM_CUDA(ctx, cudaSetDevice(ctx->device));
     HJM_CUDA(ctx, ctx->ext_raw.ensure(sizeof(double) * count));
-    HJM_CUDA(ctx, ctx->ext.ensure(sizeof(double) * (count + 2 * (size_t)n_paths)));
+    HJM_CUDA(ctx, ctx->ext.ensure(sizeof(double) * count));
     HJM_CUDA(ctx, cudaMemcpyAsync(ctx->ext_raw.p, normals_host, sizeof(double) * count, cudaMemcpyHostToDevice,
                                   ctx->stream));
-    HJM_CUDA(ctx, launch_transpose_normals((const double*)ctx->ext_raw.p, n_paths, n_steps, (double*)ctx->ext.p,
-                                           ctx->stream));
     const double q = pfe_out ? pfe_quantile : 0.0;
     hjm_status st = enqueue_impl(ctx, n_paths, n_steps, dt, 0, 0, precision, hazard_rate, recovery, q,
-                                 (const double*)ctx->ext.p);
+                                 (const double*)ctx->ext_raw.p);
     if (st != HJM_OK) return st;
-    ctx->stat_launches += 1;
     ctx->stat_h2d += (int64_t)(sizeof(double) * count);
     return hjm_fetch_results(ctx, ee_out, pfe_out, cva_out);
 }

@@ -14,8 +14,7 @@
 // FP64 accuracy from FP16 operands.  Each normal is cut into slices on fixed
 // grids, phi = a0 + a1 2^-10 + a2 2^-20 + a3 2^-30: a0, a1, a2 multiples of
 // 2^-7 (the remainder of one is scaled by 2^10 for the next, so |a1|, |a2| <=
-// 4), a3 what is left, rounded to 11 bits (exact for |phi| >= 2^-15; external
-// FP64 normals take a fifth slice).  Each response, scaled per date by a power
+// 4), a3 what is left, rounded to 11 bits (exact for |phi| >= 2^-15).  Each response, scaled per date by a power
 // of two to at most 2^8, is cut likewise into b0 .. b3 (integers up to 2^9) and
 // b4.  Every slice is exact in FP16, every product a_i b_j exact in FP32, and
 // the products of one level s = i + j share one grid, so each level has an FP32
@@ -29,6 +28,19 @@
 // then lie 1e-14 of their scale from the oracle (the convected all-FP64 step:
 // 5e-15; double-FP32 response sums on the FP32 pipe: 5e-14); with three slices
 // fewer bits (grids 2^-12 apart, four levels) it was 6e-13.
+//
+// A caller's own normals (EXT) need not average out: equal or drifting ones add
+// up coherently, 2^28 units at level 0 over a group.  So each path has a power of
+// two of its own, which brings its normals below 8 (contract_ext_scale_kernel),
+// a fifth slice for what FP32 does not hold, and levels 0 to 2 restart with every
+// k-tile: 16 products of |a0| <= 2^10, |a1| <= 2^9, |a2| <= 576 with |b0| <= 2^8,
+// |b1|, |b2| <= 2^9 add up to at most 2^23.9 units there, whatever the normals.
+// Levels 3 and 4 go on over the group, so that the generator's own draws give its
+// results bit for bit.  Constant normals of 3.65, 7.9 or 0.0039 then lie within
+// 1e-13 of the exposures, where sums over whole groups lost up to 1e-7.
+// Bound: the reads of levels 0 to 2 (three a chunk instead of one a group).
+// 100,000 paths x 1,000 steps, 10y swap: 1.24 ms (2.28 ms for double-FP32 sums on
+// the FP32 pipe; 13.4 ms with the slices cut in FP64).
 //
 // Roles of a CTA (one per SM, persistent over tiles of 128 paths):
 //   warps 0-15   normals: Philox in registers, Box-Muller, slices; warp w holds
@@ -76,7 +88,7 @@ constexpr int kMmaWarp = 20, kLoadWarp = 21;
 constexpr int kThreads = 32 * 22;
 constexpr int kAStages = 2, kBStages = 3;
 constexpr int kTmemCols = 512;
-// External FP64 normals take a fifth slice (what FP32 does not hold)
+// External normals take a fifth slice
 __host__ __device__ constexpr int slices_of(bool ext) { return ext ? kSlices + 1 : kSlices; }
 // 32-bit tensor-memory columns of a chunk's A slices; the A stages lie behind
 // the accumulators
@@ -230,22 +242,33 @@ __device__ __forceinline__ void slice_pair(float2 v, uint32_t (&out)[kSlices])
     const __half2 h = __floats2half2_rn(d.x, d.y);
     out[kSlices - 1] = *reinterpret_cast<const uint32_t*>(&h);
 }
-// ... of two FP64 normals (below 8 in magnitude), with a fifth slice for what
-// the fourth leaves; values that FP32 holds give the slices above
-__device__ __forceinline__ void slice_pair(double x, double y, uint32_t (&out)[kSlices + 1])
+// ... of two external normals hi + lo 2^-27 (contract_ext_kernel), with a fifth
+// slice for what the fourth leaves.  lo joins at the third slice, whose units are
+// 2^-27 (so |a2| <= 512 + 64); a normal that FP32 holds (lo = 0) gives the
+// slices above, bit for bit.  In FP32: with FP64 operations, which share a pipe of
+// 18 cycles an instruction, the slices of 100,000 paths x 950 steps took 13.4 ms.
+__device__ __forceinline__ void slice_pair(float2 v, float2 lo, uint32_t (&out)[kSlices + 1])
 {
-    const bool fx = (double)(float)x == x, fy = (double)(float)y == y;
-    x *= (double)kUnit;
-    y *= (double)kUnit;
-#pragma unroll
-    for (int s = 0; s <= kSlices; ++s) {
-        const double ax = s < kSlices - 1 ? rint(x) : x, ay = s < kSlices - 1 ? rint(y) : y;
-        __half2 h = __floats2half2_rn(-(float)ax, -(float)ay);
-        if (s == kSlices) h = __halves2half2(fx ? __half(0.0f) : __low2half(h), fy ? __half(0.0f) : __high2half(h));
+    const float2 g = make_float2(kGrid, kGrid), m1 = make_float2(-1.0f, -1.0f), sh = make_float2(kShift, kShift),
+                 un = make_float2(kUnit, kUnit);
+    auto put = [&](int s, float2 x) {
+        const __half2 h = __floats2half2_rn(x.x, x.y);
         out[s] = *reinterpret_cast<const uint32_t*>(&h);
-        x = (x + (double)__low2float(h)) * (double)kShift;
-        y = (y + (double)__high2float(h)) * (double)kShift;
-    }
+        return h;
+    };
+    float2 na = __ffma2_rn(__ffma2_rn(v, un, g), m1, g);
+    float2 d = __ffma2_rn(v, un, na);
+    put(0, na);
+    na = __ffma2_rn(__ffma2_rn(d, sh, g), m1, g);
+    d = __ffma2_rn(d, sh, na);
+    put(1, na);
+    na = __ffma2_rn(__fadd2_rn(__ffma2_rn(d, sh, lo), g), m1, g);
+    d = __fadd2_rn(__ffma2_rn(d, sh, na), lo);  // (both exact: multiples of lo's last bit below 2^8)
+    put(2, na);
+    d = __fmul2_rn(d, make_float2(-kShift, -kShift));
+    const __half2 h = put(3, d);
+    put(4, make_float2(lo.x == 0.0f ? 0.0f : (d.x - __low2float(h)) * kShift,
+                       lo.y == 0.0f ? 0.0f : (d.y - __high2float(h)) * kShift));
 }
 
 // Philox4x32-10 of counter (step, 0, path): what depends on the path alone is
@@ -304,6 +327,12 @@ __device__ __forceinline__ double sum_value(long long v)
 __device__ __forceinline__ void epilogue_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
 }  // namespace
+
+// Of a path with external normals: 2^e (NaN: a non-finite normal) and e
+struct ExtRow {
+    double scale;
+    int64_t e;
+};
 
 // The launch's constants besides the path parameters.  Whole tiles [0, n_tiles)
 // go to the CTAs in turn; in a split launch the accumulator groups of tiles
@@ -364,7 +393,7 @@ __device__ __forceinline__ double contract_cash_flow(const PathParams<double>& P
 template <bool EXT>
 __global__ void __launch_bounds__(kThreads, 1)
     path_kernel_contract(const __grid_constant__ ContractParams Q, const unsigned char* __restrict__ table,
-                         const double* __restrict__ ext, const double* __restrict__ ext_scale,
+                         const float2* __restrict__ ext, const ExtRow* __restrict__ ext_row,
                          double* __restrict__ partials, double* __restrict__ estore, double* __restrict__ carry,
                          double* __restrict__ result)
 {
@@ -431,8 +460,6 @@ __global__ void __launch_bounds__(kThreads, 1)
             const int64_t lp = tile * kContractTile + 32 * q + lane;
             const PathDraw pd = path_draw(P.path_offset + (uint64_t)lp, P.rk0, P.rk1);
             const int64_t lpc = lp < P.n_paths ? lp : 0;
-            double xs = 1.0;
-            if constexpr (EXT) xs = __ldg(ext_scale + 2 * lpc);
             for (; c < NC && left > 0; c += kAStages, ph ^= 1u, --left) {
 #pragma unroll 1
                 for (int half = 0; half < 2; ++half) {
@@ -440,17 +467,17 @@ __global__ void __launch_bounds__(kThreads, 1)
                     // value 3 i + k: step n0 + i, factor k; pairs of values are one column
                     uint32_t w[kSl][6];
                     if constexpr (EXT) {
-                        double z[12];
+                        float2 z[12];
                         const size_t np = (size_t)P.n_paths;
 #pragma unroll
                         for (int i = 0; i < 4; ++i)
 #pragma unroll
                             for (int k = 0; k < 3; ++k)
-                                z[3 * i + k] = __ldg(ext + (size_t)min(n0 + i, n_last) * 3 * np + k * np + lpc) * xs;
+                                z[3 * i + k] = __ldg(ext + (size_t)min(n0 + i, n_last) * 3 * np + k * np + lpc);
 #pragma unroll
                         for (int u = 0; u < 6; ++u) {
                             uint32_t o[kSl];
-                            slice_pair(z[2 * u], z[2 * u + 1], o);
+                            slice_pair(f2(z[2 * u].x, z[2 * u + 1].x), f2(z[2 * u].y, z[2 * u + 1].y), o);
 #pragma unroll
                             for (int s = 0; s < kSl; ++s) w[s][u] = o[s];
                         }
@@ -498,9 +525,9 @@ __global__ void __launch_bounds__(kThreads, 1)
         // a_s times the response slices b_0 .. b_{levels - 1 - s} gives the
         // levels s .. 4; beyond 256 columns b_4 takes an instruction of its own
         const bool split = kLevels * npad > 256;
-        uint32_t idesc[kSl];
+        uint32_t idesc[kSlices];  // (EXT: of 5 - s columns' worth, as the generator's)
 #pragma unroll
-        for (int s = 0; s < kSl; ++s) idesc[s] = tc_idesc((kLevels - s - (s == 0 && split)) * npad);
+        for (int s = 0; s < kSlices; ++s) idesc[s] = tc_idesc((kLevels - s - (s == 0 && split)) * npad);
         const uint32_t idesc1 = tc_idesc(npad);
         const uint64_t desc0 = tc_smem_desc(bs, kLevels * npad * 16);
         const uint32_t kt_step = (uint32_t)(kLevels * npad * 32) >> 4, stage_step = (uint32_t)cb >> 4;
@@ -517,11 +544,43 @@ __global__ void __launch_bounds__(kThreads, 1)
             const bool last = fl == kFlush - 1 || c == NC - 1;
             ok = mbar_wait<false>(a_full + 8 * st, ph ^ (uint32_t)(i / kAStages & 1), abort_s) &&
                  mbar_wait<false>(b_full + 8 * sb, (uint32_t)(i / kBStages & 1), abort_s) &&
-                 (!first || mbar_wait<false>(d_empty, d_ph, abort_s));
+                 (EXT || !first || mbar_wait<false>(d_empty, d_ph, abort_s));
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) return;
             tc_fence_after();
-            if (leader) {
+            if constexpr (EXT) {
+                const uint64_t bd0 = desc0 + (uint64_t)(sb * stage_step);
+                const uint32_t a0 = tmem + kACol + st * kAStageCols;
+                const uint32_t two = idesc[3], three = idesc[2];
+                for (int kt = 0; kt < 3; ++kt) {
+                    const uint64_t bd = bd0 + (uint64_t)(kt * kt_step);
+                    const uint32_t a = a0 + 8 * kt;
+                    // levels 3 and 4: a_s times b_{3-s}, b_{4-s}
+                    auto low_levels = [&](uint32_t add) {
+#pragma unroll
+                        for (int s = 0; s < kSlices; ++s)
+                            tc_mma(tmem + 3 * npad, a + 24 * s, bd + (uint64_t)((3 - s) * npad), two, s ? 1u : add);
+                        tc_mma(tmem + 4 * npad, a + 24 * kSlices, bd, idesc1, 1);
+                    };
+                    const bool fresh = first && kt == 0;
+                    if (leader && !fresh) low_levels(1);  // (the last k-tile's reader leaves these two alone)
+                    ok = __all_sync(0xffffffffu, mbar_wait<false>(d_empty, d_ph, abort_s));
+                    if (!ok) return;
+                    d_ph ^= 1u;
+                    tc_fence_after();
+                    if (leader) {
+                        if (fresh) low_levels(0);
+                        tc_mma(tmem, a, bd, three, 0);
+                        tc_mma(tmem + npad, a + 24, bd, two, 1);
+                        tc_mma(tmem + 2 * npad, a + 48, bd, idesc1, 1);
+                        tc_commit(d_full);
+                    }
+                }
+                if (leader) {
+                    tc_commit(a_empty + 8 * st);
+                    tc_commit(b_empty + 8 * sb);
+                }
+            } else if (leader) {
                 const uint64_t bd0 = desc0 + (uint64_t)(sb * stage_step);
                 const uint32_t a0 = tmem + kACol + st * kAStageCols;
 #pragma unroll
@@ -533,13 +592,13 @@ __global__ void __launch_bounds__(kThreads, 1)
                     if (split)
                         tc_mma(tmem + (kLevels - 1) * npad, a, bd + (uint64_t)((kLevels - 1) * npad), idesc1, add);
 #pragma unroll
-                    for (int s = 1; s < kSl; ++s) tc_mma(tmem + s * npad, a + 24 * s, bd, idesc[s], 1);
+                    for (int s = 1; s < kSlices; ++s) tc_mma(tmem + s * npad, a + 24 * s, bd, idesc[s], 1);
                 }
                 tc_commit(a_empty + 8 * st);
                 tc_commit(b_empty + 8 * sb);
                 if (last) tc_commit(d_full);
             }
-            if (first) d_ph ^= 1u;
+            if (!EXT && first) d_ph ^= 1u;
             ++g;
             if (++fl == kFlush || c == NC - 1) fl = 0;
             if (++c == NC) c = 0;
@@ -602,10 +661,10 @@ __global__ void __launch_bounds__(kThreads, 1)
         const int first_date = lo > 2 ? lo : 2;  // date 1 precedes any evolution
         double* e_s = cf_s + kContractTile;  // exposure row of date j: j - lo + 1 (the cash-flow row of date j + 1)
         int64_t grp = 0;
-        // waits for an accumulator group and adds it to the running sums of the live
-        // slots (fresh: the first of them), four slots at a time, padding included
-        // (its columns are zero); false if the wait ran out
-        auto drain_group = [&](bool fresh, int live) {
+        // waits for the accumulators and adds them to the running sums of the live
+        // slots (fresh: the first of them; low: levels 3 and 4 too), four slots at a
+        // time, padding included (its columns are zero); false if the wait ran out
+        auto drain = [&](bool fresh, auto low, int live) {
             const bool ok = mbar_wait<true>(d_full, (uint32_t)(grp & 1), abort_s);
             if (!__all_sync(0xffffffffu, ok)) return false;
             ++grp;
@@ -613,7 +672,11 @@ __global__ void __launch_bounds__(kThreads, 1)
             for (int r0 = 0; r0 < live; r0 += 4) {
                 float acc[kLevels][8];
 #pragma unroll
-                for (int s = 0; s < kLevels; ++s) tmem_ld8(d_addr + s * npad + 2 * r0, acc[s]);
+                for (int s = 0; s < kLevels; ++s)
+                    if (s < 3 || decltype(low)::value)
+                        tmem_ld8(d_addr + s * npad + 2 * r0, acc[s]);
+                    else
+                        for (int i = 0; i < 8; ++i) acc[s][i] = 0.0f;
                 longlong2 cell[4];
 #pragma unroll
                 for (int u = 0; u < 4; ++u)
@@ -634,6 +697,14 @@ __global__ void __launch_bounds__(kThreads, 1)
             }
             return true;
         };
+        // the accumulators of chunks [from, to), one group's: at once, or k-tile by k-tile
+        auto drain_group = [&](int from, int to, bool fresh, int live) {
+            if constexpr (EXT) {
+                for (int i = 3 * (to - from) - 1; i > 0; --i, fresh = false)
+                    if (!drain(fresh, std::false_type(), live)) return false;
+            }
+            return drain(fresh, std::true_type(), live);
+        };
         if (Q.sums) {  // ---- split tiles: this CTA's groups of each, to the tile's sums
             int64_t left = run.chunks, tile = run.first;
             for (int c = run.c0; left > 0; c = 0, ++tile) {
@@ -648,7 +719,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 bool ok = true;
                 for (int b = c; b < end && ok; b += kFlush) {
                     skip_to(b);
-                    ok = drain_group(b == c, hi - next + 1);
+                    ok = drain_group(b, min(b + kFlush, end), b == c, hi - next + 1);
                 }
                 if (!ok) break;
                 unsigned long long* to = reinterpret_cast<unsigned long long*>(
@@ -665,7 +736,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 const int64_t base = tile * kContractTile, lp = base + p;
                 const bool active = lp < P.n_paths;
                 double rs = 1.0;
-                if constexpr (EXT) rs = __ldg(ext_scale + 2 * (active ? lp : 0) + 1);
+                if constexpr (EXT) rs = ext_row[active ? lp : 0].scale;
                 auto price = [&](int i) {
                     double sx = 0.0, sa = 0.0;
                     longlong2 v = make_longlong2(0, 0);
@@ -683,7 +754,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 if (bottom) price(1);
                 int next = first_date;  // the earliest date not priced yet
                 for (int c = 0; c < NC; c += kFlush) {
-                    if (!drain_group(c == 0, hi - next + 1)) break;
+                    if (!drain_group(c, min(c + kFlush, NC), c == 0, hi - next + 1)) break;
                     // the dates whose last step this group held
                     const int done = kChunk * min(c + kFlush, NC);
                     for (; next <= hi && (next - 1) * P.stride <= done; ++next) price(next);
@@ -767,7 +838,7 @@ constexpr int kPriceWarps = 8;
 template <bool EXT>
 __global__ void __launch_bounds__(32 * kPriceWarps)
     contract_price_kernel(const __grid_constant__ ContractParams Q, const double* __restrict__ scale,
-                          const double* __restrict__ ext_scale, int64_t row0, double* __restrict__ partials,
+                          const ExtRow* __restrict__ ext_row, int64_t row0, double* __restrict__ partials,
                           double* __restrict__ estore, double* __restrict__ carry)
 {
     const PathParams<double>& P = Q.P;
@@ -780,7 +851,7 @@ __global__ void __launch_bounds__(32 * kPriceWarps)
     const bool active = lp < P.n_paths;
     const longlong2* sums = Q.sums + (size_t)(blockIdx.x / 4) * (Q.W.npad / 2) * kContractTile + in_tile;
     double rs = 1.0;
-    if constexpr (EXT) rs = __ldg(ext_scale + 2 * (active ? lp : 0) + 1);
+    if constexpr (EXT) rs = ext_row[active ? lp : 0].scale;
     for (int i = lo + warp; i <= hi; i += kPriceWarps) {
         double sx = 0.0, sa = 0.0;
         longlong2 v = make_longlong2(0, 0);
@@ -983,29 +1054,66 @@ __global__ void contract_image_kernel(int stride, int B, ContractWindow W, const
     }
 }
 
-// (values first .. per_path - 1 of a path: the steps before them are not drawn
-// upon, so nothing that a caller leaves there may set a scale)
+// The power of two 2^e of each path: e the least that brings the evolved steps'
+// normals (values first .. per_path - 1; the steps before are not drawn upon, so
+// nothing that a caller leaves there may set a scale) below 2^(3 - guard), and 0
+// where that is less and the largest is no smaller than 1/4: smaller ones are
+// brought up.  A non-finite normal makes its own path's scale, and so its curve, a NaN.
 __global__ void contract_ext_scale_kernel(const double* __restrict__ raw, int64_t n_paths, int64_t first,
-                                          int64_t per_path, double* __restrict__ out)
+                                          int64_t per_path, int guard, ExtRow* __restrict__ out)
 {
     const int lane = threadIdx.x & 31;
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
     for (int64_t p = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; p < n_paths; p += warps) {
-        int e = 0;
-        bool finite = true;  // a non-finite normal makes its own path's scale, and so its curve, a NaN
-        for (int64_t i = first + lane; i < per_path; i += 32) {
-            const uint32_t x = ((uint32_t)(__double_as_longlong(raw[p * per_path + i]) >> 52)) & 0x7ffu;
-            if (x < 0x7ffu)
-                e = max(e, (int)x - 1023 - 2);
-            else
-                finite = false;
+        uint32_t top = 0;  // biased exponents: 2047 of a non-finite normal
+#pragma unroll 4
+        for (int64_t i = first + lane; i < per_path; i += 32)
+            top = max(top, ((uint32_t)(__double_as_longlong(raw[p * per_path + i]) >> 52)) & 0x7ffu);
+        top = __reduce_max_sync(0xffffffffu, top);
+        const int x = (int)top - 1023;
+        int e = x - 2 + guard;
+        if (e < 0) e = x >= -2 ? 0 : max(e, -900);
+        if (lane == 0) out[p] = {top == 0x7ffu ? __longlong_as_double(0x7ff8000000000000ll) : scalbn(1.0, e), e};
+    }
+}
+
+// External normals [path][step][3] -> [step][3][path] as pairs {hi, lo 2^27} of the
+// scaled value hi + lo, for the evolved steps: hi its first 24 bits, lo the other 29
+// rounded to 24, by integer operations on the bits.  Tiles of 32 paths x 32 values
+// through shared memory.  Bound: memory (48 bytes a path-step).
+__global__ void __launch_bounds__(256)
+    contract_ext_kernel(const double* __restrict__ raw, int64_t n_paths, int64_t first, int64_t per_path,
+                        const ExtRow* __restrict__ row, float2* __restrict__ out)
+{
+    __shared__ float2 tile[32][33];
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const int64_t p0 = (int64_t)blockIdx.x * 32;
+    int e[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) e[u] = p0 + ty + 8 * u < n_paths ? row[p0 + ty + 8 * u].e : 0;
+    for (int64_t i0 = first + (int64_t)blockIdx.y * 32; i0 < per_path; i0 += (int64_t)gridDim.y * 32) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int64_t p = p0 + ty + 8 * u, i = i0 + tx;
+            const uint64_t b = p < n_paths && i < per_path ? (uint64_t)__double_as_longlong(raw[p * per_path + i]) : 0;
+            const int f = (int)(b >> 52 & 0x7ffu), x = f - 1023 - e[u] + 127;  // x: FP32's biased exponent
+            const uint32_t sign = (uint32_t)(b >> 63) << 31;
+            float hi = 0.0f, lo = 0.0f;
+            if (f > 0 && x > 0) {  // (else nothing beside the path's scale; x <= 129 by the choice of e)
+                hi = __uint_as_float(sign | (uint32_t)x << 23 | (uint32_t)(b >> 29 & 0x7fffffu));
+                // the low 29 bits in units of 2^(x - 127 - 52), times 2^27
+                const int y = x - 52 + 27;
+                if (y > 0) lo = (float)(uint32_t)(b & 0x1fffffffu) * __uint_as_float(sign | (uint32_t)y << 23);
+            }
+            tile[tx][ty + 8 * u] = f2(hi, lo);
         }
-        e = __reduce_max_sync(0xffffffffu, e);
-        finite = __all_sync(0xffffffffu, finite);
-        if (lane == 0) {
-            out[2 * p] = scalbn(1.0, -e);
-            out[2 * p + 1] = finite ? scalbn(1.0, e) : __longlong_as_double(0x7ff8000000000000ll);
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int64_t i = i0 + ty + 8 * u;
+            if (i < per_path && p0 + tx < n_paths) out[(size_t)i * (size_t)n_paths + (size_t)(p0 + tx)] = tile[ty + 8 * u][tx];
         }
+        __syncthreads();
     }
 }
 
@@ -1085,12 +1193,22 @@ cudaError_t launch_contract_table(int nt, double c, int stride, int n_blocks, bo
     return cudaGetLastError();
 }
 
-cudaError_t launch_contract_ext_scale(const double* raw, int64_t n_paths, int n_steps, int stride, double* out,
-                                      cudaStream_t s)
+cudaError_t launch_contract_ext(const double* raw, int64_t n_paths, int n_blocks, int stride, void* out, cudaStream_t s)
 {
-    const int64_t blocks = std::min<int64_t>((n_paths + 7) / 8, 4096);
-    contract_ext_scale_kernel<<<(unsigned)blocks, 256, 0, s>>>(raw, n_paths, (int64_t)stride * 3,
-                                                               (int64_t)n_steps * 3, out);
+    if (stride < 2) return cudaErrorInvalidValue;  // (the rows lie where the first block's normals would)
+    const int64_t first = (int64_t)stride * 3, per_path = first * n_blocks;
+    // a path's running sums stay below 2^62: values x 2^10 2^8 2^30 units
+    int guard = 0;
+    while ((per_path - first) >> (14 + guard) > 0) ++guard;
+    ExtRow* row = (ExtRow*)out;
+    contract_ext_scale_kernel<<<(unsigned)std::min<int64_t>((n_paths + 7) / 8, 4096), 256, 0, s>>>(raw, n_paths, first,
+                                                                                                   per_path, guard, row);
+    if (n_blocks > 1) {
+        const int64_t gx = (n_paths + 31) / 32, tiles = (per_path - first + 31) / 32;
+        const int64_t gy = std::max<int64_t>(1, std::min<int64_t>(tiles, 4096 / gx));
+        contract_ext_kernel<<<dim3((unsigned)gx, (unsigned)gy), 256, 0, s>>>(raw, n_paths, first, per_path, row,
+                                                                             (float2*)out);
+    }
     return cudaGetLastError();
 }
 
@@ -1122,12 +1240,13 @@ size_t contract_sums_bytes(int64_t n_paths, int n_blocks, int stride, int n_sms,
     return sizeof(longlong2) * (size_t)split_tiles(n_paths, n_blocks, stride, n_sms) * (npad / 2) * kContractTile;
 }
 
-cudaError_t launch_path_contract(int nt, const PathParams<double>& P, const void* table, const double* ext,
-                                 const double* ext_scale, double* partials, double* estore, double* carry,
-                                 longlong2* sums, double* result, int n_sms, cudaStream_t s, int* launches)
+cudaError_t launch_path_contract(int nt, const PathParams<double>& P, const void* table, const void* normals,
+                                 double* partials, double* estore, double* carry, longlong2* sums, double* result,
+                                 int n_sms, cudaStream_t s, int* launches)
 {
-    if (!path_tenor_supported(nt) || P.n_blocks < 1 || P.n_blocks >= nt || P.stride < 1 || (ext && !ext_scale))
-        return cudaErrorInvalidValue;
+    if (!path_tenor_supported(nt) || P.n_blocks < 1 || P.n_blocks >= nt || P.stride < 1) return cudaErrorInvalidValue;
+    const float2* ext = (const float2*)normals;
+    const ExtRow* ext_row = (const ExtRow*)normals;
     ContractWindow w[kMaxTenor];
     const int n = contract_windows(P.n_blocks, P.stride, ext != nullptr, w);
     if (n > 1 && !carry) return cudaErrorInvalidValue;
@@ -1149,7 +1268,7 @@ cudaError_t launch_path_contract(int nt, const PathParams<double>& P, const void
             Q.n_tiles = whole;
             Q.sums = nullptr;
             kernel<<<(unsigned)std::min<int64_t>(whole, n_sms), kThreads, smem, s>>>(
-                Q, (const unsigned char*)table, ext, ext_scale, partials, estore, carry, result);
+                Q, (const unsigned char*)table, ext, ext_row, partials, estore, carry, result);
             ++count;
         }
         if (split > 0) {
@@ -1161,10 +1280,11 @@ cudaError_t launch_path_contract(int nt, const PathParams<double>& P, const void
                 e = cudaMemsetAsync(sums, 0, sizeof(longlong2) * (size_t)split * (w[i].npad / 2) * kContractTile, s);
                 if (e != cudaSuccess) return e;
                 kernel<<<(unsigned)std::min<int64_t>(groups, n_sms), kThreads, smem, s>>>(
-                    Q, (const unsigned char*)table, ext, ext_scale, partials, estore, carry, result);
+                    Q, (const unsigned char*)table, ext, ext_row, partials, estore, carry, result);
                 ++count;
             }
-            price<<<(unsigned)(4 * split), 32 * kPriceWarps, 0, s>>>(Q, (const double*)table, ext_scale, whole, partials, estore, carry);
+            price<<<(unsigned)(4 * split), 32 * kPriceWarps, 0, s>>>(Q, (const double*)table, ext_row, whole, partials,
+                                                                    estore, carry);
             ++count;
         }
         e = cudaGetLastError();

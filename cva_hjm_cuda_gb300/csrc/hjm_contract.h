@@ -42,12 +42,10 @@ size_t contract_table_bytes(int stride, int n_blocks, bool ext);
 cudaError_t launch_contract_table(int nt, double c, int stride, int n_blocks, bool pc, bool ext, const double* sv,
                                   bool same_shape, void* table, cudaStream_t s);
 
-// Row scales of external normals [path][step][3], of the evolved steps (from
-// `stride` on; the first block holds the curve): out[2 p] = 2^-e, out[2 p +
-// 1] = 2^e with e >= 0 the least that brings every |normal| of path p below 8
-// (NaN for a path with a non-finite normal).
-cudaError_t launch_contract_ext_scale(const double* raw, int64_t n_paths, int n_steps, int stride, double* out,
-                                      cudaStream_t s);
+// External normals [path][step][3] of n_blocks blocks as launch_path_contract takes
+// them, into out (as many doubles as raw; the first block's place, whose steps no
+// valuation draws upon, holds the paths' scales).  Two launches.
+cudaError_t launch_contract_ext(const double* raw, int64_t n_paths, int n_blocks, int stride, void* out, cudaStream_t s);
 
 // Partial-sum rows of a run: one per tile of kContractTile paths, four for a tile
 // whose steps are split over the SMs (the tiles after the last whole wave, where
@@ -58,11 +56,11 @@ size_t contract_sums_bytes(int64_t n_paths, int n_blocks, int stride, int n_sms,
 
 // The valuation: per window a launch over the whole tiles and one over the split
 // ones with their pricing (carry [2][n_paths] doubles when there is more than one
-// window).  partials: contract_rows rows of n_blocks + 3 doubles.  ext: external
-// normals [step][3][path] with their row scales, or null for the generator.
+// window).  partials: contract_rows rows of n_blocks + 3 doubles.  normals:
+// launch_contract_ext's, or null for the generator.
 // result[kResErr] is set if a wait in the kernel ran out.
-cudaError_t launch_path_contract(int nt, const PathParams<double>& P, const void* table, const double* ext,
-                                 const double* ext_scale, double* partials, double* estore, double* carry,
-                                 longlong2* sums, double* result, int n_sms, cudaStream_t s, int* launches);
+cudaError_t launch_path_contract(int nt, const PathParams<double>& P, const void* table, const void* normals,
+                                 double* partials, double* estore, double* carry, longlong2* sums, double* result,
+                                 int n_sms, cudaStream_t s, int* launches);
 
 }  // namespace hjm

@@ -344,7 +344,7 @@ hjm_status hjm_run_static(void* cuda_stream, int32_t n_tenor, double dtau, const
         if (contract) {
             unsigned char* area = reinterpret_cast<unsigned char*>(resp_table);
             STATIC_CUDA(launch_contract_table(n_tenor, dt / dtau, (int)stride, B, false, false, &P.sv[0][0], false, area, s));
-            STATIC_CUDA(launch_path_contract(n_tenor, P, area, nullptr, nullptr, partials, nullptr,
+            STATIC_CUDA(launch_path_contract(n_tenor, P, area, nullptr, partials, nullptr,
                                              reinterpret_cast<double*>(area + carry_at),
                                              reinterpret_cast<longlong2*>(area + split_at), result, n_sms, s, nullptr));
         } else {
