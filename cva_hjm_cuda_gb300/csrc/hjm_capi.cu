@@ -938,7 +938,19 @@ static int mresp_run_slots(hjm_ctx* ctx, const RunShape& sh, double dt, bool pc 
     return k.ns;
 }
 
-// Its table on the stream (for the shape mresp_run_slots counted): built
+// Room for its table (for the shape mresp_run_slots counted).
+static hjm_status mresp_room(hjm_ctx* ctx)
+{
+    hjm_ctx::MrespKey& k = ctx->mresp_key;
+    const size_t bytes = sizeof(float4) * mresp_table_elems(k.stride, k.B, k.ns);
+    if (bytes > ctx->mresp.bytes) {
+        k.on_device = false;
+        HJM_CUDA(ctx, ctx->mresp.ensure(bytes));  // cudaFree waits for the device
+    }
+    return HJM_OK;
+}
+
+// The table on the stream: built
 // only when the shape changed, after the kernels of earlier valuations that
 // read the old one.
 static hjm_status ensure_mresp_table(hjm_ctx* ctx, cudaStream_t s)
@@ -946,11 +958,9 @@ static hjm_status ensure_mresp_table(hjm_ctx* ctx, cudaStream_t s)
     hjm_ctx::MrespKey& k = ctx->mresp_key;
     if (k.on_device) return HJM_OK;
     if (!ctx->resp_used) HJM_CUDA(ctx, cudaEventCreateWithFlags(&ctx->resp_used, cudaEventDisableTiming));
-    const size_t bytes = sizeof(float4) * mresp_table_elems(k.stride, k.B, k.ns);
-    if (bytes > ctx->mresp.bytes)
-        HJM_CUDA(ctx, ctx->mresp.ensure(bytes));  // cudaFree waits for the device
-    else
-        HJM_CUDA(ctx, cudaStreamWaitEvent(s, ctx->resp_used, 0));
+    const hjm_status st = mresp_room(ctx);
+    if (st != HJM_OK) return st;
+    HJM_CUDA(ctx, cudaStreamWaitEvent(s, ctx->resp_used, 0));
     HJM_CUDA(ctx, launch_mresp_table(k.nt, k.c, k.dtau, k.stride, k.B, k.ns, k.pc, (float4*)ctx->mresp.p, s));
     ctx->stat_launches += 1;
     k.on_device = true;
@@ -992,9 +1002,10 @@ static hjm_status enqueue_impl(hjm_ctx* ctx, int64_t n_paths, int32_t n_steps, d
     HJM_CUDA(ctx, ctx->sums.ensure(sizeof(double) * kSumsLen));
     HJM_CUDA(ctx, ctx->result.ensure(sizeof(double) * kResLen));
     if (store) HJM_CUDA(ctx, ctx->estore.ensure(esize * (size_t)n_dates * (size_t)ld));
-    if (want_pfe) {
-        HJM_CUDA(ctx, ctx->sel.ensure(sizeof(SelState) * kMaxTenor));
-        HJM_CUDA(ctx, ctx->hist.ensure(pfe_scratch_bytes(n_paths, n_dates, !mixed)));
+    if (want_pfe) HJM_CUDA(ctx, ctx->sel.ensure(sizeof(SelState) * kMaxTenor));
+    if (mresp_ns) {
+        st = mresp_room(ctx);
+        if (st != HJM_OK) return st;
     }
     // what the contraction needs besides: its table and carry, without which
     // the run convects, and its split tiles' sums, without which they run whole
@@ -1014,6 +1025,9 @@ static hjm_status enqueue_impl(hjm_ctx* ctx, int64_t n_paths, int32_t n_steps, d
             HJM_CUDA(ctx, ctx->partials.ensure(sizeof(double) * (size_t)n_ctas * R));
         }
     }
+    // the PFE's candidates last, in what room is left
+    size_t pfe_bytes = want_pfe ? pfe_scratch_bytes(n_paths, n_dates, !mixed) : 0;
+    while (pfe_bytes && !try_ensure(ctx->hist, pfe_bytes)) pfe_bytes = pfe_bytes > 4096 ? pfe_bytes / 2 : 0;
     cudaStream_t s = ctx->stream;
     // external normals (on the device in the caller's order) in the form's own
     const double* ext_dev = ext_raw ? (const double*)ctx->ext.p : nullptr;
@@ -1120,7 +1134,7 @@ static hjm_status enqueue_impl(hjm_ctx* ctx, int64_t n_paths, int32_t n_steps, d
         if (resp) HJM_CUDA(ctx, cudaEventRecord(ctx->resp_used, s));
     }
     HJM_CUDA(ctx, cudaEventRecord(ctx->ev[1], s));
-    HJM_CUDA(ctx, launch_reduce((const double*)ctx->partials.p, n_ctas, R, (double*)ctx->sums.p, kSumsLen, F,
+    HJM_CUDA(ctx, launch_reduce((double*)ctx->partials.p, n_ctas, R, (double*)ctx->sums.p, F,
                                 (double*)ctx->result.p, s));
     HJM_CUDA(ctx, cudaEventRecord(ctx->ev[2], s));
     if (want_pfe) {
@@ -1128,8 +1142,8 @@ static hjm_status enqueue_impl(hjm_ctx* ctx, int64_t n_paths, int32_t n_steps, d
                                             n_paths);
         int launches = 0;
         HJM_CUDA(ctx, launch_pfe(ctx->estore.p, !mixed, ld, n_paths, n_dates, (uint64_t)(k - 1),
-                                 (SelState*)ctx->sel.p, ctx->hist.p, (double*)ctx->result.p, ctx->n_sms, s,
-                                 &launches));
+                                 (SelState*)ctx->sel.p, ctx->hist.p, pfe_bytes, (double*)ctx->result.p,
+                                 ctx->n_sms, s, &launches));
         ctx->stat_launches += launches;
     }
     HJM_CUDA(ctx, cudaEventRecord(ctx->ev[3], s));
@@ -1473,7 +1487,7 @@ hjm_status hjm_run_adjoint(hjm_ctx* ctx, int64_t n_paths, int32_t n_steps, doubl
                                      K > 0 ? (float*)ctx->ck_h.p : nullptr, K > 0 ? (double*)ctx->ck_a.p : nullptr, s));
     }
     HJM_CUDA(ctx, cudaEventRecord(ctx->ev[1], s));
-    HJM_CUDA(ctx, launch_reduce((const double*)ctx->partials.p, n_ctas, R, (double*)ctx->sums.p, kSumsLen, F,
+    HJM_CUDA(ctx, launch_reduce((double*)ctx->partials.p, n_ctas, R, (double*)ctx->sums.p, F,
                                 (double*)ctx->result.p, s));
     HJM_CUDA(ctx, cudaEventRecord(ctx->ev[2], s));
     HJM_CUDA(ctx, cudaEventRecord(ctx->ev[3], s));
@@ -1688,7 +1702,7 @@ hjm_status hjm_run_mlmc(hjm_ctx* ctx, int32_t n_levels, const int64_t* n_paths, 
         else
             HJM_CUDA(ctx, launch_mlmc_level(nt, Q, use_poly_path(ctx), (double*)ctx->partials.p, s));
         HJM_CUDA(ctx, cudaEventRecord(ctx->ev[1], s));
-        HJM_CUDA(ctx, launch_reduce((const double*)ctx->partials.p, n_ctas, R, (double*)ctx->sums.p, kSumsLen, F,
+        HJM_CUDA(ctx, launch_reduce((double*)ctx->partials.p, n_ctas, R, (double*)ctx->sums.p, F,
                                     (double*)ctx->result.p, s));
         HJM_CUDA(ctx, cudaEventRecord(ctx->ev[2], s));
         HJM_CUDA(ctx, cudaEventRecord(ctx->ev[3], s));

@@ -495,7 +495,7 @@ __device__ __forceinline__ void neumaier_warp(double& s, double& comp)
 }
 
 __global__ void __launch_bounds__(kReduceThreads)
-    reduce_columns(const double* __restrict__ partials, int64_t n_rows, int R, double* __restrict__ sums,
+    reduce_columns(double* partials, int64_t n_rows, int R, double* __restrict__ sums,
                    const __grid_constant__ FinalParams F, double* __restrict__ result)
 {
     constexpr int kWarps = kReduceThreads / 32;
@@ -525,7 +525,8 @@ __global__ void __launch_bounds__(kReduceThreads)
             comp += cs[w];
             neumaier_add(s, comp, ss[w]);
         }
-        sums[(size_t)(ranges > 1 ? blockIdx.y + 1 : 0) * R + col] = s + comp;
+        // (a range's sum into its first row, which this CTA alone has read)
+        (ranges > 1 ? partials + (size_t)begin * R : sums)[col] = s + comp;
         __threadfence();
         last_s = atomicAdd(reinterpret_cast<uint32_t*>(result + kResCount), 1u) == gridDim.x * gridDim.y - 1;
     }
@@ -535,7 +536,7 @@ __global__ void __launch_bounds__(kReduceThreads)
     if (ranges > 1) {
         for (int c = t; c < R; c += kReduceThreads) {
             double a = 0.0, ca = 0.0;
-            for (int g = 1; g <= ranges; ++g) neumaier_add(a, ca, __ldcg(sums + (size_t)g * R + c));
+            for (int g = 0; g < ranges; ++g) neumaier_add(a, ca, __ldcg(partials + (size_t)(per * g) * R + c));
             sums[c] = a + ca;
         }
         __syncthreads();
@@ -701,11 +702,10 @@ int path_cta(bool mixed, int nt, int n_blocks, bool poly)
     return mixed ? mixed_cta(nt, n_blocks, poly) : kFp64Cta;
 }
 
-cudaError_t launch_reduce(const double* partials, int64_t n_rows, int R, double* sums, int64_t sums_len,
-                          const FinalParams& F, double* result, cudaStream_t s)
+cudaError_t launch_reduce(double* partials, int64_t n_rows, int R, double* sums, const FinalParams& F, double* result,
+                          cudaStream_t s)
 {
-    if (sums_len < R) return cudaErrorInvalidValue;
-    const int64_t ranges = std::max<int64_t>(1, std::min(std::min(n_rows / kReduceRows, (int64_t)kReduceRanges), sums_len / R - 1));
+    const int64_t ranges = std::max<int64_t>(1, std::min(n_rows / kReduceRows, (int64_t)kReduceRanges));
     reduce_columns<<<dim3((unsigned)R, (unsigned)ranges), kReduceThreads, 0, s>>>(partials, n_rows, R, sums, F, result);
     return cudaGetLastError();
 }

@@ -120,16 +120,17 @@ size_t path_smem(int nt, int n_blocks, bool mixed);
 int path_cta(bool mixed, int nt, int n_blocks, bool poly);
 
 // Column sums into sums[0 .. R) and the results (result cleared before on the
-// stream); sums_len doubles, more than R of them for row ranges of their own
-constexpr int64_t kSumsLen = 2048;
-cudaError_t launch_reduce(const double* partials, int64_t n_rows, int R, double* sums, int64_t sums_len,
-                          const FinalParams& F, double* result, cudaStream_t s);
+// stream); the partial rows are scratch afterwards
+constexpr int64_t kSumsLen = 4 * kMaxTenor;
+cudaError_t launch_reduce(double* partials, int64_t n_rows, int R, double* sums, const FinalParams& F, double* result,
+                          cudaStream_t s);
 // The PFE selection (hjm_pfe.cu): result[kResPFE + date] = the key of rank k0 of
-// each date's column.  scratch: pfe_scratch_bytes() of device memory; *launches:
-// kernels enqueued.
+// each date's column.  scratch: pfe_scratch_bytes() of device memory, or less (the
+// same keys, more slowly); *launches: kernels enqueued.
 size_t pfe_scratch_bytes(int64_t n_paths, int n_dates, bool fp64_keys);
 cudaError_t launch_pfe(const void* estore, bool fp64_keys, int64_t ld, int64_t n_paths, int n_dates, uint64_t k0,
-                       SelState* st, void* scratch, double* result, int n_sms, cudaStream_t s, int* launches);
+                       SelState* st, void* scratch, size_t scratch_bytes, double* result, int n_sms, cudaStream_t s,
+                       int* launches);
 cudaError_t launch_dump_normals(int64_t n_paths, uint64_t path_offset, int n_steps, uint32_t k0, uint32_t k1,
                                 double* out, cudaStream_t s);
 cudaError_t launch_philox_words(int64_t n_paths, uint64_t path_offset, uint32_t step, uint32_t k0, uint32_t k1,

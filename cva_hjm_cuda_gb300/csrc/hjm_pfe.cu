@@ -317,8 +317,8 @@ bool fits_column(int64_t n, size_t key_bytes) { return (size_t)n * key_bytes <= 
 int64_t capacity(int64_t n) { return (n / 12 + 1023) / 1024 * 1024; }
 
 template <typename K>
-cudaError_t select_t(const K* keys, int64_t ld, int64_t n, int n_dates, uint64_t k, SelState* st, K* buf, double* result,
-                     int n_sms, cudaStream_t s, int* launches)
+cudaError_t select_t(const K* keys, int64_t ld, int64_t n, int n_dates, uint64_t k, SelState* st, K* buf,
+                     size_t buf_bytes, double* result, int n_sms, cudaStream_t s, int* launches)
 {
     if (fits_column(n, sizeof(K))) {
         const size_t smem = (size_t)n * sizeof(K);
@@ -340,8 +340,9 @@ cudaError_t select_t(const K* keys, int64_t ld, int64_t n, int n_dates, uint64_t
     pfe_bracket<K><<<n_dates, kThreads, smem, s>>>(keys, ld, step, m, r0, r1, st);
     // eight CTAs per SM over all dates, each with at least a few thousand keys
     const int64_t gx = std::max<int64_t>(1, std::min<int64_t>((n + 4095) / 4096, (int64_t)n_sms * 8 / n_dates));
-    pfe_split<K><<<dim3((unsigned)gx, (unsigned)n_dates), 256, 0, s>>>(keys, ld, n, st, buf, capacity(n));
-    pfe_pick<K><<<n_dates, kThreads, 0, s>>>(keys, ld, n, n_dates, k, st, buf, capacity(n), result);
+    const int64_t cap = std::min<int64_t>(capacity(n), (int64_t)(buf_bytes / (sizeof(K) * (size_t)n_dates)));
+    pfe_split<K><<<dim3((unsigned)gx, (unsigned)n_dates), 256, 0, s>>>(keys, ld, n, st, buf, cap);
+    pfe_pick<K><<<n_dates, kThreads, 0, s>>>(keys, ld, n, n_dates, k, st, buf, cap, result);
     *launches = 3;
     return cudaGetLastError();
 }
@@ -355,12 +356,13 @@ size_t pfe_scratch_bytes(int64_t n, int n_dates, bool fp64_keys)
 }
 
 cudaError_t launch_pfe(const void* estore, bool fp64_keys, int64_t ld, int64_t n_paths, int n_dates, uint64_t k0,
-                       SelState* st, void* scratch, double* result, int n_sms, cudaStream_t s, int* launches)
+                       SelState* st, void* scratch, size_t scratch_bytes, double* result, int n_sms, cudaStream_t s,
+                       int* launches)
 {
-    return fp64_keys ? select_t((const int64_t*)estore, ld, n_paths, n_dates, k0, st, (int64_t*)scratch, result,
-                                n_sms, s, launches)
-                     : select_t((const int32_t*)estore, ld, n_paths, n_dates, k0, st, (int32_t*)scratch, result,
-                                n_sms, s, launches);
+    return fp64_keys ? select_t((const int64_t*)estore, ld, n_paths, n_dates, k0, st, (int64_t*)scratch,
+                                scratch_bytes, result, n_sms, s, launches)
+                     : select_t((const int32_t*)estore, ld, n_paths, n_dates, k0, st, (int32_t*)scratch,
+                                scratch_bytes, result, n_sms, s, launches);
 }
 
 }  // namespace hjm

@@ -351,7 +351,7 @@ hjm_status hjm_run_static(void* cuda_stream, int32_t n_tenor, double dtau, const
             STATIC_CUDA(launch_path_fp64(n_tenor, P, poly, nullptr, partials, nullptr, s));
         }
     }
-    STATIC_CUDA(launch_reduce(partials, n_ctas, R, sums, 2 * kMaxTenor, F, result, s));
+    STATIC_CUDA(launch_reduce(partials, n_ctas, R, sums, F, result, s));
     double res[kResLen];
     STATIC_CUDA(cudaMemcpyAsync(res, result, sizeof(res), cudaMemcpyDeviceToHost, s));
     STATIC_CUDA(cudaStreamSynchronize(s));
