@@ -120,8 +120,8 @@ struct hjm_ctx {
     // the tables in contract and mresp hold the run shapes of their keys;
     // resp_used is recorded after the last kernel that reads one
     struct ContractKey {  // the contraction's operand table in contract
-        bool valid = false, ext = false;
-        int nt = 0, stride = 0, B = 0, scheme = 0;
+        bool valid = false;
+        int nt = 0, stride = 0, B = 0, scheme = 0, slots = 0;
         double c = 0;
         std::vector<double> sv;
     } contract_key;
@@ -820,9 +820,10 @@ static bool use_response_form(const hjm_ctx* ctx) { return ctx->remainder != HJM
 
 // The contraction's operand table of the run shape, scheme and loadings sv
 // [kFactors][kMaxTenor] (the path parameters'), on the stream: rebuilt only
-// when it changed, after the kernels of earlier valuations that read it.
-static hjm_status ensure_contract_table(hjm_ctx* ctx, const RunShape& sh, double dt, const double* sv, bool ext,
-                                        cudaStream_t s)
+// when it changed, after the kernels of earlier valuations that read it.  (A
+// compact plan's images are built between the launches that read them.)
+static hjm_status ensure_contract_table(hjm_ctx* ctx, const RunShape& sh, double dt, const double* sv,
+                                        ContractPlan plan, cudaStream_t s)
 {
     const double c = dt / ctx->dtau;
     const int nt = ctx->nt;
@@ -832,19 +833,20 @@ static hjm_status ensure_contract_table(hjm_ctx* ctx, const RunShape& sh, double
     hjm_ctx::ContractKey& k = ctx->contract_key;
     if (!ctx->resp_used) HJM_CUDA(ctx, cudaEventCreateWithFlags(&ctx->resp_used, cudaEventDisableTiming));
     const bool same_shape = k.valid && k.nt == nt && k.stride == sh.stride && k.B == sh.B && k.c == c &&
-                            k.scheme == ctx->scheme && k.ext == ext;
+                            k.scheme == ctx->scheme && k.slots == plan.slots && !plan.compact;
     if (same_shape && k.sv == key) return HJM_OK;
     k.valid = false;
     HJM_CUDA(ctx, cudaStreamWaitEvent(s, ctx->resp_used, 0));
-    HJM_CUDA(ctx, launch_contract_table(nt, c, sh.stride, sh.B, ctx->scheme == HJM_SCHEME_PREDICTOR_CORRECTOR, ext,
+    if (plan.compact) return HJM_OK;
+    HJM_CUDA(ctx, launch_contract_table(nt, c, sh.stride, sh.B, ctx->scheme == HJM_SCHEME_PREDICTOR_CORRECTOR, plan,
                                         sv, same_shape, ctx->contract.p, s));
-    ctx->stat_launches += (same_shape ? 1 : 2) + contract_windows(sh.B, sh.stride, ext, nullptr);
+    ctx->stat_launches += (same_shape ? 1 : 2) + contract_windows(sh.B, sh.stride, plan, nullptr);
     k.nt = nt;
     k.stride = sh.stride;
     k.B = sh.B;
     k.c = c;
     k.scheme = ctx->scheme;
-    k.ext = ext;
+    k.slots = plan.slots;
     k.sv = key;
     k.valid = true;
     return HJM_OK;
@@ -857,31 +859,42 @@ static bool try_ensure(DevBuf& b, size_t bytes)
     return false;
 }
 
-// Room for the contraction's table and the carry of a windowed run.
-static bool contract_room(hjm_ctx* ctx, const RunShape& sh, int64_t n_paths, bool ext)
+// Room for the contraction's table and the carry of a windowed run: the first plan
+// that both fit, and nothing held for one that does not.
+static bool contract_room(hjm_ctx* ctx, const RunShape& sh, int64_t n_paths, bool ext, ContractPlan& plan)
 {
-    const size_t bytes = contract_table_bytes(sh.stride, sh.B, ext);
-    if (bytes > ctx->contract.bytes) {
-        ctx->contract_key.valid = false;  // (growing drops the table it held)
-        if (!try_ensure(ctx->contract, bytes)) return false;
+    const MemBudget& m = ctx->budget;
+    for (int i = 0; i < kContractPlans; ++i) {
+        plan = contract_plan(i, ext);
+        const size_t bytes = contract_table_bytes(sh.stride, sh.B, plan);
+        const size_t carry =
+            contract_windows(sh.B, sh.stride, plan, nullptr) > 1 ? sizeof(double) * 2 * (size_t)n_paths : 0;
+        const size_t grow = (bytes > ctx->contract.bytes ? bytes - ctx->contract.bytes : 0) +
+                            (carry > ctx->carry.bytes ? carry - ctx->carry.bytes : 0);
+        if (grow && m.limit && m.used + grow > m.limit) continue;
+        if (bytes > ctx->contract.bytes) ctx->contract_key.valid = false;  // (growing drops the table it held)
+        if (try_ensure(ctx->contract, bytes) && try_ensure(ctx->carry, carry)) return true;
+        ctx->contract.release();
+        ctx->contract_key.valid = false;
     }
-    return contract_windows(sh.B, sh.stride, ext, nullptr) <= 1 ||
-           try_ensure(ctx->carry, sizeof(double) * 2 * (size_t)n_paths);
+    return false;
 }
 
 // An FP64 valuation in the response form (hjm_contract.cu): the operand table
-// of the market's loadings (contract_room made room for it and the carry), the
-// launches of its windows.  P: the scheme's parameters (the predictor-corrector's N-projected
+// of the market's loadings (contract_room chose the plan that it and the carry
+// have room for), the launches of its windows.  P: the scheme's parameters (the predictor-corrector's N-projected
 // loadings and deterministic curve).  ext_dev: external normals
 // (launch_contract_ext), or null.
 static hjm_status enqueue_contract(hjm_ctx* ctx, const RunShape& sh, double dt, const PathParams<double>& P,
-                                   const double* ext_dev, double* estore, longlong2* split, cudaStream_t s)
+                                   ContractPlan plan, const double* ext_dev, double* estore, longlong2* split,
+                                   cudaStream_t s)
 {
-    hjm_status st = ensure_contract_table(ctx, sh, dt, &P.sv[0][0], ext_dev != nullptr, s);
+    hjm_status st = ensure_contract_table(ctx, sh, dt, &P.sv[0][0], plan, s);
     if (st != HJM_OK) return st;
     int launches = 0;
-    HJM_CUDA(ctx, launch_path_contract(ctx->nt, P, ctx->contract.p, ext_dev, (double*)ctx->partials.p, estore,
-                                       (double*)ctx->carry.p, split, (double*)ctx->result.p, ctx->n_sms, s, &launches));
+    HJM_CUDA(ctx, launch_contract(ctx->nt, dt / ctx->dtau, ctx->scheme == HJM_SCHEME_PREDICTOR_CORRECTOR, &P.sv[0][0], P,
+                                  plan, !plan.compact, ctx->contract.p, ext_dev, (double*)ctx->partials.p, estore,
+                                  (double*)ctx->carry.p, split, (double*)ctx->result.p, ctx->n_sms, s, &launches));
     ctx->stat_launches += launches - 1;
     return HJM_OK;
 }
@@ -1010,13 +1023,14 @@ static hjm_status enqueue_impl(hjm_ctx* ctx, int64_t n_paths, int32_t n_steps, d
     // what the contraction needs besides: its table and carry, without which
     // the run convects, and its split tiles' sums, without which they run whole
     longlong2* split = nullptr;
-    if (contract && !contract_room(ctx, sh, n_paths, ext_raw != nullptr)) {
+    ContractPlan plan = {};
+    if (contract && !contract_room(ctx, sh, n_paths, ext_raw != nullptr, plan)) {
         contract = false;
         n_ctas = (n_paths + cta - 1) / cta;
         HJM_CUDA(ctx, ctx->partials.ensure(sizeof(double) * (size_t)n_ctas * R));
     }
     if (contract) {
-        const size_t bytes = contract_sums_bytes(n_paths, sh.B, sh.stride, ctx->n_sms, ext_raw != nullptr);
+        const size_t bytes = contract_sums_bytes(n_paths, sh.B, sh.stride, ctx->n_sms, plan);
         const int64_t rows = contract_rows(n_paths, sh.B, sh.stride, ctx->n_sms);
         if (bytes && try_ensure(ctx->split, bytes) && try_ensure(ctx->partials, sizeof(double) * (size_t)rows * R)) {
             split = (longlong2*)ctx->split.p;
@@ -1088,7 +1102,7 @@ static hjm_status enqueue_impl(hjm_ctx* ctx, int64_t n_paths, int32_t n_steps, d
         ctx->stat_h2d = sizeof(Q) + sizeof(FinalParams);
         resp = contract;
         if (resp) {
-            st = enqueue_contract(ctx, sh, dt, Q.P, ext_dev, store ? (double*)ctx->estore.p : nullptr, split, s);
+            st = enqueue_contract(ctx, sh, dt, Q.P, plan, ext_dev, store ? (double*)ctx->estore.p : nullptr, split, s);
             if (st != HJM_OK) return st;
         } else {
             HJM_CUDA(ctx, launch_path_pc(ctx->nt, Q, use_poly_path(ctx), ext_dev, (double*)ctx->partials.p,
@@ -1123,7 +1137,7 @@ static hjm_status enqueue_impl(hjm_ctx* ctx, int64_t n_paths, int32_t n_steps, d
         fill_params<double>(ctx, sh, n_paths, dt, seed, path_offset, hazard, recovery, ld, store, P, F);
         resp = contract;
         if (resp) {
-            st = enqueue_contract(ctx, sh, dt, P, ext_dev, store ? (double*)ctx->estore.p : nullptr, split, s);
+            st = enqueue_contract(ctx, sh, dt, P, plan, ext_dev, store ? (double*)ctx->estore.p : nullptr, split, s);
             if (st != HJM_OK) return st;
             if (use_cubic_path(ctx)) run_form = vol_form_code(ctx);
         } else {

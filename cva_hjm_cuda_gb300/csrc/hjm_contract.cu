@@ -913,22 +913,35 @@ struct ContractLoadings {
     double sv[kFactors][kMaxTenor];
 };
 
-// weights[i M + m] = {f_m(i), G_m(i) = sum_{r <= m} f_r(i)}, i < n.  f_m are
-// the coefficients of p^m, p = a0 + a1 z + a2 z^2: from p (p^m)' = m p' p^m,
+// The power of two that maps a date's largest response into [2^7, 2^8), as a
+// multiplier back (responses below 1e-280 count as zero), by its exponent's bits:
+// FP64 instructions are what the image kernel waits for (a division and the
+// exponent functions per element: 30 us for 32 dates of the 25y run against 19).
+__device__ __forceinline__ int contract_exponent(unsigned long long top)
+{
+    const bool in = top > (unsigned long long)__double_as_longlong(1e-280) &&
+                    top < (unsigned long long)__double_as_longlong(1e300);
+    return in ? (int)(top >> 52) - 1022 - kTopBits : 0;
+}
+__device__ __forceinline__ double power_of_two(int e) { return __hiloint2double((1023 + e) << 20, 0); }
+
+// One lag's walk (hjm_walk.cuh): {f_m(i), G_m(i) = sum_{r <= m} f_r(i)}, i = 0, 1, ..
+// f_m are the coefficients of p^m, p = a0 + a1 z + a2 z^2: from p (p^m)' = m p' p^m,
 //     (i + 1) a0 f(i+1) = (m - i) a1 f(i) + (2 m - i + 1) a2 f(i-1),
 // and G those of (p^{m+1} - 1) / (p - 1), whose partial sums telescope:
 //     (a1 + a2) G(i) + a2 G(i-1) = 1 - f_{m+1}(0) - .. - f_{m+1}(i),
-// so a rounding fades by a2 / (a1 + a2) a step.  One thread per lag (hjm_walk.cuh).
-__global__ void contract_weights_kernel(const __grid_constant__ WalkParams K, int M, int n, double2* __restrict__ weights)
-{
-    const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= M) return;
-    const double md = m;
-    double f = walk_power(K, md), f1 = 0.0, h = walk_power(K, md + 1.0), h1 = 0.0, g = 0.0, tail = 1.0;
-    for (int i = 0; i < n; ++i) {
+// so a rounding fades by a2 / (a1 + a2) a step.
+struct LagWalk {
+    double md, f, f1, h, h1, g, tail;
+    __device__ __forceinline__ LagWalk(const WalkParams& K, int m)
+        : md(m), f(walk_power(K, md)), f1(0.0), h(walk_power(K, md + 1.0)), h1(0.0), g(0.0), tail(1.0)
+    {
+    }
+    __device__ __forceinline__ double2 next(const WalkParams& K, int i)
+    {
         tail -= h;
         g = fma(tail, K.inv, -(K.b2 * g));
-        weights[(size_t)i * M + m] = make_double2(f, g);
+        const double2 out = make_double2(f, g);
         const double di = i;
         const double fn = fma((md - di) * K.a1, f, (2.0 * md - di + 1.0) * K.a2 * f1) * K.rcp[i];
         const double hn = fma((md + 1.0 - di) * K.a1, h, (2.0 * md - di + 3.0) * K.a2 * h1) * K.rcp[i];
@@ -936,44 +949,40 @@ __global__ void contract_weights_kernel(const __grid_constant__ WalkParams K, in
         f = fn;
         h1 = h;
         h = hn;
+        return out;
     }
+};
+
+// weights[i M + m], i < n: the walks of all lags, a thread each
+__global__ void contract_weights_kernel(const __grid_constant__ WalkParams K, int M, int n, double2* __restrict__ weights)
+{
+    const int m = blockIdx.x * blockDim.x + threadIdx.x;
+    if (m >= M) return;
+    LagWalk walk(K, m);
+    for (int i = 0; i < n; ++i) weights[(size_t)i * M + m] = walk.next(K, i);
 }
 
-// R_jk(m) and its running sum for date j = blockIdx.y + 2 at every lag it reads
-// (m < (j - 1) stride): resp[(k (B - 1) + j - 2) M + m], and the largest
-// magnitude over lags and factors in top[2 j + {0 value, 1 sum}] (bits; cleared
-// before).
-__global__ void __launch_bounds__(128)
-    contract_response_kernel(int nt, double c, int stride, int B, const __grid_constant__ ContractLoadings S,
-                             const double2* __restrict__ weights, unsigned long long* __restrict__ top,
-                             double2* __restrict__ resp)
-{
-    __shared__ double dev_s[kFactors][kMaxTenor];
-    __shared__ double top_s[2][4];
-    const int L = nt - 1, M = (B - 1) * stride, j = blockIdx.y + 2, lags = (j - 1) * stride;
-    const int m0 = blockIdx.x * blockDim.x, m = m0 + threadIdx.x;
-    if (m0 >= lags) return;
-    for (int i = threadIdx.x; i < kFactors * nt; i += blockDim.x) {
-        const int k = i / nt, t = i % nt;
-        dev_s[k][t] = t < L - 1 ? S.sv[k][t] - (S.sv[k][L] + (double)(t - L) * (S.sv[k][L] - S.sv[k][L - 1])) : 0.0;
-    }
-    __syncthreads();
-    double best[2] = {0.0, 0.0};
-    if (m < lags) {
-        double v[kFactors], w[kFactors];
+// A date's responses to the three factors and their running sums at lag m, the
+// lags of a CTA of 128 together: v, w from the walk's weights at(i), i = 0, 1, ..
+struct DateResponse {
+    double v[kFactors], w[kFactors];
+    template <typename At>
+    __device__ __forceinline__ DateResponse(const ContractLoadings& S, const double (&dev_s)[kFactors][kMaxTenor], int L,
+                                            double c, int j, int m, int m0, int lags, At at)
+    {
         const double md = m;
 #pragma unroll
         for (int k = 0; k < kFactors; ++k) {
-            const double d = S.sv[k][L] - S.sv[k][L - 1], at = fma((double)(j - L), d, S.sv[k][L]);
-            v[k] = fma(md * c, d, at);
-            w[k] = (md + 1.0) * fma(0.5 * md * c, d, at);
+            const double d = S.sv[k][L] - S.sv[k][L - 1], x = fma((double)(j - L), d, S.sv[k][L]);
+            v[k] = fma(md * c, d, x);
+            w[k] = (md + 1.0) * fma(0.5 * md * c, d, x);
         }
         // the walk of this block's lags ends within ten standard deviations and a
         // dozen tenors of its mean (1e-22 beyond)
         const double mean = c * (double)min(m0 + (int)blockDim.x, lags);
         const int n = min(L - 1 - j, (int)(mean + 10.0 * sqrt(mean)) + 12);
         for (int i = 0; i < n; ++i) {
-            const double2 p = weights[(size_t)i * M + m];
+            const double2 p = at(i);
 #pragma unroll
             for (int k = 0; k < kFactors; ++k) {
                 const double x = dev_s[k][j + i];
@@ -981,13 +990,31 @@ __global__ void __launch_bounds__(128)
                 w[k] = fma(p.y, x, w[k]);
             }
         }
+    }
+    // its largest magnitudes into best, the CTA's into top[2 j + {0 value, 1 sum}]
+    __device__ __forceinline__ void largest(double (&best)[2]) const
+    {
 #pragma unroll
         for (int k = 0; k < kFactors; ++k) {
-            resp[((size_t)k * (B - 1) + (j - 2)) * M + m] = make_double2(v[k], w[k]);
             best[0] = fmax(best[0], fabs(v[k]));
             best[1] = fmax(best[1], fabs(w[k]));
         }
     }
+};
+// The loadings' deviations from the line through the last two tenors
+__device__ __forceinline__ void load_deviations(const ContractLoadings& S, int nt, double (&dev_s)[kFactors][kMaxTenor])
+{
+    const int L = nt - 1;
+    for (int i = threadIdx.x; i < kFactors * nt; i += blockDim.x) {
+        const int k = i / nt, t = i % nt;
+        dev_s[k][t] = t < L - 1 ? S.sv[k][t] - (S.sv[k][L] + (double)(t - L) * (S.sv[k][L] - S.sv[k][L - 1])) : 0.0;
+    }
+    __syncthreads();
+}
+// A CTA's (128 threads) largest magnitudes of date j into top (bits; cleared before)
+__device__ __forceinline__ void store_largest(double (&best)[2], int j, unsigned long long* top)
+{
+    __shared__ double top_s[2][4];
     for (int o = 16; o > 0; o >>= 1) {
         best[0] = fmax(best[0], __shfl_xor_sync(0xffffffffu, best[0], o));
         best[1] = fmax(best[1], __shfl_xor_sync(0xffffffffu, best[1], o));
@@ -1004,36 +1031,65 @@ __global__ void __launch_bounds__(128)
     }
 }
 
-// The power of two that maps a date's largest response into [2^7, 2^8), as a
-// multiplier back (responses below 1e-280 count as zero), by its exponent's bits:
-// FP64 instructions are what the image kernel waits for (a division and the
-// exponent functions per element: 30 us for 32 dates of the 25y run against 19).
-__device__ __forceinline__ int contract_exponent(unsigned long long top)
+// R_jk(m) and its running sum for date j = blockIdx.y + 2 at every lag it reads
+// (m < (j - 1) stride): resp[(k (B - 1) + j - 2) M + m], and the largest
+// magnitude over lags and factors in top.
+__global__ void __launch_bounds__(128)
+    contract_response_kernel(int nt, double c, int stride, int B, const __grid_constant__ ContractLoadings S,
+                             const double2* __restrict__ weights, unsigned long long* __restrict__ top,
+                             double2* __restrict__ resp)
 {
-    const bool in = top > (unsigned long long)__double_as_longlong(1e-280) &&
-                    top < (unsigned long long)__double_as_longlong(1e300);
-    return in ? (int)(top >> 52) - 1022 - kTopBits : 0;
+    __shared__ double dev_s[kFactors][kMaxTenor];
+    const int M = (B - 1) * stride, j = blockIdx.y + 2, lags = (j - 1) * stride;
+    const int m0 = blockIdx.x * blockDim.x, m = m0 + threadIdx.x;
+    if (m0 >= lags) return;
+    load_deviations(S, nt, dev_s);
+    double best[2] = {0.0, 0.0};
+    if (m < lags) {
+        const DateResponse r(S, dev_s, nt - 1, c, j, m, m0, lags, [&](int i) { return weights[(size_t)i * M + m]; });
+#pragma unroll
+        for (int k = 0; k < kFactors; ++k) resp[((size_t)k * (B - 1) + (j - 2)) * M + m] = make_double2(r.v[k], r.w[k]);
+        r.largest(best);
+    }
+    store_largest(best, j, top);
 }
-__device__ __forceinline__ double power_of_two(int e) { return __hiloint2double((1023 + e) << 20, 0); }
 
-// The image of one window: per chunk three k-tiles of 16 rows of the
-// contraction (value 3 i + k of the chunk: step i, factor k), per k-tile two
-// halves of 8, each holding the 4 npad rows n = slice npad + 2 slot + {0 value,
-// 1 sum} as consecutive 16-byte rows.
+// The scales of the dates from their largest responses
+__device__ __forceinline__ void store_scales(const unsigned long long* top, double* scale)
+{
+    for (int i = threadIdx.x; i < 2 * kMaxTenor; i += blockDim.x)
+        scale[i] = power_of_two(contract_exponent(top[i])) * kSumUnit;
+}
+// The slices of a scaled response x into row val (value 3 i + k of a chunk: step i,
+// factor k) and column col of the chunk's image: three k-tiles of 16 rows, each two
+// halves of 8 that hold the kLevels npad columns slice npad + 2 slot + {0 value, 1
+// sum} as consecutive 16-byte rows.
+__device__ __forceinline__ void store_slices(unsigned char* image, int npad, int chunk, int val, int col, double x)
+{
+    const int oct = val >> 3;
+    unsigned char* out = image + (size_t)chunk * chunk_bytes(npad) + (size_t)(oct >> 1) * (kLevels * npad * 32) +
+                         (size_t)(oct & 1) * (kLevels * npad * 16);
+#pragma unroll
+    for (int s = 0; s < kLevels; ++s) {
+        const double b = s < kLevels - 1 ? rint(x) : x;
+        *reinterpret_cast<__half*>(out + (size_t)(s * npad + col) * 16 + 2 * (val & 7)) = __float2half_rn((float)b);
+        x = (x - b) * (double)kShift;
+    }
+}
+
+// The image of one window from the responses, padding included
 __global__ void contract_image_kernel(int stride, int B, ContractWindow W, const unsigned long long* __restrict__ top,
                                       const double2* __restrict__ resp, double* __restrict__ scale,
                                       unsigned char* __restrict__ image)
 {
     const int M = (B - 1) * stride;
-    if (blockIdx.x == 0)
-        for (int i = threadIdx.x; i < 2 * kMaxTenor; i += blockDim.x)
-            scale[i] = power_of_two(contract_exponent(top[i])) * kSumUnit;
+    if (blockIdx.x == 0) store_scales(top, scale);
     const int64_t per_chunk = 48 * (int64_t)W.npad;
     const int64_t total = per_chunk * W.chunks;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
         const int chunk = (int)(i / per_chunk), rem = (int)(i % per_chunk);
-        const int kk = rem & 7, col = (rem >> 3) % W.npad, oct = (rem >> 3) / W.npad;  // octet of values: 0..5
-        const int val = 8 * oct + kk, step = chunk * kChunk + val / 3, k = val % 3;
+        const int col = (rem >> 3) % W.npad, val = 8 * ((rem >> 3) / W.npad) + (rem & 7);
+        const int step = chunk * kChunk + val / 3, k = val % 3;
         const int slot = col >> 1, j = W.hi - slot;
         double x = 0.0;
         if (slot < W.slots) {
@@ -1043,15 +1099,45 @@ __global__ void contract_image_kernel(int stride, int B, ContractWindow W, const
                 x = ((col & 1) ? r.y : r.x) * power_of_two(-contract_exponent(top[2 * j + (col & 1)]));
             }
         }
-        unsigned char* out = image + (size_t)chunk * chunk_bytes(W.npad) +
-                             (size_t)(oct >> 1) * (kLevels * W.npad * 32) + (size_t)(oct & 1) * (kLevels * W.npad * 16);
+        store_slices(image, W.npad, chunk, val, col, x);
+    }
+}
+
+// The image of one window with nothing kept beside it (blockIdx.y: the slot): every
+// thread walks its own lag, first (IMAGE = false) for the dates' largest responses,
+// then again for the slices (the image cleared before).  The walk's serial FP64
+// chain twice and three times the FP64 work of the two kernels above: for runs that
+// have no room for their scratch.
+template <bool IMAGE>
+__global__ void __launch_bounds__(128)
+    contract_compact_kernel(int nt, double c, int stride, const __grid_constant__ ContractLoadings S,
+                            const __grid_constant__ WalkParams K, ContractWindow W, unsigned long long* __restrict__ top,
+                            double* __restrict__ scale, unsigned char* __restrict__ image)
+{
+    __shared__ double dev_s[kFactors][kMaxTenor];
+    const int slot = blockIdx.y, j = W.hi - slot, lags = (j - 1) * stride;
+    const int m0 = blockIdx.x * blockDim.x, m = m0 + threadIdx.x;
+    if (IMAGE && blockIdx.x == 0 && slot == 0) store_scales(top, scale);
+    if (m0 >= lags) return;
+    load_deviations(S, nt, dev_s);
+    double best[2] = {0.0, 0.0};
+    if (m < lags) {
+        LagWalk walk(K, m);
+        const DateResponse r(S, dev_s, nt - 1, c, j, m, m0, lags, [&](int i) { return walk.next(K, i); });
+        if constexpr (IMAGE) {
+            const int step = lags - 1 - m;
+            const double sx = power_of_two(-contract_exponent(top[2 * j])),
+                         sa = power_of_two(-contract_exponent(top[2 * j + 1]));
 #pragma unroll
-        for (int s = 0; s < kLevels; ++s) {
-            const double b = s < kLevels - 1 ? rint(x) : x;
-            *reinterpret_cast<__half*>(out + (size_t)(s * W.npad + col) * 16 + 2 * kk) = __float2half_rn((float)b);
-            x = (x - b) * (double)kShift;
+            for (int k = 0; k < kFactors; ++k) {
+                store_slices(image, W.npad, step / kChunk, 3 * (step % kChunk) + k, 2 * slot, r.v[k] * sx);
+                store_slices(image, W.npad, step / kChunk, 3 * (step % kChunk) + k, 2 * slot + 1, r.w[k] * sa);
+            }
+        } else {
+            r.largest(best);
         }
     }
+    if constexpr (!IMAGE) store_largest(best, j, top);
 }
 
 // The power of two 2^e of each path: e the least that brings the evolved steps'
@@ -1131,9 +1217,9 @@ constexpr size_t kContractSmemMost = contract_smem(2 * kContractMaxSlots, kContr
 
 }  // namespace
 
-int contract_windows(int n_blocks, int stride, bool ext, ContractWindow* w)
+int contract_windows(int n_blocks, int stride, ContractPlan plan, ContractWindow* w)
 {
-    const int most = ext ? kContractExtSlots : kContractMaxSlots;
+    const int most = plan.slots;
     int n = 0;
     size_t image = align_up(2 * kScaleBytes);
     for (int hi = n_blocks; hi >= 1;) {
@@ -1145,7 +1231,7 @@ int contract_windows(int n_blocks, int stride, bool ext, ContractWindow* w)
         x.npad = std::max((2 * x.slots + 15) / 16 * 16, 16);
         x.chunks = ((hi - 1) * stride + kChunk - 1) / kChunk;
         x.image = image;
-        image += align_up((size_t)x.chunks * chunk_bytes(x.npad));
+        if (!plan.compact) image += align_up((size_t)x.chunks * chunk_bytes(x.npad));
         if (w) w[n] = x;
         ++n;
         hi = lo - 1;
@@ -1153,24 +1239,30 @@ int contract_windows(int n_blocks, int stride, bool ext, ContractWindow* w)
     return n;
 }
 
-size_t contract_table_bytes(int stride, int n_blocks, bool ext)
+size_t contract_table_bytes(int stride, int n_blocks, ContractPlan plan)
 {
     ContractWindow w[kMaxTenor];
-    const int n = contract_windows(n_blocks, stride, ext, w);
-    const ContractWindow& last = w[n - 1];
+    const int n = contract_windows(n_blocks, stride, plan, w);
+    size_t end = 0;
+    for (int i = 0; i < n; ++i) end = std::max(end, w[i].image + align_up((size_t)w[i].chunks * chunk_bytes(w[i].npad)));
+    if (plan.compact) return end;
     const size_t dates = std::max(n_blocks - 1, 1), lags = dates * stride;
-    return last.image + align_up((size_t)last.chunks * chunk_bytes(last.npad)) +
-           sizeof(double2) * lags * (kFactors * dates + kMaxTenor);
+    return end + sizeof(double2) * lags * (kFactors * dates + kMaxTenor);
 }
 
-cudaError_t launch_contract_table(int nt, double c, int stride, int n_blocks, bool pc, bool ext, const double* sv,
-                                  bool same_shape, void* table, cudaStream_t s)
+static bool table_shape_ok(int nt, int n_blocks, int stride)
 {
-    if (nt < 35 || nt > kMaxTenor || n_blocks < 1 || n_blocks >= nt || stride < 1) return cudaErrorInvalidValue;
+    return nt >= 35 && nt <= kMaxTenor && n_blocks >= 1 && n_blocks < nt && stride >= 1;
+}
+
+cudaError_t launch_contract_table(int nt, double c, int stride, int n_blocks, bool pc, ContractPlan plan,
+                                  const double* sv, bool same_shape, void* table, cudaStream_t s)
+{
+    if (!table_shape_ok(nt, n_blocks, stride) || plan.compact) return cudaErrorInvalidValue;
     ContractLoadings S;
     std::memcpy(S.sv, sv, sizeof(S.sv));
     ContractWindow w[kMaxTenor];
-    const int n = contract_windows(n_blocks, stride, ext, w);
+    const int n = contract_windows(n_blocks, stride, plan, w);
     if (n_blocks == 1) return cudaSuccess;  // date 1 alone: nothing evolves
     double* scale = (double*)table;
     unsigned long long* top = (unsigned long long*)((unsigned char*)table + kScaleBytes);
@@ -1190,6 +1282,26 @@ cudaError_t launch_contract_table(int nt, double c, int stride, int n_blocks, bo
         contract_image_kernel<<<(unsigned)std::min<int64_t>((total + 255) / 256, 1216), 256, 0, s>>>(
             stride, n_blocks, w[i], top, resp, scale, (unsigned char*)table + w[i].image);
     }
+    return cudaGetLastError();
+}
+
+cudaError_t launch_contract_window(int nt, double c, int stride, int n_blocks, bool pc, const ContractWindow& W,
+                                   const double* sv, void* table, cudaStream_t s)
+{
+    if (!table_shape_ok(nt, n_blocks, stride)) return cudaErrorInvalidValue;
+    if (W.slots == 0) return cudaSuccess;  // date 1 alone: nothing evolves
+    ContractLoadings S;
+    std::memcpy(S.sv, sv, sizeof(S.sv));
+    const WalkParams K = walk_params(c, pc);
+    double* scale = (double*)table;
+    unsigned long long* top = (unsigned long long*)((unsigned char*)table + kScaleBytes);
+    unsigned char* image = (unsigned char*)table + W.image;
+    // (the image lies behind the scales and the largest responses)
+    cudaError_t e = cudaMemsetAsync(table, 0, W.image + (size_t)W.chunks * chunk_bytes(W.npad), s);
+    if (e != cudaSuccess) return e;
+    const dim3 grid(((W.hi - 1) * stride + 127) / 128, W.slots);
+    contract_compact_kernel<false><<<grid, 128, 0, s>>>(nt, c, stride, S, K, W, top, scale, image);
+    contract_compact_kernel<true><<<grid, 128, 0, s>>>(nt, c, stride, S, K, W, top, scale, image);
     return cudaGetLastError();
 }
 
@@ -1231,66 +1343,79 @@ int64_t contract_rows(int64_t n_paths, int n_blocks, int stride, int n_sms, bool
     return (n_paths + kContractTile - 1) / kContractTile + 3 * split;
 }
 
-size_t contract_sums_bytes(int64_t n_paths, int n_blocks, int stride, int n_sms, bool ext)
+size_t contract_sums_bytes(int64_t n_paths, int n_blocks, int stride, int n_sms, ContractPlan plan)
 {
     ContractWindow w[kMaxTenor];
-    const int n = contract_windows(n_blocks, stride, ext, w);
+    const int n = contract_windows(n_blocks, stride, plan, w);
     int npad = 0;
     for (int i = 0; i < n; ++i) npad = std::max(npad, w[i].npad);
     return sizeof(longlong2) * (size_t)split_tiles(n_paths, n_blocks, stride, n_sms) * (npad / 2) * kContractTile;
 }
 
-cudaError_t launch_path_contract(int nt, const PathParams<double>& P, const void* table, const void* normals,
-                                 double* partials, double* estore, double* carry, longlong2* sums, double* result,
-                                 int n_sms, cudaStream_t s, int* launches)
+cudaError_t launch_path_contract(int nt, const PathParams<double>& P, const ContractWindow& W, const void* table,
+                                 const void* normals, double* partials, double* estore, double* carry, longlong2* sums,
+                                 double* result, int n_sms, cudaStream_t s, int* launches)
 {
     if (!path_tenor_supported(nt) || P.n_blocks < 1 || P.n_blocks >= nt || P.stride < 1) return cudaErrorInvalidValue;
+    if ((W.lo != 1 || W.hi != P.n_blocks) && !carry) return cudaErrorInvalidValue;
     const float2* ext = (const float2*)normals;
     const ExtRow* ext_row = (const ExtRow*)normals;
-    ContractWindow w[kMaxTenor];
-    const int n = contract_windows(P.n_blocks, P.stride, ext != nullptr, w);
-    if (n > 1 && !carry) return cudaErrorInvalidValue;
     auto kernel = ext ? path_kernel_contract<true> : path_kernel_contract<false>;
     auto price = ext ? contract_price_kernel<true> : contract_price_kernel<false>;
-    const cudaError_t allowed = allow_dynamic_smem(kernel, kContractSmemMost);
-    if (allowed != cudaSuccess) return allowed;
+    cudaError_t e = allow_dynamic_smem(kernel, kContractSmemMost);
+    if (e != cudaSuccess) return e;
     ContractParams Q;
     Q.P = P;
+    Q.W = W;
     const int64_t tiles = (P.n_paths + kContractTile - 1) / kContractTile;
     const int64_t split = sums ? split_tiles(P.n_paths, P.n_blocks, P.stride, n_sms) : 0, whole = tiles - split;
+    const size_t smem = contract_smem(W.npad, W.hi - W.lo + 1);
     int count = 0;
-    for (int i = 0; i < n; ++i) {
-        Q.W = w[i];
-        const size_t smem = contract_smem(w[i].npad, w[i].hi - w[i].lo + 1);
-        cudaError_t e;
-        if (whole > 0) {
-            Q.tile0 = 0;
-            Q.n_tiles = whole;
-            Q.sums = nullptr;
-            kernel<<<(unsigned)std::min<int64_t>(whole, n_sms), kThreads, smem, s>>>(
+    if (whole > 0) {
+        Q.tile0 = 0;
+        Q.n_tiles = whole;
+        Q.sums = nullptr;
+        kernel<<<(unsigned)std::min<int64_t>(whole, n_sms), kThreads, smem, s>>>(
+            Q, (const unsigned char*)table, ext, ext_row, partials, estore, carry, result);
+        ++count;
+    }
+    if (split > 0) {
+        Q.tile0 = whole;
+        Q.n_tiles = split;
+        Q.sums = sums;
+        const int64_t groups = split * tile_groups(W.chunks);
+        if (groups > 0) {
+            e = cudaMemsetAsync(sums, 0, sizeof(longlong2) * (size_t)split * (W.npad / 2) * kContractTile, s);
+            if (e != cudaSuccess) return e;
+            kernel<<<(unsigned)std::min<int64_t>(groups, n_sms), kThreads, smem, s>>>(
                 Q, (const unsigned char*)table, ext, ext_row, partials, estore, carry, result);
             ++count;
         }
-        if (split > 0) {
-            Q.tile0 = whole;
-            Q.n_tiles = split;
-            Q.sums = sums;
-            const int64_t groups = split * tile_groups(w[i].chunks);
-            if (groups > 0) {
-                e = cudaMemsetAsync(sums, 0, sizeof(longlong2) * (size_t)split * (w[i].npad / 2) * kContractTile, s);
-                if (e != cudaSuccess) return e;
-                kernel<<<(unsigned)std::min<int64_t>(groups, n_sms), kThreads, smem, s>>>(
-                    Q, (const unsigned char*)table, ext, ext_row, partials, estore, carry, result);
-                ++count;
-            }
-            price<<<(unsigned)(4 * split), 32 * kPriceWarps, 0, s>>>(Q, (const double*)table, ext_row, whole, partials,
-                                                                    estore, carry);
-            ++count;
+        price<<<(unsigned)(4 * split), 32 * kPriceWarps, 0, s>>>(Q, (const double*)table, ext_row, whole, partials,
+                                                                estore, carry);
+        ++count;
+    }
+    *launches += count;
+    return cudaGetLastError();
+}
+
+cudaError_t launch_contract(int nt, double c, bool pc, const double* sv, const PathParams<double>& P, ContractPlan plan,
+                            bool have_table, void* table, const void* normals, double* partials, double* estore,
+                            double* carry, longlong2* sums, double* result, int n_sms, cudaStream_t s, int* launches)
+{
+    ContractWindow w[kMaxTenor];
+    const int n = contract_windows(P.n_blocks, P.stride, plan, w);
+    *launches = 0;
+    for (int i = 0; i < n; ++i) {
+        if (!have_table) {
+            const cudaError_t e = launch_contract_window(nt, c, P.stride, P.n_blocks, pc, w[i], sv, table, s);
+            if (e != cudaSuccess) return e;
+            *launches += w[i].slots > 0 ? 2 : 0;
         }
-        e = cudaGetLastError();
+        const cudaError_t e = launch_path_contract(nt, P, w[i], table, normals, partials, estore, carry, sums, result,
+                                                   n_sms, s, launches);
         if (e != cudaSuccess) return e;
     }
-    if (launches) *launches = count;
     return cudaSuccess;
 }
 

@@ -18,10 +18,11 @@
 // cudaGetSymbolAddress, with that device current, and passes it to the same
 // path and reduction kernels that hjm_run launches.
 //
-// FP64 runs take the contraction (hjm_contract.cu) as hjm_run does, whenever
-// its operand table (rebuilt on the device at every call), the carry between
-// windows and the split tiles' sums fit a second static array (48 MB); the
-// others the convected step (quadratic factors decomposed, else the table).
+// FP64 runs take the contraction (hjm_contract.cu) as hjm_run does, by the first
+// of its plans whose operand table (rebuilt on the device at every call) and carry
+// between windows fit a second static array (48 MB); only what exceeds even one
+// window of eight dates takes the convected step (quadratic factors decomposed,
+// else the table).
 // Mixed precision with polynomial factors takes the FP32 response form where
 // hjm_run does (its table in the same array), else the convected pairs.
 //
@@ -87,7 +88,9 @@ hjm_status static_fail(hjm_status st, const char* fmt, ...)
 static __device__ __align__(256) double g_hjm_static_scratch[kScratchDoubles];
 // ... and 48 MB for a response form's table (FP64: also the carry between
 // windows, 16 MB at HJM_STATIC_MAX_PATHS, and the split tiles' sums, 10 MB).
-// The 25y run at dt = 0.01 takes 41 MB at most, the 10y run down to dt = 0.001.
+// The 25y run at dt = 0.01 takes 41 MB at most, the 10y run down to dt = 0.001; one
+// image at a time the 10y run down to dt = 0.0004 and, in windows of eight dates, the
+// 30y run down to dt = 0.0005.
 static __device__ __align__(256) double2 g_hjm_static_resp[kStaticRespBytes / sizeof(double2)];
 
 #define STATIC_CUDA(call)                                                                          \
@@ -262,24 +265,30 @@ hjm_status hjm_run_static(void* cuda_stream, int32_t n_tenor, double dtau, const
         (precision == HJM_PRECISION_MIXED && (poly || cub)) ? mresp_slots(n_tenor, dt / dtau, dtau, (int)stride, B, false, &live) : 0;
     const bool mresp =
         mresp_ns > 0 && sizeof(float4) * mresp_table_elems((int)stride, B, mresp_ns) <= kStaticRespBytes;
-    // FP64: the contraction where its table, the carry of several windows and
-    // the split tiles' sums fit the static array
+    // FP64: the contraction by the first plan whose table and carry of several
+    // windows fit the static array, the steps of leftover tiles split where their
+    // sums fit it too
     int n_sms = 0;
     const size_t align = 256;
     size_t carry_at = 0, split_at = 0;
-    bool contract = false;
+    bool contract = false, split = false;
+    ContractPlan plan = {};
     if (precision == HJM_PRECISION_FP64) {
         int dev = 0;
         STATIC_CUDA(cudaGetDevice(&dev));
         STATIC_CUDA(cudaDeviceGetAttribute(&n_sms, cudaDevAttrMultiProcessorCount, dev));
-        carry_at = (contract_table_bytes((int)stride, B, false) + align - 1) / align * align;
-        const bool windows = contract_windows(B, (int)stride, false, nullptr) > 1;
-        split_at = carry_at + (windows ? (sizeof(double) * 2 * (size_t)n_paths + align - 1) / align * align : 0);
-        contract = split_at + contract_sums_bytes(n_paths, B, (int)stride, n_sms, false) <= kStaticRespBytes;
+        for (int i = 0; i < kContractPlans && !contract; ++i) {
+            plan = contract_plan(i, false);
+            carry_at = (contract_table_bytes((int)stride, B, plan) + align - 1) / align * align;
+            const bool windows = contract_windows(B, (int)stride, plan, nullptr) > 1;
+            split_at = carry_at + (windows ? (sizeof(double) * 2 * (size_t)n_paths + align - 1) / align * align : 0);
+            contract = split_at <= kStaticRespBytes;
+        }
+        split = split_at + contract_sums_bytes(n_paths, B, (int)stride, n_sms, plan) <= kStaticRespBytes;
     }
     const int cta = mresp ? kCta : path_cta(precision == HJM_PRECISION_MIXED, n_tenor, B, poly || cub);
     const int64_t n_ctas =
-        contract ? contract_rows(n_paths, B, (int)stride, n_sms) : (n_paths + cta - 1) / cta;
+        contract ? contract_rows(n_paths, B, (int)stride, n_sms, split) : (n_paths + cta - 1) / cta;
     if (R > kStaticCols || n_ctas > kStaticCtas)
         return static_fail(HJM_ERR_INVALID_ARGUMENT, "run exceeds the static scratch");
 
@@ -343,10 +352,14 @@ hjm_status hjm_run_static(void* cuda_stream, int32_t n_tenor, double dtau, const
                 for (int d = 0; d < 3; ++d) P.svc[k][d] = sq * coef[k * 3 + d];
         if (contract) {
             unsigned char* area = reinterpret_cast<unsigned char*>(resp_table);
-            STATIC_CUDA(launch_contract_table(n_tenor, dt / dtau, (int)stride, B, false, false, &P.sv[0][0], false, area, s));
-            STATIC_CUDA(launch_path_contract(n_tenor, P, area, nullptr, partials, nullptr,
-                                             reinterpret_cast<double*>(area + carry_at),
-                                             reinterpret_cast<longlong2*>(area + split_at), result, n_sms, s, nullptr));
+            const double c = dt / dtau;
+            int launches;
+            if (!plan.compact)
+                STATIC_CUDA(launch_contract_table(n_tenor, c, (int)stride, B, false, plan, &P.sv[0][0], false, area, s));
+            STATIC_CUDA(launch_contract(n_tenor, c, false, &P.sv[0][0], P, plan, !plan.compact, area, nullptr, partials,
+                                        nullptr, reinterpret_cast<double*>(area + carry_at),
+                                        split ? reinterpret_cast<longlong2*>(area + split_at) : nullptr, result, n_sms, s,
+                                        &launches));
         } else {
             STATIC_CUDA(launch_path_fp64(n_tenor, P, poly, nullptr, partials, nullptr, s));
         }
