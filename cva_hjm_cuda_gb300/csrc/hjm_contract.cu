@@ -913,14 +913,15 @@ struct ContractLoadings {
     double sv[kFactors][kMaxTenor];
 };
 
-// The power of two that maps a date's largest response into [2^7, 2^8), as a
-// multiplier back (responses below 1e-280 count as zero), by its exponent's bits:
+// The power of two that maps a date's largest response (finite) into [2^7, 2^8), as
+// a multiplier back (responses below 1e-280 count as zero), by its exponent's bits:
 // FP64 instructions are what the image kernel waits for (a division and the
 // exponent functions per element: 30 us for 32 dates of the 25y run against 19).
+constexpr unsigned long long kInfBits = 0x7ff0000000000000ull;
 __device__ __forceinline__ int contract_exponent(unsigned long long top)
 {
     const bool in = top > (unsigned long long)__double_as_longlong(1e-280) &&
-                    top < (unsigned long long)__double_as_longlong(1e300);
+                    top < kInfBits;
     return in ? (int)(top >> 52) - 1022 - kTopBits : 0;
 }
 __device__ __forceinline__ double power_of_two(int e) { return __hiloint2double((1023 + e) << 20, 0); }
@@ -996,8 +997,8 @@ struct DateResponse {
     {
 #pragma unroll
         for (int k = 0; k < kFactors; ++k) {
-            best[0] = fmax(best[0], fabs(v[k]));
-            best[1] = fmax(best[1], fabs(w[k]));
+            best[0] = isfinite(v[k]) ? fmax(best[0], fabs(v[k])) : __longlong_as_double(kInfBits);
+            best[1] = isfinite(w[k]) ? fmax(best[1], fabs(w[k])) : __longlong_as_double(kInfBits);
         }
     }
 };
@@ -1054,11 +1055,14 @@ __global__ void __launch_bounds__(128)
     store_largest(best, j, top);
 }
 
-// The scales of the dates from their largest responses
+// The scales of the dates from their largest responses.  A date with a response that
+// overflowed has a NaN for a scale and so for its values (its slices, NaN too, would
+// come out of the integer sums as zero: a curve without noise).
 __device__ __forceinline__ void store_scales(const unsigned long long* top, double* scale)
 {
     for (int i = threadIdx.x; i < 2 * kMaxTenor; i += blockDim.x)
-        scale[i] = power_of_two(contract_exponent(top[i])) * kSumUnit;
+        scale[i] = top[i] < kInfBits ? power_of_two(contract_exponent(top[i])) * kSumUnit
+                                     : __longlong_as_double(0x7ff8000000000000ll);
 }
 // The slices of a scaled response x into row val (value 3 i + k of a chunk: step i,
 // factor k) and column col of the chunk's image: three k-tiles of 16 rows, each two

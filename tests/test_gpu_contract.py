@@ -192,3 +192,24 @@ def test_table_of_another_market_in_the_same_shape():
     for v in got:
         np.testing.assert_array_equal(v.ee, want.ee)
         assert v.cva == want.cva
+
+
+@pytest.mark.parametrize("size", [1e100, 1e301])
+def test_loadings_near_overflow(engine, size):
+    """Volatilities whose responses come near FP64's limit: the exposures (0, inf) are
+    those of the convected step, not those of a curve without noise."""
+    mk = _table_market(51)
+    engine.set_market(Market(vol=mk.vol * size, drift=np.zeros(51)))
+    engine.set_swap(Swap(n_periods=8, strike=0.01))
+    (v, x), (c, xc) = _both(engine, lambda: engine.run(RunConfig(n_paths=300, n_steps=200, dt=0.02, seed=3), "fp64"))
+    np.testing.assert_array_equal(x, xc)
+    assert not np.any(np.isfinite(x) & (x > 0.0))
+
+
+def test_responses_that_overflow(engine):
+    """Volatilities whose responses leave FP64's range give no finite positive exposure."""
+    mk = _table_market(51)
+    engine.set_market(Market(vol=mk.vol * 1e307, drift=np.zeros(51)))
+    engine.set_swap(Swap(n_periods=30, strike=0.01))
+    (v, x), _ = _both(engine, lambda: engine.run(RunConfig(n_paths=300, n_steps=750, dt=0.02, seed=3), "fp64"))
+    assert not np.any(np.isfinite(x) & (x > 0.0))
