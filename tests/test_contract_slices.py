@@ -173,3 +173,25 @@ def test_walk_tails_equal_the_recursion_over_the_lags(nt, c, stride, B, pc):
             want = [hist[0, m, j], cum[0, m, j], hist[1, m, j], cum[1, m, j], hist[0, m + 1, j]]
             for x, y in list(zip(got, want))[: 5 if pc else 2]:
                 assert abs(x - float(y)) <= max(2.0 ** -24 * abs(float(y)), 2.0 ** -54), (j, m, x, y)
+
+
+@pytest.mark.parametrize("pc", [False, True], ids=["euler", "predictor-corrector"])
+@pytest.mark.parametrize("c,M", [(0.02, 2450), (0.5, 98), (0.1, 290)])
+def test_walk_form_of_the_running_sums(pc, c, M):
+    """The responses' running sums against the cumulated recursion in extended
+    precision: the responses' bound, and 48 roundings of the walk's upper tail
+    (2^-53 each) that every sum's weight carries, 1 / (a1 + a2) <= 1 / (c - c^2 / 2) times."""
+    T = 0.5 * np.arange(51)
+    for S in (0.002 - 0.0006 * T + 2e-5 * T**2, 0.004 * np.cos(np.arange(51) / 7.0)):
+        _, C = _walk(S, c, M, pc)
+        v, total = S.astype(np.longdouble), np.zeros(51, dtype=np.longdouble)
+        want = np.zeros((M, 51), dtype=np.longdouble)
+        for m in range(M):
+            total = total + v
+            want[m] = total
+            v = _advance(v, np.longdouble(c), pc)
+        line = S[50] + (np.arange(51) - 50) * (S[50] - S[49])
+        dev = np.cumsum(np.abs(S - line)[::-1])[::-1]
+        for j in range(2, 51):
+            bound = 48 * 4 * 2.0**-53 * np.max(np.abs(want[:, j])) + 48 * 2.0**-53 / (c - 0.5 * c * c) * dev[j]
+            assert np.max(np.abs(C[:, j] - want[:, j])) <= bound
