@@ -161,7 +161,8 @@ __global__ void __launch_bounds__(kAdjCta, adj_min_ctas<NT>())
     const int64_t ld = A.ck_ld;
 
     // ---------------------------------------------------------------- forward
-    // The same arithmetic as path_kernel_mixed, plus what the sweep needs.
+    // The convected valuation's arithmetic (path_kernel_mixed_conv's with polynomial
+    // factors, else path_kernel_mixed's), plus what the sweep needs.
     constexpr int W1 = conv_window(NT, 0), W2 = conv_window(NT, 1);
     MixedPath<NT, POLY> x;
     x.reset();

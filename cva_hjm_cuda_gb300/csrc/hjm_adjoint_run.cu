@@ -20,9 +20,9 @@
 // loading.  Y_k = sum_n {kappa G_j, kappa CG_j}(n) r0(n) is the remainder's
 // response to W = r0: the table row and the slots of A, once per factor.
 // The twelve sums of a date go to memory (a part of sens per CTA, rewritten
-// tile by tile, 71 MB for 20 dates: it stays in the second-level cache) until
-// the seeds {xbar_i, abar_i}, which need the exposures of the whole path,
-// weigh them.
+// tile by tile, 71 MB for 20 dates: 95 MB of write-backs to DRAM at 262,144 paths, reads
+// from the second-level cache) until the seeds {xbar_i, abar_i}, which need the exposures
+// of the whole path, weigh them.
 //
 // Bounds: the generator (115 of ~165 issue cycles per 32 path-steps), then the
 // packed FMAs of Y.  10y swap, 1M paths: 8.35 ms -> 5.75 ms against the

@@ -85,12 +85,10 @@ struct hjm_ctx {
     bool have_poly = false;       // coefficients given by hjm_set_market_poly (sensitivities)
     bool poly_path = false;       // the kernels run the polynomial decomposition (coef)
     bool allow_poly_path = true;  // hjm_ctx_set_vol_decomposition
-    // cubic factors up to a small residual table (a PCA table printed to a
-    // few decimals): the FP64 Euler response form's decomposition
+    // cubic factors up to a residual below FP32's resolution of them (a PCA table
+    // printed to a few decimals): the mixed-precision Euler step's cubic form
     bool cubic_path = false;
     double cubic[HJM_N_FACTOR][4] = {};  // coefficients of (T - T_L)^d
-    int cubic_degs[HJM_N_FACTOR] = {};
-    std::vector<double> resid;            // [3][nt] sigma_k - cubic_k (unscaled)
     int scheme = HJM_SCHEME_EULER;  // hjm_ctx_set_scheme
     int remainder = HJM_REMAINDER_AUTO;  // hjm_ctx_set_remainder_form
     int nt = 0;
@@ -295,9 +293,9 @@ static bool use_poly_path(const hjm_ctx* ctx) { return ctx->poly_path && ctx->al
 
 static bool use_cubic_path(const hjm_ctx* ctx) { return !ctx->poly_path && ctx->cubic_path && ctx->allow_poly_path; }
 
-// 0: table step, 1: quadratic factors, 2: factor k of degree <= k, 3: cubic
-// factors with a residual table (FP64 Euler valuations; the other modes run
-// the table step on such a market)
+// 0: table, 1: quadratic factors, 2: factor k of degree <= k, 3: cubic factors up to
+// a residual.  What the mixed and the convected forms make of the market; the FP64
+// contraction takes the table itself, whatever its shape.
 static int vol_form_code(const hjm_ctx* ctx)
 {
     if (!ctx->have_market) return 0;
@@ -389,18 +387,16 @@ __attribute__((visibility("hidden"))) bool fit_quadratic_vols(const double* vol,
     return true;
 }
 
-// Cubic factors up to a residual table.  Each factor row is fitted by least
+// Cubic factors up to a residual.  Each factor row is fitted by least
 // squares (modified Gram-Schmidt on 1, u, u^2, u^3 with u = (T - T_L) / T_L in
 // [-1, 0], then scaled to powers of t = T - T_L) with the lowest degree <= 3
 // whose largest residual is at most 2^-20 of the row's largest magnitude;
-// coef[k * 4 + d] multiplies t^d, degs[k] is the degree, resid[k * nt + t] =
-// sigma_k(T_t) - poly_k(T_t) in FP64.  False when some row needs more than a
+// coef[k * 4 + d] multiplies t^d.  False when some row needs more than a
 // cubic.  A PCA table printed to a fixed number of decimals (the reference's,
 // simulation_gpu_testing.cpp:47-63: its factors 2 and 3 are cubics to the
 // 9-decimal rounding, 1.1e-7 of their scale) fits with a residual of that
 // rounding's size.  Internal to the library.
-__attribute__((visibility("hidden"))) bool fit_cubic_resid(const double* vol, int nt, double dtau, double* coef,
-                                                            int* degs, double* resid)
+__attribute__((visibility("hidden"))) bool fit_cubic(const double* vol, int nt, double dtau, double* coef)
 {
     if (nt < 5) return false;
     if (nt > HJM_MAX_TENOR) return false;
@@ -452,14 +448,11 @@ __attribute__((visibility("hidden"))) bool fit_cubic_resid(const double* vol, in
             for (int t = 0; t < nt; ++t) {
                 const double x = dtau * t - TL;
                 const double pv = ((a[3] * x + a[2]) * x + a[1]) * x + a[0];
-                r[t] = v[t] - pv;
-                worst = std::max(worst, std::fabs(r[t]));
+                worst = std::max(worst, std::fabs(v[t] - pv));
             }
             if (worst <= tol * scale) {
                 found = true;
-                degs[k] = d;
                 for (int i = 0; i < 4; ++i) coef[k * 4 + i] = a[i];
-                for (int t = 0; t < nt; ++t) resid[(size_t)k * nt + t] = r[t];
             }
         }
         if (!found) return false;
@@ -507,10 +500,7 @@ hjm_status hjm_set_market(hjm_ctx* ctx, int32_t n_tenor, double dtau, const doub
     ctx->have_market = true;
     ctx->have_poly = false;
     ctx->poly_path = fit_quadratic_vols(ctx->vol.data(), n_tenor, dtau, ctx->coef);
-    ctx->resid.assign((size_t)HJM_N_FACTOR * n_tenor, 0.0);
-    ctx->cubic_path = !ctx->poly_path &&
-                      fit_cubic_resid(ctx->vol.data(), n_tenor, dtau, &ctx->cubic[0][0], ctx->cubic_degs,
-                                      ctx->resid.data());
+    ctx->cubic_path = !ctx->poly_path && fit_cubic(ctx->vol.data(), n_tenor, dtau, &ctx->cubic[0][0]);
     if (ctx->have_product && (int)ctx->payA.size() != n_tenor) ctx->have_product = false;
     return HJM_OK;
 }
@@ -909,7 +899,7 @@ static hjm_status enqueue_contract(hjm_ctx* ctx, const RunShape& sh, double dt, 
 // input perturbation of that size, far inside the mixed precision's 1e-4.
 namespace hjm {
 // (Shared with hjm_run_static; internal to the library.)  cubic: [3][4]
-// coefficients of (T - T_L)^d as fit_cubic_resid gives them.
+// coefficients of (T - T_L)^d as fit_cubic gives them.
 __attribute__((visibility("hidden"))) void mixed_cubic_params(int nt, double dtau, double dt, int n_blocks,
                                                               const double* cubic, MixedParams& M)
 {
@@ -1060,9 +1050,9 @@ static hjm_status enqueue_impl(hjm_ctx* ctx, int64_t n_paths, int32_t n_steps, d
     ctx->stat_d2h = 0;
     HJM_CUDA(ctx, cudaEventRecord(ctx->ev[0], s));
     bool resp = false;
-    // the volatility form this run takes (vol_form_code's values): a cubic
-    // market runs its decomposition in the Euler step only (FP64: the response
-    // form with the residual; mixed precision: the cubic polynomial form)
+    // the market's volatility form under this scheme (vol_form_code's values) for
+    // the report: a cubic market's counts in the Euler step only, where mixed
+    // precision runs it (the FP64 contraction takes any table as it is)
     int run_form = use_poly_path(ctx) ? vol_form_code(ctx) : 0;
     if (pc && mixed) {
         PathParams<float> P;

@@ -50,7 +50,7 @@ using namespace hjm;
 namespace hjm {
 void set_thread_error(const char* msg);  // hjm_capi.cu: the message hjm_last_error(NULL) returns
 bool fit_quadratic_vols(const double* vol, int nt, double dtau, double* coef);  // hjm_capi.cu
-bool fit_cubic_resid(const double* vol, int nt, double dtau, double* coef, int* degs, double* resid);  // hjm_capi.cu
+bool fit_cubic(const double* vol, int nt, double dtau, double* coef);  // hjm_capi.cu
 void mixed_cubic_params(int nt, double dtau, double dt, int n_blocks, const double* cubic, MixedParams& M);  // hjm_capi.cu
 }
 
@@ -253,11 +253,9 @@ hjm_status hjm_run_static(void* cuda_stream, int32_t n_tenor, double dtau, const
     double coef[HJM_N_VOL_COEF];
     const bool poly = fit_quadratic_vols(vol_host, n_tenor, dtau, coef);
     // a table that is a cubic up to a small residual (the reference's own PCA
-    // table): FP64 the response form with the residual, mixed precision the
-    // cubic polynomial form, as hjm_run
-    double cubic[HJM_N_FACTOR * 4], resid[HJM_N_FACTOR * HJM_MAX_TENOR];
-    int cdegs[HJM_N_FACTOR];
-    const bool cub = !poly && fit_cubic_resid(vol_host, n_tenor, dtau, cubic, cdegs, resid);
+    // table): mixed precision runs the cubic polynomial form, as hjm_run
+    double cubic[HJM_N_FACTOR * 4];
+    const bool cub = !poly && fit_cubic(vol_host, n_tenor, dtau, cubic);
     // mixed precision with polynomial factors: the response form when the
     // dates its remainder reaches fit its slots and its table the static array
     RespLive live = {};

@@ -148,9 +148,11 @@ class HJMEngine:
         return self.vol_form() != "table"
 
     def vol_form(self) -> str:
-        """The step the current market runs: "table", "poly" (quadratic factors),
+        """The current market's volatility form: "table", "poly" (quadratic factors),
         "poly_tri" (factor k of degree <= k) or "cubic_resid" (cubic factors up to a
-        residual table: the FP64 Euler valuations; other modes run the table step)."""
+        residual).  The mixed-precision and the convected forms decompose the market by
+        it (a cubic one in mixed-precision Euler valuations only); the FP64 response form takes the
+        table as it is."""
         active = C.c_int32(0)
         self._check(self.lib.hjm_ctx_vol_decomposition(self.ctx, C.byref(active)))
         return ("table", "poly", "poly_tri", "cubic_resid")[active.value]

@@ -105,23 +105,22 @@ hjm_status hjm_ctx_set_scheme(hjm_ctx* ctx, int32_t scheme);
 /* Polynomial volatility decomposition.  When every volatility factor is a
  * polynomial of degree <= 2 in the tenor T (given by hjm_set_market_poly, or a
  * table that hjm_set_market finds to be one to 1e-12 of each row's scale, as
- * the configured workloads' synthetic factors are), the kernels
- * carry the stochastic curve as S + U T + W T^2 plus a remainder driven only at
- * the last tenor, instead of adding the three factor columns to every tenor
- * each step (simulation_gpu.cu:153-180).  enable = 0 forces the generic
- * table-driven step; default 1.  A table that is no quadratic but a cubic in
- * each factor up to a residual of at most 2^-20 of the factor's scale (a PCA
+ * the configured workloads' synthetic factors are), mixed precision and the
+ * convected forms carry the stochastic curve as S + U T + W T^2 plus a remainder
+ * driven only at the last tenor, instead of adding the three factor columns to
+ * every tenor each step (simulation_gpu.cu:153-180).  enable = 0 forces the
+ * generic table-driven step; default 1.  A table that is no quadratic but a cubic
+ * in each factor up to a residual of at most 2^-20 of the factor's scale (a PCA
  * table printed to a fixed number of decimals, as the reference's own
  * simulation_gpu_testing.cpp:47-63, whose factors 2 and 3 are cubics to
- * 1.1e-7) runs, in Euler valuations, the cubic decomposition: in FP64 with
- * the residual's impulse responses carried beside the remainder's, in mixed
- * precision without the residual (below FP32's resolution of the loadings);
- * the predictor-corrector scheme, the adjoint and MLMC run the table step on
- * it.
- * hjm_ctx_vol_decomposition reports what the current market runs: 0 the
- * table step, 1 the decomposition, 2 the decomposition with factor k of
- * degree <= k (three zero coefficients), 3 the cubic decomposition with a
- * residual table. */
+ * 1.1e-7) runs the cubic decomposition in mixed-precision Euler valuations,
+ * without the residual (below FP32's resolution of the loadings); the
+ * predictor-corrector scheme, the adjoint and MLMC run the table step on it.
+ * FP64 valuations in the response form (below) take any table as it is.
+ * hjm_ctx_vol_decomposition reports the market's form, as a valuation's report
+ * does ("vol_form"; a cubic market under the predictor-corrector: table): 0 table,
+ * 1 quadratic factors, 2 factor k of degree <= k (three zero coefficients), 3
+ * cubic factors up to a residual. */
 hjm_status hjm_ctx_set_vol_decomposition(hjm_ctx* ctx, int32_t enable);
 hjm_status hjm_ctx_vol_decomposition(hjm_ctx* ctx, int32_t* active);
 
@@ -134,9 +133,11 @@ hjm_status hjm_ctx_vol_decomposition(hjm_ctx* ctx, int32_t* active);
  * FP64: for any market and either scheme the sums over steps and factors of
  * normal times response are a contraction, which the tensor cores run exactly
  * on 10-bit slices of both (per-path exposures within ~1e-14 of the exposure
- * scale of the exact sums); any number of dates, in launches of at most 32
- * (external normals: 24).  AUTO (default) takes it for every FP64 valuation
- * whose tables the memory limit allows.
+ * scale of the exact sums, on the generator's draws and on any normals of the
+ * caller's); any number of dates, in launches of at most 32 (external normals:
+ * 24).  AUTO (default) takes it for every FP64 valuation whose operands the memory
+ * limit allows: the whole table (3.2 MB for the 10y swap, 14 MB at 25y), or one
+ * launch's image at a time (1.4 and 4.7 MB), or that of eight dates (0.5 and 1.2 MB).
  * Mixed precision with the decomposition carries the remainder as FP32
  * impulse-response sums (one packed FMA per date per step) when the dates
  * whose responses ever reach 2^-30 of the source fit 16 slots (the 10y swap's
@@ -205,7 +206,8 @@ hjm_status hjm_fetch_results(hjm_ctx* ctx, double* ee_out, double* pfe_out, doub
 
 /* The valuation on caller-supplied normals, normals_host[path][step][3]
  * (the reference's layout, simulation_cpu.h:205-207, simulation_gpu.cu:410).
- * Used to feed the reference's own draws to the kernels. */
+ * Used to feed the reference's own draws to the kernels.  The first block's
+ * normals (steps below stride) are not read: the curve stands at spot there. */
 hjm_status hjm_run_with_normals(hjm_ctx* ctx, int64_t n_paths, int32_t n_steps, double dt,
                                 const double* normals_host, int32_t precision, double hazard_rate,
                                 double recovery, double pfe_quantile, double* ee_out,
@@ -307,7 +309,8 @@ hjm_status hjm_run_adjoint(hjm_ctx* ctx, int64_t n_paths, int32_t n_steps, doubl
  * when ee_out [n_tenor] and cva_out [HJM_CVA_OUT_LEN] hold the results.  Its
  * device memory is two fixed static arrays that each GPU loading the library
  * keeps until exit: 8.4 MB of scratch and 48 MB for a response form's table
- * (FP64: also the sums that its launches pass on), 57 MB in all; it calls no
+ * (FP64: also the sums that its launches pass on; runs of very many steps build it
+ * piece by piece), 57 MB in all; it calls no
  * cudaMalloc, cudaFree or allocating library routine.  Limits: at most
  * HJM_STATIC_MAX_PATHS paths per call (larger runs fail with
  * HJM_ERR_INVALID_ARGUMENT), EE and CVA only (no PFE).  The first call on a
