@@ -242,19 +242,18 @@ def adjoint_response_flops_per_path(n_tenor: int, n_steps: int, stride: int, for
 
 
 def contraction_flops_per_path(n_steps: int, stride: int) -> int:
-    """Tensor-core flops per path of the FP64 contraction (path_kernel_contract)
-    as its instructions run them: windows of at most 32 dates, latest first,
-    each over the steps up to its last date in chunks of 16 (48 normals), per
-    chunk the 14 products of normal slice i and response slice j with i + j <=
-    4 and i <= 3 over the window's columns (value and running sum per date,
-    padded to 16)."""
+    """Tensor-core flops per path of the FP64 contraction (path_kernel_contract):
+    windows of at most 32 dates, latest first, each over the steps up to its
+    last date in chunks of 16 (48 normals), per chunk the 14 products of normal
+    slice i and response slice j with i + j <= 4 and i <= 3 over the columns that
+    hold dates (value and running sum; the instructions' padding to 16 columns is
+    not counted)."""
     total, hi = 0, n_steps // stride
     while hi >= 1:
         lo = 1 if hi - 1 <= 32 else hi - 31
         slots = max(hi - max(lo, 2) + 1, 0)
-        npad = max((2 * slots + 15) // 16 * 16, 16)
         chunks = ((hi - 1) * stride + 15) // 16
-        total += chunks * 48 * 14 * npad * 2
+        total += chunks * 48 * 14 * (2 * slots) * 2
         hi = lo - 1
     return total
 
